@@ -78,6 +78,12 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
+// One lane of a converged warp.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t chosen;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
+  return chosen;
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -392,7 +398,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       if (n_item >= 1) ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(ACC_EMPTY, 0), (n_item - 1) & 1u, deadline, aborted));  // the previous item's accumulators are in registers
       PF_TICK(m1);
       PF_ADD(3, m0, m1);
-      if (lane == 0 && ok) {
+      // The whole warp walks the K blocks and waits; one elected lane issues.  An MMA's descriptors live in
+      // uniform registers, and only code that the compiler can see to be warp-uniform keeps them there:
+      // issued from an `if (lane == 0)` branch an MMA cost 79 cycles of the issuing thread whatever its
+      // size, issued under elect.sync it costs what the tensor core takes (16 cycles at 32 columns, 64 at 128).
+      if (ok) {
         // N = 2 * n_pad: the high-byte rows and the low-byte rows of the routes are one B operand
         // accumulator s32, A unsigned bytes (the nibble decoder's u = q + 8), B signed bytes
         const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(n_pad >> 2) << 17) | ((PF_ROWS >> 4) << 24);
@@ -400,30 +410,33 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         for (int kb = 0; kb < k_blocks && ok; ++kb) {
           const uint32_t sa = issue_a, sb = issue_b;
           PF_TICK(m2);
-          ok = mbar_wait(bar(A_FULL, sa), issue_a_phase, deadline, aborted);
+          ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(A_FULL, sa), issue_a_phase, deadline, aborted));
           PF_TICK(m3);
-          ok = ok && mbar_wait(bar(B_FULL, sb), issue_b_phase, deadline, aborted);
+          ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(bar(B_FULL, sb), issue_b_phase, deadline, aborted));
           PF_TICK(m4);
           PF_ADD(0, m2, m3); PF_ADD(1, m3, m4);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_cols = tmem + A_COL0 + sa * A_STAGE_COLS;
           const uint64_t b_desc = umma_desc(b_stage_addr(sb));
+          if (elect_one()) {
 #pragma unroll
-          for (int m = 0; m < M; ++m) {
+            for (int m = 0; m < M; ++m) {
 #pragma unroll
-            for (int k = 0; k < 4 && diag != 4; ++k)  // 32 bytes of K per instruction: 8 columns of A, 2 x 16 bytes of the B start address
-              umma_i8_ts(tmem + m * (2 * PF_N_MAX), a_cols + m * PF_A_TILE_COLS + 8 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
+              for (int k = 0; k < 4 && diag != 4; ++k)  // 32 bytes of K per instruction: 8 columns of A, 2 x 16 bytes of the B start address
+                umma_i8_ts(tmem + m * (2 * PF_N_MAX), a_cols + m * PF_A_TILE_COLS + 8 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
+            }
+            umma_commit(bar(A_EMPTY, sa));  // the stages may be refilled once these MMAs have read them
+            umma_commit(bar(B_EMPTY, sb));
+            if (kb == k_blocks - 1) umma_commit(bar(ACC_FULL, 0));
           }
+          __syncwarp();
           mma_issued = true;
-          umma_commit(bar(A_EMPTY, sa));  // the stages may be refilled once these MMAs have read them
-          umma_commit(bar(B_EMPTY, sb));
           if (++issue_a == PF_A_STAGES) { issue_a = 0; issue_a_phase ^= 1u; }
           if (++issue_b == PF_B_STAGES) { issue_b = 0; issue_b_phase ^= 1u; }
           PF_TICK(m5);
           PF_ADD(2, m4, m5);
         }
-        if (ok) umma_commit(bar(ACC_FULL, 0));
       }
       // The other lanes wait here for the issuing lane.  Without this they would run one item ahead
       // and refill the per-route buffer of item n - 1 while that item's drain is still doing the
@@ -469,7 +482,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   if (*aborted) {
     if (tid == 0 && status) atomicExch(status, window_ok ? 1 : 2);
     // MMAs may still be in flight: one more commit arrives when they are all done; wait for it, bounded as every wait
-    if (warp == PF_MMA_WARP && lane == 0 && mma_issued) {
+    if (warp == PF_MMA_WARP && mma_issued && elect_one()) {  // the lane that issued: a commit follows its own thread's MMAs
       umma_commit(bar(DRAINED, 0));
       const uint64_t grace = global_timer_ns() + 100000000ull;
       for (uint32_t spin = 0; spin < (1u << 22); ++spin) {
