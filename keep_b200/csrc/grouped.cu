@@ -5,7 +5,7 @@
 // out[r] = W[rhs[r]] @ x[r] for r < routes; x holds one activation row per route (the caller
 // gathers them, as the reference does before its kernels, src/ramp/ops/vq_switch.py:758-761).
 // The sequence is the down projection of the layer call: quantise the rows, group the routes by
-// expert on the device, then the tcgen05 kernel (24 or more routes per expert on average) or the
+// expert on the device, then the tcgen05 kernel (8 or more routes per expert on average) or the
 // mma.sync one.  Routes need not be sorted; a route with expert 0xFFFFFFFF gives a zero row.
 #include "moe_fast.cuh"
 
@@ -80,19 +80,20 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
   fast::RouteGroups groups = {reinterpret_cast<int32_t*>(ws + sc.gcount), reinterpret_cast<int32_t*>(ws + sc.gslot),
                               reinterpret_cast<int32_t*>(ws + sc.gstart), reinterpret_cast<int32_t*>(ws + sc.gsize),
                               reinterpret_cast<int32_t*>(ws + sc.groutes)};
-  const bool many = !residual && a.routes >= 1024 && a.routes >= 24 * a.slots && fast::prefill_supported(a.out_dim, a.in_dim, a.groups);
+  const bool many = !residual && a.routes >= 1024 && a.routes >= 8 * a.slots && fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups);
   // (the sums region has room for a scale group per codeword; these kernels' rows have at most one
   // per 256 inputs, and their sums per 256 inputs go behind those)
   fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + sc.xq), reinterpret_cast<float*>(ws + sc.xscale), reinterpret_cast<int32_t*>(ws + sc.xsums),
                         many ? nullptr : reinterpret_cast<int32_t*>(ws + sc.xsums) + (x_rows + 1) * a.groups};
   int32_t* wait_status = reinterpret_cast<int32_t*>(ws + sc.status);
   int rc;
-  const int group_cols = many ? fast::PREFILL_GROUP_ROUTES : fast::decode_group_routes(a.routes, a.slots, a.in_dim);
+  const int group_cols = many ? fast::prefill_group_routes(a.routes, a.slots, a.groups > 1) : fast::decode_group_routes(a.routes, a.slots, a.in_dim);
   if ((rc = fast::group_routes(a.rhs, a.routes, a.slots, group_cols, groups, wait_status, s))) return rc;
   if (many) {  // the tcgen05 kernels copy rows in grouped order
     if ((rc = fast::quantize_rows_sorted(a.x, a.x_dtype, a.routes, a.in_dim, a.groups, xq, {groups.routes, groups.count, static_cast<int32_t>(x_div)}, s))) return rc;
   } else if ((rc = fast::quantize_rows(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, false, s))) return rc;
   fast::FastProjectionArgs p = {};
+  p.slots = a.slots;
   p.a = {a.codes, a.scales, a.res_codes, a.res_scales}; p.b = {nullptr, nullptr, nullptr, nullptr};
   if (residual) { p.res_groups = a.res_groups; p.hot_of_slot = a.hot_of_slot; p.res_table = a.res_table; }
   p.scales_dtype = a.scales_dtype; p.codebook = a.codebook; p.groups_of_routes = groups; p.max_routes = a.routes; p.group_cols = group_cols; p.status = wait_status;
@@ -133,17 +134,17 @@ extern "C" int keepvq_wait_selftest(void* workspace, int64_t workspace_bytes, in
   char* ws = reinterpret_cast<char*>(workspace);
   cudaError_t e = cudaMemsetAsync(ws, 0, SELFTEST_BYTES, s);
   if (e != cudaSuccess) return note_cuda_error(e);
-  // status 0 | groups 256.. | routes 1280 | table 2048 | scales 3072 | codes 4096 | planes 8192 | x scale 16384 | x sums 16640 | out 20480
+  // status 0 | groups 256.. | routes 1280 | table 2048 | scales 3072 | codes 4096 | planes 12288 | x scale 21248 | x sums 21504 | out 22528
   fast::RouteGroups groups = {reinterpret_cast<int32_t*>(ws + 256), reinterpret_cast<int32_t*>(ws + 512), reinterpret_cast<int32_t*>(ws + 768),
                               reinterpret_cast<int32_t*>(ws + 1024), reinterpret_cast<int32_t*>(ws + 1280)};
-  fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + 8192), reinterpret_cast<float*>(ws + 16384), reinterpret_cast<int32_t*>(ws + 16640), nullptr};
+  fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + 12288), reinterpret_cast<float*>(ws + 21248), reinterpret_cast<int32_t*>(ws + 21504), nullptr};
   selftest_init_kernel<<<1, 32, 0, s>>>(groups.count, groups.size, groups.routes, xq.scale);
   KEEPVQ_CHECK_LAUNCH();
   fast::FastProjectionArgs p = {};
   p.a = {reinterpret_cast<const uint16_t*>(ws + 4096), ws + 3072, nullptr, nullptr};
-  p.scales_dtype = KEEPVQ_F16; p.out_dim = 128; p.in_dim = 128; p.groups = 1;
+  p.scales_dtype = KEEPVQ_F16; p.slots = 1; p.out_dim = 128; p.in_dim = 256; p.groups = 1;
   p.codebook = reinterpret_cast<const uint32_t*>(ws + 2048);
   p.x = xq; p.x_zero_row = 16; p.x_div = 1; p.groups_of_routes = groups; p.max_routes = 16; p.group_cols = fast::PREFILL_GROUP_ROUTES;
-  p.out = ws + 20480; p.out_dtype = KEEPVQ_BF16;
+  p.out = ws + 22528; p.out_dtype = KEEPVQ_BF16;
   return fast::prefill_wait_selftest(p, reinterpret_cast<int32_t*>(ws), static_cast<uint64_t>(wait_ns), s);
 }

@@ -21,6 +21,8 @@ constexpr int SMALL_CALL_ROUTES = 48;   // calls with fewer routes never run the
 constexpr int FEW_ROUTE_GROUPS = 96;    // below this many route groups a CTA's warps share rows AND inputs (sweep kernel, split slab kernel)
 constexpr int PAIRED_GROUP_ROUTES = 4;  // ... when a route's two byte planes take a column each (one MMA per step)
 constexpr int PREFILL_GROUP_ROUTES = 96;   // routes of one expert per tcgen05 item (its accumulators and two operand stages fill tensor memory)
+constexpr int PREFILL_GROUP_ROUTES_SMALL = 48;  // ... for calls with fewer routes per expert, and for rows with several scale groups
+constexpr int PREFILL_FEW_ROUTES_MEAN = 32;     // routes per expert on average up to which a call counts as the former
 
 
 // ------------------------------------------------------------------------------------------
@@ -194,6 +196,7 @@ struct FastProjectionArgs {
   Projection a;           // gate (or down)
   Projection b;           // up, or {nullptr, nullptr} for a single projection
   int32_t scales_dtype;
+  int64_t slots;          // rows of `codes` are slots * out_dim
   int64_t out_dim, in_dim, groups;
   const uint32_t* codebook;
   QuantRows x;            // activations
@@ -267,7 +270,9 @@ int sweep_down(const FastProjectionArgs& args, cudaStream_t s);
 
 // tcgen05 kernels for many routes per expert (prefill_umma.cu).  `status` is a device word that
 // a CTA sets to 1 if one of its bounded waits expires.
-bool prefill_supported(int64_t out_dim, int64_t in_dim, int64_t groups);
+bool prefill_supported(int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups);
+// Routes per item (group_routes' max_group) of a call with `live` routes; a kernel takes p.group_cols.
+int prefill_group_routes(int64_t live, int64_t slots, bool several_groups);
 int prefill_gate_up(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);
 int prefill_down(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);
 // One CTA whose activation loaders never publish, with a deadline of wait_ns: the wait runs out, the CTA sets *status = 1 and returns.

@@ -35,13 +35,14 @@ struct dtype_tag_of {
 
 static inline int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
-// The tcgen05 kernels decode a code once per 96 routes of an expert but cost the same for one
-// route as for 96; the mma.sync kernels stream an expert's codes once per 8 routes.  Which one
-// pays depends on routes per expert, and the host only knows its upper bound routes / slots
-// (reading the routing back would stall the stream): from 24 on, three passes of the decode
-// kernels cost more than the one pass of the tcgen05 kernels.
+// The tcgen05 kernels decode a code once per 48 or 96 routes of an expert and cost nearly the same
+// for one route as for 48; the mma.sync kernels stream an expert's codes once per 4 or 8 routes.
+// Which one pays depends on routes per expert, and the host only knows its upper bound
+// routes / slots (reading the routing back would stall the stream): from 8 on, the two passes of
+// the decode kernels cost more than the one pass of the tcgen05 kernels (1000 tokens of top-6 over
+// 384 experts, 15.6 routes each: 1069 against 2019 us for the layer).
 constexpr int64_t PREFILL_MIN_ROUTES = 1024;
-constexpr int64_t PREFILL_MIN_ROUTES_PER_SLOT = 24;
+constexpr int64_t PREFILL_MIN_ROUTES_PER_SLOT = 8;
 
 struct LayerScratch {
   int64_t logits, gate, up, h, down;
@@ -62,7 +63,7 @@ static LayerScratch plan_scratch(int64_t tokens, int64_t hidden, int64_t inter, 
   const int64_t x_rows = routes >= PREFILL_MIN_ROUTES ? routes : tokens;
   s.xq = at;     at += align256((x_rows + 1) * hidden * 2);  // + the zero row
   s.xscale = at; at += align256((x_rows + 1) * 4);
-  s.xsums = at;  at += align256(std::max((tokens + 1) * (hidden / 8) * 4, (x_rows + 1) * 4));  // room for one scale group per codeword (one per row in grouped order)
+  s.xsums = at;  at += align256(std::max((tokens + 1) * (hidden / 8) * 4, (x_rows + 1) * std::max<int64_t>(hidden / 256, 1) * 4));  // room for one scale group per codeword (one per 256 inputs in grouped order)
   s.hq = at;     at += align256((routes + 1) * inter * 2);
   s.hscale = at; at += align256((routes + 1) * 4);
   s.hsums = at;  at += align256((routes + 1) * (inter / 8) * 4);
@@ -205,10 +206,10 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
   const bool tensor_path = a.x_dtype != KEEPVQ_F32 && a.codebook_all_odd && residual_fits && fast::shapes_supported(a.inter, a.hidden, a.w1.groups) &&
                            fast::shapes_supported(a.hidden, a.inter, a.w2.groups);
   int rc = KEEPVQ_OK;
-  // many routes per expert: the tcgen05 kernels, which decode a code once per 96 routes
+  // many routes per expert: the tcgen05 kernels
   const int64_t live = a.expected_routes > 0 && a.expected_routes < routes ? a.expected_routes : routes;
   const bool prefill = tensor_path && !residual && live >= PREFILL_MIN_ROUTES && live >= PREFILL_MIN_ROUTES_PER_SLOT * a.slots &&
-                       fast::prefill_supported(a.inter, a.hidden, a.w1.groups) && fast::prefill_supported(a.hidden, a.inter, a.w2.groups);
+                       fast::prefill_supported(a.slots, a.inter, a.hidden, a.w1.groups) && fast::prefill_supported(a.slots, a.hidden, a.inter, a.w2.groups);
   // (the sums regions have room for a scale group per codeword; the tensor-core kernels' rows have at
   // most one per 256 inputs, and their sums per 256 inputs go behind those)
   fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + sc.xq), reinterpret_cast<float*>(ws + sc.xscale), reinterpret_cast<int32_t*>(ws + sc.xsums),
@@ -247,7 +248,7 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
     fast::QuantRows hq = {reinterpret_cast<uint8_t*>(ws + sc.hq), reinterpret_cast<float*>(ws + sc.hscale), reinterpret_cast<int32_t*>(ws + sc.hsums),
                           prefill ? nullptr : reinterpret_cast<int32_t*>(ws + sc.hsums) + (routes + 1) * a.w2.groups};
     int32_t* wait_status = reinterpret_cast<int32_t*>(ws + sc.status);
-    const int group_cols = prefill ? fast::PREFILL_GROUP_ROUTES : fast::decode_group_routes(live, a.slots, std::max(a.hidden, a.inter));
+    const int group_cols = prefill ? fast::prefill_group_routes(live, a.slots, a.w1.groups > 1 || a.w2.groups > 1) : fast::decode_group_routes(live, a.slots, std::max(a.hidden, a.inter));
     if (stages & KEEPVQ_STAGE_PREPARE) {
       if (!x_quantized && !prefill && fast::group_with_quantize_supported(routes, a.slots)) {  // one launch for both
         if ((rc = fast::quantize_rows_and_group(a.x, a.x_dtype, a.tokens, a.hidden, a.w1.groups, xq, false, s, padded, a.top_k, a.slots,
@@ -260,6 +261,7 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
       }
     }
     fast::FastProjectionArgs p = {};
+    p.slots = a.slots;
     p.scales_dtype = a.scales_dtype; p.codebook = a.codebook; p.groups_of_routes = groups; p.max_routes = routes; p.group_cols = group_cols; p.status = wait_status;
     p.few_groups = prefill ? 0 : fast::few_route_groups(live, a.slots);
     p.out_dtype = a.x_dtype; p.swiglu_limit = a.swiglu_limit; p.route_weight = a.served_weight;

@@ -188,6 +188,24 @@ def test_many_routes_per_expert_take_the_tcgen05_kernels(cuda, tokens, experts, 
     check_layer(cfg, x, out, routing, top_k=top_k)
 
 
+@pytest.mark.parametrize("tokens,experts,top_k,hidden,inter,group_hidden,group_inter", [
+    (300, 8, 4, 512, 256, 256, None),    # two segments of two K blocks (each warp's share is one), one in the down projection
+    (700, 5, 2, 1024, 512, 256, 256),    # several 48-route items per expert
+    (260, 24, 4, 1536, 768, 512, 256),   # three segments of four K blocks; partial last row tiles of a 256-row item
+    (171, 40, 6, 512, 512, None, 256),   # 26 routes per expert: the 48-route items of rows with one scale group
+])
+def test_scale_groups_and_short_groups_on_the_tcgen05_kernels(cuda, tokens, experts, top_k, hidden, inter, group_hidden, group_inter):
+    """Rows with several scale groups (accumulators drained once per group into fp32 sums) and
+    items of at most 48 routes; bound: the layer's own (three roundings to bf16)."""
+    cfg = synthetic.layer(seed=51, experts=experts, hidden=hidden, inter=inter, group_hidden=group_hidden, group_inter=group_inter)
+    x = synthetic.tokens(52, tokens, hidden)
+    layer = build_layer(cuda, cfg, top_k=top_k)
+    assert layer.kernel_path == "tensor" and tokens * top_k >= 1024
+    out, routing = layer.decode(x.to(cuda))
+    assert not layer.wait_expired(tokens, x.dtype)
+    check_layer(cfg, x, out, routing, top_k=top_k)
+
+
 def test_many_routes_spread_over_many_experts_stay_on_the_decode_kernels(cuda):
     """1200 routes over 64 experts (under 24 per expert on average): the mma.sync kernels, with
     several 8-route groups per expert."""

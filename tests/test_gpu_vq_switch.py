@@ -135,6 +135,23 @@ def test_sorted_routes_on_the_tensor_core_kernels(cuda, routes, experts, dtype):
         assert direct is not None and torch.equal(direct, got)  # the operator did take this entry point
 
 
+@pytest.mark.parametrize("out,inp,group", [(100, 256, 256), (200, 512, 256), (300, 768, 256), (640, 512, 512)])
+def test_sorted_routes_with_ragged_rows_and_scale_groups(cuda, out, inp, group):
+    """Row counts that no tile divides (the tcgen05 kernels' code boxes then run into the next
+    expert's rows, or past the last), one item tile and several, one scale group and several."""
+    rng = np.random.default_rng(23)
+    experts, routes = 7, 1100
+    codes = rng.integers(0, 1 << 16, (experts, out, inp // 8), dtype=np.uint16)
+    scales = (0.02 * rng.uniform(0.5, 1.5, (experts, out, inp // group))).astype(np.float16)
+    x = torch.from_numpy(rng.normal(size=(routes, inp)).astype(np.float32)).to(torch.bfloat16)
+    rhs = np.sort(rng.integers(0, experts, routes)).astype(np.int64)
+    lhs = np.arange(routes)
+    want = ops.gather_vqmm(x.float().numpy(), codes, scales, None, rhs, lhs_indices=lhs, code_bits=16)
+    got = vq_switch.gather_vqmm_sorted_routes(x.to(cuda), codes, scales, None, rhs, lhs, input_dims=inp, output_dims=out,
+                                              group_size=group, code_bits=16, validate_indices=True)
+    np.testing.assert_allclose(f32(got), want, rtol=1e-2, atol=1e-2)
+
+
 def test_routes_without_an_expert_give_zero_rows_on_every_path(cuda):
     """A route whose index names no expert (0xFFFFFFFF, or any value past the last expert) returns
     a row of zeros from the tensor-core kernels and from the general kernel alike."""
