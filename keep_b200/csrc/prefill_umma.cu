@@ -60,8 +60,7 @@ constexpr int PF_A_TILE_COLS = PF_KBLOCK_CODES * 2;   // a decoded K block of on
 constexpr uint32_t PF_TMEM_COLS = 512;
 constexpr uint32_t PF_CODE_UNIT_BYTES = PF_ROWS * 64; // two K blocks of one tile's codes, 64 bytes per row
 constexpr uint32_t PF_TABLE_BYTES = 64 * 1024;  // the nibble decoder's two tables, interleaved (moe_fast.cuh)
-constexpr uint32_t PF_LOW_UNITS = 6;            // code units below the tables
-constexpr uint32_t PF_LOW_BYTES = PF_LOW_UNITS * PF_CODE_UNIT_BYTES;
+constexpr uint32_t PF_LOW_BYTES = 48 * 1024;    // what lies below the tables: B stages
 constexpr int PF_INFO_BUFFERS = 3;
 constexpr int PF_SMEM_BYTES = 220 * 1024;       // dynamic request: covers A0 + 160 KB from any base below A0 - 48 KB
 constexpr uint64_t PF_DEFAULT_WAIT_NS = 2000000000ull;
@@ -71,7 +70,7 @@ constexpr uint64_t PF_DEFAULT_WAIT_NS = 2000000000ull;
 // decoded A stages of 32 columns per tile.  With several scale groups per row the accumulators are
 // drained once per group, so there are two sets; with one, a single set leaves room for more A stages.
 // Shared window, absolute addresses; A0 = the 64 KB boundary the tables sit on:
-//   [A0 - 48 KB, A0) code units 0-5 | [A0, +64 KB) tables | B stages | code units 6, 7
+//   [A0 - 48 KB, A0) the first B stages | [A0, +64 KB) tables | code stages | the other B stages
 template <int M, int N_MAX, bool GROUPED>
 struct PrefillPlan {
   static_assert(N_MAX % 16 == 0, "an item's routes pad to a multiple of sixteen columns");
@@ -82,9 +81,11 @@ struct PrefillPlan {
   static constexpr uint32_t A_STAGES = (PF_TMEM_COLS - A_COL0) / A_STAGE_COLS >= 4 ? 4 : 2;
   static_assert(A_COL0 + A_STAGES * A_STAGE_COLS <= PF_TMEM_COLS, "tensor memory holds the accumulators and the A stages");
   static constexpr uint32_t B_STAGE_BYTES = 2 * N_MAX * 128;  // high-byte rows of the routes, then their low-byte rows
-  static constexpr uint32_t B_STAGES = N_MAX > 48 ? 4 : 6;
-  static constexpr uint32_t CODE_STAGES = N_MAX > 48 ? 3 : 4;  // units of every tile in flight
-  static constexpr uint32_t HIGH_BYTES = PF_TABLE_BYTES + B_STAGES * B_STAGE_BYTES + (CODE_STAGES * 2 - PF_LOW_UNITS) * PF_CODE_UNIT_BYTES;
+  static constexpr uint32_t LOW_B_STAGES = PF_LOW_BYTES / B_STAGE_BYTES;
+  static constexpr uint32_t B_STAGES = 4;
+  static constexpr uint32_t CODE_STAGE_BYTES = M * PF_CODE_UNIT_BYTES;
+  static constexpr uint32_t CODE_STAGES = N_MAX > 48 ? 3 : 5;
+  static constexpr uint32_t HIGH_BYTES = PF_TABLE_BYTES + CODE_STAGES * CODE_STAGE_BYTES + (B_STAGES - LOW_B_STAGES) * B_STAGE_BYTES;
   static_assert(HIGH_BYTES <= 160 * 1024, "the window above A0");
 };
 
@@ -213,11 +214,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   const uint32_t dyn_base = smem_addr(smem_raw);
   const uint32_t a0 = (dyn_base + PF_LOW_BYTES + 0xFFFFu) & ~0xFFFFu;
   const bool window_ok = a0 + Plan::HIGH_BYTES <= dyn_base + PF_SMEM_BYTES;  // uniform over the grid
-  auto b_stage_addr = [&](uint32_t stage) { return a0 + PF_TABLE_BYTES + stage * Plan::B_STAGE_BYTES; };
-  auto code_unit_addr = [&](uint32_t stage, uint32_t m) {
-    const uint32_t unit = 2 * stage + m;
-    return unit < PF_LOW_UNITS ? a0 - PF_LOW_BYTES + unit * PF_CODE_UNIT_BYTES
-                               : a0 + PF_TABLE_BYTES + B_STAGES * Plan::B_STAGE_BYTES + (unit - PF_LOW_UNITS) * PF_CODE_UNIT_BYTES;
+  const uint32_t code_base = a0 + PF_TABLE_BYTES;
+  auto b_stage_addr = [&](uint32_t stage) {
+    return stage < Plan::LOW_B_STAGES ? a0 - PF_LOW_BYTES + stage * Plan::B_STAGE_BYTES
+                                      : code_base + CODE_STAGES * Plan::CODE_STAGE_BYTES + (stage - Plan::LOW_B_STAGES) * Plan::B_STAGE_BYTES;
   };
 
   // ---- set-up: tables, barriers, tensor memory ------------------------------------------------
@@ -259,8 +259,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     const int row = quadrant * 32 + lane;
     const uint32_t abs_lane = a0 + lane * 4u, sign_lane = a0 + 128u + lane * 4u;
     const uint32_t lane_tmem = tmem + (static_cast<uint32_t>(quadrant * 32) << 16);
-    const uint32_t code_chunk0 = row * 64u + (((2u * parity) ^ ((row >> 1) & 3u)) << 4);  // 64-byte swizzle: 16-byte chunk ^ (row / 2) % 4
-    const uint32_t code_chunk1 = row * 64u + (((2u * parity + 1u) ^ ((row >> 1) & 3u)) << 4);
+    const uint32_t code_chunk0 = code_base + m * PF_CODE_UNIT_BYTES + row * 64u + (((2u * parity) ^ ((row >> 1) & 3u)) << 4);  // 64-byte swizzle: 16-byte chunk ^ (row / 2) % 4
+    const uint32_t code_chunk1 = code_base + m * PF_CODE_UNIT_BYTES + row * 64u + (((2u * parity + 1u) ^ ((row >> 1) & 3u)) << 4);
     const Projection mats[2] = {p.a, GLU ? p.b : p.a};
     const bool scales32 = p.scales_dtype == KEEPVQ_F32;
     const float limit = p.swiglu_limit > 0.0f ? p.swiglu_limit : INFINITY;
@@ -399,6 +399,16 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
 #pragma unroll
         for (int c = 0; c < N_MAX / 4; ++c) sum[mm][c] = 0.0f;
     }
+    // The codes of this warp's next K block are read ahead, while the current one goes to tensor memory.
+    int blocks_left = m < M && blockIdx.x < items ? ((items - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1) * code_units : 0;
+    uint32_t w[8];
+    auto read_codes = [&]() {
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(CODE_FULL, code.index), code.phase, deadline, aborted));
+      const uint32_t at = code.index * Plan::CODE_STAGE_BYTES;
+      asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(code_chunk0 + at));
+      asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(code_chunk1 + at));
+    };
+    if (blocks_left > 0) read_codes();
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
       const int gi = item / row_tiles, tile = item - gi * row_tiles;
       const int64_t slot = p.groups_of_routes.slot[gi];
@@ -406,12 +416,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       for (int segment = 0; segment < segments && ok; ++segment) {
         if (m < M) {
           for (int b = parity; b < segment_blocks; b += 2) {
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(CODE_FULL, code.index), code.phase, deadline, aborted));
-            if (!ok) break;
-            const uint32_t unit = code_unit_addr(code.index, m);
-            uint32_t w[8], q[32];
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(unit + code_chunk0));
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(unit + code_chunk1));
+            uint32_t q[32];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               decode_codeword_nibble<false>(w[i], abs_lane, sign_lane, q[4 * i], q[4 * i + 1]);
@@ -420,7 +425,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(CODE_EMPTY, code.index));
             code.advance();
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(A_EMPTY, stage.index), stage.phase ^ 1u, deadline, aborted));
+            if (--blocks_left > 0) read_codes();
+            ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(bar(A_EMPTY, stage.index), stage.phase ^ 1u, deadline, aborted));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             tmem_st32(lane_tmem + Plan::A_COL0 + stage.index * Plan::A_STAGE_COLS + m * PF_A_TILE_COLS, q);
@@ -562,7 +568,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         const uint32_t full = bar(CODE_FULL, code.index);
         mbar_expect_tx(full, M * PF_CODE_UNIT_BYTES);
 #pragma unroll
-        for (int m = 0; m < M; ++m) tma_box_2d(code_unit_addr(code.index, m), GLU && m ? &b_map : &a_map, u * 64, row0 + m * TILE_STEP, full);
+        for (int m = 0; m < M; ++m) tma_box_2d(code_base + code.index * Plan::CODE_STAGE_BYTES + m * PF_CODE_UNIT_BYTES, GLU && m ? &b_map : &a_map, u * 64, row0 + m * TILE_STEP, full);
         ++used;
         code.advance();
       }

@@ -139,6 +139,8 @@ def test_sorted_routes_on_the_tensor_core_kernels(cuda, routes, experts, dtype):
 def test_sorted_routes_with_ragged_rows_and_scale_groups(cuda, out, inp, group):
     """Row counts that no tile divides (the tcgen05 kernels' code boxes then run into the next
     expert's rows, or past the last), one item tile and several, one scale group and several."""
+    from keep_b200 import vq_switch
+
     rng = np.random.default_rng(23)
     experts, routes = 7, 1100
     codes = rng.integers(0, 1 << 16, (experts, out, inp // 8), dtype=np.uint16)
