@@ -82,9 +82,9 @@ struct PrefillPlan {
   static_assert(A_COL0 + A_STAGES * A_STAGE_COLS <= PF_TMEM_COLS, "tensor memory holds the accumulators and the A stages");
   static constexpr uint32_t B_STAGE_BYTES = 2 * N_MAX * 128;  // high-byte rows of the routes, then their low-byte rows
   static constexpr uint32_t LOW_B_STAGES = PF_LOW_BYTES / B_STAGE_BYTES;
-  static constexpr uint32_t B_STAGES = 4;
+  static constexpr uint32_t B_STAGES = N_MAX > 48 ? 4 : 6;
   static constexpr uint32_t CODE_STAGE_BYTES = M * PF_CODE_UNIT_BYTES;
-  static constexpr uint32_t CODE_STAGES = N_MAX > 48 ? 3 : 5;
+  static constexpr uint32_t CODE_STAGES = N_MAX > 48 ? 3 : 4;
   static constexpr uint32_t HIGH_BYTES = PF_TABLE_BYTES + CODE_STAGES * CODE_STAGE_BYTES + (B_STAGES - LOW_B_STAGES) * B_STAGE_BYTES;
   static_assert(HIGH_BYTES <= 160 * 1024, "the window above A0");
 };
@@ -108,20 +108,25 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Wait bounded by time.  Returns false when the deadline passes (the caller's CTA then gives up:
-// the flag is raised for every role) or when another thread of the CTA already gave up.
+// the flag is raised for every role) or when another thread of the CTA already gave up.  RELAXED is
+// for the loaders, which run stages ahead: their polls would take issue slots from the decode warps.
+template <bool RELAXED = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t deadline, volatile int* abort_flag) {
   for (uint32_t spin = 0;; ++spin) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (done) return true;
+    if (RELAXED) __nanosleep(40);
     if ((spin & 31u) == 31u) {
       if (*abort_flag) return false;
       if (global_timer_ns() > deadline) { *abort_flag = 1; return false; }
     }
   }
 }
-
+// A value that is the same in every lane, in a form the compiler knows to be: what depends on it
+// (loop bounds, descriptors of MMAs and copies) then lives in uniform registers.
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
 // The wait of a CTA that has given up, for what it still has in flight: bounded by 100 ms.
 __device__ __forceinline__ void mbar_wait_grace(uint32_t bar, uint32_t parity) {
   const uint64_t grace = global_timer_ns() + 100000000ull;
@@ -170,6 +175,10 @@ __device__ __forceinline__ void tma_box_2d(uint32_t dst, const CUtensorMap* map,
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void tma_box_3d(uint32_t dst, const CUtensorMap* map, int32_t x, int32_t y, int32_t z, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+               ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -191,8 +200,12 @@ struct RingPlace {
 // the K blocks) into fp32 sums that the drain warps keep in registers.
 // `stall` != 0 is the wait self-test: the activation loader never publishes, so the MMA issuer's
 // first wait runs into the deadline.
+// Boxes over the activations, one map per padded number of routes: [2 planes][16 (i + 1) rows][128 bytes].
+template <int N_MAX>
+struct ActivationMaps { CUtensorMap rows[N_MAX / 16]; };
+
 template <int M, bool GLU, int N_MAX, bool GROUPED>
-__global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastProjectionArgs p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap a_map,
+__global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastProjectionArgs p, const __grid_constant__ ActivationMaps<N_MAX> x_maps, const __grid_constant__ CUtensorMap a_map,
                                                                            const __grid_constant__ CUtensorMap b_map, int32_t* status, int stall, uint64_t wait_ns) {
   using Plan = PrefillPlan<M, N_MAX, GROUPED>;
   constexpr int ITEM_ROWS = GLU ? PF_ROWS : PF_ROWS * M;
@@ -239,7 +252,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_base_slot;
+  const bool set_up_ok = window_ok && tmem_base_slot == 0;  // uniform over the block
+  if (!set_up_ok && tid == 0) abort_flag = 1;
+  // an allocation of all 512 columns starts at column 0 of lane 0: a constant, which keeps the MMAs' operands in uniform registers
+  constexpr uint32_t tmem = 0;
 
   const int64_t N_out = p.out_dim;
   const int k_blocks = static_cast<int>(p.in_dim / (8 * PF_KBLOCK_CODES));
@@ -247,8 +263,9 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   const int segments = GROUPED ? static_cast<int>(p.groups) : 1;  // drains per item
   const int segment_blocks = k_blocks / segments;
   const int row_tiles = static_cast<int>((N_out + ITEM_ROWS - 1) / ITEM_ROWS);
-  const int items = p.groups_of_routes.count[0] * row_tiles;
+  const int items = warp_uniform(p.groups_of_routes.count[0]) * row_tiles;
   volatile int* aborted = &abort_flag;
+  const int items_here = set_up_ok ? items : 0;
   bool mma_issued = false;
 
   // Every role walks the same item list on its own clock; barriers carry the dependencies.
@@ -399,24 +416,19 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
 #pragma unroll
         for (int c = 0; c < N_MAX / 4; ++c) sum[mm][c] = 0.0f;
     }
-    // The codes of this warp's next K block are read ahead, while the current one goes to tensor memory.
-    int blocks_left = m < M && blockIdx.x < items ? ((items - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1) * code_units : 0;
-    uint32_t w[8];
-    auto read_codes = [&]() {
-      ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(CODE_FULL, code.index), code.phase, deadline, aborted));
-      const uint32_t at = code.index * Plan::CODE_STAGE_BYTES;
-      asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(code_chunk0 + at));
-      asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(code_chunk1 + at));
-    };
-    if (blocks_left > 0) read_codes();
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+    for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
       const int gi = item / row_tiles, tile = item - gi * row_tiles;
       const int64_t slot = p.groups_of_routes.slot[gi];
       const int gsize = p.groups_of_routes.size[gi], gstart = p.groups_of_routes.start[gi];
       for (int segment = 0; segment < segments && ok; ++segment) {
         if (m < M) {
           for (int b = parity; b < segment_blocks; b += 2) {
-            uint32_t q[32];
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(CODE_FULL, code.index), code.phase, deadline, aborted));
+            if (!ok) break;
+            const uint32_t at = code.index * Plan::CODE_STAGE_BYTES;
+            uint32_t w[8], q[32];
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(code_chunk0 + at));
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(code_chunk1 + at));
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               decode_codeword_nibble<false>(w[i], abs_lane, sign_lane, q[4 * i], q[4 * i + 1]);
@@ -425,8 +437,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(CODE_EMPTY, code.index));
             code.advance();
-            if (--blocks_left > 0) read_codes();
-            ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(bar(A_EMPTY, stage.index), stage.phase ^ 1u, deadline, aborted));
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(A_EMPTY, stage.index), stage.phase ^ 1u, deadline, aborted));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             tmem_st32(lane_tmem + Plan::A_COL0 + stage.index * Plan::A_STAGE_COLS + m * PF_A_TILE_COLS, q);
@@ -467,9 +478,9 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     RingPlace<ACC_SETS> acc;
     uint32_t info_index = 0;
     bool ok = true, first_round = true;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+    for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
       const int gi = item / row_tiles;
-      const int gsize = p.groups_of_routes.size[gi], gstart = p.groups_of_routes.start[gi];
+      const int gsize = warp_uniform(p.groups_of_routes.size[gi]), gstart = p.groups_of_routes.start[gi];
       const int n_pad = (gsize + 15) & ~15;  // the N of the MMA
       // The facts go into the buffer of item n - 3.  Behind every MMA of item n - 1 stand all decode
       // warps' K blocks of that item, and a warp produces those only after its drain of item n - 3
@@ -522,28 +533,27 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       }
       __syncwarp();
     }
-  } else if (warp == PF_B_WARP && lane == 0) {
+  } else if (warp == PF_B_WARP) {
     // ================= activation (B operand) loader: TMA ====================================
-    // Rows gstart .. gstart + n_pad - 1 of the high-byte plane and of the low-byte plane, 16 rows
-    // per box (a box lands swizzled at a 2 KB step of the tile); rows past the group's own belong
-    // to the next group or to nobody, and nobody looks at their columns.  One thread issues.
+    // Rows gstart .. gstart + n_pad - 1 of the high-byte plane and of the low-byte plane in one box,
+    // which lands swizzled as the operand tile it is; rows past the group's own belong to the next
+    // group or to nobody, and nobody looks at their columns.  The whole warp walks and one elected
+    // lane issues: from a branch of one lane a copy cost some 150 cycles of its issue.
     RingPlace<B_STAGES> b;
     uint32_t used = 0;
     bool ok = true;
-    const int32_t plane_rows = static_cast<int32_t>(p.x_zero_row + 1);
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+    for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
       const int gi = item / row_tiles;
-      const int gsize = p.groups_of_routes.size[gi], gstart = p.groups_of_routes.start[gi];
+      const int gsize = warp_uniform(p.groups_of_routes.size[gi]), gstart = warp_uniform(p.groups_of_routes.start[gi]);
       const int n_pad = (gsize + 15) & ~15;
+      const CUtensorMap* map = &x_maps.rows[(n_pad >> 4) - 1];
       for (int kb = 0; kb < k_blocks; ++kb) {
-        ok = mbar_wait(bar(B_EMPTY, b.index), b.phase ^ 1u, deadline, aborted);
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait<true>(bar(B_EMPTY, b.index), b.phase ^ 1u, deadline, aborted));
         if (!ok) break;
         if (!stall) {  // (the wait self-test: nothing is ever published)
-          const uint32_t b_stage = b_stage_addr(b.index), full = bar(B_FULL, b.index);
-          mbar_expect_tx(full, static_cast<uint32_t>(2 * n_pad * 128));
-          for (int r = 0; r < n_pad; r += 16) {
-            tma_box_2d(b_stage + r * 128, &x_map, kb * 128, gstart + r, full);
-            tma_box_2d(b_stage + (n_pad + r) * 128, &x_map, kb * 128, plane_rows + gstart + r, full);
+          if (elect_one()) {
+            mbar_expect_tx(bar(B_FULL, b.index), static_cast<uint32_t>(2 * n_pad * 128));
+            tma_box_3d(b_stage_addr(b.index), map, kb * 128, gstart, 0, bar(B_FULL, b.index));
           }
           ++used;
         }
@@ -551,7 +561,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       }
     }
     if (*aborted) wait_copies_landed<B_STAGES>(bar(B_FULL, 0), used);
-  } else if (warp == PF_CODE_WARP && lane == 0) {
+  } else if (warp == PF_CODE_WARP) {
     // ================= code loader: TMA ======================================================
     // Two K blocks (64 bytes of a row's codes) of every tile per stage, straight from the caller's
     // layout seen as one [slots * out_dim, in_dim / 4] byte matrix; rows past a slot's last tile are
@@ -559,16 +569,18 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     RingPlace<CODE_STAGES> code;
     uint32_t used = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+    for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
       const int gi = item / row_tiles, tile = item - gi * row_tiles;
-      const int32_t row0 = static_cast<int32_t>(p.groups_of_routes.slot[gi] * N_out + static_cast<int64_t>(tile) * ITEM_ROWS);
+      const int row0 = warp_uniform(static_cast<int>(p.groups_of_routes.slot[gi] * N_out + static_cast<int64_t>(tile) * ITEM_ROWS));
       for (int u = 0; u < code_units; ++u) {
-        ok = mbar_wait(bar(CODE_EMPTY, code.index), code.phase ^ 1u, deadline, aborted);
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait<true>(bar(CODE_EMPTY, code.index), code.phase ^ 1u, deadline, aborted));
         if (!ok) break;
-        const uint32_t full = bar(CODE_FULL, code.index);
-        mbar_expect_tx(full, M * PF_CODE_UNIT_BYTES);
-#pragma unroll
-        for (int m = 0; m < M; ++m) tma_box_2d(code_base + code.index * Plan::CODE_STAGE_BYTES + m * PF_CODE_UNIT_BYTES, GLU && m ? &b_map : &a_map, u * 64, row0 + m * TILE_STEP, full);
+        if (elect_one()) {
+          const uint32_t full = bar(CODE_FULL, code.index);
+          mbar_expect_tx(full, Plan::CODE_STAGE_BYTES);
+          tma_box_2d(code_base + code.index * Plan::CODE_STAGE_BYTES, &a_map, u * 64, row0, full);
+          if (GLU) tma_box_2d(code_base + code.index * Plan::CODE_STAGE_BYTES + PF_CODE_UNIT_BYTES, &b_map, u * 64, row0, full);
+        }
         ++used;
         code.advance();
       }
@@ -579,7 +591,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   // ---- teardown ------------------------------------------------------------------------------
   __syncwarp();
   if (*aborted) {
-    if (tid == 0 && status) atomicExch(status, window_ok ? 1 : 2);
+    if (tid == 0 && status) atomicExch(status, set_up_ok ? 1 : 2);
     // MMAs may still be in flight: one more commit arrives when they are all done; wait for it, bounded as every wait
     if (warp == PF_MMA_WARP && mma_issued && elect_one()) {  // the lane that issued: a commit follows its own thread's MMAs
       umma_commit(bar(DRAINED, 0));
@@ -588,7 +600,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == PF_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PF_TMEM_COLS) : "memory");
+  if (warp == PF_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_slot), "r"(PF_TMEM_COLS) : "memory");
 }
 
 bool prefill_supported(int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups) {
@@ -605,8 +617,9 @@ int prefill_group_routes(int64_t live, int64_t slots, bool several_groups) {
   return several_groups || live <= PREFILL_FEW_ROUTES_MEAN * slots ? PREFILL_GROUP_ROUTES_SMALL : PREFILL_GROUP_ROUTES;
 }
 
-// A tensor map of bytes in this GPU's own memory: [rows, row_bytes], boxes of box_rows x box_bytes.
-static int byte_map(CUtensorMap* map, const void* base, int64_t row_bytes, int64_t rows, uint32_t box_bytes, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
+// A tensor map of bytes in this GPU's own memory: `planes` matrices of [rows, row_bytes] one after the
+// other, boxes of planes x box_rows x box_bytes.
+static int byte_map(CUtensorMap* map, const void* base, int64_t row_bytes, int64_t rows, uint32_t planes, uint32_t box_bytes, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
   typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
   static EncodeTiled encode = nullptr;
@@ -619,29 +632,28 @@ static int byte_map(CUtensorMap* map, const void* base, int64_t row_bytes, int64
     encode = reinterpret_cast<EncodeTiled>(fn);
   }
   if (row_bytes % 16 != 0 || (reinterpret_cast<uintptr_t>(base) & 15u) != 0) return KEEPVQ_ERR_ALIGN;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(row_bytes), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
-  const cuuint32_t box[2] = {box_bytes, box_rows}, element_strides[2] = {1, 1};
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(row_bytes), static_cast<cuuint64_t>(rows), planes};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(row_bytes), static_cast<cuuint64_t>(row_bytes * rows)};
+  const cuuint32_t box[3] = {box_bytes, box_rows, planes}, element_strides[3] = {1, 1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, planes > 1 ? 3 : 2, const_cast<void*>(base), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? KEEPVQ_OK : KEEPVQ_ERR_LAUNCH;
 }
-// A projection's quantised activations: a [2 * (rows + 1), in_dim] byte matrix (the high-byte plane
-// over the low-byte plane).
-static int activation_map(const FastProjectionArgs& p, CUtensorMap* map) {
-  return byte_map(map, p.x.q, p.in_dim, 2 * (p.x_zero_row + 1), 128, 16, CU_TENSOR_MAP_SWIZZLE_128B);
-}
 // A projection's codes: a [slots * out_dim, in_dim / 4] byte matrix.
-static int code_map(const FastProjectionArgs& p, const uint16_t* codes, CUtensorMap* map) {
-  return byte_map(map, codes, p.in_dim / 4, p.slots * p.out_dim, 64, PF_ROWS, CU_TENSOR_MAP_SWIZZLE_64B);
+static int code_map(const FastProjectionArgs& p, const uint16_t* codes, uint32_t box_rows, CUtensorMap* map) {
+  return byte_map(map, codes, p.in_dim / 4, p.slots * p.out_dim, 1, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 template <int M, bool GLU, int N_MAX, bool GROUPED>
 static int launch_prefill(const FastProjectionArgs& p, int32_t* status, cudaStream_t s, int stall = 0, uint64_t wait_ns = 0, int ctas = 0) {
-  CUtensorMap x_map, a_map, b_map;
-  if (const int rc = activation_map(p, &x_map)) return rc;
-  if (const int rc = code_map(p, p.a.codes, &a_map)) return rc;
-  if (const int rc = code_map(p, GLU ? p.b.codes : p.a.codes, &b_map)) return rc;
+  ActivationMaps<N_MAX> x_maps;  // the quantised activations: the high-byte plane, then the low-byte plane, each [rows + 1, in_dim]
+  for (int i = 0; i < N_MAX / 16; ++i)
+    if (const int rc = byte_map(&x_maps.rows[i], p.x.q, p.in_dim, p.x_zero_row + 1, 2, 128, 16 * (i + 1), CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+  CUtensorMap a_map, b_map;
+  if (const int rc = code_map(p, p.a.codes, GLU ? PF_ROWS : PF_ROWS * M, &a_map)) return rc;
+  if (GLU) {
+    if (const int rc = code_map(p, p.b.codes, PF_ROWS, &b_map)) return rc;
+  } else b_map = a_map;
   auto kernel = prefill_projection_kernel<M, GLU, N_MAX, GROUPED>;
   static uint64_t configured = 0;  // one bit per device: the shared-memory opt-in is a per-device attribute of the function
   int dev = 0, sms = 148;
@@ -652,7 +664,7 @@ static int launch_prefill(const FastProjectionArgs& p, int32_t* status, cudaStre
     if (dev >= 0 && dev < 64) configured |= 1ull << dev;
   }
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  kernel<<<ctas > 0 ? ctas : sms, PF_THREADS, PF_SMEM_BYTES, s>>>(p, x_map, a_map, b_map, status, stall, wait_ns);
+  kernel<<<ctas > 0 ? ctas : sms, PF_THREADS, PF_SMEM_BYTES, s>>>(p, x_maps, a_map, b_map, status, stall, wait_ns);
   KEEPVQ_CHECK_LAUNCH();
   return KEEPVQ_OK;
 }
