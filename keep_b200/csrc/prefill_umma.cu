@@ -60,17 +60,20 @@ constexpr int PF_A_TILE_COLS = PF_KBLOCK_CODES * 2;   // a decoded K block of on
 constexpr uint32_t PF_TMEM_COLS = 512;
 constexpr uint32_t PF_CODE_UNIT_BYTES = PF_ROWS * 64; // two K blocks of one tile's codes, 64 bytes per row
 constexpr uint32_t PF_TABLE_BYTES = 64 * 1024;  // the nibble decoder's two tables, interleaved (moe_fast.cuh)
+// Shared window, absolute addresses (compile-time constants: the operands of the MMAs, copies and
+// barriers are then immediates); a block whose window lies elsewhere reports and does nothing.
+constexpr uint32_t PF_A0 = 64 * 1024;           // the 64 KB boundary the tables sit on
 constexpr uint32_t PF_LOW_BYTES = 48 * 1024;    // what lies below the tables: B stages
+constexpr uint32_t PF_BARS = PF_A0 - PF_LOW_BYTES - 1024;  // the mbarriers, below those
 constexpr int PF_INFO_BUFFERS = 3;
-constexpr int PF_SMEM_BYTES = 220 * 1024;       // dynamic request: covers A0 + 160 KB from any base below A0 - 48 KB
+constexpr int PF_SMEM_BYTES = 222 * 1024;       // dynamic request: reaches A0 + 160 KB behind the 3 to 5 KB of static and reserved shared memory
 constexpr uint64_t PF_DEFAULT_WAIT_NS = 2000000000ull;
 
 // What a kernel that takes up to N_MAX routes per item keeps in tensor memory and shared memory.
 // Tensor memory (512 columns): per accumulator set 2 byte planes x M tiles x N_MAX columns, the rest
 // decoded A stages of 32 columns per tile.  With several scale groups per row the accumulators are
 // drained once per group, so there are two sets; with one, a single set leaves room for more A stages.
-// Shared window, absolute addresses; A0 = the 64 KB boundary the tables sit on:
-//   [A0 - 48 KB, A0) the first B stages | [A0, +64 KB) tables | code stages | the other B stages
+// Shared window: [A0 - 48 KB, A0) the first B stages | [A0, +64 KB) tables | code stages | the other B stages
 template <int M, int N_MAX, bool GROUPED>
 struct PrefillPlan {
   static_assert(N_MAX % 16 == 0, "an item's routes pad to a multiple of sixteen columns");
@@ -82,11 +85,16 @@ struct PrefillPlan {
   static_assert(A_COL0 + A_STAGES * A_STAGE_COLS <= PF_TMEM_COLS, "tensor memory holds the accumulators and the A stages");
   static constexpr uint32_t B_STAGE_BYTES = 2 * N_MAX * 128;  // high-byte rows of the routes, then their low-byte rows
   static constexpr uint32_t LOW_B_STAGES = PF_LOW_BYTES / B_STAGE_BYTES;
-  static constexpr uint32_t B_STAGES = N_MAX > 48 ? 4 : 6;
+  static constexpr uint32_t B_STAGES = N_MAX > 48 ? 4 : 8;    // one ring of barriers for A and B: a K block's A stage is its B stage modulo A_STAGES
+  static_assert(B_STAGES % A_STAGES == 0, "");
   static constexpr uint32_t CODE_STAGE_BYTES = M * PF_CODE_UNIT_BYTES;
-  static constexpr uint32_t CODE_STAGES = N_MAX > 48 ? 3 : 4;
+  static constexpr uint32_t CODE_STAGES = 3;
   static constexpr uint32_t HIGH_BYTES = PF_TABLE_BYTES + CODE_STAGES * CODE_STAGE_BYTES + (B_STAGES - LOW_B_STAGES) * B_STAGE_BYTES;
   static_assert(HIGH_BYTES <= 160 * 1024, "the window above A0");
+  static constexpr uint32_t CODE_BASE = PF_A0 + PF_TABLE_BYTES;
+  static constexpr __host__ __device__ uint32_t b_stage(uint32_t stage) {
+    return stage < LOW_B_STAGES ? PF_A0 - PF_LOW_BYTES + stage * B_STAGE_BYTES : CODE_BASE + CODE_STAGES * CODE_STAGE_BYTES + (stage - LOW_B_STAGES) * B_STAGE_BYTES;
+  }
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -107,20 +115,21 @@ __device__ __forceinline__ uint32_t elect_one() {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Wait bounded by time.  Returns false when the deadline passes (the caller's CTA then gives up:
-// the flag is raised for every role) or when another thread of the CTA already gave up.  RELAXED is
-// for the loaders, which run stages ahead: their polls would take issue slots from the decode warps.
+// Wait of a whole warp, bounded by time.  Returns false (in every lane) when the deadline passes (the
+// caller's CTA then gives up: the flag is raised for every role) or when another warp of the CTA
+// already gave up.  RELAXED is for the loaders, which run stages ahead: their polls would take issue
+// slots from the decode warps.
 template <bool RELAXED = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t deadline, volatile int* abort_flag) {
   for (uint32_t spin = 0;; ++spin) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
+    if (__all_sync(0xFFFFFFFFu, done)) return true;
     if (RELAXED) __nanosleep(40);
     if ((spin & 31u) == 31u) {
-      if (*abort_flag) return false;
-      if (global_timer_ns() > deadline) { *abort_flag = 1; return false; }
+      if (__any_sync(0xFFFFFFFFu, *abort_flag)) return false;
+      if (__any_sync(0xFFFFFFFFu, global_timer_ns() > deadline)) { *abort_flag = 1; return false; }
     }
   }
 }
@@ -212,37 +221,31 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   constexpr int A_STAGES = Plan::A_STAGES, B_STAGES = Plan::B_STAGES, CODE_STAGES = Plan::CODE_STAGES, ACC_SETS = Plan::ACC_SETS;
   constexpr int TILE_STEP = GLU ? 0 : PF_ROWS;  // rows between the A tiles of an item
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  enum { A_FULL = 0, A_EMPTY = A_FULL + A_STAGES, B_FULL = A_EMPTY + A_STAGES, B_EMPTY = B_FULL + B_STAGES, CODE_FULL = B_EMPTY + B_STAGES, CODE_EMPTY = CODE_FULL + CODE_STAGES,
+  // STAGE_FULL: the decode warps' A tiles and the activations of a K block are in place; STAGE_EMPTY: its MMAs have read them
+  enum { STAGE_FULL = 0, STAGE_EMPTY = STAGE_FULL + B_STAGES, CODE_FULL = STAGE_EMPTY + B_STAGES, CODE_EMPTY = CODE_FULL + CODE_STAGES,
          ACC_FULL = CODE_EMPTY + CODE_STAGES, ACC_EMPTY = ACC_FULL + ACC_SETS, INFO_FULL = ACC_EMPTY + ACC_SETS, DRAINED = INFO_FULL + PF_INFO_BUFFERS, N_BARS = DRAINED + 1 };
-  __shared__ __align__(8) uint64_t bars[N_BARS];
+  static_assert(N_BARS * 8 <= 1024, "");
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
   __shared__ int4 route_info[PF_INFO_BUFFERS][N_MAX];  // per item (three in flight): route, x scale, x sum (one scale group only), gate weight
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t bar0 = smem_addr(&bars[0]);
-  auto bar = [&](int which, uint32_t index) { return bar0 + 8u * (static_cast<uint32_t>(which) + index); };
+  auto bar = [](int which, uint32_t index) { return PF_BARS + 8u * (static_cast<uint32_t>(which) + index); };
   const uint64_t deadline = global_timer_ns() + (wait_ns ? wait_ns : PF_DEFAULT_WAIT_NS);
 
-  // ---- the shared window --------------------------------------------------------------------------
   const uint32_t dyn_base = smem_addr(smem_raw);
-  const uint32_t a0 = (dyn_base + PF_LOW_BYTES + 0xFFFFu) & ~0xFFFFu;
-  const bool window_ok = a0 + Plan::HIGH_BYTES <= dyn_base + PF_SMEM_BYTES;  // uniform over the grid
-  const uint32_t code_base = a0 + PF_TABLE_BYTES;
-  auto b_stage_addr = [&](uint32_t stage) {
-    return stage < Plan::LOW_B_STAGES ? a0 - PF_LOW_BYTES + stage * Plan::B_STAGE_BYTES
-                                      : code_base + CODE_STAGES * Plan::CODE_STAGE_BYTES + (stage - Plan::LOW_B_STAGES) * Plan::B_STAGE_BYTES;
-  };
+  const bool window_ok = dyn_base <= PF_BARS && PF_A0 + Plan::HIGH_BYTES <= dyn_base + PF_SMEM_BYTES;  // uniform over the grid
 
   // ---- set-up: tables, barriers, tensor memory ------------------------------------------------
-  if (window_ok) build_nibble_tables(a0, p.codebook, tid, PF_THREADS);
+  if (window_ok) build_nibble_tables(PF_A0, p.codebook, tid, PF_THREADS);
   if (tid == 0) {
     abort_flag = window_ok ? 0 : 1;
-    for (int s = 0; s < A_STAGES; ++s) { mbar_init(bar(A_FULL, s), M * 4); mbar_init(bar(A_EMPTY, s), 1); }
-    for (int s = 0; s < B_STAGES; ++s) { mbar_init(bar(B_FULL, s), 1); mbar_init(bar(B_EMPTY, s), 1); }
-    for (int s = 0; s < CODE_STAGES; ++s) { mbar_init(bar(CODE_FULL, s), 1); mbar_init(bar(CODE_EMPTY, s), M * 8); }
-    for (int s = 0; s < ACC_SETS; ++s) { mbar_init(bar(ACC_FULL, s), 1); mbar_init(bar(ACC_EMPTY, s), PF_DECODE_WARPS); }
-    for (int s = 0; s < PF_INFO_BUFFERS; ++s) mbar_init(bar(INFO_FULL, s), 1);
-    mbar_init(bar(DRAINED, 0), 1);
+    if (window_ok) {
+      for (int s = 0; s < B_STAGES; ++s) { mbar_init(bar(STAGE_FULL, s), M * 4 + 1); mbar_init(bar(STAGE_EMPTY, s), 1); }
+      for (int s = 0; s < CODE_STAGES; ++s) { mbar_init(bar(CODE_FULL, s), 1); mbar_init(bar(CODE_EMPTY, s), M * 8); }
+      for (int s = 0; s < ACC_SETS; ++s) { mbar_init(bar(ACC_FULL, s), 1); mbar_init(bar(ACC_EMPTY, s), PF_DECODE_WARPS); }
+      for (int s = 0; s < PF_INFO_BUFFERS; ++s) mbar_init(bar(INFO_FULL, s), 1);
+      mbar_init(bar(DRAINED, 0), 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == PF_MMA_WARP) {
@@ -274,16 +277,18 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     const int quadrant = warp & 3, part = warp >> 2;    // part: which quarter of the columns this warp drains
     const int m = warp >> 3, parity = (warp >> 2) & 1;  // decodes every other K block of tile m
     const int row = quadrant * 32 + lane;
-    const uint32_t abs_lane = a0 + lane * 4u, sign_lane = a0 + 128u + lane * 4u;
+    const uint32_t abs_lane = PF_A0 + lane * 4u, sign_lane = PF_A0 + 128u + lane * 4u;
     const uint32_t lane_tmem = tmem + (static_cast<uint32_t>(quadrant * 32) << 16);
-    const uint32_t code_chunk0 = code_base + m * PF_CODE_UNIT_BYTES + row * 64u + (((2u * parity) ^ ((row >> 1) & 3u)) << 4);  // 64-byte swizzle: 16-byte chunk ^ (row / 2) % 4
-    const uint32_t code_chunk1 = code_base + m * PF_CODE_UNIT_BYTES + row * 64u + (((2u * parity + 1u) ^ ((row >> 1) & 3u)) << 4);
+    const uint32_t code_chunk0 = Plan::CODE_BASE + m * PF_CODE_UNIT_BYTES + row * 64u + (((2u * parity) ^ ((row >> 1) & 3u)) << 4);  // 64-byte swizzle: 16-byte chunk ^ (row / 2) % 4
+    const uint32_t code_chunk1 = Plan::CODE_BASE + m * PF_CODE_UNIT_BYTES + row * 64u + (((2u * parity + 1u) ^ ((row >> 1) & 3u)) << 4);
     const Projection mats[2] = {p.a, GLU ? p.b : p.a};
     const bool scales32 = p.scales_dtype == KEEPVQ_F32;
     const float limit = p.swiglu_limit > 0.0f ? p.swiglu_limit : INFINITY;
     RingPlace<CODE_STAGES> code;
-    RingPlace<A_STAGES> stage;
+    RingPlace<B_STAGES> stage, freed;  // of this warp's K block, and of the one A_STAGES before it
     stage.advance(parity);
+    freed.advance(parity);
+    int fresh = A_STAGES / 2;          // this warp's first K blocks find their A stages free
     RingPlace<ACC_SETS> acc;
     RingPlace<PF_INFO_BUFFERS> info;
     bool ok = true;
@@ -394,8 +399,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     };
     auto drain = [&]() {
       pending = false;
-      ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(bar(INFO_FULL, info.index), info.phase, deadline, aborted));
-      ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(bar(ACC_FULL, acc.index), acc.phase, deadline, aborted));
+      ok = ok && mbar_wait(bar(INFO_FULL, info.index), info.phase, deadline, aborted);
+      ok = ok && mbar_wait(bar(ACC_FULL, acc.index), acc.phase, deadline, aborted);
       if (!ok) return;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (p.out_dtype == KEEPVQ_BF16)
@@ -423,7 +428,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       for (int segment = 0; segment < segments && ok; ++segment) {
         if (m < M) {
           for (int b = parity; b < segment_blocks; b += 2) {
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(CODE_FULL, code.index), code.phase, deadline, aborted));
+            ok = mbar_wait(bar(CODE_FULL, code.index), code.phase, deadline, aborted);
             if (!ok) break;
             const uint32_t at = code.index * Plan::CODE_STAGE_BYTES;
             uint32_t w[8], q[32];
@@ -437,14 +442,19 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(CODE_EMPTY, code.index));
             code.advance();
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(A_EMPTY, stage.index), stage.phase ^ 1u, deadline, aborted));
-            if (!ok) break;
+            if (fresh > 0) {
+              --fresh;
+            } else {
+              ok = mbar_wait(bar(STAGE_EMPTY, freed.index), freed.phase, deadline, aborted);
+              if (!ok) break;
+              freed.advance(2);
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tmem_st32(lane_tmem + Plan::A_COL0 + stage.index * Plan::A_STAGE_COLS + m * PF_A_TILE_COLS, q);
+            tmem_st32(lane_tmem + Plan::A_COL0 + (stage.index % A_STAGES) * Plan::A_STAGE_COLS + m * PF_A_TILE_COLS, q);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(A_FULL, stage.index));
+            if (lane == 0) mbar_arrive(bar(STAGE_FULL, stage.index));
             stage.advance(2);
             // the previous segment's MMAs have had this K block's decode to finish under
             if (pending) drain();
@@ -472,66 +482,77 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     }
     if (pending && ok) drain();
   } else if (warp == PF_MMA_WARP) {
-    // ================= per-route facts for the drain, then the MMAs ============================
-    RingPlace<A_STAGES> a;
-    RingPlace<B_STAGES> b;
+    // ================= per-route facts for the drain, and the MMAs =============================
+    // One loop over all K blocks of the block's items, unrolled over the stage ring: this warp's own
+    // instructions between two K blocks are on the critical path.  The whole warp walks and waits,
+    // one elected lane issues, and the addresses are immediates: an MMA's descriptors live in uniform
+    // registers, and code that moves them there for each MMA cost more than the MMAs themselves
+    // (79 cycles each from a lane's branch; 610 cycles of issue per K block of eight MMAs with two
+    // waits, two commits and addresses worked out inside the elected branch, where the tensor core
+    // takes 128 to 256 at 16 to 32 routes).
     RingPlace<ACC_SETS> acc;
-    uint32_t info_index = 0;
+    uint32_t info_index = 0, phase = 0, idesc = 0, d_cols = 0;
     bool ok = true, first_round = true;
-    for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
-      const int gi = item / row_tiles;
-      const int gsize = warp_uniform(p.groups_of_routes.size[gi]), gstart = p.groups_of_routes.start[gi];
-      const int n_pad = (gsize + 15) & ~15;  // the N of the MMA
-      // The facts go into the buffer of item n - 3.  Behind every MMA of item n - 1 stand all decode
-      // warps' K blocks of that item, and a warp produces those only after its drain of item n - 3
-      // (it drains an item no later than behind its first K block of the next one; a warp without K
-      // blocks must have handed back the accumulators of item n - 2, which it does after item n - 3).
-      for (int n = lane; n < n_pad; n += 32) {
-        const int route = n < gsize ? p.groups_of_routes.routes[gstart + n] : -1;
-        const int64_t xrow = route < 0 ? p.x_zero_row : static_cast<int64_t>(gstart + n);  // the activation rows were quantised in grouped order
-        const float weight = (GLU && route >= 0) ? p.route_weight[route] : 1.0f;
-        route_info[info_index][n] = make_int4(route, __float_as_int(p.x.scale[xrow]), GROUPED ? 0 : p.x.sums[xrow], __float_as_int(weight));
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(INFO_FULL, info_index));
-      if (++info_index == PF_INFO_BUFFERS) info_index = 0;
-      // The whole warp walks the K blocks and waits; one elected lane issues.  An MMA's descriptors live in
-      // uniform registers, and only code that the compiler can see to be warp-uniform keeps them there:
-      // issued from an `if (lane == 0)` branch an MMA cost 79 cycles of the issuing thread whatever its
-      // size, issued under elect.sync it costs what the tensor core takes (16 cycles at 32 columns, 64 at 128).
-      // N = 2 * n_pad: the high-byte rows and the low-byte rows of the routes are one B operand
-      // accumulator s32, A unsigned bytes (the nibble decoder's u = q + 8), B signed bytes
-      const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(n_pad >> 2) << 17) | ((PF_ROWS >> 4) << 24);
-      for (int segment = 0; segment < segments && ok; ++segment) {
-        if (!first_round) ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(ACC_EMPTY, acc.index), acc.phase ^ 1u, deadline, aborted));  // the set's last accumulators are in registers
-        const uint32_t d_cols = tmem + acc.index * Plan::ACC_SET_COLS;
-        for (int kb = 0; kb < segment_blocks && ok; ++kb) {
-          ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar(A_FULL, a.index), a.phase, deadline, aborted));
-          ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(bar(B_FULL, b.index), b.phase, deadline, aborted));
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_cols = tmem + Plan::A_COL0 + a.index * Plan::A_STAGE_COLS;
-          const uint64_t b_desc = umma_desc(b_stage_addr(b.index));
-          if (elect_one()) {
-#pragma unroll
-            for (int m = 0; m < M; ++m) {
-#pragma unroll
-              for (int k = 0; k < 4; ++k)  // 32 bytes of K per instruction: 8 columns of A, 2 x 16 bytes of the B start address
-                umma_i8_ts(d_cols + m * (2 * N_MAX), a_cols + m * PF_A_TILE_COLS + 8 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
-            }
-            umma_commit(bar(A_EMPTY, a.index));  // the stages may be refilled once these MMAs have read them
-            umma_commit(bar(B_EMPTY, b.index));
-            if (kb == segment_blocks - 1) umma_commit(bar(ACC_FULL, acc.index));
-          }
-          __syncwarp();
-          mma_issued = true;
-          a.advance();
-          b.advance();
+    int item = static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x), segment = segments - 1, kb = segment_blocks - 1;
+    // the next segment: its accumulators, and at the start of an item its facts
+    auto next_segment = [&]() {
+      kb = 0;
+      if (++segment == segments) {
+        segment = 0;
+        item += gridDim.x;
+        if (item >= items_here) return false;
+        const int gi = item / row_tiles;
+        const int gsize = warp_uniform(p.groups_of_routes.size[gi]), gstart = p.groups_of_routes.start[gi];
+        const int n_pad = (gsize + 15) & ~15;  // the N of the MMA
+        // The facts go into the buffer of item n - 3.  Behind every MMA of item n - 1 stand all decode
+        // warps' K blocks of that item, and a warp produces those only after its drain of item n - 3
+        // (it drains an item no later than behind its first K block of the next one; a warp without K
+        // blocks must have handed back the accumulators of item n - 2, which it does after item n - 3).
+        for (int n = lane; n < n_pad; n += 32) {
+          const int route = n < gsize ? p.groups_of_routes.routes[gstart + n] : -1;
+          const int64_t xrow = route < 0 ? p.x_zero_row : static_cast<int64_t>(gstart + n);  // the activation rows were quantised in grouped order
+          const float weight = (GLU && route >= 0) ? p.route_weight[route] : 1.0f;
+          route_info[info_index][n] = make_int4(route, __float_as_int(p.x.scale[xrow]), GROUPED ? 0 : p.x.sums[xrow], __float_as_int(weight));
         }
-        acc.advance();
-        if (acc.index == 0) first_round = false;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(INFO_FULL, info_index));
+        if (++info_index == PF_INFO_BUFFERS) info_index = 0;
+        // N = 2 * n_pad: the high-byte rows and the low-byte rows of the routes are one B operand;
+        // accumulator s32, A unsigned bytes (the nibble decoder's u = q + 8), B signed bytes
+        idesc = (2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(n_pad >> 2) << 17) | ((PF_ROWS >> 4) << 24);
       }
-      __syncwarp();
+      if (!first_round && !mbar_wait(bar(ACC_EMPTY, acc.index), acc.phase ^ 1u, deadline, aborted)) return false;  // the set's last accumulators are in registers
+      d_cols = acc.index * Plan::ACC_SET_COLS;
+      return true;
+    };
+    while (ok) {
+#pragma unroll
+      for (uint32_t st = 0; st < B_STAGES; ++st) {
+        if (++kb == segment_blocks) ok = ok && next_segment();
+        ok = ok && mbar_wait(bar(STAGE_FULL, st), phase, deadline, aborted);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t accumulate = kb != 0;
+        const bool last = kb == segment_blocks - 1;
+        if (elect_one()) {
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)  // 32 bytes of K per instruction: 8 columns of A, 2 x 16 bytes of the B start address
+              umma_i8_ts(d_cols + m * (2 * N_MAX), Plan::A_COL0 + (st % A_STAGES) * Plan::A_STAGE_COLS + m * PF_A_TILE_COLS + 8 * k,
+                         umma_desc(Plan::b_stage(st)) + 2 * k, idesc, accumulate | static_cast<uint32_t>(k));
+          }
+          umma_commit(bar(STAGE_EMPTY, st));  // the stage may be refilled once these MMAs have read it
+          if (last) umma_commit(bar(ACC_FULL, acc.index));
+        }
+        __syncwarp();
+        mma_issued = true;
+        if (last) {
+          acc.advance();
+          if (acc.index == 0) first_round = false;
+        }
+      }
+      phase ^= 1u;
     }
   } else if (warp == PF_B_WARP) {
     // ================= activation (B operand) loader: TMA ====================================
@@ -548,19 +569,20 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       const int n_pad = (gsize + 15) & ~15;
       const CUtensorMap* map = &x_maps.rows[(n_pad >> 4) - 1];
       for (int kb = 0; kb < k_blocks; ++kb) {
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait<true>(bar(B_EMPTY, b.index), b.phase ^ 1u, deadline, aborted));
+        ok = mbar_wait<true>(bar(STAGE_EMPTY, b.index), b.phase ^ 1u, deadline, aborted);
         if (!ok) break;
         if (!stall) {  // (the wait self-test: nothing is ever published)
           if (elect_one()) {
-            mbar_expect_tx(bar(B_FULL, b.index), static_cast<uint32_t>(2 * n_pad * 128));
-            tma_box_3d(b_stage_addr(b.index), map, kb * 128, gstart, 0, bar(B_FULL, b.index));
+            mbar_expect_tx(bar(STAGE_FULL, b.index), static_cast<uint32_t>(2 * n_pad * 128));
+            tma_box_3d(Plan::b_stage(b.index), map, kb * 128, gstart, 0, bar(STAGE_FULL, b.index));
           }
           ++used;
         }
         b.advance();
       }
     }
-    if (*aborted) wait_copies_landed<B_STAGES>(bar(B_FULL, 0), used);
+    // (a stage's barrier also waits for the decode warps, so here the copies just get the time they need at most)
+    if (*aborted && used) __nanosleep(1000000);
   } else if (warp == PF_CODE_WARP) {
     // ================= code loader: TMA ======================================================
     // Two K blocks (64 bytes of a row's codes) of every tile per stage, straight from the caller's
@@ -573,13 +595,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       const int gi = item / row_tiles, tile = item - gi * row_tiles;
       const int row0 = warp_uniform(static_cast<int>(p.groups_of_routes.slot[gi] * N_out + static_cast<int64_t>(tile) * ITEM_ROWS));
       for (int u = 0; u < code_units; ++u) {
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait<true>(bar(CODE_EMPTY, code.index), code.phase ^ 1u, deadline, aborted));
+        ok = mbar_wait<true>(bar(CODE_EMPTY, code.index), code.phase ^ 1u, deadline, aborted);
         if (!ok) break;
         if (elect_one()) {
           const uint32_t full = bar(CODE_FULL, code.index);
           mbar_expect_tx(full, Plan::CODE_STAGE_BYTES);
-          tma_box_2d(code_base + code.index * Plan::CODE_STAGE_BYTES, &a_map, u * 64, row0, full);
-          if (GLU) tma_box_2d(code_base + code.index * Plan::CODE_STAGE_BYTES + PF_CODE_UNIT_BYTES, &b_map, u * 64, row0, full);
+          tma_box_2d(Plan::CODE_BASE + code.index * Plan::CODE_STAGE_BYTES, &a_map, u * 64, row0, full);
+          if (GLU) tma_box_2d(Plan::CODE_BASE + code.index * Plan::CODE_STAGE_BYTES + PF_CODE_UNIT_BYTES, &b_map, u * 64, row0, full);
         }
         ++used;
         code.advance();
