@@ -112,8 +112,9 @@ __device__ __forceinline__ uint32_t elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
   return chosen;
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+// One arrival for the warp, predicated instead of a branch.
+__device__ __forceinline__ void mbar_arrive_warp(uint32_t bar, int lane) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
 }
 // Wait of a whole warp, bounded by time.  Returns false (in every lane) when the deadline passes (the
 // caller's CTA then gives up: the flag is raised for every role) or when another warp of the CTA
@@ -126,16 +127,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (__all_sync(0xFFFFFFFFu, done)) return true;
-    if (RELAXED) __nanosleep(40);
+    if (RELAXED) __nanosleep(160);
     if ((spin & 31u) == 31u) {
       if (__any_sync(0xFFFFFFFFu, *abort_flag)) return false;
       if (__any_sync(0xFFFFFFFFu, global_timer_ns() > deadline)) { *abort_flag = 1; return false; }
     }
   }
 }
-// A value that is the same in every lane, in a form the compiler knows to be: what depends on it
-// (loop bounds, descriptors of MMAs and copies) then lives in uniform registers.
-__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+// A value that is the same in every lane, in a form the compiler knows to be (the result of a warp
+// reduction): what depends on it (loop bounds, descriptors of MMAs and copies) then lives in uniform
+// registers.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_or_sync(0xFFFFFFFFu, v); }
 // The wait of a CTA that has given up, for what it still has in flight: bounded by 100 ms.
 __device__ __forceinline__ void mbar_wait_grace(uint32_t bar, uint32_t parity) {
   const uint64_t grace = global_timer_ns() + 100000000ull;
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   const int segments = GROUPED ? static_cast<int>(p.groups) : 1;  // drains per item
   const int segment_blocks = k_blocks / segments;
   const int row_tiles = static_cast<int>((N_out + ITEM_ROWS - 1) / ITEM_ROWS);
-  const int items = warp_uniform(p.groups_of_routes.count[0]) * row_tiles;
+  const int items = static_cast<int>(warp_uniform(p.groups_of_routes.count[0])) * row_tiles;
   volatile int* aborted = &abort_flag;
   const int items_here = set_up_ok ? items : 0;
   bool mma_issued = false;
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     auto release_accumulators = [&]() {
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(ACC_EMPTY, acc.index));
+      mbar_arrive_warp(bar(ACC_EMPTY, acc.index), lane);
     };
     auto finish_column = [&](const int4& pr, const float (&y)[M], auto round_out, auto store_out) {
       if (GLU) {  // round G and U to the activation dtype first, as the separate kernels of the reference do
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
               decode_codeword_nibble<true>(w[i], abs_lane, sign_lane, q[4 * i + 2], q[4 * i + 3]);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(CODE_EMPTY, code.index));
+            mbar_arrive_warp(bar(CODE_EMPTY, code.index), lane);
             code.advance();
             if (fresh > 0) {
               --fresh;
@@ -454,7 +456,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(STAGE_FULL, stage.index));
+            mbar_arrive_warp(bar(STAGE_FULL, stage.index), lane);
             stage.advance(2);
             // the previous segment's MMAs have had this K block's decode to finish under
             if (pending) drain();
@@ -515,14 +517,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
           route_info[info_index][n] = make_int4(route, __float_as_int(p.x.scale[xrow]), GROUPED ? 0 : p.x.sums[xrow], __float_as_int(weight));
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(INFO_FULL, info_index));
+        mbar_arrive_warp(bar(INFO_FULL, info_index), lane);
         if (++info_index == PF_INFO_BUFFERS) info_index = 0;
         // N = 2 * n_pad: the high-byte rows and the low-byte rows of the routes are one B operand;
         // accumulator s32, A unsigned bytes (the nibble decoder's u = q + 8), B signed bytes
-        idesc = (2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(n_pad >> 2) << 17) | ((PF_ROWS >> 4) << 24);
+        idesc = warp_uniform((2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(n_pad >> 2) << 17) | ((PF_ROWS >> 4) << 24));
       }
       if (!first_round && !mbar_wait(bar(ACC_EMPTY, acc.index), acc.phase ^ 1u, deadline, aborted)) return false;  // the set's last accumulators are in registers
-      d_cols = acc.index * Plan::ACC_SET_COLS;
+      if (ACC_SETS > 1) d_cols = warp_uniform(acc.index * Plan::ACC_SET_COLS);
       return true;
     };
     while (ok) {
@@ -593,7 +595,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     bool ok = true;
     for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
       const int gi = item / row_tiles, tile = item - gi * row_tiles;
-      const int row0 = warp_uniform(static_cast<int>(p.groups_of_routes.slot[gi] * N_out + static_cast<int64_t>(tile) * ITEM_ROWS));
+      const int row0 = warp_uniform(static_cast<uint32_t>(p.groups_of_routes.slot[gi] * N_out + static_cast<int64_t>(tile) * ITEM_ROWS));
       for (int u = 0; u < code_units; ++u) {
         ok = mbar_wait<true>(bar(CODE_EMPTY, code.index), code.phase ^ 1u, deadline, aborted);
         if (!ok) break;
