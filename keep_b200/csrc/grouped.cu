@@ -86,11 +86,12 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
   fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + sc.xq), reinterpret_cast<float*>(ws + sc.xscale), reinterpret_cast<int32_t*>(ws + sc.xsums),
                         many ? nullptr : reinterpret_cast<int32_t*>(ws + sc.xsums) + (x_rows + 1) * a.groups};
   int32_t* wait_status = reinterpret_cast<int32_t*>(ws + sc.status);
+  if (many) groups.position = reinterpret_cast<int32_t*>(ws + sc.xsums) + (a.routes + 1) * a.groups;  // behind the sums, as well
   int rc;
   const int group_cols = many ? fast::prefill_group_routes(a.routes, a.slots, a.groups > 1) : fast::decode_group_routes(a.routes, a.slots, a.in_dim);
   if ((rc = fast::group_routes(a.rhs, a.routes, a.slots, group_cols, groups, wait_status, s))) return rc;
   if (many) {  // the tcgen05 kernels copy rows in grouped order
-    if ((rc = fast::quantize_rows_sorted(a.x, a.x_dtype, a.routes, a.in_dim, a.groups, xq, {groups.routes, groups.count, static_cast<int32_t>(x_div)}, s))) return rc;
+    if ((rc = fast::quantize_rows_sorted(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, groups.position, x_div, s))) return rc;
   } else if ((rc = fast::quantize_rows(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, false, s))) return rc;
   fast::FastProjectionArgs p = {};
   p.slots = a.slots;

@@ -14,6 +14,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "moe_fast.cuh"
 #include "router_logits.cuh"
@@ -24,94 +25,176 @@ namespace fast {
 // ------------------------------------------------------------------------------------------
 // Activation quantisation: x -> 16-bit fixed point with a power-of-two scale per row.
 // ------------------------------------------------------------------------------------------
-// One row per block of 256 threads; row == rows is the extra all-zero row.
-template <typename XT>
-__device__ __forceinline__ void quantize_row(const XT* __restrict__ x, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, int planes, int64_t row, int64_t source_row) {
-  __shared__ float warp_max[8];
-  __shared__ float row_scale;
-  extern __shared__ int32_t group_sum[];
-  const int64_t cw = in_dim / 8, per_group = cw / groups;
-  if (row == rows) {  // one extra all-zero row: the B operand of MMA columns that carry no route
-    // (both layouts: the buffer is (rows + 1) * cw * 16 bytes either way)
-    for (int64_t c = threadIdx.x; c < cw; c += 256) {
-      if (planes) {
-        reinterpret_cast<uint2*>(out.q)[row * cw + c] = make_uint2(0, 0);
-        reinterpret_cast<uint2*>(out.q + (rows + 1) * cw * 8)[row * cw + c] = make_uint2(0, 0);
-      } else {
-        reinterpret_cast<uint4*>(out.q)[row * cw + c] = make_uint4(0, 0, 0, 0);
-      }
-    }
-    for (int64_t g = threadIdx.x; g < groups; g += 256) out.sums[row * groups + g] = 0;
-    if (out.chunk_sums)
-      for (int64_t c = threadIdx.x; c < cw / 32; c += 256) out.chunk_sums[row * (cw / 32) + c] = 0;
-    if (threadIdx.x == 0) out.scale[row] = 1.0f;
-    return;
-  }
-  const XT* xr = x + source_row * in_dim;
-  for (int64_t g = threadIdx.x; g < groups; g += 256) group_sum[g] = 0;
-
+// One row per team of THREADS threads, the whole block or (THREADS = 32) one warp of it.  What bounds it is bytes and, before that, instructions: an
+// element costs about six (widen, one fused multiply-add whose magic addend leaves the rounded integer
+// in the low bits, one add, one and a half byte permutes, half an add for the sums; the first form's
+// conversions, clamps, shifts and shared-memory atomics took 138 us for the 4096 tokens of a 4096-wide
+// call, written once per route).  The row stays in registers between the maximum and the conversion.
+//
+// Where a row's values go: `targets` rows of the output, target(j) its index or a negative value for
+// none.  Inputs come in multiples of 256 (shapes_supported), so a warp's 32 codewords are one chunk of
+// 256 inputs and a scale group is a whole number of chunks.  `sm`: in_dim / 256 ints.
+template <typename XT, int THREADS, typename Target>
+__device__ __forceinline__ void quantize_row(const XT* __restrict__ xr, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, int planes, int32_t* sm, int targets, Target target) {
+  constexpr int KEEP = THREADS == 32 ? 10 : 8;  // vectors of eight values a thread keeps
+  constexpr bool PAIRS = sizeof(XT) == 2;  // 16-bit values: kept as they are, maximum taken on pairs
+  __shared__ float warp_max[THREADS / 32];  // (a warp on its own has none to share)
+  auto team_sync = [] { if (THREADS > 32) __syncthreads(); else __syncwarp(); };
+  const int cw = static_cast<int>(in_dim / 8), chunks = cw / 32, per_group = chunks / static_cast<int>(groups);
+  const int tid = threadIdx.x % THREADS, lane = tid & 31, warp = tid >> 5;
+  uint4 raw[KEEP];
+  // largest magnitude; a NaN or an infinity anywhere gives a value that is not finite
   float amax = 0.0f;
-  for (int64_t c = threadIdx.x; c < cw; c += 256) {
-    float v[8];
-    load8_as_float<XT>(xr + c * 8, v);
+  bool odd = false;
+  if constexpr (PAIRS) {
+    typedef typename std::conditional<std::is_same<XT, __half>::value, __half2, __nv_bfloat162>::type Pair;
+    uint32_t top = 0;
+    auto take = [&](const uint4& r) {
+      const uint32_t word[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-    for (int d = 0; d < 8; ++d) amax = fmaxf(amax, fabsf(v[d]));
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t magnitude = word[k] & 0x7FFF7FFFu;
+        const Pair m = __hmax2_nan(*reinterpret_cast<const Pair*>(&top), *reinterpret_cast<const Pair*>(&magnitude));
+        top = *reinterpret_cast<const uint32_t*>(&m);
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) {
+      const int c = tid + i * THREADS;
+      if (c < cw) raw[i] = *reinterpret_cast<const uint4*>(xr + c * 8);
+    }
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+      if (tid + i * THREADS < cw) take(raw[i]);
+    for (int c = tid + KEEP * THREADS; c < cw; c += THREADS) take(*reinterpret_cast<const uint4*>(xr + c * 8));
+    const Pair pair = *reinterpret_cast<const Pair*>(&top);
+    const float a = std::is_same<XT, __half>::value ? __half2float(*reinterpret_cast<const __half*>(&pair.x)) : __uint_as_float(top << 16);
+    const float b = std::is_same<XT, __half>::value ? __half2float(*reinterpret_cast<const __half*>(&pair.y)) : __uint_as_float(top & 0xFFFF0000u);
+    odd = !(isfinite(a) && isfinite(b));
+    amax = fmaxf(a, b);
+  } else {
+    for (int c = tid; c < cw; c += THREADS) {
+      float v[8];
+      load8_as_float<XT>(xr + c * 8, v);
+#pragma unroll
+      for (int d = 0; d < 8; ++d) { odd = odd || !isfinite(v[d]); amax = fmaxf(amax, fabsf(v[d])); }
+    }
+  }
+  odd = THREADS > 32 ? __syncthreads_or(odd) : __any_sync(0xFFFFFFFFu, odd);
+  if (odd) {  // rows with a NaN or an infinity: the maximum leaves the NaNs out
+    amax = 0.0f;
+    for (int c = tid; c < cw; c += THREADS) {
+      float v[8];
+      load8_as_float<XT>(xr + c * 8, v);
+#pragma unroll
+      for (int d = 0; d < 8; ++d) amax = fmaxf(amax, fabsf(v[d]));
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = amax;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float m = 0.0f;
-    for (int w = 0; w < 8; ++w) m = fmaxf(m, warp_max[w]);
-    float s = 1.0f;
-    if (m > 0.0f && isfinite(m)) {
-      int ex;
-      frexpf(m, &ex);            // m < 2^ex
-      s = ldexpf(1.0f, ex - 15);  // |x| / s < 2^15
-      if (m / s > 32639.0f) s *= 2.0f;  // 127 * 256 + 127: the largest value two signed bytes hold
-    }
-    row_scale = s;
-    out.scale[row] = s;
+  float m = amax;
+  if (THREADS > 32) {
+    if (lane == 0) warp_max[warp] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) m = fmaxf(m, warp_max[w]);
   }
-  __syncthreads();
-  const float inv = 1.0f / row_scale;  // exact: a power of two
+  float s = 1.0f;
+  if (m > 0.0f && isfinite(m)) {
+    int ex;
+    frexpf(m, &ex);            // m < 2^ex
+    s = ldexpf(1.0f, ex - 15);  // |x| / s < 2^15
+    if (m / s > 32639.0f) s *= 2.0f;  // 127 * 256 + 127: the largest value two signed bytes hold
+  }
+  const float inv = 1.0f / s;  // exact: a power of two
+  const bool plain = !odd && isfinite(inv);
 
-  for (int64_t c = threadIdx.x; c < cw; c += 256) {
+  auto convert = [&](const float (&v)[8], int c) {
+    uint32_t t[8];  // the low 16 bits: x' in two's complement
+    int total = 0;
+    if (plain) {    // |x / s| <= 32639: 2^23 + 2^22 added to it rounds it to nearest even, as a conversion would
+#pragma unroll
+      for (int d = 0; d < 8; ++d) {
+        t[d] = __float_as_uint(fmaf(v[d], inv, 12582912.0f));
+        total += static_cast<int>(t[d]);
+      }
+      total -= static_cast<int>(8u * 0x4B400000u);
+    } else {
+#pragma unroll
+      for (int d = 0; d < 8; ++d) {
+        const int q = max(-32639, min(32639, __float2int_rn(v[d] * inv)));
+        t[d] = static_cast<uint32_t>(q);
+        total += q;
+      }
+    }
+    const int chunk_total = __reduce_add_sync(0xFFFFFFFFu, total);
+    if (lane == 0) sm[c >> 5] = chunk_total;
+    // x' = 256 * hi + lo with both bytes signed: lo is the low byte, hi the second byte of x' + 128.
+    // byte j of word 0 pairs with table nibble 3-j = dim 6-2j; of word 1 with nibble 7-j = dim 7-2j
+    const uint32_t lo0 = __byte_perm(__byte_perm(t[6], t[4], 0x0040), __byte_perm(t[2], t[0], 0x0040), 0x5410);
+    const uint32_t lo1 = __byte_perm(__byte_perm(t[7], t[5], 0x0040), __byte_perm(t[3], t[1], 0x0040), 0x5410);
+#pragma unroll
+    for (int d = 0; d < 8; ++d) t[d] += 128u;
+    const uint32_t hi0 = __byte_perm(__byte_perm(t[6], t[4], 0x0051), __byte_perm(t[2], t[0], 0x0051), 0x5410);
+    const uint32_t hi1 = __byte_perm(__byte_perm(t[7], t[5], 0x0051), __byte_perm(t[3], t[1], 0x0051), 0x5410);
+    for (int j = 0; j < targets; ++j) {
+      const int64_t row = target(j);
+      if (row < 0) continue;
+      if (planes) {  // high bytes of every row first, then the low bytes: what the tcgen05 B tiles copy from
+        reinterpret_cast<uint2*>(out.q)[row * cw + c] = make_uint2(hi0, hi1);
+        reinterpret_cast<uint2*>(out.q + (rows + 1) * cw * 8)[row * cw + c] = make_uint2(lo0, lo1);
+      } else {
+        reinterpret_cast<uint4*>(out.q)[row * cw + c] = make_uint4(hi0, hi1, lo0, lo1);
+      }
+    }
+  };
+  if constexpr (PAIRS) {
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) {
+      const int c = tid + i * THREADS;
+      if (c < cw) {
+        float v[8];
+        load8_as_float<XT>(reinterpret_cast<const XT*>(&raw[i]), v);
+        convert(v, c);
+      }
+    }
+  }
+  for (int c = tid + (PAIRS ? KEEP * THREADS : 0); c < cw; c += THREADS) {
     float v[8];
     load8_as_float<XT>(xr + c * 8, v);
-    int q[8], total = 0;
-#pragma unroll
-    for (int d = 0; d < 8; ++d) {
-      q[d] = max(-32639, min(32639, __float2int_rn(v[d] * inv)));
-      total += q[d];
+    convert(v, c);
+  }
+  team_sync();
+  for (int j = 0; j < targets; ++j) {
+    const int64_t row = target(j);
+    if (row < 0) continue;
+    if (tid == 0) out.scale[row] = s;
+    for (int g = tid; g < groups; g += THREADS) {
+      int total = 0;
+      for (int c = 0; c < per_group; ++c) total += sm[g * per_group + c];
+      out.sums[row * groups + g] = total;
     }
-    atomicAdd(&group_sum[c / per_group], total);
-    if (out.chunk_sums) {  // a warp's 32 codewords are one chunk of 256 inputs (the row is a multiple of that when these are asked for)
-      const int chunk_total = __reduce_add_sync(0xFFFFFFFFu, total);
-      if ((threadIdx.x & 31) == 0) out.chunk_sums[row * (cw / 32) + c / 32] = chunk_total;
-    }
-    // byte j of word 0 pairs with table nibble 3-j = dim 6-2j; of word 1 with nibble 7-j = dim 7-2j
-    uint32_t hi0 = 0, hi1 = 0, lo0 = 0, lo1 = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      // x' = 256 * hi + lo with both bytes signed, so the two MMAs are the same s8 x s8 kind
-      const int e = q[6 - 2 * j], o = q[7 - 2 * j];
-      const int eh = (e + 128) >> 8, oh = (o + 128) >> 8;
-      hi0 |= static_cast<uint32_t>(eh & 0xFF) << (8 * j);
-      lo0 |= static_cast<uint32_t>((e - 256 * eh) & 0xFF) << (8 * j);
-      hi1 |= static_cast<uint32_t>(oh & 0xFF) << (8 * j);
-      lo1 |= static_cast<uint32_t>((o - 256 * oh) & 0xFF) << (8 * j);
-    }
-    if (planes) {  // high bytes of every row first, then the low bytes: what the tcgen05 B tiles copy from
-      reinterpret_cast<uint2*>(out.q)[row * cw + c] = make_uint2(hi0, hi1);
-      reinterpret_cast<uint2*>(out.q + (rows + 1) * cw * 8)[row * cw + c] = make_uint2(lo0, lo1);
+    if (out.chunk_sums)
+      for (int c = tid; c < chunks; c += THREADS) out.chunk_sums[row * chunks + c] = sm[c];
+  }
+}
+// The extra all-zero row: the B operand of MMA columns that carry no route.
+template <int THREADS>
+__device__ __forceinline__ void zero_row(int64_t row, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, int planes) {
+  const int64_t cw = in_dim / 8;
+  // (both layouts: the buffer is (rows + 1) * cw * 16 bytes either way)
+  for (int64_t c = threadIdx.x; c < cw; c += THREADS) {
+    if (planes) {
+      reinterpret_cast<uint2*>(out.q)[row * cw + c] = make_uint2(0, 0);
+      reinterpret_cast<uint2*>(out.q + (rows + 1) * cw * 8)[row * cw + c] = make_uint2(0, 0);
     } else {
-      reinterpret_cast<uint4*>(out.q)[row * cw + c] = make_uint4(hi0, hi1, lo0, lo1);
+      reinterpret_cast<uint4*>(out.q)[row * cw + c] = make_uint4(0, 0, 0, 0);
     }
   }
-  __syncthreads();
-  for (int64_t g = threadIdx.x; g < groups; g += 256) out.sums[row * groups + g] = group_sum[g];
+  for (int64_t g = threadIdx.x; g < groups; g += THREADS) out.sums[row * groups + g] = 0;
+  if (out.chunk_sums)
+    for (int64_t c = threadIdx.x; c < cw / 32; c += THREADS) out.chunk_sums[row * (cw / 32) + c] = 0;
+  if (threadIdx.x == 0) out.scale[row] = 1.0f;
 }
 
 // `live` (may be null): the slots of the routes that read the rows, `per_row` of them per row; a row
@@ -127,28 +210,40 @@ template <typename XT>
 __global__ void __launch_bounds__(256) quantize_rows_kernel(const XT* __restrict__ x, int64_t rows, int64_t in_dim, int64_t groups, QuantRows out, int planes, LiveRows live, GroupJob job) {
   grid_launch_dependents();
   grid_wait();
+  extern __shared__ int32_t sm[];
   const int64_t row = blockIdx.x;
   if (row > rows) {  // only launched when there is a job
-    extern __shared__ int32_t group_scratch[];
-    group_routes_block<256>(job.served_slot, job.routes, job.slots, job.max_group, job.out, job.clear, group_scratch);
+    group_routes_block<256>(job.served_slot, job.routes, job.slots, job.max_group, job.out, job.clear, sm);
     return;
   }
-  if (live.slot && row < rows) {
+  if (row == rows) return zero_row<256>(row, rows, in_dim, groups, out, planes);
+  if (live.slot) {
     bool any = false;
     for (int j = 0; j < live.per_row; ++j) any = any || live.slot[row * live.per_row + j] < static_cast<uint64_t>(live.slots);
     if (!any) return;  // uniform over the block
   }
-  quantize_row<XT>(x, rows, in_dim, groups, out, planes, row, row);
+  quantize_row<XT, 256>(x + row * in_dim, rows, in_dim, groups, out, planes, sm, 1, [&](int) { return row; });
 }
 
-// Byte planes with the rows in grouped order (what the tcgen05 kernels' TMA boxes copy).
-template <typename XT>
-__global__ void __launch_bounds__(256) quantize_rows_sorted_kernel(const XT* __restrict__ x, int64_t rows, int64_t in_dim, int64_t groups, QuantRows out, SortedRows sorted) {
+// Byte planes with a row per route in grouped order (what the tcgen05 kernels' TMA boxes copy).  Blocks
+// of 128 threads; a row takes all of them or, up to QS_WARP_ROW inputs, one warp, which needs no block
+// barrier.
+constexpr int QS_THREADS = 128;
+constexpr int64_t QS_WARP_ROW = 2560;
+template <typename XT, int TEAM>
+__global__ void __launch_bounds__(QS_THREADS) quantize_rows_sorted_kernel(const XT* __restrict__ x, int64_t x_rows, int64_t in_dim, int64_t groups, QuantRows out, const int32_t* __restrict__ position, int x_div) {
   grid_launch_dependents();
   grid_wait();
-  const int64_t row = blockIdx.x;
-  if (row < rows && row >= sorted.count[1]) return;  // not a grouped route: nothing reads the row (uniform over the block)
-  quantize_row<XT>(x, rows, in_dim, groups, out, 1, row, row < rows ? sorted.routes[row] / sorted.x_div : 0);
+  extern __shared__ int32_t sm[];
+  constexpr int TEAMS = QS_THREADS / TEAM;
+  const int team = threadIdx.x / TEAM;
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * TEAMS + team, rows = x_rows * x_div;
+  if (blockIdx.x == gridDim.x - 1) return zero_row<QS_THREADS>(rows, rows, in_dim, groups, out, 1);
+  if (r >= x_rows) return;
+  bool any = false;
+  for (int j = 0; j < x_div; ++j) any = any || position[r * x_div + j] >= 0;
+  if (!any) return;  // nothing reads the row (uniform over the team)
+  quantize_row<XT, TEAM>(x + r * in_dim, rows, in_dim, groups, out, 1, sm + team * (in_dim / 256), x_div, [&](int j) { return static_cast<int64_t>(position[r * x_div + j]); });
 }
 
 // The front of a decode layer call in one launch: the router's logits (the few-token kernel's
@@ -162,7 +257,12 @@ __global__ void __launch_bounds__(256) logits_and_quantize_kernel(keepvq_router_
   grid_wait();
   const int b = static_cast<int>(blockIdx.x);
   if (b < logit_blocks) router_logits_block<XT, WT>(a, b % logit_blocks_x, b / logit_blocks_x);
-  else quantize_row<XT>(reinterpret_cast<const XT*>(a.x), a.tokens, a.hidden, groups, out, 0, b - logit_blocks, b - logit_blocks);
+  else {
+    extern __shared__ int32_t sm[];
+    const int64_t row = b - logit_blocks;
+    if (row == a.tokens) zero_row<256>(row, a.tokens, a.hidden, groups, out, 0);
+    else quantize_row<XT, 256>(reinterpret_cast<const XT*>(a.x) + row * a.hidden, a.tokens, a.hidden, groups, out, 0, sm, 1, [&](int) { return row; });
+  }
 }
 
 template <typename XT>
@@ -173,14 +273,16 @@ static cudaError_t launch_front(const keepvq_router_logits_args& a, int bx, int 
   return launch_after(true, logits_and_quantize_kernel<XT, __nv_bfloat16>, grid, 256, smem, s, a, bx, blocks, groups, out);
 }
 
+static size_t chunk_bytes(int64_t in_dim) { return static_cast<size_t>(in_dim / 256) * sizeof(int32_t); }  // quantize_row's shared memory
+
 bool logits_and_quantize_supported(const keepvq_router_logits_args& a, int64_t groups) {
-  return a.tokens > 0 && a.tokens <= FRONT_MAX_TOKENS && a.x_dtype != KEEPVQ_F32 && a.hidden % 8 == 0 && groups * sizeof(int32_t) <= 40 * 1024 &&
+  return a.tokens > 0 && a.tokens <= FRONT_MAX_TOKENS && a.x_dtype != KEEPVQ_F32 && a.hidden % 256 == 0 && chunk_bytes(a.hidden) <= 40 * 1024 &&
          (a.pool + RL_ROWS - 1) / RL_ROWS * ((a.tokens + RL_TOKENS - 1) / RL_TOKENS) <= EARLY_LAUNCH_MAX_BLOCKS;
 }
 
 int logits_and_quantize(const keepvq_router_logits_args& a, int64_t groups, const QuantRows& out, cudaStream_t s) {
   const int bx = static_cast<int>((a.pool + RL_ROWS - 1) / RL_ROWS), by = static_cast<int>((a.tokens + RL_TOKENS - 1) / RL_TOKENS);
-  const size_t smem = static_cast<size_t>(groups) * sizeof(int32_t);
+  const size_t smem = chunk_bytes(a.hidden);
   const cudaError_t err = a.x_dtype == KEEPVQ_F16 ? launch_front<__half>(a, bx, bx * by, groups, out, smem, s) : launch_front<__nv_bfloat16>(a, bx, bx * by, groups, out, smem, s);
   if (err != cudaSuccess) return note_cuda_error(err);
   return KEEPVQ_OK;
@@ -191,14 +293,20 @@ int quantize_rows(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, 
   return quantize_rows_and_group(x, x_dtype, rows, in_dim, groups, out, planes, s, live_slot, per_row, slots, nullptr, 0, 0, RouteGroups{}, nullptr);
 }
 
-int quantize_rows_sorted(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, const SortedRows& sorted, cudaStream_t s) {
-  const size_t smem = static_cast<size_t>(groups) * sizeof(int32_t);
-  if (smem > 40 * 1024) return KEEPVQ_ERR_CAPACITY;
-  const unsigned grid = static_cast<unsigned>(rows + 1);  // + the zero row
+template <typename XT>
+static cudaError_t launch_sorted(const void* x, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s) {
+  const bool warps = in_dim <= QS_WARP_ROW;
+  const int64_t teams = warps ? QS_THREADS / 32 : 1;
+  const unsigned grid = static_cast<unsigned>((x_rows + teams - 1) / teams + 1);  // + the zero row
+  return launch_after(grid < EARLY_LAUNCH_MAX_BLOCKS, warps ? quantize_rows_sorted_kernel<XT, 32> : quantize_rows_sorted_kernel<XT, QS_THREADS>, grid, QS_THREADS,
+                      chunk_bytes(in_dim) * teams, s, static_cast<const XT*>(x), x_rows, in_dim, groups, out, position, x_div);
+}
+int quantize_rows_sorted(const void* x, int32_t x_dtype, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s) {
+  if (chunk_bytes(in_dim) > 40 * 1024) return KEEPVQ_ERR_CAPACITY;
   cudaError_t err;
-  if (x_dtype == KEEPVQ_F32) err = launch_after(false, quantize_rows_sorted_kernel<float>, grid, 256, smem, s, reinterpret_cast<const float*>(x), rows, in_dim, groups, out, sorted);
-  else if (x_dtype == KEEPVQ_F16) err = launch_after(false, quantize_rows_sorted_kernel<__half>, grid, 256, smem, s, reinterpret_cast<const __half*>(x), rows, in_dim, groups, out, sorted);
-  else err = launch_after(false, quantize_rows_sorted_kernel<__nv_bfloat16>, grid, 256, smem, s, reinterpret_cast<const __nv_bfloat16*>(x), rows, in_dim, groups, out, sorted);
+  if (x_dtype == KEEPVQ_F32) err = launch_sorted<float>(x, x_rows, in_dim, groups, out, position, x_div, s);
+  else if (x_dtype == KEEPVQ_F16) err = launch_sorted<__half>(x, x_rows, in_dim, groups, out, position, x_div, s);
+  else err = launch_sorted<__nv_bfloat16>(x, x_rows, in_dim, groups, out, position, x_div, s);
   if (err != cudaSuccess) return note_cuda_error(err);
   return KEEPVQ_OK;
 }
@@ -210,7 +318,7 @@ int quantize_rows_and_group(const void* x, int32_t x_dtype, int64_t rows, int64_
                             const uint32_t* served_slot, int64_t routes, int max_group, const RouteGroups& route_groups, int32_t* clear) {
   const LiveRows live = {live_slot, per_row, slots};
   const GroupJob job = {served_slot, static_cast<int32_t>(routes), static_cast<int32_t>(slots), max_group, route_groups, clear};
-  size_t smem = static_cast<size_t>(groups) * sizeof(int32_t);
+  size_t smem = chunk_bytes(in_dim);
   if (smem > 40 * 1024) return KEEPVQ_ERR_CAPACITY;
   if (served_slot) {
     if (!group_with_quantize_supported(routes, slots)) return KEEPVQ_ERR_UNSUPPORTED;

@@ -118,6 +118,7 @@ struct RouteGroups {
   int32_t* start;        // [max_groups] first entry in `routes`
   int32_t* size;         // [max_groups] 1..max_group
   int32_t* routes;       // [routes] route ids ordered by group
+  int32_t* position = nullptr;  // [routes], may be null: where a route stands in `routes`, -1 for one without a slot
 };
 
 // ------------------------------------------------------------------------------------------
@@ -181,7 +182,9 @@ __device__ __forceinline__ void group_routes_block(const uint32_t* __restrict__ 
   __syncthreads();
   for (int r = tid; r < routes; r += GR_THREADS) {
     const uint32_t s = served_slot[r];
-    if (s < static_cast<uint32_t>(slots)) out.routes[first[s] + atomicAdd(&count[s], 1)] = r;
+    const int at = s < static_cast<uint32_t>(slots) ? first[s] + atomicAdd(&count[s], 1) : -1;
+    if (at >= 0) out.routes[at] = r;
+    if (out.position) out.position[r] = at;
   }
 }
 
@@ -229,11 +232,10 @@ bool residual_supported(int64_t routes, int64_t in_dim, int64_t res_groups);
 int quantize_rows(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, bool planes, cudaStream_t s,
                   const uint32_t* live_slot = nullptr, int32_t per_row = 1, int64_t slots = 0);
 // What the tcgen05 kernels' TMA boxes copy: byte planes (all high bytes [rows + 1, in_dim], then all
-// low bytes) with the rows IN GROUPED ORDER: output row r is input row sorted.routes[r] / x_div for
-// r below sorted.count[1] (group_routes must have run), rows beyond that are left alone; scale and
-// sums are per output row.
-struct SortedRows { const int32_t* routes; const int32_t* count; int32_t x_div; };
-int quantize_rows_sorted(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, const SortedRows& sorted, cudaStream_t s);
+// low bytes) with a row per route IN GROUPED ORDER: input row r is quantised once and written to the
+// rows position[r * x_div ...] of its x_div routes (group_routes must have run); rows of routes
+// without a slot are left alone; scale and sums are per output row.  rows = x_rows * x_div.
+int quantize_rows_sorted(const void* x, int32_t x_dtype, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s);
 // `clear` (may be null): a status word the kernel zeroes for the projection kernels that follow it.
 // The router's logits and quantize_rows (planes = false) of the same token rows in one launch, for
 // calls of at most FRONT_MAX_TOKENS tokens with fp16 / bf16 activations.

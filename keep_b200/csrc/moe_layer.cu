@@ -245,6 +245,7 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
     fast::RouteGroups groups = {reinterpret_cast<int32_t*>(ws + sc.gcount), reinterpret_cast<int32_t*>(ws + sc.gslot),
                                 reinterpret_cast<int32_t*>(ws + sc.gstart), reinterpret_cast<int32_t*>(ws + sc.gsize),
                                 reinterpret_cast<int32_t*>(ws + sc.groutes)};
+    if (prefill) groups.position = reinterpret_cast<int32_t*>(ws + sc.gate);  // (only the general kernel uses the gate rows)
     fast::QuantRows hq = {reinterpret_cast<uint8_t*>(ws + sc.hq), reinterpret_cast<float*>(ws + sc.hscale), reinterpret_cast<int32_t*>(ws + sc.hsums),
                           prefill ? nullptr : reinterpret_cast<int32_t*>(ws + sc.hsums) + (routes + 1) * a.w2.groups};
     int32_t* wait_status = reinterpret_cast<int32_t*>(ws + sc.status);
@@ -256,7 +257,7 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
       } else {
         if ((rc = fast::group_routes(a.served_slot, routes, a.slots, group_cols, groups, wait_status, s))) return rc;
         if (prefill) {
-          if ((rc = fast::quantize_rows_sorted(a.x, a.x_dtype, routes, a.hidden, a.w1.groups, xq, {groups.routes, groups.count, a.top_k}, s))) return rc;
+          if ((rc = fast::quantize_rows_sorted(a.x, a.x_dtype, a.tokens, a.hidden, a.w1.groups, xq, groups.position, a.top_k, s))) return rc;
         } else if (!x_quantized && (rc = fast::quantize_rows(a.x, a.x_dtype, a.tokens, a.hidden, a.w1.groups, xq, false, s, padded, a.top_k, a.slots))) return rc;
       }
     }
@@ -273,7 +274,7 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
     }
     if (stages & KEEPVQ_STAGE_DOWN) {
       if (prefill) {
-        if ((rc = fast::quantize_rows_sorted(ws + sc.h, a.x_dtype, routes, a.inter, a.w2.groups, hq, {groups.routes, groups.count, 1}, s))) return rc;
+        if ((rc = fast::quantize_rows_sorted(ws + sc.h, a.x_dtype, routes, a.inter, a.w2.groups, hq, groups.position, 1, s))) return rc;
       } else if ((rc = fast::quantize_rows(ws + sc.h, a.x_dtype, routes, a.inter, a.w2.groups, hq, false, s, padded, 1, a.slots))) return rc;
       p.a = {a.w2.codes, a.w2.scales, a.w2.res_codes, a.w2.res_scales}; p.b = {nullptr, nullptr, nullptr, nullptr};
       if (residual) { p.res_groups = a.w2.res_groups; p.hot_of_slot = a.hot_of_slot; p.res_table = a.res_table; }

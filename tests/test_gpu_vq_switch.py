@@ -176,6 +176,37 @@ def test_routes_without_an_expert_give_zero_rows_on_every_path(cuda):
         assert bool((general[dead] == 0).all()) and bool((general[0] != 0).any())
 
 
+@pytest.mark.parametrize("routes,inp", [(6, 256), (64, 2560), (64, 8448), (1100, 2560), (1100, 2816)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_activation_rows_as_fixed_point(cuda, dtype, routes, inp):
+    """The 16-bit fixed-point rows behind every tensor-core projection, through products whose sums
+    are exact: codes that decode to one of two rows, inputs that are whole steps.  Widths at the
+    edges of what a warp or a block keeps in registers; a row with an infinity (step 1, clamped to
+    +-32639), a NaN (counts as zero), all zeros, and the largest value two signed bytes hold."""
+    from keep_b200 import prefill, vq
+
+    rng = np.random.default_rng(24)
+    experts, out = 2, 64
+    codes = rng.integers(0, 1 << 16, (experts, out, inp // 8), dtype=np.uint16)
+    scales = np.full((experts, out, 1), 2.0 ** -6, dtype=np.float16)
+    dense = ops.dense_experts(codes, scales, dtype=np.float64)
+    x = rng.integers(-64, 65, (routes, inp)).astype(np.float32)
+    x[0] = 0.0
+    x[1, 5], x[1, 9] = np.inf, -np.inf
+    x[2, 3] = np.nan
+    x[3, 7] = 65280.0 if dtype == torch.bfloat16 else 65504.0  # in fixed point past 127 * 256 + 127: the step doubles
+    fixed = np.nan_to_num(x.astype(np.float64), nan=0.0, posinf=32639.0, neginf=-32639.0)
+    step = 4.0  # of the row with the large value: 65280 / 2 and 65504 / 2 exceed 32639
+    fixed[3] = np.round(fixed[3] / step) * step
+    rhs = (np.arange(routes) % experts).astype(np.int32)
+    got = prefill.tensor_core_projection(torch.from_numpy(x).to(cuda).to(dtype), torch.from_numpy(codes).to(cuda), torch.from_numpy(scales).to(cuda),
+                                         vq.table_on(cuda, "e8p"), torch.from_numpy(rhs).to(cuda)).double().cpu().numpy()
+    want = np.stack([dense[rhs[r]] @ fixed[r] for r in range(routes)])
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10  # the output's own rounding; fp32 sums are far below it
+    top = np.abs(want[np.isfinite(want)]).max() if dtype == torch.bfloat16 else 65504.0
+    np.testing.assert_allclose(np.clip(got, -top, top), np.clip(want, -top, top), rtol=eps, atol=1e-3 * step)
+
+
 @pytest.mark.parametrize("factor", [300.0, 3000.0])
 def test_one_outlier_channel_costs_what_the_header_says(cuda, factor):
     """fp16 / bf16 rows are held as 16-bit fixed point with one power-of-two step per row, so a
