@@ -103,6 +103,26 @@ __device__ __forceinline__ void build_nibble_tables(uint32_t region, const uint3
     }
   }
 }
+// 8-bit codes: a table word holds dim d in nibble d, and byte j of the operand's low word is dim
+// 6 - 2j, of the high word dim 7 - 2j, so an entry is the word with its bytes reversed; 32 replicas at
+// region + code * 256 + lane * 4.  The operand bytes are the nibbles themselves, u = q + 8.
+__device__ __forceinline__ void build_byte_code_table(uint32_t region, const uint32_t* __restrict__ table, int tid, int threads) {
+  const int lane = tid & 31;
+  for (int first = tid - lane; first < 256; first += threads) {
+    const uint32_t v = __byte_perm(table[first + lane], 0, 0x0123);
+#pragma unroll 8
+    for (int i = 0; i < 32; ++i) {
+      const uint32_t vi = __shfl_sync(0xFFFFFFFFu, v, i);
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(region + (first + i) * 256 + lane * 4), "r"(vi) : "memory");
+    }
+  }
+}
+__device__ __forceinline__ void decode_byte_code(uint32_t word, int byte, uint32_t table_lane, uint32_t& lo, uint32_t& hi) {
+  uint32_t e;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(e) : "r"(__byte_perm(word, table_lane, 0x7604 | (byte << 4))));
+  lo = e & 0x0F0F0F0Fu;
+  hi = (e >> 4) & 0x0F0F0F0Fu;
+}
 // Quantised activation rows: the B operand of the projections.
 struct QuantRows {
   uint8_t* q;       // [rows + 1, in_dim/8, 16] (last row all zero): per codeword 4 words: hi(dims 6,4,2,0) hi(7,5,3,1) lo(...) lo(...)
@@ -277,6 +297,7 @@ bool prefill_supported(int64_t slots, int64_t out_dim, int64_t in_dim, int64_t g
 int prefill_group_routes(int64_t live, int64_t slots, bool several_groups);
 int prefill_gate_up(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);
 int prefill_down(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);
+int prefill_byte_codes(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);
 // One CTA whose activation loaders never publish, with a deadline of wait_ns: the wait runs out, the CTA sets *status = 1 and returns.
 int prefill_wait_selftest(const FastProjectionArgs& args, int32_t* status, uint64_t wait_ns, cudaStream_t s);
 

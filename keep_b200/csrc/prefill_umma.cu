@@ -58,7 +58,6 @@ constexpr int PF_ROWS = 128;                    // output rows per tile
 constexpr int PF_KBLOCK_CODES = 16;             // codewords of a row per K block = 128 bytes of int8
 constexpr int PF_A_TILE_COLS = PF_KBLOCK_CODES * 2;   // a decoded K block of one tile: 128 bytes per row = 32 columns
 constexpr uint32_t PF_TMEM_COLS = 512;
-constexpr uint32_t PF_CODE_UNIT_BYTES = PF_ROWS * 64; // two K blocks of one tile's codes, 64 bytes per row
 constexpr uint32_t PF_TABLE_BYTES = 64 * 1024;  // the nibble decoder's two tables, interleaved (moe_fast.cuh)
 // Shared window, absolute addresses (compile-time constants: the operands of the MMAs, copies and
 // barriers are then immediates); a block whose window lies elsewhere reports and does nothing.
@@ -74,7 +73,7 @@ constexpr uint64_t PF_DEFAULT_WAIT_NS = 2000000000ull;
 // decoded A stages of 32 columns per tile.  With several scale groups per row the accumulators are
 // drained once per group, so there are two sets; with one, a single set leaves room for more A stages.
 // Shared window: [A0 - 48 KB, A0) the first B stages | [A0, +64 KB) tables | code stages | the other B stages
-template <int M, int N_MAX, bool GROUPED>
+template <int M, int N_MAX, bool GROUPED, int BITS>
 struct PrefillPlan {
   static_assert(N_MAX % 16 == 0, "an item's routes pad to a multiple of sixteen columns");
   static constexpr uint32_t ACC_SET_COLS = 2 * M * N_MAX;
@@ -87,8 +86,10 @@ struct PrefillPlan {
   static constexpr uint32_t LOW_B_STAGES = PF_LOW_BYTES / B_STAGE_BYTES;
   static constexpr uint32_t B_STAGES = N_MAX > 48 ? 4 : 8;    // one ring of barriers for A and B: a K block's A stage is its B stage modulo A_STAGES
   static_assert(B_STAGES % A_STAGES == 0, "");
-  static constexpr uint32_t CODE_STAGE_BYTES = M * PF_CODE_UNIT_BYTES;
-  static constexpr uint32_t CODE_STAGES = 3;
+  static constexpr uint32_t CODE_ROW_BYTES = 2 * PF_KBLOCK_CODES * BITS / 8;  // two K blocks of a row's codes
+  static constexpr uint32_t CODE_UNIT_BYTES = PF_ROWS * CODE_ROW_BYTES;       // ... of a tile's
+  static constexpr uint32_t CODE_STAGE_BYTES = M * CODE_UNIT_BYTES;
+  static constexpr uint32_t CODE_STAGES = BITS == 16 ? 3 : 6;
   static constexpr uint32_t HIGH_BYTES = PF_TABLE_BYTES + CODE_STAGES * CODE_STAGE_BYTES + (B_STAGES - LOW_B_STAGES) * B_STAGE_BYTES;
   static_assert(HIGH_BYTES <= 160 * 1024, "the window above A0");
   static constexpr uint32_t CODE_BASE = PF_A0 + PF_TABLE_BYTES;
@@ -209,16 +210,19 @@ struct RingPlace {
 // and its activation (B) stages serve all of them (the copies are what bounds a single projection).
 // GROUPED: several scale groups per row.  The accumulators are drained once per group (a segment of
 // the K blocks) into fp32 sums that the drain warps keep in registers.
+// BITS: 16-bit E8P codes, or 8-bit codes of a table whose word holds dim d in nibble d, value
+// (nibble - 8) / 2.  There a codeword is ONE table read, w = q / 2 without the quarter, and any table
+// will do.
 // `stall` != 0 is the wait self-test: the activation loader never publishes, so the MMA issuer's
 // first wait runs into the deadline.
 // Boxes over the activations, one map per padded number of routes: [2 planes][16 (i + 1) rows][128 bytes].
 template <int N_MAX>
 struct ActivationMaps { CUtensorMap rows[N_MAX / 16]; };
 
-template <int M, bool GLU, int N_MAX, bool GROUPED>
+template <int M, bool GLU, int N_MAX, bool GROUPED, int BITS>
 __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastProjectionArgs p, const __grid_constant__ ActivationMaps<N_MAX> x_maps, const __grid_constant__ CUtensorMap a_map,
                                                                            const __grid_constant__ CUtensorMap b_map, int32_t* status, int stall, uint64_t wait_ns) {
-  using Plan = PrefillPlan<M, N_MAX, GROUPED>;
+  using Plan = PrefillPlan<M, N_MAX, GROUPED, BITS>;
   constexpr int ITEM_ROWS = GLU ? PF_ROWS : PF_ROWS * M;
   constexpr int A_STAGES = Plan::A_STAGES, B_STAGES = Plan::B_STAGES, CODE_STAGES = Plan::CODE_STAGES, ACC_SETS = Plan::ACC_SETS;
   constexpr int TILE_STEP = GLU ? 0 : PF_ROWS;  // rows between the A tiles of an item
@@ -238,7 +242,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   const bool window_ok = dyn_base <= PF_BARS && PF_A0 + Plan::HIGH_BYTES <= dyn_base + PF_SMEM_BYTES;  // uniform over the grid
 
   // ---- set-up: tables, barriers, tensor memory ------------------------------------------------
-  if (window_ok) build_nibble_tables(PF_A0, p.codebook, tid, PF_THREADS);
+  if (window_ok) {
+    if (BITS == 16) build_nibble_tables(PF_A0, p.codebook, tid, PF_THREADS);
+    else build_byte_code_table(PF_A0, p.codebook, tid, PF_THREADS);
+  }
   if (tid == 0) {
     abort_flag = window_ok ? 0 : 1;
     if (window_ok) {
@@ -281,8 +288,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     const int row = quadrant * 32 + lane;
     const uint32_t abs_lane = PF_A0 + lane * 4u, sign_lane = PF_A0 + 128u + lane * 4u;
     const uint32_t lane_tmem = tmem + (static_cast<uint32_t>(quadrant * 32) << 16);
-    const uint32_t code_chunk0 = Plan::CODE_BASE + m * PF_CODE_UNIT_BYTES + row * 64u + (((2u * parity) ^ ((row >> 1) & 3u)) << 4);  // 64-byte swizzle: 16-byte chunk ^ (row / 2) % 4
-    const uint32_t code_chunk1 = Plan::CODE_BASE + m * PF_CODE_UNIT_BYTES + row * 64u + (((2u * parity + 1u) ^ ((row >> 1) & 3u)) << 4);
+    // the rows of a code tile are swizzled in 16-byte chunks: 64-byte rows chunk ^ (row / 2) % 4, 32-byte rows chunk ^ (row / 4) % 2
+    const uint32_t code_row = Plan::CODE_BASE + m * Plan::CODE_UNIT_BYTES + row * Plan::CODE_ROW_BYTES;
+    const uint32_t code_chunk0 = BITS == 16 ? code_row + (((2u * parity) ^ ((row >> 1) & 3u)) << 4) : code_row + ((parity ^ ((row >> 2) & 1u)) << 4);
+    const uint32_t code_chunk1 = code_row + (((2u * parity + 1u) ^ ((row >> 1) & 3u)) << 4);
     const Projection mats[2] = {p.a, GLU ? p.b : p.a};
     const bool scales32 = p.scales_dtype == KEEPVQ_F32;
     const float limit = p.swiglu_limit > 0.0f ? p.swiglu_limit : INFINITY;
@@ -354,7 +363,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint32_t offset = 8u * static_cast<uint32_t>(x_sums[c + j]);
-            const float x_sum4 = 0.25f * static_cast<float>(x_sums[c + j]);
+            const float x_sum4 = BITS == 16 ? 0.25f * static_cast<float>(x_sums[c + j]) : 0.0f;
 #pragma unroll
             for (int mm = 0; mm < M; ++mm) {
               const int dot = static_cast<int>(v[mm][0][j] * 256u + v[mm][1][j] - offset);
@@ -385,7 +394,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int4 pr = per_route[c_first + c + j];
-            const float x_scale = __int_as_float(pr.y), x_sum4 = 0.25f * static_cast<float>(pr.z);
+            const float x_scale = __int_as_float(pr.y), x_sum4 = BITS == 16 ? 0.25f * static_cast<float>(pr.z) : 0.0f;
             const uint32_t offset = 8u * static_cast<uint32_t>(pr.z);  // the A operand was u = q + 8: 8 * sum(x') too much
             float y[M];
 #pragma unroll
@@ -435,11 +444,16 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             const uint32_t at = code.index * Plan::CODE_STAGE_BYTES;
             uint32_t w[8], q[32];
             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(code_chunk0 + at));
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(code_chunk1 + at));
+            if constexpr (BITS == 16) {
+              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(code_chunk1 + at));
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              decode_codeword_nibble<false>(w[i], abs_lane, sign_lane, q[4 * i], q[4 * i + 1]);
-              decode_codeword_nibble<true>(w[i], abs_lane, sign_lane, q[4 * i + 2], q[4 * i + 3]);
+              for (int i = 0; i < 8; ++i) {
+                decode_codeword_nibble<false>(w[i], abs_lane, sign_lane, q[4 * i], q[4 * i + 1]);
+                decode_codeword_nibble<true>(w[i], abs_lane, sign_lane, q[4 * i + 2], q[4 * i + 3]);
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) decode_byte_code(w[i >> 2], i & 3, abs_lane, q[2 * i], q[2 * i + 1]);
             }
             __syncwarp();
             mbar_arrive_warp(bar(CODE_EMPTY, code.index), lane);
@@ -587,8 +601,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     if (*aborted && used) __nanosleep(1000000);
   } else if (warp == PF_CODE_WARP) {
     // ================= code loader: TMA ======================================================
-    // Two K blocks (64 bytes of a row's codes) of every tile per stage, straight from the caller's
-    // layout seen as one [slots * out_dim, in_dim / 4] byte matrix; rows past a slot's last tile are
+    // Two K blocks of every tile per stage, straight from the caller's
+    // layout seen as one byte matrix of slots * out_dim rows; rows past a slot's last tile are
     // the next slot's (or zeros past the end) and their outputs are never stored.
     RingPlace<CODE_STAGES> code;
     uint32_t used = 0;
@@ -602,8 +616,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         if (elect_one()) {
           const uint32_t full = bar(CODE_FULL, code.index);
           mbar_expect_tx(full, Plan::CODE_STAGE_BYTES);
-          tma_box_2d(Plan::CODE_BASE + code.index * Plan::CODE_STAGE_BYTES, &a_map, u * 64, row0, full);
-          if (GLU) tma_box_2d(Plan::CODE_BASE + code.index * Plan::CODE_STAGE_BYTES + PF_CODE_UNIT_BYTES, &b_map, u * 64, row0, full);
+          tma_box_2d(Plan::CODE_BASE + code.index * Plan::CODE_STAGE_BYTES, &a_map, u * static_cast<int>(Plan::CODE_ROW_BYTES), row0, full);
+          if (GLU) tma_box_2d(Plan::CODE_BASE + code.index * Plan::CODE_STAGE_BYTES + Plan::CODE_UNIT_BYTES, &b_map, u * static_cast<int>(Plan::CODE_ROW_BYTES), row0, full);
         }
         ++used;
         code.advance();
@@ -663,22 +677,22 @@ static int byte_map(CUtensorMap* map, const void* base, int64_t row_bytes, int64
                             swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? KEEPVQ_OK : KEEPVQ_ERR_LAUNCH;
 }
-// A projection's codes: a [slots * out_dim, in_dim / 4] byte matrix.
-static int code_map(const FastProjectionArgs& p, const uint16_t* codes, uint32_t box_rows, CUtensorMap* map) {
-  return byte_map(map, codes, p.in_dim / 4, p.slots * p.out_dim, 1, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_64B);
+// A projection's codes: a byte matrix of slots * out_dim rows, two K blocks of a row's codes per box row.
+static int code_map(const FastProjectionArgs& p, const void* codes, int bits, uint32_t box_rows, CUtensorMap* map) {
+  return byte_map(map, codes, p.in_dim / 8 * (bits / 8), p.slots * p.out_dim, 1, 2 * PF_KBLOCK_CODES * bits / 8, box_rows, bits == 16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-template <int M, bool GLU, int N_MAX, bool GROUPED>
+template <int M, bool GLU, int N_MAX, bool GROUPED, int BITS = 16>
 static int launch_prefill(const FastProjectionArgs& p, int32_t* status, cudaStream_t s, int stall = 0, uint64_t wait_ns = 0, int ctas = 0) {
   ActivationMaps<N_MAX> x_maps;  // the quantised activations: the high-byte plane, then the low-byte plane, each [rows + 1, in_dim]
   for (int i = 0; i < N_MAX / 16; ++i)
     if (const int rc = byte_map(&x_maps.rows[i], p.x.q, p.in_dim, p.x_zero_row + 1, 2, 128, 16 * (i + 1), CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
   CUtensorMap a_map, b_map;
-  if (const int rc = code_map(p, p.a.codes, GLU ? PF_ROWS : PF_ROWS * M, &a_map)) return rc;
+  if (const int rc = code_map(p, p.a.codes, BITS, GLU ? PF_ROWS : PF_ROWS * M, &a_map)) return rc;
   if (GLU) {
-    if (const int rc = code_map(p, p.b.codes, PF_ROWS, &b_map)) return rc;
+    if (const int rc = code_map(p, p.b.codes, BITS, PF_ROWS, &b_map)) return rc;
   } else b_map = a_map;
-  auto kernel = prefill_projection_kernel<M, GLU, N_MAX, GROUPED>;
+  auto kernel = prefill_projection_kernel<M, GLU, N_MAX, GROUPED, BITS>;
   static uint64_t configured = 0;  // one bit per device: the shared-memory opt-in is a per-device attribute of the function
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -703,6 +717,11 @@ int prefill_gate_up(const FastProjectionArgs& p, int32_t* status, cudaStream_t s
 // a single projection takes two row tiles per item when it has them (the activation copies serve both)
 int prefill_down(const FastProjectionArgs& p, int32_t* status, cudaStream_t s) {
   return p.out_dim > PF_ROWS ? launch_prefill_any<2, false>(p, status, s) : launch_prefill_any<1, false>(p, status, s);
+}
+// 8-bit codes (p.a.codes holds bytes, p.codebook their table); p.group_cols is PREFILL_GROUP_ROUTES_SMALL.
+int prefill_byte_codes(const FastProjectionArgs& p, int32_t* status, cudaStream_t s) {
+  if (p.groups > 1) return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, true, 8>(p, status, s);
+  return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, false, 8>(p, status, s);
 }
 // One CTA of the single-projection kernel whose activation loader never publishes, with a short
 // deadline: the wait runs out, the CTA reports and returns.  `p` must describe a valid problem.

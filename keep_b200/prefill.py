@@ -37,13 +37,13 @@ def _table_all_odd(table: torch.Tensor) -> bool:
     return _all_odd[key][2]
 
 
-def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, residual=None, hot_of_slot=None):
+def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, code_bits: int = 16, residual=None, hot_of_slot=None):
     """``keepvq_grouped_projection``: route ``r`` against activation row ``r // x_div`` of ``rows``
     (fp16 / bf16), optionally with a nested residual ``(res_codes, res_scales, res_table)``.
     Returns None when the library says these shapes are not for the tensor-core kernels."""
     routes, in_dim = int(rhs.numel()), int(rows.shape[1])
     slots, out_dim, groups = int(codes.shape[0]), int(codes.shape[1]), int(scales.shape[2])
-    if codes.dtype != torch.uint16 or in_dim % 256 or rows.dtype not in (torch.float16, torch.bfloat16):
+    if codes.dtype != (torch.uint8 if code_bits == 8 else torch.uint16) or in_dim % 256 or rows.dtype not in (torch.float16, torch.bfloat16):
         return None
     if int(rows.shape[0]) * x_div != routes:
         return None
@@ -61,10 +61,12 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, r
     out_dtype = qmv_output_dtype(rows.dtype)
     out = torch.empty((routes, out_dim), dtype=out_dtype, device=device)
     rows, rhs = rows.contiguous(), rhs.to(torch.int32).contiguous()
+    if rows.data_ptr() % 16:  # a view that starts inside an allocation: the kernels read 16 bytes at a time
+        rows = rows.clone()
     args = _lib.GroupedProjectionArgs(
         x=_lib.ptr(rows), x_dtype=_lib.dtype_tag(rows.dtype), routes=routes, rhs=_lib.ptr(rhs), codes=_lib.ptr(codes), scales=_lib.ptr(scales),
         scales_dtype=_lib.dtype_tag(scales.dtype), slots=slots, out_dim=out_dim, in_dim=in_dim, groups=groups, codebook=_lib.ptr(table),
-        codebook_all_odd=int(_table_all_odd(table)), out=_lib.ptr(out), out_dtype=_lib.dtype_tag(out_dtype),
+        codebook_all_odd=int(code_bits == 16 and _table_all_odd(table)), code_bits=code_bits, out=_lib.ptr(out), out_dtype=_lib.dtype_tag(out_dtype),
         workspace=_lib.ptr(ws), workspace_bytes=int(ws.numel()), x_div=int(x_div))
     keep = [rows, rhs]
     if residual is not None:
@@ -88,9 +90,9 @@ def grouped_matmul_sorted(x, codes, scales, table, sorted_rhs, sorted_lhs, *, co
     ``[routes, out]`` in the given order.  ``tile_descriptors`` is accepted for callers that
     pre-build it; the CUDA kernels derive their own grouping from ``sorted_rhs``."""
     del tile_descriptors
-    if code_bits == 16 and x.dtype in (torch.float16, torch.bfloat16) and scales.dtype in (torch.float32, torch.float16, torch.bfloat16):
+    if x.dtype in (torch.float16, torch.bfloat16) and scales.dtype in (torch.float32, torch.float16, torch.bfloat16):
         rows = x if sorted_lhs is None else x[sorted_lhs.long()]  # the gather the reference does before its kernels
-        out = tensor_core_projection(rows, codes, scales, table, sorted_rhs)
+        out = tensor_core_projection(rows, codes, scales, table, sorted_rhs, code_bits=code_bits)
         if out is not None:
             return out
     return routed_matvec(x, codes, scales, table, sorted_rhs, lhs=sorted_lhs, x_div=1, code_bits=code_bits)

@@ -276,14 +276,14 @@ def gather_vqmm(x, codes, scales, codebook, rhs_indices, *, lhs_indices=None, in
             _check_range(flat_lhs, int(x_t.shape[0]), "lhs_indices")
         return _dense_routes(x_t[rows], codes_t, scales_t, table, flat_rhs, code_bits).reshape(output_shape)
 
-    if code_bits == 16 and flat_lhs is None and x_t.dtype in (torch.float16, torch.bfloat16) and scales_t.dtype in (torch.float32, torch.float16, torch.bfloat16):
+    if flat_lhs is None and x_t.dtype in (torch.float16, torch.bfloat16) and scales_t.dtype in (torch.float32, torch.float16, torch.bfloat16):
         # token layout with 16-bit rows: the int8 tensor-core kernels, which group the routes by
         # expert on the device, in whatever order they come, and read each touched expert's codes
         # once: sorting them here first, gathering a row per route and scattering the outputs back
         # cost 200 of the 445 us of a 1024-token call
         from .prefill import tensor_core_projection
 
-        out = tensor_core_projection(x_t, codes_t.contiguous(), scales_t.contiguous(), table, flat_rhs, x_div=x_div)
+        out = tensor_core_projection(x_t, codes_t.contiguous(), scales_t.contiguous(), table, flat_rhs, x_div=x_div, code_bits=code_bits)
         if out is not None:
             return out.reshape(output_shape)
 

@@ -176,6 +176,57 @@ def test_routes_without_an_expert_give_zero_rows_on_every_path(cuda):
         assert bool((general[dead] == 0).all()) and bool((general[0] != 0).any())
 
 
+@pytest.mark.parametrize("routes,experts,out,inp,group", [
+    (12, 3, 100, 256, 256),     # the fewest routes, one partial row tile
+    (144, 96, 384, 1024, 1024),  # about a route per expert, a partial item
+    (130, 2, 256, 512, 256),    # two 48-route items and a short one per expert, two scale groups of two K blocks
+    (600, 40, 300, 768, 256),   # ragged rows, three scale groups
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_8bit_codes_on_the_tcgen05_kernel(cuda, dtype, routes, experts, out, inp, group):
+    """8-bit codes with enough routes for the grouped kernel, through both operators, and the same
+    routes on the general kernel: two 16-bit fixed-point paths, apart by the output's rounding."""
+    from keep_b200 import kernels, prefill, vq, vq_switch
+
+    rng = np.random.default_rng(25)
+    codes = rng.integers(0, 256, (experts, out, inp // 8), dtype=np.uint8)
+    scales = (0.02 * rng.uniform(0.5, 1.5, (experts, out, inp // group))).astype(np.float16)
+    table = vq.table_on(cuda, "e8_1bit")
+    dev = lambda a: torch.from_numpy(a).to(cuda)  # noqa: E731
+    rhs = rng.integers(0, experts, routes).astype(np.int32)
+    x = torch.from_numpy(rng.normal(size=(routes, inp)).astype(np.float32)).to(dtype)
+    want = ops.gather_vqmm(x.float().numpy(), codes, scales, None, rhs.astype(np.int64), lhs_indices=np.arange(routes), code_bits=8)
+    named = dict(input_dims=inp, output_dims=out, group_size=group, code_bits=8)
+    tokens = vq_switch.gather_vqmm(x.to(cuda), dev(codes), dev(scales), table, dev(rhs).reshape(routes, 1), **named)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10
+    atol = 2.0 ** -14 * np.abs(want).max() * 8  # the fixed-point step of a row against its largest output
+    np.testing.assert_allclose(f32(tokens).reshape(routes, out), want, rtol=eps, atol=atol)
+    general = kernels.routed_matvec(x.to(cuda), dev(codes), dev(scales), table, dev(rhs), code_bits=8)
+    np.testing.assert_allclose(f32(tokens).reshape(routes, out), f32(general), rtol=eps, atol=atol)
+    direct = prefill.tensor_core_projection(x.to(cuda), dev(codes), dev(scales), table, dev(rhs), code_bits=8)
+    assert direct is not None and torch.equal(direct, tokens.reshape(routes, out))
+    dead = rhs.copy()
+    dead[1] = experts + 2
+    with_dead = prefill.tensor_core_projection(x.to(cuda), dev(codes), dev(scales), table, dev(dead), code_bits=8)
+    assert bool((with_dead[1] == 0).all()) and torch.equal(with_dead[2:], direct[2:])
+
+
+def test_rows_that_start_inside_an_allocation(cuda):
+    """A view whose first row is not on a 16-byte boundary, few routes and many: the same outputs."""
+    from keep_b200 import vq, vq_switch
+
+    rng = np.random.default_rng(26)
+    codes = torch.from_numpy(rng.integers(0, 1 << 16, (4, 128, 32), dtype=np.uint16)).to(cuda)
+    scales = torch.full((4, 128, 1), 0.02, dtype=torch.float16, device=cuda)
+    for tokens in (4, 100):
+        base = torch.from_numpy(rng.normal(size=tokens * 256 + 1).astype(np.float32)).to(cuda).to(torch.bfloat16)
+        view = base[1:].reshape(tokens, 256)
+        rhs = torch.from_numpy(rng.integers(0, 4, (tokens, 2)).astype(np.int32)).to(cuda)
+        named = dict(input_dims=256, output_dims=128, group_size=256, code_bits=16)
+        table = vq.table_on(cuda, "e8p")
+        assert torch.equal(vq_switch.gather_vqmm(view, codes, scales, table, rhs, **named), vq_switch.gather_vqmm(view.clone(), codes, scales, table, rhs, **named))
+
+
 @pytest.mark.parametrize("routes,inp", [(6, 256), (64, 2560), (64, 8448), (1100, 2560), (1100, 2816)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_activation_rows_as_fixed_point(cuda, dtype, routes, inp):
