@@ -30,8 +30,7 @@
 //                An item's accumulators are drained (tcgen05.ld: same lanes; each of the four warps
 //                of a quadrant takes a quarter of the columns) behind the warp's first K block of the
 //                NEXT item, so nobody waits for the tail of the MMAs.
-//   warp  16     issues the MMAs: A from tensor memory, B from shared memory.  Its lanes also gather
-//                what the drain needs per route (route id, activation scale and sum, gate weight).
+//   warp  16     issues the MMAs: A from tensor memory, B from shared memory.
 //   warp  17     one thread brings the routes' quantised activations into the B tiles with TMA: the
 //                rows were quantised in grouped order, so a group's high bytes and its low bytes are
 //                two runs of rows of one [2 x rows, K] byte matrix, and a K block of them is a handful
@@ -39,6 +38,7 @@
 //                for the MMA; the boxes report to the stage's mbarrier (expect_tx / complete_tx).
 //   warp  18     one thread brings the codes with TMA: boxes of 128 rows x 64 bytes (two K blocks of
 //                a tile), 64-byte swizzle, so a thread reads its row's 32 bytes without bank conflicts.
+//   warp  19     gathers what the drain needs per route (route id, activation scale and sums, gate weight).
 // mbarrier full/empty pairs carry every dependency.  Every wait is bounded by a deadline on the
 // global timer: on expiry the CTA raises a flag in `status`, stops issuing work, waits (bounded)
 // for the MMAs in flight, frees its tensor memory and returns.
@@ -53,7 +53,10 @@ constexpr int PF_DECODE_WARPS = 16;
 constexpr int PF_MMA_WARP = PF_DECODE_WARPS;
 constexpr int PF_B_WARP = PF_DECODE_WARPS + 1;     // activations by TMA
 constexpr int PF_CODE_WARP = PF_DECODE_WARPS + 2;  // codes by TMA
-constexpr int PF_THREADS = (PF_DECODE_WARPS + 3) * 32;  // 608
+constexpr int PF_INFO_WARP = PF_DECODE_WARPS + 3;  // per-route facts
+constexpr int PF_THREADS = (PF_DECODE_WARPS + 4) * 32;  // 640
+constexpr int PF_MAX_SEGMENTS = 32;             // most scale groups of a row
+constexpr int64_t PF_MAX_SEGMENT_INPUTS = 4096; // ... and most inputs of one, where a row has several: sum(4w x') fits 32 bits
 constexpr int PF_ROWS = 128;                    // output rows per tile
 constexpr int PF_KBLOCK_CODES = 16;             // codewords of a row per K block = 128 bytes of int8
 constexpr int PF_A_TILE_COLS = PF_KBLOCK_CODES * 2;   // a decoded K block of one tile: 128 bytes per row = 32 columns
@@ -80,17 +83,19 @@ struct PrefillPlan {
   static constexpr uint32_t ACC_SETS = GROUPED ? 2 : 1;
   static constexpr uint32_t A_STAGE_COLS = M * PF_A_TILE_COLS;
   static constexpr uint32_t A_COL0 = ACC_SETS * ACC_SET_COLS;
-  static constexpr uint32_t A_STAGES = (PF_TMEM_COLS - A_COL0) / A_STAGE_COLS >= 4 ? 4 : 2;
+  static constexpr uint32_t A_STAGES = GROUPED || N_MAX > 48 ? 2 : 4;
   static_assert(A_COL0 + A_STAGES * A_STAGE_COLS <= PF_TMEM_COLS, "tensor memory holds the accumulators and the A stages");
   static constexpr uint32_t B_STAGE_BYTES = 2 * N_MAX * 128;  // high-byte rows of the routes, then their low-byte rows
   static constexpr uint32_t LOW_B_STAGES = PF_LOW_BYTES / B_STAGE_BYTES;
-  static constexpr uint32_t B_STAGES = N_MAX > 48 ? 4 : 8;    // one ring of barriers for A and B: a K block's A stage is its B stage modulo A_STAGES
+  static constexpr uint32_t B_STAGES = N_MAX > 48 ? 4 : GROUPED ? 6 : 8;    // one ring of barriers for A and B: a K block's A stage is its B stage modulo A_STAGES
   static_assert(B_STAGES % A_STAGES == 0, "");
   static constexpr uint32_t CODE_ROW_BYTES = 2 * PF_KBLOCK_CODES * BITS / 8;  // two K blocks of a row's codes
   static constexpr uint32_t CODE_UNIT_BYTES = PF_ROWS * CODE_ROW_BYTES;       // ... of a tile's
   static constexpr uint32_t CODE_STAGE_BYTES = M * CODE_UNIT_BYTES;
   static constexpr uint32_t CODE_STAGES = BITS == 16 ? 3 : 6;
-  static constexpr uint32_t HIGH_BYTES = PF_TABLE_BYTES + CODE_STAGES * CODE_STAGE_BYTES + (B_STAGES - LOW_B_STAGES) * B_STAGE_BYTES;
+  static constexpr uint32_t SUMS_OFFSET = PF_TABLE_BYTES + CODE_STAGES * CODE_STAGE_BYTES + (B_STAGES - LOW_B_STAGES) * B_STAGE_BYTES;
+  static constexpr uint32_t SUMS = PF_A0 + SUMS_OFFSET;  // [item buffers][segments][routes]: what comes off the segment's integer sums
+  static constexpr uint32_t HIGH_BYTES = SUMS_OFFSET + (GROUPED ? PF_INFO_BUFFERS * PF_MAX_SEGMENTS * N_MAX * 4 : 0);
   static_assert(HIGH_BYTES <= 160 * 1024, "the window above A0");
   static constexpr uint32_t CODE_BASE = PF_A0 + PF_TABLE_BYTES;
   static constexpr __host__ __device__ uint32_t b_stage(uint32_t stage) {
@@ -229,7 +234,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   extern __shared__ __align__(16) uint8_t smem_raw[];
   // STAGE_FULL: the decode warps' A tiles and the activations of a K block are in place; STAGE_EMPTY: its MMAs have read them
   enum { STAGE_FULL = 0, STAGE_EMPTY = STAGE_FULL + B_STAGES, CODE_FULL = STAGE_EMPTY + B_STAGES, CODE_EMPTY = CODE_FULL + CODE_STAGES,
-         ACC_FULL = CODE_EMPTY + CODE_STAGES, ACC_EMPTY = ACC_FULL + ACC_SETS, INFO_FULL = ACC_EMPTY + ACC_SETS, DRAINED = INFO_FULL + PF_INFO_BUFFERS, N_BARS = DRAINED + 1 };
+         ACC_FULL = CODE_EMPTY + CODE_STAGES, ACC_EMPTY = ACC_FULL + ACC_SETS, INFO_FULL = ACC_EMPTY + ACC_SETS, INFO_EMPTY = INFO_FULL + PF_INFO_BUFFERS, DRAINED = INFO_EMPTY + PF_INFO_BUFFERS, N_BARS = DRAINED + 1 };
   static_assert(N_BARS * 8 <= 1024, "");
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
@@ -252,7 +257,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       for (int s = 0; s < B_STAGES; ++s) { mbar_init(bar(STAGE_FULL, s), M * 4 + 1); mbar_init(bar(STAGE_EMPTY, s), 1); }
       for (int s = 0; s < CODE_STAGES; ++s) { mbar_init(bar(CODE_FULL, s), 1); mbar_init(bar(CODE_EMPTY, s), M * 8); }
       for (int s = 0; s < ACC_SETS; ++s) { mbar_init(bar(ACC_FULL, s), 1); mbar_init(bar(ACC_EMPTY, s), PF_DECODE_WARPS); }
-      for (int s = 0; s < PF_INFO_BUFFERS; ++s) mbar_init(bar(INFO_FULL, s), 1);
+      for (int s = 0; s < PF_INFO_BUFFERS; ++s) { mbar_init(bar(INFO_FULL, s), 1); mbar_init(bar(INFO_EMPTY, s), PF_DECODE_WARPS); }
       mbar_init(bar(DRAINED, 0), 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -306,10 +311,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
 
     // the segment that waits for its drain
     bool pending = false, last_segment = false;
+    int pending_segment = 0;
     int n_pad = 0, quarter = 0;
     int64_t erow = 0;
     uint32_t raw_scale[M];
-    int x_sums[GROUPED ? N_MAX / 4 : 1];
     float sum[GROUPED ? M : 1][GROUPED ? N_MAX / 4 : 1];
 
     auto load_scale = [&](int64_t index, int mm) -> uint32_t {
@@ -356,18 +361,19 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
 #pragma unroll
         for (int c = 0; c < N_MAX / 4; c += 4) {
           if (c >= quarter) break;
-          uint32_t v[M][2][4];
+          uint32_t v[M][2][4], less[4];
           load_columns(v, c_first + c);
+          asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(less[0]), "=r"(less[1]), "=r"(less[2]), "=r"(less[3])
+                       : "r"(Plan::SUMS + ((info.index * PF_MAX_SEGMENTS + pending_segment) * N_MAX + c_first + c) * 4u));
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if (c + 4 >= quarter) release_accumulators();
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const uint32_t offset = 8u * static_cast<uint32_t>(x_sums[c + j]);
-            const float x_sum4 = BITS == 16 ? 0.25f * static_cast<float>(x_sums[c + j]) : 0.0f;
 #pragma unroll
             for (int mm = 0; mm < M; ++mm) {
-              const int dot = static_cast<int>(v[mm][0][j] * 256u + v[mm][1][j] - offset);
-              sum[mm][c + j] += scale[mm] * (0.5f * static_cast<float>(dot) + x_sum4);
+              // 4 sum(w x') in wrapping 32-bit arithmetic, which the true value fits: four instructions a value and segment
+              const int dot4 = static_cast<int>(v[mm][0][j] * 512u + (v[mm][1][j] * 2u + less[j]));
+              sum[mm][c + j] += scale[mm] * static_cast<float>(dot4);
             }
           }
         }
@@ -378,7 +384,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
               const int4 pr = per_route[c_first + c];
               float y[M];
 #pragma unroll
-              for (int mm = 0; mm < M; ++mm) y[mm] = __int_as_float(pr.y) * sum[mm][c];
+              for (int mm = 0; mm < M; ++mm) y[mm] = 0.25f * __int_as_float(pr.y) * sum[mm][c];
               finish_column(pr, y, round_out, store_out);
             }
 #pragma unroll
@@ -423,7 +429,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       else
         drain_as([](float v) { return v; }, [&](int64_t i, float v) { static_cast<float*>(p.out)[i] = v; });
       acc.advance();
-      if (last_segment) info.advance();
+      if (last_segment) {
+        __syncwarp();
+        mbar_arrive_warp(bar(INFO_EMPTY, info.index), lane);
+        info.advance();
+      }
     };
 
     if constexpr (GROUPED) {
@@ -435,7 +445,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
       const int gi = item / row_tiles, tile = item - gi * row_tiles;
       const int64_t slot = p.groups_of_routes.slot[gi];
-      const int gsize = p.groups_of_routes.size[gi], gstart = p.groups_of_routes.start[gi];
+      const int gsize = p.groups_of_routes.size[gi];
       for (int segment = 0; segment < segments && ok; ++segment) {
         if (m < M) {
           for (int b = parity; b < segment_blocks; b += 2) {
@@ -479,6 +489,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         if (pending) drain();  // a warp without K blocks
         // this segment is the next to be drained; what its drain needs from memory is asked for now
         pending = true;
+        pending_segment = segment;
         last_segment = segment == segments - 1;
         if (segment == 0) {
           n_pad = (gsize + 15) & ~15;
@@ -487,18 +498,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         }
 #pragma unroll
         for (int mm = 0; mm < M; ++mm) raw_scale[mm] = load_scale((slot * N_out + min(erow + mm * TILE_STEP, N_out - 1)) * segments + segment, mm);
-        if constexpr (GROUPED) {
-#pragma unroll
-          for (int c = 0; c < N_MAX / 4; ++c) {
-            const int n = part * quarter + c;
-            x_sums[c] = c < quarter && n < gsize ? p.x.sums[static_cast<int64_t>(gstart + n) * segments + segment] : 0;
-          }
-        }
       }
     }
     if (pending && ok) drain();
   } else if (warp == PF_MMA_WARP) {
-    // ================= per-route facts for the drain, and the MMAs =============================
+    // ================= the MMAs ================================================================
     // One loop over all K blocks of the block's items, unrolled over the stage ring: this warp's own
     // instructions between two K blocks are on the critical path.  The whole warp walks and waits,
     // one elected lane issues, and the addresses are immediates: an MMA's descriptors live in uniform
@@ -507,10 +511,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     // waits, two commits and addresses worked out inside the elected branch, where the tensor core
     // takes 128 to 256 at 16 to 32 routes).
     RingPlace<ACC_SETS> acc;
-    uint32_t info_index = 0, phase = 0, idesc = 0, d_cols = 0;
+    uint32_t phase = 0, idesc = 0, d_cols = 0;
     bool ok = true, first_round = true;
     int item = static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x), segment = segments - 1, kb = segment_blocks - 1;
-    // the next segment: its accumulators, and at the start of an item its facts
+    // the next segment: its accumulators, and at the start of an item its width
     auto next_segment = [&]() {
       kb = 0;
       if (++segment == segments) {
@@ -518,21 +522,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         item += gridDim.x;
         if (item >= items_here) return false;
         const int gi = item / row_tiles;
-        const int gsize = warp_uniform(p.groups_of_routes.size[gi]), gstart = p.groups_of_routes.start[gi];
-        const int n_pad = (gsize + 15) & ~15;  // the N of the MMA
-        // The facts go into the buffer of item n - 3.  Behind every MMA of item n - 1 stand all decode
-        // warps' K blocks of that item, and a warp produces those only after its drain of item n - 3
-        // (it drains an item no later than behind its first K block of the next one; a warp without K
-        // blocks must have handed back the accumulators of item n - 2, which it does after item n - 3).
-        for (int n = lane; n < n_pad; n += 32) {
-          const int route = n < gsize ? p.groups_of_routes.routes[gstart + n] : -1;
-          const int64_t xrow = route < 0 ? p.x_zero_row : static_cast<int64_t>(gstart + n);  // the activation rows were quantised in grouped order
-          const float weight = (GLU && route >= 0) ? p.route_weight[route] : 1.0f;
-          route_info[info_index][n] = make_int4(route, __float_as_int(p.x.scale[xrow]), GROUPED ? 0 : p.x.sums[xrow], __float_as_int(weight));
-        }
-        __syncwarp();
-        mbar_arrive_warp(bar(INFO_FULL, info_index), lane);
-        if (++info_index == PF_INFO_BUFFERS) info_index = 0;
+        const int n_pad = (p.groups_of_routes.size[gi] + 15) & ~15;
         // N = 2 * n_pad: the high-byte rows and the low-byte rows of the routes are one B operand;
         // accumulator s32, A unsigned bytes (the nibble decoder's u = q + 8), B signed bytes
         idesc = warp_uniform((2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(n_pad >> 2) << 17) | ((PF_ROWS >> 4) << 24));
@@ -626,6 +616,41 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     if (*aborted) wait_copies_landed<CODE_STAGES>(bar(CODE_FULL, 0), used);
   }
 
+  if (warp == PF_INFO_WARP) {
+    // ================= what the drain needs per route, up to three items ahead ==================
+    RingPlace<PF_INFO_BUFFERS> info;
+    bool ok = true;
+    for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
+      const int gi = item / row_tiles;
+      const int gsize = p.groups_of_routes.size[gi], gstart = p.groups_of_routes.start[gi];
+      const int n_pad = (gsize + 15) & ~15;
+      ok = mbar_wait<true>(bar(INFO_EMPTY, info.index), info.phase ^ 1u, deadline, aborted);
+      if (!ok) break;
+      for (int n = lane; n < n_pad; n += 32) {
+        const int route = n < gsize ? p.groups_of_routes.routes[gstart + n] : -1;
+        const int64_t xrow = route < 0 ? p.x_zero_row : static_cast<int64_t>(gstart + n);  // the activation rows were quantised in grouped order
+        const float weight = (GLU && route >= 0) ? p.route_weight[route] : 1.0f;
+        route_info[info.index][n] = make_int4(route, __float_as_int(p.x.scale[xrow]), GROUPED ? 0 : p.x.sums[xrow], __float_as_int(weight));
+      }
+      if constexpr (GROUPED) {
+        // the A operand is u = q + 8 (4w = 2q + 1; 2q for 8-bit codes): 2 D - 15 sum(x') = sum(4w x'), or 2 D - 16 sum(x')
+        const int step_n = 32 / segments, step_segment = 32 % segments;
+        int n = lane / segments, segment = lane % segments;
+        while (n < n_pad) {
+          const int x_sum = n < gsize ? p.x.sums[static_cast<int64_t>(gstart + n) * segments + segment] : 0;
+          asm volatile("st.shared.u32 [%0], %1;" ::"r"(Plan::SUMS + ((info.index * PF_MAX_SEGMENTS + segment) * N_MAX + n) * 4u),
+                       "r"((BITS == 16 ? 15u : 16u) * (0u - static_cast<uint32_t>(x_sum))) : "memory");
+          n += step_n;
+          segment += step_segment;
+          if (segment >= segments) { segment -= segments; ++n; }
+        }
+      }
+      __syncwarp();
+      mbar_arrive_warp(bar(INFO_FULL, info.index), lane);
+      info.advance();
+    }
+  }
+
   // ---- teardown ------------------------------------------------------------------------------
   __syncwarp();
   if (*aborted) {
@@ -643,7 +668,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
 
 bool prefill_supported(int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups) {
   // code rows are addressed by a 32-bit box coordinate that may run past the last row by an item
-  return shapes_supported(out_dim, in_dim, groups) && slots * out_dim < (int64_t{1} << 31) - 4 * PF_ROWS;
+  return shapes_supported(out_dim, in_dim, groups) && slots * out_dim < (int64_t{1} << 31) - 4 * PF_ROWS &&
+         (groups == 1 || (groups <= PF_MAX_SEGMENTS && in_dim / groups <= PF_MAX_SEGMENT_INPUTS));
 }
 
 // Routes per item.  96 fill tensor memory (accumulators of two byte planes and two tiles, two A
