@@ -5,7 +5,7 @@
 // out[r] = W[rhs[r]] @ x[r] for r < routes; x holds one activation row per route (the caller
 // gathers them, as the reference does before its kernels, src/ramp/ops/vq_switch.py:758-761).
 // The sequence is the down projection of the layer call: quantise the rows, group the routes by
-// expert on the device, then the tcgen05 kernel (8 or more routes per expert on average) or the
+// expert on the device, then the tcgen05 kernel (5 or more routes per expert on average) or the
 // mma.sync one.  Routes need not be sorted; a route with expert 0xFFFFFFFF gives a zero row.
 #include "moe_fast.cuh"
 
@@ -20,13 +20,6 @@ struct GroupedScratch {
 };
 
 static inline int64_t up256(int64_t v) { return (v + 255) / 256 * 256; }
-
-// The grouped kernels never touch the output row of a route that names no expert: this does.
-__global__ void __launch_bounds__(128) zero_dead_rows_kernel(const uint32_t* __restrict__ rhs, int64_t slots, void* out, int64_t row_bytes) {
-  if (rhs[blockIdx.x] < static_cast<uint64_t>(slots)) return;
-  uint8_t* row = reinterpret_cast<uint8_t*>(out) + static_cast<int64_t>(blockIdx.x) * row_bytes;
-  for (int64_t i = threadIdx.x * 2; i < row_bytes; i += 256) *reinterpret_cast<uint16_t*>(row + i) = 0;
-}
 
 static GroupedScratch plan_grouped(int64_t routes, int64_t in_dim) {
   GroupedScratch s;
@@ -89,7 +82,7 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
   fast::RouteGroups groups = {reinterpret_cast<int32_t*>(ws + sc.gcount), reinterpret_cast<int32_t*>(ws + sc.gslot),
                               reinterpret_cast<int32_t*>(ws + sc.gstart), reinterpret_cast<int32_t*>(ws + sc.gsize),
                               reinterpret_cast<int32_t*>(ws + sc.groutes)};
-  const bool many = byte_codes || (!residual && a.routes >= 1024 && a.routes >= 8 * a.slots && fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups));
+  const bool many = byte_codes || (!residual && fast::prefill_pays(a.routes, a.slots, a.groups > 1) && fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups));
   // (the sums region has room for a scale group per codeword; these kernels' rows have at most one
   // per 256 inputs, and their sums per 256 inputs go behind those)
   fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + sc.xq), reinterpret_cast<float*>(ws + sc.xscale), reinterpret_cast<int32_t*>(ws + sc.xsums),
@@ -98,10 +91,15 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
   if (many) groups.position = reinterpret_cast<int32_t*>(ws + sc.xsums) + (a.routes + 1) * a.groups;  // behind the sums, as well
   int rc;
   const int group_cols = byte_codes ? fast::PREFILL_GROUP_ROUTES_SMALL : many ? fast::prefill_group_routes(a.routes, a.slots, a.groups > 1) : fast::decode_group_routes(a.routes, a.slots, a.in_dim);
-  if ((rc = fast::group_routes(a.rhs, a.routes, a.slots, group_cols, groups, wait_status, s))) return rc;
-  if (many) {  // the tcgen05 kernels copy rows in grouped order
-    if ((rc = fast::quantize_rows_sorted(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, groups.position, x_div, s))) return rc;
-  } else if ((rc = fast::quantize_rows(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, false, s))) return rc;
+  const fast::DeadRows dead = {a.rhs, x_div, a.slots, a.out, a.out_dim * dtype_size(a.out_dtype)};
+  if (!many && fast::group_with_quantize_supported(a.routes, a.slots)) {  // one launch for both
+    if ((rc = fast::quantize_rows_and_group(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, false, s, nullptr, 1, a.slots, a.rhs, a.routes, group_cols, groups, wait_status, dead))) return rc;
+  } else {
+    if ((rc = fast::group_routes(a.rhs, a.routes, a.slots, group_cols, groups, wait_status, s))) return rc;
+    if (many) rc = fast::quantize_rows_sorted(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, groups.position, x_div, s, dead);
+    else rc = fast::quantize_rows_and_group(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, false, s, nullptr, 1, a.slots, nullptr, 0, 0, {}, nullptr, dead);
+    if (rc) return rc;
+  }
   fast::FastProjectionArgs p = {};
   p.slots = a.slots;
   p.a = {static_cast<const uint16_t*>(a.codes), a.scales, a.res_codes, a.res_scales}; p.b = {nullptr, nullptr, nullptr, nullptr};
@@ -110,9 +108,6 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
   p.few_groups = many ? 0 : fast::few_route_groups(a.routes, a.slots);
   p.out_dim = a.out_dim; p.in_dim = a.in_dim; p.groups = a.groups; p.x = xq; p.x_zero_row = many ? a.routes : x_rows; p.x_div = x_div;
   p.out = a.out; p.out_dtype = a.out_dtype; p.swiglu_limit = 0.0f; p.route_weight = nullptr;
-  if (a.routes > 0x7FFFFFFFll) return KEEPVQ_ERR_CAPACITY;
-  zero_dead_rows_kernel<<<static_cast<unsigned>(a.routes), 128, 0, s>>>(a.rhs, a.slots, a.out, a.out_dim * dtype_size(a.out_dtype));
-  KEEPVQ_CHECK_LAUNCH();
   if (byte_codes) return fast::prefill_byte_codes(p, wait_status, s);
   return many ? fast::prefill_down(p, wait_status, s) : fast::down(p, s);
 }

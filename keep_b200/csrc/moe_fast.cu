@@ -36,16 +36,18 @@ namespace fast {
 // 256 inputs and a scale group is a whole number of chunks.  `sm`: in_dim / 256 ints.
 template <typename XT, int THREADS, typename Target>
 __device__ __forceinline__ void quantize_row(const XT* __restrict__ xr, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, int planes, int32_t* sm, int targets, Target target) {
-  constexpr int KEEP = THREADS == 32 ? 10 : 8;  // vectors of eight values a thread keeps
+  // Vectors of eight values a thread keeps.  Blocks of 256 serve calls of a few rows, where the code a
+  // cold launch has to fetch counts (eight copies of the conversion cost such a call a microsecond).
+  constexpr int KEEP = THREADS == 32 ? 10 : THREADS == 128 ? 5 : 2;
   constexpr bool PAIRS = sizeof(XT) == 2;  // 16-bit values: kept as they are, maximum taken on pairs
-  __shared__ float warp_max[THREADS / 32];  // (a warp on its own has none to share)
+  __shared__ uint32_t warp_max[THREADS / 32];  // (a warp on its own has none to share)
   auto team_sync = [] { if (THREADS > 32) __syncthreads(); else __syncwarp(); };
   const int cw = static_cast<int>(in_dim / 8), chunks = cw / 32, per_group = chunks / static_cast<int>(groups);
   const int tid = threadIdx.x % THREADS, lane = tid & 31, warp = tid >> 5;
   uint4 raw[KEEP];
-  // largest magnitude; a NaN or an infinity anywhere gives a value that is not finite
-  float amax = 0.0f;
-  bool odd = false;
+  // largest magnitude, as the bits of a float (they order like the values): a NaN or an infinity
+  // anywhere gives the bits of an infinity or more
+  uint32_t top_bits = 0;
   if constexpr (PAIRS) {
     typedef typename std::conditional<std::is_same<XT, __half>::value, __half2, __nv_bfloat162>::type Pair;
     uint32_t top = 0;
@@ -66,44 +68,48 @@ __device__ __forceinline__ void quantize_row(const XT* __restrict__ xr, int64_t 
 #pragma unroll
     for (int i = 0; i < KEEP; ++i)
       if (tid + i * THREADS < cw) take(raw[i]);
+#pragma unroll 1
     for (int c = tid + KEEP * THREADS; c < cw; c += THREADS) take(*reinterpret_cast<const uint4*>(xr + c * 8));
     const Pair pair = *reinterpret_cast<const Pair*>(&top);
     const float a = std::is_same<XT, __half>::value ? __half2float(*reinterpret_cast<const __half*>(&pair.x)) : __uint_as_float(top << 16);
     const float b = std::is_same<XT, __half>::value ? __half2float(*reinterpret_cast<const __half*>(&pair.y)) : __uint_as_float(top & 0xFFFF0000u);
-    odd = !(isfinite(a) && isfinite(b));
-    amax = fmaxf(a, b);
+    top_bits = max(__float_as_uint(a) & 0x7FFFFFFFu, __float_as_uint(b) & 0x7FFFFFFFu);
   } else {
     for (int c = tid; c < cw; c += THREADS) {
       float v[8];
       load8_as_float<XT>(xr + c * 8, v);
 #pragma unroll
-      for (int d = 0; d < 8; ++d) { odd = odd || !isfinite(v[d]); amax = fmaxf(amax, fabsf(v[d])); }
+      for (int d = 0; d < 8; ++d) top_bits = max(top_bits, __float_as_uint(v[d]) & 0x7FFFFFFFu);
     }
   }
-  odd = THREADS > 32 ? __syncthreads_or(odd) : __any_sync(0xFFFFFFFFu, odd);
+  auto team_max = [&](uint32_t bits) {
+    bits = __reduce_max_sync(0xFFFFFFFFu, bits);
+    if (THREADS > 32) {
+      if (lane == 0) warp_max[warp] = bits;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < THREADS / 32; ++w) bits = max(bits, warp_max[w]);
+    }
+    return bits;
+  };
+  top_bits = team_max(top_bits);
+  const bool odd = top_bits >= 0x7F800000u;
   if (odd) {  // rows with a NaN or an infinity: the maximum leaves the NaNs out
-    amax = 0.0f;
+    float amax = 0.0f;
     for (int c = tid; c < cw; c += THREADS) {
       float v[8];
       load8_as_float<XT>(xr + c * 8, v);
 #pragma unroll
       for (int d = 0; d < 8; ++d) amax = fmaxf(amax, fabsf(v[d]));
     }
+    team_sync();  // everyone has read warp_max
+    top_bits = team_max(__float_as_uint(amax));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-  float m = amax;
-  if (THREADS > 32) {
-    if (lane == 0) warp_max[warp] = amax;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < THREADS / 32; ++w) m = fmaxf(m, warp_max[w]);
-  }
+  const float m = __uint_as_float(top_bits);
   float s = 1.0f;
   if (m > 0.0f && isfinite(m)) {
-    int ex;
-    frexpf(m, &ex);            // m < 2^ex
-    s = ldexpf(1.0f, ex - 15);  // |x| / s < 2^15
+    // |x| / s < 2^15 with s a power of two: the exponent of m, less 14
+    s = top_bits >= (16u << 23) ? __uint_as_float((top_bits & 0x7F800000u) - (14u << 23)) : ldexpf(1.0f, ilogbf(m) - 14);
     if (m / s > 32639.0f) s *= 2.0f;  // 127 * 256 + 127: the largest value two signed bytes hold
   }
   const float inv = 1.0f / s;  // exact: a power of two
@@ -159,6 +165,7 @@ __device__ __forceinline__ void quantize_row(const XT* __restrict__ xr, int64_t 
       }
     }
   }
+#pragma unroll 1
   for (int c = tid + (PAIRS ? KEEP * THREADS : 0); c < cw; c += THREADS) {
     float v[8];
     load8_as_float<XT>(xr + c * 8, v);
@@ -169,10 +176,11 @@ __device__ __forceinline__ void quantize_row(const XT* __restrict__ xr, int64_t 
     const int64_t row = target(j);
     if (row < 0) continue;
     if (tid == 0) out.scale[row] = s;
-    for (int g = tid; g < groups; g += THREADS) {
+    for (int g = warp; g < groups; g += THREADS / 32) {
       int total = 0;
-      for (int c = 0; c < per_group; ++c) total += sm[g * per_group + c];
-      out.sums[row * groups + g] = total;
+      for (int c = lane; c < per_group; c += 32) total += sm[g * per_group + c];
+      total = __reduce_add_sync(0xFFFFFFFFu, total);
+      if (lane == 0) out.sums[row * groups + g] = total;
     }
     if (out.chunk_sums)
       for (int c = tid; c < chunks; c += THREADS) out.chunk_sums[row * chunks + c] = sm[c];
@@ -197,6 +205,18 @@ __device__ __forceinline__ void zero_row(int64_t row, int64_t rows, int64_t in_d
   if (threadIdx.x == 0) out.scale[row] = 1.0f;
 }
 
+// Zeroes the output rows of the dead routes that read activation row `row`.
+template <int THREADS>
+__device__ __forceinline__ void zero_dead_rows(const DeadRows& dead, int64_t row) {
+  if (!dead.slot) return;
+  for (int j = 0; j < dead.per_row; ++j) {
+    const int64_t route = row * dead.per_row + j;
+    if (dead.slot[route] < static_cast<uint64_t>(dead.slots)) continue;
+    uint16_t* out = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(dead.out) + route * dead.row_bytes);
+    for (int64_t i = threadIdx.x % THREADS; i < dead.row_bytes / 2; i += THREADS) out[i] = 0;
+  }
+}
+
 // `live` (may be null): the slots of the routes that read the rows, `per_row` of them per row; a row
 // none of whose routes has a slot below `slots` is skipped (no kernel reads it: projections only
 // follow live routes).  An expert-parallel rank quantises 8 x capacity rows of which an eighth is live.
@@ -207,7 +227,7 @@ struct LiveRows { const uint32_t* slot; int32_t per_row; int64_t slots; };
 struct GroupJob { const uint32_t* served_slot; int32_t routes, slots, max_group; RouteGroups out; int32_t* clear; };
 
 template <typename XT>
-__global__ void __launch_bounds__(256) quantize_rows_kernel(const XT* __restrict__ x, int64_t rows, int64_t in_dim, int64_t groups, QuantRows out, int planes, LiveRows live, GroupJob job) {
+__global__ void __launch_bounds__(256) quantize_rows_kernel(const XT* __restrict__ x, int64_t rows, int64_t in_dim, int64_t groups, QuantRows out, int planes, LiveRows live, GroupJob job, DeadRows dead) {
   grid_launch_dependents();
   grid_wait();
   extern __shared__ int32_t sm[];
@@ -217,6 +237,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const XT* __restrict
     return;
   }
   if (row == rows) return zero_row<256>(row, rows, in_dim, groups, out, planes);
+  zero_dead_rows<256>(dead, row);
   if (live.slot) {
     bool any = false;
     for (int j = 0; j < live.per_row; ++j) any = any || live.slot[row * live.per_row + j] < static_cast<uint64_t>(live.slots);
@@ -231,7 +252,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const XT* __restrict
 constexpr int QS_THREADS = 128;
 constexpr int64_t QS_WARP_ROW = 2560;
 template <typename XT, int TEAM>
-__global__ void __launch_bounds__(QS_THREADS) quantize_rows_sorted_kernel(const XT* __restrict__ x, int64_t x_rows, int64_t in_dim, int64_t groups, QuantRows out, const int32_t* __restrict__ position, int x_div) {
+__global__ void __launch_bounds__(QS_THREADS) quantize_rows_sorted_kernel(const XT* __restrict__ x, int64_t x_rows, int64_t in_dim, int64_t groups, QuantRows out, const int32_t* __restrict__ position, int x_div, DeadRows dead) {
   grid_launch_dependents();
   grid_wait();
   extern __shared__ int32_t sm[];
@@ -240,6 +261,7 @@ __global__ void __launch_bounds__(QS_THREADS) quantize_rows_sorted_kernel(const 
   const int64_t r = static_cast<int64_t>(blockIdx.x) * TEAMS + team, rows = x_rows * x_div;
   if (blockIdx.x == gridDim.x - 1) return zero_row<QS_THREADS>(rows, rows, in_dim, groups, out, 1);
   if (r >= x_rows) return;
+  zero_dead_rows<TEAM>(dead, r);
   bool any = false;
   for (int j = 0; j < x_div; ++j) any = any || position[r * x_div + j] >= 0;
   if (!any) return;  // nothing reads the row (uniform over the team)
@@ -294,19 +316,19 @@ int quantize_rows(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, 
 }
 
 template <typename XT>
-static cudaError_t launch_sorted(const void* x, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s) {
+static cudaError_t launch_sorted(const void* x, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s, const DeadRows& dead) {
   const bool warps = in_dim <= QS_WARP_ROW;
   const int64_t teams = warps ? QS_THREADS / 32 : 1;
   const unsigned grid = static_cast<unsigned>((x_rows + teams - 1) / teams + 1);  // + the zero row
   return launch_after(grid < EARLY_LAUNCH_MAX_BLOCKS, warps ? quantize_rows_sorted_kernel<XT, 32> : quantize_rows_sorted_kernel<XT, QS_THREADS>, grid, QS_THREADS,
-                      chunk_bytes(in_dim) * teams, s, static_cast<const XT*>(x), x_rows, in_dim, groups, out, position, x_div);
+                      chunk_bytes(in_dim) * teams, s, static_cast<const XT*>(x), x_rows, in_dim, groups, out, position, x_div, dead);
 }
-int quantize_rows_sorted(const void* x, int32_t x_dtype, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s) {
+int quantize_rows_sorted(const void* x, int32_t x_dtype, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s, const DeadRows& dead) {
   if (chunk_bytes(in_dim) > 40 * 1024) return KEEPVQ_ERR_CAPACITY;
   cudaError_t err;
-  if (x_dtype == KEEPVQ_F32) err = launch_sorted<float>(x, x_rows, in_dim, groups, out, position, x_div, s);
-  else if (x_dtype == KEEPVQ_F16) err = launch_sorted<__half>(x, x_rows, in_dim, groups, out, position, x_div, s);
-  else err = launch_sorted<__nv_bfloat16>(x, x_rows, in_dim, groups, out, position, x_div, s);
+  if (x_dtype == KEEPVQ_F32) err = launch_sorted<float>(x, x_rows, in_dim, groups, out, position, x_div, s, dead);
+  else if (x_dtype == KEEPVQ_F16) err = launch_sorted<__half>(x, x_rows, in_dim, groups, out, position, x_div, s, dead);
+  else err = launch_sorted<__nv_bfloat16>(x, x_rows, in_dim, groups, out, position, x_div, s, dead);
   if (err != cudaSuccess) return note_cuda_error(err);
   return KEEPVQ_OK;
 }
@@ -315,7 +337,7 @@ bool group_with_quantize_supported(int64_t routes, int64_t slots) { return route
 
 int quantize_rows_and_group(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, bool planes, cudaStream_t s,
                             const uint32_t* live_slot, int32_t per_row, int64_t slots,
-                            const uint32_t* served_slot, int64_t routes, int max_group, const RouteGroups& route_groups, int32_t* clear) {
+                            const uint32_t* served_slot, int64_t routes, int max_group, const RouteGroups& route_groups, int32_t* clear, const DeadRows& dead) {
   const LiveRows live = {live_slot, per_row, slots};
   const GroupJob job = {served_slot, static_cast<int32_t>(routes), static_cast<int32_t>(slots), max_group, route_groups, clear};
   size_t smem = chunk_bytes(in_dim);
@@ -327,9 +349,9 @@ int quantize_rows_and_group(const void* x, int32_t x_dtype, int64_t rows, int64_
   const unsigned grid = static_cast<unsigned>(rows + 1 + (served_slot ? 1 : 0));  // + the zero row (+ the grouping block)
   const bool early = rows < EARLY_LAUNCH_MAX_BLOCKS;
   cudaError_t err;
-  if (x_dtype == KEEPVQ_F32) err = launch_after(early, quantize_rows_kernel<float>, grid, 256, smem, s, reinterpret_cast<const float*>(x), rows, in_dim, groups, out, planes ? 1 : 0, live, job);
-  else if (x_dtype == KEEPVQ_F16) err = launch_after(early, quantize_rows_kernel<__half>, grid, 256, smem, s, reinterpret_cast<const __half*>(x), rows, in_dim, groups, out, planes ? 1 : 0, live, job);
-  else err = launch_after(early, quantize_rows_kernel<__nv_bfloat16>, grid, 256, smem, s, reinterpret_cast<const __nv_bfloat16*>(x), rows, in_dim, groups, out, planes ? 1 : 0, live, job);
+  if (x_dtype == KEEPVQ_F32) err = launch_after(early, quantize_rows_kernel<float>, grid, 256, smem, s, reinterpret_cast<const float*>(x), rows, in_dim, groups, out, planes ? 1 : 0, live, job, dead);
+  else if (x_dtype == KEEPVQ_F16) err = launch_after(early, quantize_rows_kernel<__half>, grid, 256, smem, s, reinterpret_cast<const __half*>(x), rows, in_dim, groups, out, planes ? 1 : 0, live, job, dead);
+  else err = launch_after(early, quantize_rows_kernel<__nv_bfloat16>, grid, 256, smem, s, reinterpret_cast<const __nv_bfloat16*>(x), rows, in_dim, groups, out, planes ? 1 : 0, live, job, dead);
   if (err != cudaSuccess) return note_cuda_error(err);
   return KEEPVQ_OK;
 }

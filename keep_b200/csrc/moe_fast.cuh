@@ -246,6 +246,9 @@ bool shapes_supported(int64_t out_dim, int64_t in_dim, int64_t groups);
 // True when gate_up / down can also add a nested residual with these scale groups to `routes` routes.
 bool residual_supported(int64_t routes, int64_t in_dim, int64_t res_groups);
 
+// Output rows of routes that name no expert: the projection kernels never touch them, so a caller
+// that promises zeros there has the quantisation kernels write them.  slot == nullptr: no such promise.
+struct DeadRows { const uint32_t* slot = nullptr; int32_t per_row = 1; int64_t slots = 0; void* out = nullptr; int64_t row_bytes = 0; };
 // planes = false: 16 bytes per codeword (hi 8, lo 8), what the mma.sync kernels read;
 // planes = true: all high bytes [rows + 1, in_dim] then all low bytes (quantize_rows_sorted writes that form).
 // live_slot (may be null): [rows, per_row] slots of the routes that read the rows; rows whose routes are all dead (slot >= slots) are skipped.
@@ -255,7 +258,8 @@ int quantize_rows(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, 
 // low bytes) with a row per route IN GROUPED ORDER: input row r is quantised once and written to the
 // rows position[r * x_div ...] of its x_div routes (group_routes must have run); rows of routes
 // without a slot are left alone; scale and sums are per output row.  rows = x_rows * x_div.
-int quantize_rows_sorted(const void* x, int32_t x_dtype, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s);
+int quantize_rows_sorted(const void* x, int32_t x_dtype, int64_t x_rows, int64_t in_dim, int64_t groups, const QuantRows& out, const int32_t* position, int32_t x_div, cudaStream_t s,
+                         const DeadRows& dead = {});
 // `clear` (may be null): a status word the kernel zeroes for the projection kernels that follow it.
 // The router's logits and quantize_rows (planes = false) of the same token rows in one launch, for
 // calls of at most FRONT_MAX_TOKENS tokens with fp16 / bf16 activations.
@@ -266,7 +270,7 @@ int logits_and_quantize(const keepvq_router_logits_args& logits, int64_t groups,
 bool group_with_quantize_supported(int64_t routes, int64_t slots);
 int quantize_rows_and_group(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, bool planes, cudaStream_t s,
                             const uint32_t* live_slot, int32_t per_row, int64_t slots,
-                            const uint32_t* served_slot, int64_t routes, int max_group, const RouteGroups& route_groups, int32_t* clear);
+                            const uint32_t* served_slot, int64_t routes, int max_group, const RouteGroups& route_groups, int32_t* clear, const DeadRows& dead = {});
 int group_routes(const uint32_t* served_slot, int64_t routes, int64_t slots, int max_group, const RouteGroups& out, int32_t* clear, cudaStream_t s);
 // Routes per group for a decode call: four while experts rarely get more (the kernels then run one
 // MMA per step for both byte planes), eight beyond.  `live` = routes expected to carry a slot.
@@ -293,6 +297,14 @@ int sweep_down(const FastProjectionArgs& args, cudaStream_t s);
 // tcgen05 kernels for many routes per expert (prefill_umma.cu).  `status` is a device word that
 // a CTA sets to 1 if one of its bounded waits expires.
 bool prefill_supported(int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups);
+// The tcgen05 kernels decode a code once per 48 or 96 routes of an expert and cost nearly the same for
+// one route as for 48; the mma.sync kernels stream an expert's codes once per 4 or 8 routes.  Which
+// one pays depends on routes per expert, and the host only knows their number over the call (reading
+// the routing back would stall the stream).  Whole layers, mma.sync against tcgen05: 384 experts of
+// 4096 x 2048, one scale group: 825 / 834 us at 4 routes an expert, 870 / 855 at 5, 1136 / 869 at 7.5;
+// 192 experts of 5120 x 2304 in groups of 512 and 256: 713 / 971 us at 4, 961 / 962 at 8, 4459 / 1119 at 32.
+constexpr int64_t PREFILL_MIN_ROUTES = 1024;
+inline bool prefill_pays(int64_t live, int64_t slots, bool several_groups) { return live >= PREFILL_MIN_ROUTES && live >= (several_groups ? 8 : 5) * slots; }
 // Routes per item (group_routes' max_group) of a call with `live` routes; a kernel takes p.group_cols.
 int prefill_group_routes(int64_t live, int64_t slots, bool several_groups);
 int prefill_gate_up(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);

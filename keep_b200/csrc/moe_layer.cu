@@ -35,15 +35,6 @@ struct dtype_tag_of {
 
 static inline int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
-// The tcgen05 kernels decode a code once per 48 or 96 routes of an expert and cost nearly the same
-// for one route as for 48; the mma.sync kernels stream an expert's codes once per 4 or 8 routes.
-// Which one pays depends on routes per expert, and the host only knows its upper bound
-// routes / slots (reading the routing back would stall the stream): from 8 on, the two passes of
-// the decode kernels cost more than the one pass of the tcgen05 kernels (1000 tokens of top-6 over
-// 384 experts, 15.6 routes each: 1069 against 2019 us for the layer).
-constexpr int64_t PREFILL_MIN_ROUTES = 1024;
-constexpr int64_t PREFILL_MIN_ROUTES_PER_SLOT = 8;
-
 struct LayerScratch {
   int64_t logits, gate, up, h, down;
   int64_t xq, xscale, xsums, hq, hscale, hsums, gcount, gslot, gstart, gsize, groutes, status;
@@ -60,7 +51,7 @@ static LayerScratch plan_scratch(int64_t tokens, int64_t hidden, int64_t inter, 
   s.h = at;      at += align256(routes * inter * 4);
   s.down = at;   at += align256(routes * hidden * 4);
   // calls large enough for the tcgen05 kernels quantise the token rows once per route, in grouped order
-  const int64_t x_rows = routes >= PREFILL_MIN_ROUTES ? routes : tokens;
+  const int64_t x_rows = routes >= fast::PREFILL_MIN_ROUTES ? routes : tokens;
   s.xq = at;     at += align256((x_rows + 1) * hidden * 2);  // + the zero row
   s.xscale = at; at += align256((x_rows + 1) * 4);
   s.xsums = at;  at += align256(std::max((tokens + 1) * (hidden / 8) * 4, (x_rows + 1) * std::max<int64_t>(hidden / 256, 1) * 4));  // room for one scale group per codeword (one per 256 inputs in grouped order)
@@ -208,7 +199,7 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
   int rc = KEEPVQ_OK;
   // many routes per expert: the tcgen05 kernels
   const int64_t live = a.expected_routes > 0 && a.expected_routes < routes ? a.expected_routes : routes;
-  const bool prefill = tensor_path && !residual && live >= PREFILL_MIN_ROUTES && live >= PREFILL_MIN_ROUTES_PER_SLOT * a.slots &&
+  const bool prefill = tensor_path && !residual && fast::prefill_pays(live, a.slots, a.w1.groups > 1 || a.w2.groups > 1) &&
                        fast::prefill_supported(a.slots, a.inter, a.hidden, a.w1.groups) && fast::prefill_supported(a.slots, a.hidden, a.inter, a.w2.groups);
   // (the sums regions have room for a scale group per codeword; the tensor-core kernels' rows have at
   // most one per 256 inputs, and their sums per 256 inputs go behind those)

@@ -232,6 +232,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   constexpr int A_STAGES = Plan::A_STAGES, B_STAGES = Plan::B_STAGES, CODE_STAGES = Plan::CODE_STAGES, ACC_SETS = Plan::ACC_SETS;
   constexpr int TILE_STEP = GLU ? 0 : PF_ROWS;  // rows between the A tiles of an item
   extern __shared__ __align__(16) uint8_t smem_raw[];
+  grid_launch_dependents();
   // STAGE_FULL: the decode warps' A tiles and the activations of a K block are in place; STAGE_EMPTY: its MMAs have read them
   enum { STAGE_FULL = 0, STAGE_EMPTY = STAGE_FULL + B_STAGES, CODE_FULL = STAGE_EMPTY + B_STAGES, CODE_EMPTY = CODE_FULL + CODE_STAGES,
          ACC_FULL = CODE_EMPTY + CODE_STAGES, ACC_EMPTY = ACC_FULL + ACC_SETS, INFO_FULL = ACC_EMPTY + ACC_SETS, INFO_EMPTY = INFO_FULL + PF_INFO_BUFFERS, DRAINED = INFO_EMPTY + PF_INFO_BUFFERS, N_BARS = DRAINED + 1 };
@@ -273,6 +274,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   if (!set_up_ok && tid == 0) abort_flag = 1;
   // an allocation of all 512 columns starts at column 0 of lane 0: a constant, which keeps the MMAs' operands in uniform registers
   constexpr uint32_t tmem = 0;
+  grid_wait();  // the tables come from constants; everything below reads what the kernels before this one wrote
 
   const int64_t N_out = p.out_dim;
   const int k_blocks = static_cast<int>(p.in_dim / (8 * PF_KBLOCK_CODES));
@@ -728,9 +730,8 @@ static int launch_prefill(const FastProjectionArgs& p, int32_t* status, cudaStre
     if (dev >= 0 && dev < 64) configured |= 1ull << dev;
   }
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  kernel<<<ctas > 0 ? ctas : sms, PF_THREADS, PF_SMEM_BYTES, s>>>(p, x_maps, a_map, b_map, status, stall, wait_ns);
-  KEEPVQ_CHECK_LAUNCH();
-  return KEEPVQ_OK;
+  const cudaError_t err = launch_after(true, kernel, ctas > 0 ? ctas : sms, PF_THREADS, PF_SMEM_BYTES, s, p, x_maps, a_map, b_map, status, stall, wait_ns);
+  return err == cudaSuccess ? KEEPVQ_OK : note_cuda_error(err);
 }
 
 template <int M, bool GLU>
