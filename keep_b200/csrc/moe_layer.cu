@@ -99,12 +99,28 @@ __global__ void __launch_bounds__(256) combine_kernel(const T* __restrict__ down
   for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < total; i += 256ll * gridDim.x) {
     const int64_t t = i / vectors, d = (i - t * vectors) * 8;
     float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < top_k; ++j) {
-      if (served_slot[t * top_k + j] >= static_cast<uint64_t>(slots)) continue;
-      float v[8];
-      load8_as_float<T>(down + (t * top_k + j) * hidden + d, v);
+    // Six at a time: their slots, then their rows, are all in flight together, and are added in pick
+    // order.  (Pick by pick, a slot and then its row, a call of one token waited for twelve reads in turn.)
+    constexpr int AT_ONCE = 6;
+    constexpr int WORDS = 8 * sizeof(T) / 16;
+    for (int j0 = 0; j0 < top_k; j0 += AT_ONCE) {
+      bool live[AT_ONCE];
+      uint4 raw[AT_ONCE][WORDS];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) y[q] += v[q];
+      for (int j = 0; j < AT_ONCE; ++j) live[j] = j0 + j < top_k && served_slot[t * top_k + j0 + j] < static_cast<uint64_t>(slots);
+#pragma unroll
+      for (int j = 0; j < AT_ONCE; ++j)
+#pragma unroll
+        for (int w = 0; w < WORDS; ++w)
+          if (live[j]) raw[j][w] = reinterpret_cast<const uint4*>(down + (t * top_k + j0 + j) * hidden + d)[w];
+#pragma unroll
+      for (int j = 0; j < AT_ONCE; ++j) {
+        if (!live[j]) continue;
+        float v[8];
+        load8_as_float<T>(reinterpret_cast<const T*>(raw[j]), v);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) y[q] += v[q];
+      }
     }
     if (shared) {
       const float4 lo = *reinterpret_cast<const float4*>(shared + t * hidden + d), hi = *reinterpret_cast<const float4*>(shared + t * hidden + d + 4);

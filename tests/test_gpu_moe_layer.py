@@ -55,6 +55,16 @@ def test_small_layer_all_resident(cuda, tokens):
     check_layer(cfg, x, out, routing, top_k=3)
 
 
+@pytest.mark.parametrize("top_k", [1, 6, 7, 13])
+def test_sum_over_picks_in_blocks_of_six(cuda, top_k):
+    """The last kernel reads a token's picks six at a time: fewer, exactly six, and a ragged rest."""
+    cfg = synthetic.layer(seed=6, experts=20, hidden=256, inter=256)
+    x = synthetic.tokens(11, 3, 256)
+    layer = build_layer(cuda, cfg, top_k=top_k)
+    out, routing = layer.decode(x.to(cuda))
+    check_layer(cfg, x, out, routing, top_k=top_k)
+
+
 def test_small_layer_grouped_scales_and_fp16(cuda):
     cfg = synthetic.layer(seed=4, experts=10, hidden=512, inter=256, group_hidden=64, group_inter=128)
     x = synthetic.tokens(9, 4, 512)
