@@ -6,7 +6,7 @@
 // gathers them, as the reference does before its kernels, src/ramp/ops/vq_switch.py:758-761).
 // The sequence is the down projection of the layer call: quantise the rows, group the routes by
 // expert on the device, then the tcgen05 kernel (5 or more routes per expert on average) or the
-// mma.sync one.  Routes need not be sorted; a route with expert 0xFFFFFFFF gives a zero row.
+// mma.sync one; 8-bit codes run on the tcgen05 kernel alone.  Routes need not be sorted; a route with expert 0xFFFFFFFF gives a zero row.
 #include "moe_fast.cuh"
 
 namespace keepvq {

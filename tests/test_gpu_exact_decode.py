@@ -64,7 +64,7 @@ def test_single_projection_kernels_return_scale_times_weight_exactly(cuda, famil
     """The M = 1 (down-shaped) kernels through ``keepvq_grouped_projection``.  The route count and
     the expert count pick the kernel: under 48 routes the sweep kernel ("few" below), from there the
     slab kernel with eight routes per group (many routes per expert) or four (few), and from 1024
-    routes with 24 per expert the tcgen05 kernel."""
+    routes with 5 per expert the tcgen05 kernel."""
     copies = {"few": 1, "slab8": 1, "slab4": 32, "tcgen05": 1}[family]
     codes, scales = all_codes_experts(copies), None
     scales = scales_for(codes.shape[0], 1)

@@ -217,14 +217,24 @@ def test_scale_groups_and_short_groups_on_the_tcgen05_kernels(cuda, tokens, expe
 
 
 def test_many_routes_spread_over_many_experts_stay_on_the_decode_kernels(cuda):
-    """1200 routes over 64 experts (under 24 per expert on average): the mma.sync kernels, with
-    several 8-route groups per expert."""
+    """1200 routes over 64 experts, 19 per expert on average: the tcgen05 kernels' 48-route items.
+    (The mma.sync kernels with several 8-route groups per expert: the next test.)"""
     cfg = synthetic.layer(seed=43, experts=64, hidden=512, inter=256)
     x = synthetic.tokens(44, 400, 512)
     layer = build_layer(cuda, cfg, top_k=3)
     assert layer.kernel_path == "tensor"
     out, routing = layer.decode(x.to(cuda))
     check_layer(cfg, x, out, routing, top_k=3)
+
+
+def test_under_1024_routes_the_decode_kernels_take_several_groups_per_expert(cuda):
+    """1000 routes over 20 experts: too few for the tcgen05 kernels, six 8-route groups per expert."""
+    cfg = synthetic.layer(seed=45, experts=20, hidden=512, inter=256)
+    x = synthetic.tokens(46, 250, 512)
+    layer = build_layer(cuda, cfg, top_k=4)
+    assert layer.kernel_path == "tensor"
+    out, routing = layer.decode(x.to(cuda))
+    check_layer(cfg, x, out, routing, top_k=4)
 
 
 @pytest.mark.parametrize("tokens", [2, 10])
