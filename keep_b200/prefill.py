@@ -12,6 +12,8 @@ else (fp32 activations, odd shapes, custom 16-bit tables with even nibbles) to t
 
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -19,7 +21,7 @@ from .kernels import qmv_output_dtype, routed_matvec
 
 _UNSUPPORTED = -5  # KEEPVQ_ERR_UNSUPPORTED
 _all_odd: dict = {}     # table data_ptr -> (the tensor, its version, every nibble odd): read back once per table, never per call
-_workspaces: dict = {}  # (device, routes, in_dim) -> scratch tensor; the most recent shapes only
+_workspaces: dict = {}  # (device, stream, routes, in_dim) -> scratch tensor, one per stream so that calls may overlap; the most recent only
 _MAX_CACHED = 8
 
 
@@ -49,7 +51,8 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
         return None
     lib = _lib.load()
     device = rows.device
-    key = (str(device), routes, in_dim)
+    stream = torch.cuda.current_stream(device).cuda_stream
+    key = (str(device), stream, routes, in_dim)
     if key not in _workspaces:
         nbytes = int(lib.keepvq_grouped_projection_workspace_bytes(routes, in_dim))
         if nbytes < 0:
@@ -77,7 +80,7 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
         args.res_rows, args.res_groups, args.hot_of_slot = int(res_codes.shape[0]), int(res_scales.shape[2]), _lib.ptr(hot_of_slot)
         keep += [res_codes, res_scales, res_table, hot_of_slot]
     with torch.cuda.device(device):
-        status = lib.keepvq_grouped_projection(args, _lib.stream_handle(device))
+        status = lib.keepvq_grouped_projection(args, ctypes.c_void_p(stream))
     del keep
     if status == _UNSUPPORTED:
         return None

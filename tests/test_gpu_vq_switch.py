@@ -211,6 +211,29 @@ def test_8bit_codes_on_the_tcgen05_kernel(cuda, dtype, routes, experts, out, inp
     assert bool((with_dead[1] == 0).all()) and torch.equal(with_dead[2:], direct[2:])
 
 
+def test_calls_on_two_streams_do_not_share_scratch(cuda):
+    """The same shapes on two streams that may overlap, 8-bit and 16-bit codes: each call's own result."""
+    from keep_b200 import vq, vq_switch
+
+    rng = np.random.default_rng(27)
+    named = dict(input_dims=512, output_dims=1024, group_size=512)
+    streams = [torch.cuda.Stream(cuda) for _ in range(2)]
+    for bits, table in ((8, vq.table_on(cuda, "e8_1bit")), (16, vq.table_on(cuda, "e8p"))):
+        codes = torch.from_numpy(rng.integers(0, 1 << bits, (8, 1024, 64), dtype=np.uint8 if bits == 8 else np.uint16)).to(cuda)
+        scales = torch.full((8, 1024, 1), 0.02, dtype=torch.float16, device=cuda)
+        xs = [torch.from_numpy(rng.normal(size=(64, 512)).astype(np.float32)).to(cuda).to(torch.bfloat16) for _ in range(2)]
+        rhs = [torch.from_numpy(rng.integers(0, 8, (64, 2)).astype(np.int32)).to(cuda) for _ in range(2)]
+        want = [vq_switch.gather_vqmm(xs[i], codes, scales, table, rhs[i], code_bits=bits, **named) for i in range(2)]
+        torch.cuda.synchronize()
+        got = [[], []]
+        for _ in range(20):
+            for i, s in enumerate(streams):
+                with torch.cuda.stream(s):
+                    got[i].append(vq_switch.gather_vqmm(xs[i], codes, scales, table, rhs[i], code_bits=bits, **named))
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i])
+
+
 def test_rows_that_start_inside_an_allocation(cuda):
     """A view whose first row is not on a 16-byte boundary, few routes and many: the same outputs."""
     from keep_b200 import vq, vq_switch
