@@ -389,7 +389,7 @@ constexpr int CHUNK_CODES = 32;               // codewords of a row a warp consu
 bool shapes_supported(int64_t out_dim, int64_t in_dim, int64_t groups) {
   if (in_dim % (8 * CHUNK_CODES) != 0 || groups <= 0) return false;
   const int64_t chunks = in_dim / (8 * CHUNK_CODES);
-  return chunks % groups == 0 && out_dim > 0;
+  return chunks % groups == 0 && in_dim / groups <= MAX_GROUP_INPUTS && out_dim > 0;
 }
 
 // Enough routes to give every CTA of the machine its own (group, slab) items, and activations

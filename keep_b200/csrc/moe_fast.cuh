@@ -20,6 +20,8 @@ constexpr int MAX_GROUP_ROUTES = 8;     // routes of one expert that share an mm
 constexpr int SMALL_CALL_ROUTES = 48;   // calls with fewer routes never run the plain slab kernel
 constexpr int FEW_ROUTE_GROUPS = 96;    // below this many route groups a CTA's warps share rows AND inputs (sweep kernel, split slab kernel)
 constexpr int PAIRED_GROUP_ROUTES = 4;  // ... when a route's two byte planes take a column each (one MMA per step)
+constexpr int64_t MAX_GROUP_INPUTS = 65536;  // inputs of a scale group: sum(x') with |x'| <= 32639 fits the 32 bits it is kept in
+static_assert(32639 * MAX_GROUP_INPUTS < (int64_t{1} << 31), "");
 constexpr int PREFILL_GROUP_ROUTES = 96;   // routes of one expert per tcgen05 item (its accumulators and two operand stages fill tensor memory)
 constexpr int PREFILL_GROUP_ROUTES_SMALL = 48;  // ... for calls with fewer routes per expert, and for rows with several scale groups
 constexpr int PREFILL_FEW_ROUTES_MEAN = 32;     // routes per expert on average up to which a call counts as the former
@@ -241,7 +243,8 @@ struct FastProjectionArgs {
   const uint32_t* res_table;
 };
 
-// True when the shapes fit the tensor-core path (in_dim % 256 == 0, group size % 256 == 0, ...).
+// True when the shapes fit the tensor-core path (in_dim % 256 == 0, group size % 256 == 0, at most
+// MAX_GROUP_INPUTS inputs in a scale group, ...).
 bool shapes_supported(int64_t out_dim, int64_t in_dim, int64_t groups);
 // True when gate_up / down can also add a nested residual with these scale groups to `routes` routes.
 bool residual_supported(int64_t routes, int64_t in_dim, int64_t res_groups);

@@ -58,6 +58,11 @@ constexpr int PF_INFO_WARP = PF_DECODE_WARPS + 3;  // per-route facts
 constexpr int PF_THREADS = (PF_DECODE_WARPS + 4) * 32;  // 640
 constexpr int PF_MAX_SEGMENTS = 32;             // most scale groups of a row
 constexpr int64_t PF_MAX_SEGMENT_INPUTS = 4096; // ... and most inputs of one, where a row has several: sum(4w x') fits 32 bits
+// One scale group per row, |u - 8| <= 8 for any table and |x'| <= 32639: sum(q x') fits 32 bits up to here ...
+constexpr int64_t PF_EXACT32_INPUTS = 8192;
+// ... and the two byte planes' sums and sum(x'), which meet in 64 bits beyond that, up to MAX_GROUP_INPUTS.
+static_assert(8 * 32639 * PF_EXACT32_INPUTS < (int64_t{1} << 31) && 16 * 32639 * PF_MAX_SEGMENT_INPUTS < (int64_t{1} << 31), "");
+static_assert(15 * 128 * MAX_GROUP_INPUTS < (int64_t{1} << 31), "");
 constexpr int PF_ROWS = 128;                    // output rows per tile
 constexpr int PF_KBLOCK_CODES = 16;             // codewords of a row per K block = 128 bytes of int8
 constexpr int PF_A_TILE_COLS = PF_KBLOCK_CODES * 2;   // a decoded K block of one tile: 128 bytes per row = 32 columns
@@ -218,14 +223,16 @@ struct RingPlace {
 // the K blocks) into fp32 sums that the drain warps keep in registers.
 // BITS: 16-bit E8P codes, or 8-bit codes of a table whose word holds dim d in nibble d, value
 // (nibble - 8) / 2.  There a codeword is ONE table read, w = q / 2 without the quarter, and any table
-// will do.
+// will do (the integer sums are bounded for |q| <= 8, not for the shipped table's codewords).
 // `stall` != 0 is the wait self-test: the activation loader never publishes, so the MMA issuer's
 // first wait runs into the deadline.
 // Boxes over the activations, one map per padded number of routes: [2 planes][16 (i + 1) rows][128 bytes].
 template <int N_MAX>
 struct ActivationMaps { CUtensorMap rows[N_MAX / 16]; };
 
-template <int M, bool GLU, int N_MAX, bool GROUPED, int BITS>
+// WIDE: one scale group of more than PF_EXACT32_INPUTS inputs, whose sums meet in 64 bits (as a branch
+// inside the drain that cost the other calls 1 to 2 %).
+template <int M, bool GLU, int N_MAX, bool GROUPED, int BITS, bool WIDE>
 __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastProjectionArgs p, const __grid_constant__ ActivationMaps<N_MAX> x_maps, const __grid_constant__ CUtensorMap a_map,
                                                                            const __grid_constant__ CUtensorMap b_map, int32_t* status, int stall, uint64_t wait_ns) {
   using Plan = PrefillPlan<M, N_MAX, GROUPED, BITS>;
@@ -408,9 +415,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             float y[M];
 #pragma unroll
             for (int mm = 0; mm < M; ++mm) {
-              // 256 high + low - 8 sum(x') in wrapping 32-bit arithmetic: the true value, sum(q x'), fits
-              const int dot = static_cast<int>(v[mm][0][j] * 256u + v[mm][1][j] - offset);
-              y[mm] = scale[mm] * x_scale * (0.5f * static_cast<float>(dot) + x_sum4);
+              // 256 high + low - 8 sum(x') = sum(q x'), in wrapping 32-bit arithmetic where the true value fits that
+              const float dot = WIDE ? static_cast<float>(256 * static_cast<int64_t>(static_cast<int>(v[mm][0][j])) + static_cast<int>(v[mm][1][j]) - 8 * static_cast<int64_t>(pr.z))
+                                     : static_cast<float>(static_cast<int>(v[mm][0][j] * 256u + v[mm][1][j] - offset));
+              y[mm] = scale[mm] * x_scale * (0.5f * dot + x_sum4);
             }
             finish_column(pr, y, round_out, store_out);
           }
@@ -711,8 +719,8 @@ static int code_map(const FastProjectionArgs& p, const void* codes, int bits, ui
   return byte_map(map, codes, p.in_dim / 8 * (bits / 8), p.slots * p.out_dim, 1, 2 * PF_KBLOCK_CODES * bits / 8, box_rows, bits == 16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-template <int M, bool GLU, int N_MAX, bool GROUPED, int BITS = 16>
-static int launch_prefill(const FastProjectionArgs& p, int32_t* status, cudaStream_t s, int stall = 0, uint64_t wait_ns = 0, int ctas = 0) {
+template <int M, bool GLU, int N_MAX, bool GROUPED, int BITS, bool WIDE>
+static int launch_prefill_kernel(const FastProjectionArgs& p, int32_t* status, cudaStream_t s, int stall = 0, uint64_t wait_ns = 0, int ctas = 0) {
   ActivationMaps<N_MAX> x_maps;  // the quantised activations: the high-byte plane, then the low-byte plane, each [rows + 1, in_dim]
   for (int i = 0; i < N_MAX / 16; ++i)
     if (const int rc = byte_map(&x_maps.rows[i], p.x.q, p.in_dim, p.x_zero_row + 1, 2, 128, 16 * (i + 1), CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
@@ -721,7 +729,7 @@ static int launch_prefill(const FastProjectionArgs& p, int32_t* status, cudaStre
   if (GLU) {
     if (const int rc = code_map(p, p.b.codes, BITS, PF_ROWS, &b_map)) return rc;
   } else b_map = a_map;
-  auto kernel = prefill_projection_kernel<M, GLU, N_MAX, GROUPED, BITS>;
+  auto kernel = prefill_projection_kernel<M, GLU, N_MAX, GROUPED, BITS, WIDE>;
   static uint64_t configured = 0;  // one bit per device: the shared-memory opt-in is a per-device attribute of the function
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -733,6 +741,12 @@ static int launch_prefill(const FastProjectionArgs& p, int32_t* status, cudaStre
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const cudaError_t err = launch_after(true, kernel, ctas > 0 ? ctas : sms, PF_THREADS, PF_SMEM_BYTES, s, p, x_maps, a_map, b_map, status, stall, wait_ns);
   return err == cudaSuccess ? KEEPVQ_OK : note_cuda_error(err);
+}
+
+template <int M, bool GLU, int N_MAX, bool GROUPED, int BITS = 16>
+static int launch_prefill(const FastProjectionArgs& p, int32_t* status, cudaStream_t s, int stall = 0, uint64_t wait_ns = 0, int ctas = 0) {
+  if (!GROUPED && p.in_dim > PF_EXACT32_INPUTS) return launch_prefill_kernel<M, GLU, N_MAX, GROUPED, BITS, !GROUPED>(p, status, s, stall, wait_ns, ctas);
+  return launch_prefill_kernel<M, GLU, N_MAX, GROUPED, BITS, false>(p, status, s, stall, wait_ns, ctas);
 }
 
 template <int M, bool GLU>

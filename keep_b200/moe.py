@@ -195,7 +195,7 @@ class RoutedMoELayer:
         residual tier the inputs may be at most 6144 wide (the residual pass lives in the slab
         kernels, whose split form for small calls keeps 48 KB of activations in shared memory);
         wider layers with a residual tier run the general kernels."""
-        ok = lambda inp, groups: inp % 256 == 0 and (inp // 256) % groups == 0  # noqa: E731
+        ok = lambda inp, groups: inp % 256 == 0 and (inp // 256) % groups == 0 and inp // groups <= 65536  # noqa: E731
         fits = ok(self.hidden, int(self.w1.scales.shape[2])) and ok(self.inter, int(self.w2.scales.shape[2]))
         if self.res_rows:
             tiers = (self.w1, self.w3, self.w2)

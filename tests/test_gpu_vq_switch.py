@@ -211,6 +211,29 @@ def test_8bit_codes_on_the_tcgen05_kernel(cuda, dtype, routes, experts, out, inp
     assert bool((with_dead[1] == 0).all()) and torch.equal(with_dead[2:], direct[2:])
 
 
+@pytest.mark.parametrize("bits,inp,word,code", [
+    (8, 8192, 0x00000000, 0), (8, 8704, 0x00000000, 0), (8, 66560, 0x00000000, 0),  # every weight -4
+    (16, 8192, 0x11111111, 0), (16, 10240, 0x11111111, 0),  # an all-odd table: every weight -3.25
+    (16, 66560, 0x11111111, 0),  # wider than the tcgen05 kernel's sums: another kernel takes it
+])
+def test_wide_rows_keep_their_integer_sums(cuda, bits, inp, word, code):
+    """The largest sums a caller's own table allows: constant rows against constant weights.  From
+    8257 inputs on 8 * 32,512 * inputs passes 32 bits, from 66,053 on sum(x') itself."""
+    from keep_b200 import vq_switch
+
+    routes, out = 1024, 32
+    table = np.full(256, word, dtype=np.uint32)
+    codes = np.full((1, out, inp // 8), code, dtype=np.uint8 if bits == 8 else np.uint16)
+    scales = np.full((1, out, 1), 2.0 ** -12, dtype=np.float16)
+    weight = ops.dense_experts(codes[:, :1], scales[:, :1], code_bits=bits, codebook=table, dtype=np.float64)[0, 0]
+    value = 127 / 64  # 32,512 steps of 2^-14: a bf16 value near the top of the fixed-point range (32,639)
+    x = torch.full((routes, inp), value, dtype=torch.bfloat16, device=cuda)
+    got = vq_switch.gather_vqmm(x, torch.from_numpy(codes).to(cuda), torch.from_numpy(scales).to(cuda), torch.from_numpy(table.view(np.int32)).to(cuda),
+                                torch.zeros((routes, 1), dtype=torch.int32, device=cuda), input_dims=inp, output_dims=out, group_size=inp, code_bits=bits)
+    want = np.full((routes, 1, out), weight.sum() * value)
+    np.testing.assert_allclose(f32(got), want, rtol=2.0 ** -8)  # exact sums, one rounding to bf16
+
+
 def test_calls_on_two_streams_do_not_share_scratch(cuda):
     """The same shapes on two streams that may overlap, 8-bit and 16-bit codes: each call's own result."""
     from keep_b200 import vq, vq_switch
