@@ -13,6 +13,7 @@ else (fp32 activations, odd shapes, custom 16-bit tables with even nibbles) to t
 from __future__ import annotations
 
 import ctypes
+from functools import lru_cache
 
 import torch
 
@@ -21,7 +22,6 @@ from .kernels import qmv_output_dtype, routed_matvec
 
 _UNSUPPORTED = -5  # KEEPVQ_ERR_UNSUPPORTED
 _all_odd: dict = {}     # table data_ptr -> (the tensor, its version, every nibble odd): read back once per table, never per call
-_workspaces: dict = {}  # (device, stream, routes, in_dim) -> scratch tensor, one per stream so that calls may overlap; the most recent only
 _MAX_CACHED = 8
 
 
@@ -39,6 +39,14 @@ def _table_all_odd(table: torch.Tensor) -> bool:
     return _all_odd[key][2]
 
 
+@lru_cache(maxsize=256)
+def _scratch_bytes(routes: int, in_dim: int) -> int:
+    nbytes = int(_lib.load().keepvq_grouped_projection_workspace_bytes(routes, in_dim))
+    if nbytes < 0:
+        _lib.check(nbytes, "keepvq_grouped_projection_workspace_bytes")
+    return nbytes
+
+
 def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, code_bits: int = 16, residual=None, hot_of_slot=None):
     """``keepvq_grouped_projection``: route ``r`` against activation row ``r // x_div`` of ``rows``
     (fp16 / bf16), optionally with a nested residual ``(res_codes, res_scales, res_table)``.
@@ -52,15 +60,10 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
     lib = _lib.load()
     device = rows.device
     stream = torch.cuda.current_stream(device).cuda_stream
-    key = (str(device), stream, routes, in_dim)
-    if key not in _workspaces:
-        nbytes = int(lib.keepvq_grouped_projection_workspace_bytes(routes, in_dim))
-        if nbytes < 0:
-            _lib.check(nbytes, "keepvq_grouped_projection_workspace_bytes")
-        if len(_workspaces) >= _MAX_CACHED:  # varying route counts must not pile up scratch
-            _workspaces.pop(next(iter(_workspaces)))
-        _workspaces[key] = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    ws = _workspaces[key]
+    nbytes = _scratch_bytes(routes, in_dim)
+    # Scratch of this call alone, from the caching allocator: calls of other threads, of other streams
+    # and of other captured graphs have their own, and a graph's stays the graph's.
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     out_dtype = qmv_output_dtype(rows.dtype)
     out = torch.empty((routes, out_dim), dtype=out_dtype, device=device)
     rows, rhs = rows.contiguous(), rhs.to(torch.int32).contiguous()

@@ -257,6 +257,60 @@ def test_calls_on_two_streams_do_not_share_scratch(cuda):
         assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i])
 
 
+def _calls_of_one_shape(cuda, count):
+    """``count`` argument lists of one shape (100 tokens of top-2 over 8 experts) with inputs of their own, and their results."""
+    from keep_b200 import vq, vq_switch
+
+    rng = np.random.default_rng(28)
+    table = vq.table_on(cuda, "e8p")
+    codes = torch.from_numpy(rng.integers(0, 1 << 16, (8, 1024, 64), dtype=np.uint16)).to(cuda)
+    scales = torch.full((8, 1024, 1), 0.02, dtype=torch.float16, device=cuda)
+    named = dict(input_dims=512, output_dims=1024, group_size=512, code_bits=16)
+    calls = []
+    for _ in range(count):
+        x = torch.from_numpy(rng.normal(size=(100, 512)).astype(np.float32)).to(cuda).to(torch.bfloat16)
+        rhs = torch.from_numpy(rng.integers(0, 8, (100, 2)).astype(np.int32)).to(cuda)
+        calls.append(lambda x=x, rhs=rhs: vq_switch.gather_vqmm(x, codes, scales, table, rhs, **named))
+    want = [call() for call in calls]
+    torch.cuda.synchronize()
+    return calls, want
+
+
+def test_two_host_threads_on_one_stream_do_not_share_scratch(cuda):
+    """Threads start on the same (default) stream; each call's launches may fall between another's."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    calls, want = _calls_of_one_shape(cuda, 2)
+    with ThreadPoolExecutor(2) as pool:
+        got = list(pool.map(lambda i: [calls[i]() for _ in range(200)], range(2)))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i])
+
+
+def test_captured_graphs_of_one_shape_replay_side_by_side(cuda):
+    """Two graphs captured one after the other (torch captures both on one stream), replayed on two
+    streams with calls of many other shapes in between."""
+    from keep_b200 import kernels
+
+    calls, want = _calls_of_one_shape(cuda, 2)
+    graphs, outs = [], []
+    for call in calls:
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            outs.append([call() for _ in range(10)])
+    codes, scales = torch.zeros((64, 32), dtype=torch.uint16, device=cuda), torch.ones((64, 1), dtype=torch.float16, device=cuda)
+    for rows in range(50, 70):
+        kernels.vq_qmm(torch.ones((rows, 256), dtype=torch.bfloat16, device=cuda), codes, scales, in_dim=256, out_dim=64, group_size=256, code_bits=16)
+    streams = [torch.cuda.Stream(cuda) for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(10):
+        for s, g in zip(streams, graphs):
+            with torch.cuda.stream(s):
+                g.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i]) for i in range(2) for y in outs[i])
+
+
 def test_rows_that_start_inside_an_allocation(cuda):
     """A view whose first row is not on a 16-byte boundary, few routes and many: the same outputs."""
     from keep_b200 import vq, vq_switch

@@ -1,0 +1,35 @@
+"""Scratch of the operators' grouped kernels: every call has its own (host logic, no GPU)."""
+
+import contextlib
+import ctypes
+from types import SimpleNamespace
+
+import torch
+
+
+def test_calls_in_flight_together_do_not_share_scratch(monkeypatch):
+    """A second call of the same shape on the same stream, made while the first is still enqueueing
+    its launches (another host thread: the library call releases the interpreter lock), must not
+    be handed the first one's scratch.  The library is a stand-in that makes that second call."""
+    from keep_b200 import _lib, prefill
+
+    nbytes, seen = 4096, []
+    rows = torch.zeros((2, 256), dtype=torch.bfloat16)
+    codes, scales = torch.zeros((1, 32, 32), dtype=torch.uint16), torch.ones((1, 32, 1), dtype=torch.float16)
+    table, rhs = torch.full((256,), 0x11111111, dtype=torch.int32), torch.zeros(2, dtype=torch.int32)
+
+    def project(args, stream):
+        first = not seen
+        seen.append(ctypes.cast(args.workspace, ctypes.c_void_p).value)
+        assert args.workspace_bytes >= nbytes
+        if first:
+            assert prefill.tensor_core_projection(rows, codes, scales, table, rhs) is not None
+        return 0
+
+    fake = SimpleNamespace(keepvq_grouped_projection=project)
+    monkeypatch.setattr(_lib, "load", lambda: fake)
+    monkeypatch.setattr(prefill, "_scratch_bytes", lambda routes, in_dim: nbytes)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: SimpleNamespace(cuda_stream=0))
+    monkeypatch.setattr(torch.cuda, "device", lambda device: contextlib.nullcontext())
+    prefill.tensor_core_projection(rows, codes, scales, table, rhs)
+    assert len(seen) == 2 and abs(seen[0] - seen[1]) >= nbytes
