@@ -13,6 +13,7 @@ else (fp32 activations, odd shapes, custom 16-bit tables with even nibbles) to t
 from __future__ import annotations
 
 import ctypes
+import threading
 from functools import lru_cache
 
 import torch
@@ -21,22 +22,27 @@ from . import _lib
 from .kernels import qmv_output_dtype, routed_matvec
 
 _UNSUPPORTED = -5  # KEEPVQ_ERR_UNSUPPORTED
-_all_odd: dict = {}     # table data_ptr -> (the tensor, its version, every nibble odd): read back once per table, never per call
+_all_odd: dict = {}     # table data_ptr, device -> (the tensor, its version, every nibble odd): read back once per table, never per call
+_all_odd_lock = threading.Lock()  # of the entries' insertion and eviction
 _MAX_CACHED = 8
 
 
 def _table_all_odd(table: torch.Tensor) -> bool:
     """Whether every nibble of the table is odd (what the int8 kernels need).  The cache holds the
     tensor itself, so its address cannot be handed to another table while the entry lives, and an
-    in-place change of the table (a new version) is looked at again."""
-    key = (table.data_ptr(), str(table.device))
+    in-place change of the table (a new version) is looked at again.  Another thread may drop the
+    entry at any time: the answer comes from what was looked up or worked out here."""
+    key = (table.data_ptr(), table.get_device())
     hit = _all_odd.get(key)
     if hit is None or hit[0] is not table or hit[1] != table._version:
+        version = table._version
         nibbles = (table.cpu().to(torch.int64) & 0xFFFFFFFF)[:, None] >> (4 * torch.arange(8))[None] & 1
-        if len(_all_odd) >= _MAX_CACHED:
-            _all_odd.pop(next(iter(_all_odd)))
-        _all_odd[key] = (table, table._version, bool(nibbles.all()))
-    return _all_odd[key][2]
+        hit = (table, version, bool(nibbles.all()))
+        with _all_odd_lock:
+            if len(_all_odd) >= _MAX_CACHED and key not in _all_odd:
+                _all_odd.pop(next(iter(_all_odd)))
+            _all_odd[key] = hit
+    return hit[2]
 
 
 @lru_cache(maxsize=256)

@@ -33,3 +33,17 @@ def test_calls_in_flight_together_do_not_share_scratch(monkeypatch):
     monkeypatch.setattr(torch.cuda, "device", lambda device: contextlib.nullcontext())
     prefill.tensor_core_projection(rows, codes, scales, table, rhs)
     assert len(seen) == 2 and abs(seen[0] - seen[1]) >= nbytes
+
+
+def test_the_answer_about_a_table_survives_an_eviction(monkeypatch):
+    """Whether a table's nibbles are all odd is remembered for a few tables; another thread may evict
+    the entry between its insertion and the answer."""
+    from keep_b200 import prefill
+
+    class Forgetful(dict):
+        def __setitem__(self, key, value):
+            pass
+
+    monkeypatch.setattr(prefill, "_all_odd", Forgetful())
+    assert prefill._table_all_odd(torch.full((256,), 0x11111111, dtype=torch.int32)) is True
+    assert prefill._table_all_odd(torch.full((256,), 0x11111112, dtype=torch.int32)) is False
