@@ -554,12 +554,14 @@ int keepvq_moe_decode_layer_static(const keepvq_moe_layer_args* args, void* stre
 
 /* ------------------------------------------------------------------------------------------
  * Self-test of the bounded waits of the tcgen05 kernels.  Runs one thread block of the prefill
- * projection kernel on a tiny problem laid out inside `workspace`, with the producers of its
- * activation tiles told never to publish.  The consumer's wait must run into its deadline
- * (`wait_ns` nanoseconds on the GPU's global timer, at most one second), after which the block
- * writes 1 into the first int32 of `workspace`, releases its tensor memory and returns; the
- * device stays usable.  A host checks that word after synchronising.  No counterpart in the
- * reference.
+ * projection kernel on a tiny problem laid out inside `workspace`, with one of its loaders told
+ * never to publish: first the activations of the form for rows with one scale group (a wait must
+ * run into its deadline, `wait_ns` nanoseconds on the GPU's global timer, at most one second),
+ * then the codes of the forms for rows with several scale groups and for 8-bit codes, whose
+ * activation copies are in flight when they give up (at most 5 ms each).  Run i writes 1 into the
+ * i-th int32 of `workspace`, waits for its copies, releases its tensor memory and returns; the
+ * device stays usable.  A host checks those three words after synchronising.  No counterpart in
+ * the reference.
  * ------------------------------------------------------------------------------------------ */
 int64_t keepvq_wait_selftest_workspace_bytes(void);
 int keepvq_wait_selftest(void* workspace, int64_t workspace_bytes, int64_t wait_ns, void* stream);

@@ -7,6 +7,8 @@
 // The sequence is the down projection of the layer call: quantise the rows, group the routes by
 // expert on the device, then the tcgen05 kernel (5 or more routes per expert on average) or the
 // mma.sync one; 8-bit codes run on the tcgen05 kernel alone.  Routes need not be sorted; a route with expert 0xFFFFFFFF gives a zero row.
+#include <algorithm>
+
 #include "moe_fast.cuh"
 
 namespace keepvq {
@@ -113,14 +115,15 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
 }
 
 // ------------------------------------------------------------------------------------------
-// Self-test of the bounded waits of the tcgen05 kernel: one CTA on a tiny problem laid out in the
-// caller's scratch, whose activation loaders never publish their tiles.  The MMA issuer's first
-// wait then runs into its deadline (wait_ns on the global timer); the CTA must set the status
-// word to 1, free its tensor memory and return, and the context must stay usable.  Nothing
-// faults and nothing spins without a limit.  No counterpart in the reference.
+// Self-test of the bounded waits of the tcgen05 kernel: runs of one CTA on a tiny problem laid out in
+// the caller's scratch, one of whose loaders never publishes its tiles.  A wait then runs into its
+// deadline (on the global timer); the CTA must set its status word to 1, wait for what the other
+// loader still has in flight, free its tensor memory and return, and the context must stay usable.
+// Nothing faults and nothing spins without a limit.  No counterpart in the reference.
 // ------------------------------------------------------------------------------------------
 namespace keepvq {
-constexpr int64_t SELFTEST_BYTES = 32 * 1024;
+constexpr int64_t SELFTEST_BYTES = 192 * 1024;
+constexpr int64_t SELFTEST_SHORT_NS = 5000000;  // the runs behind the first take no longer than this each
 __global__ void selftest_init_kernel(int32_t* count, int32_t* size, int32_t* routes, float* x_scale) {
   if (threadIdx.x == 0) { count[0] = 1; size[0] = 16; }
   if (threadIdx.x < 16) routes[threadIdx.x] = threadIdx.x;
@@ -135,22 +138,30 @@ extern "C" int keepvq_wait_selftest(void* workspace, int64_t workspace_bytes, in
   if (!workspace) return KEEPVQ_ERR_NULL;
   if (workspace_bytes < SELFTEST_BYTES) return KEEPVQ_ERR_CAPACITY;
   if (!aligned_to(workspace, 256)) return KEEPVQ_ERR_ALIGN;
-  if (wait_ns <= 0 || wait_ns > 1000000000ll) return KEEPVQ_ERR_SHAPE;  // a self-test may hold the GPU for a second at most
+  if (wait_ns <= 0 || wait_ns > 1000000000ll) return KEEPVQ_ERR_SHAPE;  // a self-test may hold the GPU for about a second at most
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* ws = reinterpret_cast<char*>(workspace);
+  int32_t* status = reinterpret_cast<int32_t*>(ws);
   cudaError_t e = cudaMemsetAsync(ws, 0, SELFTEST_BYTES, s);
   if (e != cudaSuccess) return note_cuda_error(e);
-  // status 0 | groups 256.. | routes 1280 | table 2048 | scales 3072 | codes 4096 | planes 12288 | x scale 21248 | x sums 21504 | out 22528
+  // status words 0 | groups 256.. | routes 1280 | table 2048 | x scale 3072 | x sums 4096 | scales 8192 | out 16384 | planes 32768 | codes 65536
   fast::RouteGroups groups = {reinterpret_cast<int32_t*>(ws + 256), reinterpret_cast<int32_t*>(ws + 512), reinterpret_cast<int32_t*>(ws + 768),
                               reinterpret_cast<int32_t*>(ws + 1024), reinterpret_cast<int32_t*>(ws + 1280)};
-  fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + 12288), reinterpret_cast<float*>(ws + 21248), reinterpret_cast<int32_t*>(ws + 21504), nullptr};
+  fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + 32768), reinterpret_cast<float*>(ws + 3072), reinterpret_cast<int32_t*>(ws + 4096), nullptr};
   selftest_init_kernel<<<1, 32, 0, s>>>(groups.count, groups.size, groups.routes, xq.scale);
   KEEPVQ_CHECK_LAUNCH();
   fast::FastProjectionArgs p = {};
-  p.a = {reinterpret_cast<const uint16_t*>(ws + 4096), ws + 3072, nullptr, nullptr};
-  p.scales_dtype = KEEPVQ_F16; p.slots = 1; p.out_dim = 128; p.in_dim = 256; p.groups = 1;
+  p.a = {reinterpret_cast<const uint16_t*>(ws + 65536), ws + 8192, nullptr, nullptr};
+  p.scales_dtype = KEEPVQ_F16; p.slots = 1; p.in_dim = 512;  // two planes of 17 rows of 512 inputs
   p.codebook = reinterpret_cast<const uint32_t*>(ws + 2048);
-  p.x = xq; p.x_zero_row = 16; p.x_div = 1; p.groups_of_routes = groups; p.max_routes = 16; p.group_cols = fast::PREFILL_GROUP_ROUTES;
-  p.out = ws + 22528; p.out_dtype = KEEPVQ_BF16;
-  return fast::prefill_wait_selftest(p, reinterpret_cast<int32_t*>(ws), static_cast<uint64_t>(wait_ns), s);
+  p.x = xq; p.x_zero_row = 16; p.x_div = 1; p.groups_of_routes = groups; p.max_routes = 16;
+  p.out = ws + 16384; p.out_dtype = KEEPVQ_BF16;
+  for (int form = 0; form < 3; ++form) {
+    p.out_dim = form == 0 ? 128 : 512;  // (the other forms take 256 rows an item: two items)
+    p.groups = form == 1 ? 2 : 1;
+    p.group_cols = form == 0 ? fast::PREFILL_GROUP_ROUTES : fast::PREFILL_GROUP_ROUTES_SMALL;
+    const int rc = fast::prefill_wait_selftest(form, p, status + form, static_cast<uint64_t>(form == 0 ? wait_ns : std::min(wait_ns, SELFTEST_SHORT_NS)), s);
+    if (rc) return rc;
+  }
+  return KEEPVQ_OK;
 }

@@ -313,8 +313,8 @@ int prefill_group_routes(int64_t live, int64_t slots, bool several_groups);
 int prefill_gate_up(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);
 int prefill_down(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);
 int prefill_byte_codes(const FastProjectionArgs& args, int32_t* status, cudaStream_t s);
-// One CTA whose activation loaders never publish, with a deadline of wait_ns: the wait runs out, the CTA sets *status = 1 and returns.
-int prefill_wait_selftest(const FastProjectionArgs& args, int32_t* status, uint64_t wait_ns, cudaStream_t s);
+// One CTA one of whose loaders never publishes, with a deadline of wait_ns: the wait runs out, the CTA sets *status = 1 and returns.
+int prefill_wait_selftest(int form, const FastProjectionArgs& args, int32_t* status, uint64_t wait_ns, cudaStream_t s);
 
 }  // namespace fast
 }  // namespace keepvq

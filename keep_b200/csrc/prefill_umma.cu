@@ -42,7 +42,7 @@
 //   warp  19     gathers what the drain needs per route (route id, activation scale and sums, gate weight).
 // mbarrier full/empty pairs carry every dependency.  Every wait is bounded by a deadline on the
 // global timer: on expiry the CTA raises a flag in `status`, stops issuing work, waits (bounded)
-// for the MMAs in flight, frees its tensor memory and returns.
+// for the MMAs and the copies in flight, frees its tensor memory and returns.
 #include <cuda.h>  // CUtensorMap (types only: the one driver entry point is looked up through the runtime)
 
 #include "moe_fast.cuh"
@@ -124,9 +124,16 @@ __device__ __forceinline__ uint32_t elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
   return chosen;
 }
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // One arrival for the warp, predicated instead of a branch.
 __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar, int lane) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
+}
+__device__ __forceinline__ bool mbar_complete(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
 }
 // Wait of a whole warp, bounded by time.  Returns false (in every lane) when the deadline passes (the
 // caller's CTA then gives up: the flag is raised for every role) or when another warp of the CTA
@@ -135,10 +142,7 @@ __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar, int lane) {
 template <bool RELAXED = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t deadline, volatile int* abort_flag) {
   for (uint32_t spin = 0;; ++spin) {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (__all_sync(0xFFFFFFFFu, done)) return true;
+    if (__all_sync(0xFFFFFFFFu, mbar_complete(bar, parity))) return true;
     if (RELAXED) __nanosleep(160);
     if ((spin & 31u) == 31u) {
       if (__any_sync(0xFFFFFFFFu, *abort_flag)) return false;
@@ -154,16 +158,29 @@ __device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_o
 __device__ __forceinline__ void mbar_wait_grace(uint32_t bar, uint32_t parity) {
   const uint64_t grace = global_timer_ns() + 100000000ull;
   for (uint32_t spin = 0; spin < (1u << 22); ++spin) {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done || ((spin & 31u) == 31u && global_timer_ns() > grace)) return;
+    if (mbar_complete(bar, parity) || ((spin & 31u) == 31u && global_timer_ns() > grace)) return;
   }
 }
-// A loader that gives up waits for the copies it has issued (`used` stage fills so far) before the CTA's shared memory goes.
+// A CTA that gives up waits for the copies of its code loader (`used` stage fills) before its shared memory goes.
 template <uint32_t STAGES>
-__device__ __forceinline__ void wait_copies_landed(uint32_t full_bars, uint32_t used) {
+__device__ __forceinline__ void wait_codes_landed(uint32_t full_bars, uint32_t used) {
   for (uint32_t i = used > STAGES ? used - STAGES : 0; i < used; ++i) mbar_wait_grace(full_bars + 8u * (i % STAGES), (i / STAGES) & 1u);
+}
+// ... and for those of its activation loader (`used` K blocks).  A K block's barrier also counts the
+// decode warps that fill its A stage, so the arrivals they did not come to make are made for them:
+// place[w] is where decode warp w stopped, its next K block modulo 2 STAGES.  A K block whose barrier
+// is not complete has not been read, so no decode warp is as far as STAGES beyond it, none STAGES behind.
+template <uint32_t STAGES>
+__device__ __forceinline__ void wait_activations_landed(uint32_t full_bars, uint32_t used, const uint32_t* place, int decode_warps) {
+  for (uint32_t i = used > STAGES ? used - STAGES : 0; i < used; ++i) {
+    const uint32_t bar = full_bars + 8u * (i % STAGES), phase = (i / STAGES) & 1u;
+    if (mbar_complete(bar, phase)) continue;
+    for (int w = 0; w < decode_warps; ++w) {
+      const uint32_t ahead = (place[w] + 2 * STAGES - i % (2 * STAGES)) % (2 * STAGES);  // its next K block less this one
+      if (((static_cast<uint32_t>(w) >> 2) & 1u) == (i & 1u) && (ahead == 0 || ahead > STAGES)) mbar_arrive(bar);
+    }
+    mbar_wait_grace(bar, phase);
+  }
 }
 
 // K-major SWIZZLE_128B operand tile: rows of 128 bytes, 8-row groups 1024 bytes apart.
@@ -224,8 +241,8 @@ struct RingPlace {
 // BITS: 16-bit E8P codes, or 8-bit codes of a table whose word holds dim d in nibble d, value
 // (nibble - 8) / 2.  There a codeword is ONE table read, w = q / 2 without the quarter, and any table
 // will do (the integer sums are bounded for |q| <= 8, not for the shipped table's codewords).
-// `stall` != 0 is the wait self-test: the activation loader never publishes, so the MMA issuer's
-// first wait runs into the deadline.
+// `stall` != 0 is the wait self-test: a loader never publishes, and a wait runs into the deadline.
+enum { STALL_ACTIVATIONS = 1, STALL_CODES = 2 };
 // Boxes over the activations, one map per padded number of routes: [2 planes][16 (i + 1) rows][128 bytes].
 template <int N_MAX>
 struct ActivationMaps { CUtensorMap rows[N_MAX / 16]; };
@@ -247,6 +264,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   static_assert(N_BARS * 8 <= 1024, "");
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ uint32_t decode_place[PF_DECODE_WARPS], codes_issued, activations_issued;  // where the roles stopped
   __shared__ int4 route_info[PF_INFO_BUFFERS][N_MAX];  // per item (three in flight): route, x scale, x sum (one scale group only), gate weight
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   auto bar = [](int which, uint32_t index) { return PF_BARS + 8u * (static_cast<uint32_t>(which) + index); };
@@ -512,6 +530,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       }
     }
     if (pending && ok) drain();
+    if (lane == 0) decode_place[warp] = (freed.phase * B_STAGES + freed.index + A_STAGES - 2 * fresh) % (2 * B_STAGES);  // its next K block
   } else if (warp == PF_MMA_WARP) {
     // ================= the MMAs ================================================================
     // One loop over all K blocks of the block's items, unrolled over the stage ring: this warp's own
@@ -588,7 +607,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       for (int kb = 0; kb < k_blocks; ++kb) {
         ok = mbar_wait<true>(bar(STAGE_EMPTY, b.index), b.phase ^ 1u, deadline, aborted);
         if (!ok) break;
-        if (!stall) {  // (the wait self-test: nothing is ever published)
+        if (stall != STALL_ACTIVATIONS) {
           if (elect_one()) {
             mbar_expect_tx(bar(STAGE_FULL, b.index), static_cast<uint32_t>(2 * n_pad * 128));
             tma_box_3d(Plan::b_stage(b.index), map, kb * 128, gstart, 0, bar(STAGE_FULL, b.index));
@@ -598,8 +617,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         b.advance();
       }
     }
-    // (a stage's barrier also waits for the decode warps, so here the copies just get the time they need at most)
-    if (*aborted && used) __nanosleep(1000000);
+    if (lane == 0) activations_issued = used;
   } else if (warp == PF_CODE_WARP) {
     // ================= code loader: TMA ======================================================
     // Two K blocks of every tile per stage, straight from the caller's
@@ -614,6 +632,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       for (int u = 0; u < code_units; ++u) {
         ok = mbar_wait<true>(bar(CODE_EMPTY, code.index), code.phase ^ 1u, deadline, aborted);
         if (!ok) break;
+        if (stall == STALL_CODES) continue;
         if (elect_one()) {
           const uint32_t full = bar(CODE_FULL, code.index);
           mbar_expect_tx(full, Plan::CODE_STAGE_BYTES);
@@ -624,7 +643,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         code.advance();
       }
     }
-    if (*aborted) wait_copies_landed<CODE_STAGES>(bar(CODE_FULL, 0), used);
+    if (lane == 0) codes_issued = used;
   }
 
   if (warp == PF_INFO_WARP) {
@@ -663,14 +682,17 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   }
 
   // ---- teardown ------------------------------------------------------------------------------
-  __syncwarp();
+  __syncthreads();  // every role has left its loop: nothing is issued any more, and the flag is what it will be
   if (*aborted) {
     if (tid == 0 && status) atomicExch(status, set_up_ok ? 1 : 2);
-    // MMAs may still be in flight: one more commit arrives when they are all done; wait for it, bounded as every wait
+    // What may still be in flight is waited for, bounded as every wait: MMAs (one more commit arrives
+    // when they are all done), codes, activations.
     if (warp == PF_MMA_WARP && mma_issued && elect_one()) {  // the lane that issued: a commit follows its own thread's MMAs
       umma_commit(bar(DRAINED, 0));
       mbar_wait_grace(bar(DRAINED, 0), 0u);
     }
+    if (warp == PF_CODE_WARP && lane == 0) wait_codes_landed<CODE_STAGES>(bar(CODE_FULL, 0), codes_issued);
+    if (warp == PF_B_WARP && lane == 0) wait_activations_landed<B_STAGES>(bar(STAGE_FULL, 0), activations_issued, decode_place, M * 8);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -765,10 +787,13 @@ int prefill_byte_codes(const FastProjectionArgs& p, int32_t* status, cudaStream_
   if (p.groups > 1) return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, true, 8>(p, status, s);
   return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, false, 8>(p, status, s);
 }
-// One CTA of the single-projection kernel whose activation loader never publishes, with a short
-// deadline: the wait runs out, the CTA reports and returns.  `p` must describe a valid problem.
-int prefill_wait_selftest(const FastProjectionArgs& p, int32_t* status, uint64_t wait_ns, cudaStream_t s) {
-  return launch_prefill<1, false, PREFILL_GROUP_ROUTES, false>(p, status, s, 1, wait_ns, 1);
+// One CTA of a single-projection kernel, one of whose loaders never publishes, with a short deadline:
+// a wait runs out, the CTA reports and returns.  `p` must describe a valid problem.
+// 0: the 96-route form without activations; 1: the scale-group form without codes; 2: the 8-bit form without codes.
+int prefill_wait_selftest(int form, const FastProjectionArgs& p, int32_t* status, uint64_t wait_ns, cudaStream_t s) {
+  if (form == 1) return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, true>(p, status, s, STALL_CODES, wait_ns, 1);
+  if (form == 2) return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, false, 8>(p, status, s, STALL_CODES, wait_ns, 1);
+  return launch_prefill<1, false, PREFILL_GROUP_ROUTES, false>(p, status, s, STALL_ACTIVATIONS, wait_ns, 1);
 }
 
 }  // namespace fast

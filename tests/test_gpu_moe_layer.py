@@ -284,6 +284,32 @@ def test_a_wait_that_nothing_satisfies_runs_out_and_the_kernel_returns(cuda):
     assert lib.keepvq_wait_selftest(_lib.ptr(ws), nbytes, 0, _lib.stream_handle(cuda)) == -2  # a deadline is mandatory (and at most a second)
 
 
+def _wait_selftest(cuda):
+    """The self-test's words, and the milliseconds its runs took."""
+    from keep_b200 import _lib
+
+    lib = _lib.load()
+    nbytes = int(lib.keepvq_wait_selftest_workspace_bytes())
+    ws = torch.full((nbytes,), 0x5A, dtype=torch.uint8, device=cuda)
+    for _ in range(2):  # the first call also loads the kernels
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        with torch.cuda.device(cuda):
+            start.record()
+            _lib.check(lib.keepvq_wait_selftest(_lib.ptr(ws), nbytes, 2_000_000, _lib.stream_handle(cuda)), "keepvq_wait_selftest")
+            end.record()
+        torch.cuda.synchronize()
+    return ws[:64].view(torch.int32).tolist(), start.elapsed_time(end)
+
+
+def test_every_form_that_gives_up_waits_for_its_copies(cuda):
+    """The scale-group form and the 8-bit form give up while the activation loader has a ring full of
+    copies under way, on barriers that also count decode warps which never came.  Each reports,
+    and finds its copies landed: one that did not would sit out its 100 ms of grace."""
+    words, ms = _wait_selftest(cuda)
+    assert words[:3] == [1, 1, 1]
+    assert ms < 3 * 2 + 50, ms  # three waits of 2 ms
+
+
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 256, 128), (7, 512, 256), (300, 512, 256)])
 def test_shared_expert_joins_the_routed_sum_before_the_one_rounding(cuda, tokens, hidden, inter):
     """``decode(x, shared=s)``: out = bf16(sum over the picks of the routes' bf16 outputs, in pick
