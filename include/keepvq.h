@@ -558,10 +558,11 @@ int keepvq_moe_decode_layer_static(const keepvq_moe_layer_args* args, void* stre
  * never to publish: first the activations of the form for rows with one scale group (a wait must
  * run into its deadline, `wait_ns` nanoseconds on the GPU's global timer, at most one second),
  * then the codes of the forms for rows with several scale groups and for 8-bit codes, whose
- * activation copies are in flight when they give up (at most 5 ms each).  Run i writes 1 into the
- * i-th int32 of `workspace`, waits for its copies, releases its tensor memory and returns; the
- * device stays usable.  A host checks those three words after synchronising.  No counterpart in
- * the reference.
+ * activation copies are in flight when they give up, and a run whose per-route facts come only
+ * after a warp gave up on them (at most 5 ms each).  Run i writes 1 into the i-th int32 of
+ * `workspace`, waits for its copies, releases its tensor memory and returns; the device stays
+ * usable.  Word 4 counts outputs that the last of them stored although their products were never
+ * formed: 0.  A host checks the words after synchronising.  No counterpart in the reference.
  * ------------------------------------------------------------------------------------------ */
 int64_t keepvq_wait_selftest_workspace_bytes(void);
 int keepvq_wait_selftest(void* workspace, int64_t workspace_bytes, int64_t wait_ns, void* stream);

@@ -129,6 +129,11 @@ __global__ void selftest_init_kernel(int32_t* count, int32_t* size, int32_t* rou
   if (threadIdx.x < 16) routes[threadIdx.x] = threadIdx.x;
   if (threadIdx.x < 17) x_scale[threadIdx.x] = 1.0f;
 }
+// How many values of columns first .. 511 of 16 output rows are not `want`.
+__global__ void selftest_check_kernel(const uint16_t* out, int first, uint32_t want, int32_t* wrong) {
+  for (int i = threadIdx.x; i < 16 * (512 - first); i += 256)
+    if (out[i / (512 - first) * 512 + first + i % (512 - first)] != want) atomicAdd(wrong, 1);
+}
 }  // namespace keepvq
 
 extern "C" int64_t keepvq_wait_selftest_workspace_bytes(void) { return keepvq::SELFTEST_BYTES; }
@@ -156,12 +161,16 @@ extern "C" int keepvq_wait_selftest(void* workspace, int64_t workspace_bytes, in
   p.codebook = reinterpret_cast<const uint32_t*>(ws + 2048);
   p.x = xq; p.x_zero_row = 16; p.x_div = 1; p.groups_of_routes = groups; p.max_routes = 16;
   p.out = ws + 16384; p.out_dtype = KEEPVQ_BF16;
-  for (int form = 0; form < 3; ++form) {
+  for (int form = 0; form < 4; ++form) {
+    if (form == 3 && (e = cudaMemsetAsync(p.out, 0xFF, 16 * 512 * 2, s)) != cudaSuccess) return note_cuda_error(e);
     p.out_dim = form == 0 ? 128 : 512;  // (the other forms take 256 rows an item: two items)
     p.groups = form == 1 ? 2 : 1;
     p.group_cols = form == 0 ? fast::PREFILL_GROUP_ROUTES : fast::PREFILL_GROUP_ROUTES_SMALL;
     const int rc = fast::prefill_wait_selftest(form, p, status + form, static_cast<uint64_t>(form == 0 ? wait_ns : std::min(wait_ns, SELFTEST_SHORT_NS)), s);
     if (rc) return rc;
   }
+  // nothing of the second item (rows 256 on) may have been stored: its drain had nothing to store
+  selftest_check_kernel<<<1, 256, 0, s>>>(static_cast<const uint16_t*>(p.out), 256, 0xFFFFu, status + 4);
+  KEEPVQ_CHECK_LAUNCH();
   return KEEPVQ_OK;
 }

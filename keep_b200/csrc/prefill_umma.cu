@@ -241,8 +241,9 @@ struct RingPlace {
 // BITS: 16-bit E8P codes, or 8-bit codes of a table whose word holds dim d in nibble d, value
 // (nibble - 8) / 2.  There a codeword is ONE table read, w = q / 2 without the quarter, and any table
 // will do (the integer sums are bounded for |q| <= 8, not for the shipped table's codewords).
-// `stall` != 0 is the wait self-test: a loader never publishes, and a wait runs into the deadline.
-enum { STALL_ACTIVATIONS = 1, STALL_CODES = 2 };
+// `stall` != 0 is the wait self-test: a loader never publishes, or the per-route facts come only after
+// somebody gave up, and a wait runs into the deadline.
+enum { STALL_ACTIVATIONS = 1, STALL_CODES = 2, STALL_FACTS = 3 };
 // Boxes over the activations, one map per padded number of routes: [2 planes][16 (i + 1) rows][128 bytes].
 template <int N_MAX>
 struct ActivationMaps { CUtensorMap rows[N_MAX / 16]; };
@@ -512,7 +513,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             mbar_arrive_warp(bar(STAGE_FULL, stage.index), lane);
             stage.advance(2);
             // the previous segment's MMAs have had this K block's decode to finish under
-            if (pending) drain();
+            if (pending) {
+              drain();
+              if (!ok) break;  // (the next wait would find its barrier complete and carry on)
+            }
           }
         }
         if (pending) drain();  // a warp without K blocks
@@ -675,6 +679,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
           if (segment >= segments) { segment -= segments; ++n; }
         }
       }
+      while (stall == STALL_FACTS && !*aborted && global_timer_ns() <= deadline + 1000000) __nanosleep(1000);
       __syncwarp();
       mbar_arrive_warp(bar(INFO_FULL, info.index), lane);
       info.advance();
@@ -789,10 +794,12 @@ int prefill_byte_codes(const FastProjectionArgs& p, int32_t* status, cudaStream_
 }
 // One CTA of a single-projection kernel, one of whose loaders never publishes, with a short deadline:
 // a wait runs out, the CTA reports and returns.  `p` must describe a valid problem.
-// 0: the 96-route form without activations; 1: the scale-group form without codes; 2: the 8-bit form without codes.
+// 0: the 96-route form without activations; 1: the scale-group form without codes; 2: the 8-bit form without codes;
+// 3: the 48-route form whose per-route facts come too late.
 int prefill_wait_selftest(int form, const FastProjectionArgs& p, int32_t* status, uint64_t wait_ns, cudaStream_t s) {
   if (form == 1) return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, true>(p, status, s, STALL_CODES, wait_ns, 1);
   if (form == 2) return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, false, 8>(p, status, s, STALL_CODES, wait_ns, 1);
+  if (form == 3) return launch_prefill<2, false, PREFILL_GROUP_ROUTES_SMALL, false>(p, status, s, STALL_FACTS, wait_ns, 1);
   return launch_prefill<1, false, PREFILL_GROUP_ROUTES, false>(p, status, s, STALL_ACTIVATIONS, wait_ns, 1);
 }
 

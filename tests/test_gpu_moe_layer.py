@@ -307,7 +307,16 @@ def test_every_form_that_gives_up_waits_for_its_copies(cuda):
     and finds its copies landed: one that did not would sit out its 100 ms of grace."""
     words, ms = _wait_selftest(cuda)
     assert words[:3] == [1, 1, 1]
-    assert ms < 3 * 2 + 50, ms  # three waits of 2 ms
+    assert ms < 4 * 2 + 50, ms  # four waits of 2 ms
+
+
+def test_a_warp_that_gave_up_stores_nothing_any_more(cuda):
+    """The per-route facts of an item come only after a decode warp gave up waiting for them.  That
+    warp must not go on to the next item, whose drain would find the facts and the first item's
+    accumulators, and store them as the second item's rows."""
+    words, _ = _wait_selftest(cuda)
+    assert words[3] == 1
+    assert words[4] == 0
 
 
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 256, 128), (7, 512, 256), (300, 512, 256)])
