@@ -269,7 +269,6 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   __shared__ int4 route_info[PF_INFO_BUFFERS][N_MAX];  // per item (three in flight): route, x scale, x sum (one scale group only), gate weight
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   auto bar = [](int which, uint32_t index) { return PF_BARS + 8u * (static_cast<uint32_t>(which) + index); };
-  const uint64_t deadline = global_timer_ns() + (wait_ns ? wait_ns : PF_DEFAULT_WAIT_NS);
 
   const uint32_t dyn_base = smem_addr(smem_raw);
   const bool window_ok = dyn_base <= PF_BARS && PF_A0 + Plan::HIGH_BYTES <= dyn_base + PF_SMEM_BYTES;  // uniform over the grid
@@ -302,6 +301,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   // an allocation of all 512 columns starts at column 0 of lane 0: a constant, which keeps the MMAs' operands in uniform registers
   constexpr uint32_t tmem = 0;
   grid_wait();  // the tables come from constants; everything below reads what the kernels before this one wrote
+  const uint64_t deadline = global_timer_ns() + (wait_ns ? wait_ns : PF_DEFAULT_WAIT_NS);  // (the time spent waiting for those is not this kernel's)
 
   const int64_t N_out = p.out_dim;
   const int k_blocks = static_cast<int>(p.in_dim / (8 * PF_KBLOCK_CODES));

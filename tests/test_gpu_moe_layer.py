@@ -319,6 +319,14 @@ def test_a_warp_that_gave_up_stores_nothing_any_more(cuda):
     assert words[4] == 0
 
 
+def test_the_time_a_kernel_waits_for_its_predecessor_is_not_its_own(cuda):
+    """The kernels are launched early and wait, resident, for the kernel before them.  Each run of the
+    self-test starts while the one before it sits out its 2 ms, and must have 2 ms of its own."""
+    words, ms = _wait_selftest(cuda)
+    assert words[:4] == [1, 1, 1, 1]
+    assert ms >= 4 * 2, ms
+
+
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 256, 128), (7, 512, 256), (300, 512, 256)])
 def test_shared_expert_joins_the_routed_sum_before_the_one_rounding(cuda, tokens, hidden, inter):
     """``decode(x, shared=s)``: out = bf16(sum over the picks of the routes' bf16 outputs, in pick
