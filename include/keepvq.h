@@ -405,11 +405,11 @@ typedef struct keepvq_grouped_projection_args {
   int32_t x_dtype;
   int64_t routes;
   const uint32_t* rhs;       /* [routes] expert (slot) of each route */
-  const void* codes;         /* [slots, out_dim, in_dim/8], uint16 or (code_bits 8) uint8 */
+  const uint16_t* codes;     /* [slots, out_dim, in_dim/8] */
   const void* scales;        /* [slots, out_dim, groups] */
   int32_t scales_dtype;
   int64_t slots, out_dim, in_dim, groups;
-  const uint32_t* codebook;  /* E8P packed abs grid, or (code_bits 8) the table words, dim d in nibble d */
+  const uint32_t* codebook;  /* E8P packed abs grid */
   int32_t codebook_all_odd;  /* as in keepvq_moe_layer_args */
   void* out;                 /* [routes, out_dim] */
   int32_t out_dtype;
@@ -418,9 +418,6 @@ typedef struct keepvq_grouped_projection_args {
   /* Route r reads activation row r / x_div: 1 (or 0) = a row per route, top_k = the token layout
      of e8p_m1_token_layout (src/ramp/kernels/e8p_m1.py:134-157).  x_rows = routes / x_div. */
   int32_t x_div;
-  /* 0 or 16: 16-bit E8P codes.  8: 8-bit codes, no residual; calls of a few routes and unaligned codes
-     are KEEPVQ_ERR_UNSUPPORTED (keepvq_routed_matvec takes them). */
-  int32_t code_bits;
   /* Optional nested residual, as in keepvq_matvec_args (e8p_nested_m1.py:90-112); res_codes == NULL
      turns it off.  Needs at least 48 routes and whole residual scale groups per 256 inputs,
      otherwise KEEPVQ_ERR_UNSUPPORTED. */
@@ -435,6 +432,12 @@ typedef struct keepvq_grouped_projection_args {
 int64_t keepvq_grouped_projection_workspace_bytes(int64_t routes, int64_t in_dim);
 int64_t keepvq_grouped_projection_status_offset(int64_t routes, int64_t in_dim);
 int keepvq_grouped_projection(const keepvq_grouped_projection_args* args, void* stream);
+/* The same for 8-bit codes: `codes` is the address of uint8 [slots, out_dim, in_dim/8], `codebook` the
+ * table words (dim d in nibble d), codebook_all_odd is not looked at, and there is no residual.  Calls
+ * that the general kernel serves as fast (few routes) and unaligned codes are KEEPVQ_ERR_UNSUPPORTED:
+ * keepvq_routed_matvec takes them.  (An entry point of its own: keepvq_grouped_projection_args stays
+ * as callers of this ABI version lay it out.) */
+int keepvq_grouped_projection_bytes(const keepvq_grouped_projection_args* args, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Expert parallelism: packing routes for the dispatch all-to-all and summing them after the

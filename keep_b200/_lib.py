@@ -107,7 +107,7 @@ class GroupedProjectionArgs(Structure):
         ("x", c_void_p), ("x_dtype", c_int32), ("routes", c_int64), ("rhs", c_void_p), ("codes", c_void_p), ("scales", c_void_p),
         ("scales_dtype", c_int32), ("slots", c_int64), ("out_dim", c_int64), ("in_dim", c_int64), ("groups", c_int64),
         ("codebook", c_void_p), ("codebook_all_odd", c_int32), ("out", c_void_p), ("out_dtype", c_int32),
-        ("workspace", c_void_p), ("workspace_bytes", c_int64), ("x_div", c_int32), ("code_bits", c_int32),
+        ("workspace", c_void_p), ("workspace_bytes", c_int64), ("x_div", c_int32),
         ("res_codes", c_void_p), ("res_scales", c_void_p), ("res_rows", c_int64), ("res_groups", c_int64),
         ("res_table", c_void_p), ("hot_of_slot", c_void_p),
     ]
@@ -166,6 +166,7 @@ _SIGNATURES = {
     "keepvq_grouped_projection_workspace_bytes": (c_int64, [c_int64, c_int64]),
     "keepvq_grouped_projection_status_offset": (c_int64, [c_int64, c_int64]),
     "keepvq_grouped_projection": (c_int, [POINTER(GroupedProjectionArgs), c_void_p]),
+    "keepvq_grouped_projection_bytes": (c_int, [POINTER(GroupedProjectionArgs), c_void_p]),
     "keepvq_wait_selftest_workspace_bytes": (c_int64, []),
     "keepvq_wait_selftest": (c_int, [c_void_p, c_int64, c_int64, c_void_p]),
     "keepvq_ep_pack": (c_int, [POINTER(EpPackArgs), c_void_p]),

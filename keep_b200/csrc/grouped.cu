@@ -51,8 +51,9 @@ extern "C" int64_t keepvq_grouped_projection_status_offset(int64_t routes, int64
   return keepvq::plan_grouped(routes, in_dim).status;
 }
 
-extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* args, void* stream) {
-  using namespace keepvq;
+namespace keepvq {
+
+static int grouped_projection(const keepvq_grouped_projection_args* args, bool byte_codes, void* stream) {
   if (!args) return KEEPVQ_ERR_NULL;
   const keepvq_grouped_projection_args& a = *args;
   if (!valid_dtype(a.x_dtype) || !valid_dtype(a.scales_dtype)) return KEEPVQ_ERR_DTYPE;
@@ -60,8 +61,6 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
   if (a.routes == 0) return KEEPVQ_OK;
   if (!a.x || !a.rhs || !a.codes || !a.scales || !a.codebook || !a.out || !a.workspace) return KEEPVQ_ERR_NULL;
   if (a.x_dtype == KEEPVQ_F32) return KEEPVQ_ERR_UNSUPPORTED;  // these kernels keep 16 bits of a row: not what an fp32 caller asked for
-  if (a.code_bits != 0 && a.code_bits != 16 && a.code_bits != 8) return KEEPVQ_ERR_SHAPE;
-  const bool byte_codes = a.code_bits == 8;
   if ((!byte_codes && !a.codebook_all_odd) || !fast::shapes_supported(a.out_dim, a.in_dim, a.groups)) return KEEPVQ_ERR_UNSUPPORTED;
   if (byte_codes && (a.res_codes || a.routes < BYTE_CODES_MIN_ROUTES || !fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups) || !aligned_to(a.codes, 16) ||
                      a.routes > (1 << 20) || a.slots > 16384))
@@ -104,7 +103,7 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
   }
   fast::FastProjectionArgs p = {};
   p.slots = a.slots;
-  p.a = {static_cast<const uint16_t*>(a.codes), a.scales, a.res_codes, a.res_scales}; p.b = {nullptr, nullptr, nullptr, nullptr};
+  p.a = {a.codes, a.scales, a.res_codes, a.res_scales}; p.b = {nullptr, nullptr, nullptr, nullptr};
   if (residual) { p.res_groups = a.res_groups; p.hot_of_slot = a.hot_of_slot; p.res_table = a.res_table; }
   p.scales_dtype = a.scales_dtype; p.codebook = a.codebook; p.groups_of_routes = groups; p.max_routes = a.routes; p.group_cols = group_cols; p.status = wait_status;
   p.few_groups = many ? 0 : fast::few_route_groups(a.routes, a.slots);
@@ -113,6 +112,11 @@ extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* a
   if (byte_codes) return fast::prefill_byte_codes(p, wait_status, s);
   return many ? fast::prefill_down(p, wait_status, s) : fast::down(p, s);
 }
+
+}  // namespace keepvq
+
+extern "C" int keepvq_grouped_projection(const keepvq_grouped_projection_args* args, void* stream) { return keepvq::grouped_projection(args, false, stream); }
+extern "C" int keepvq_grouped_projection_bytes(const keepvq_grouped_projection_args* args, void* stream) { return keepvq::grouped_projection(args, true, stream); }
 
 // ------------------------------------------------------------------------------------------
 // Self-test of the bounded waits of the tcgen05 kernel: runs of one CTA on a tiny problem laid out in

@@ -54,7 +54,7 @@ def _scratch_bytes(routes: int, in_dim: int) -> int:
 
 
 def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, code_bits: int = 16, residual=None, hot_of_slot=None):
-    """``keepvq_grouped_projection``: route ``r`` against activation row ``r // x_div`` of ``rows``
+    """``keepvq_grouped_projection`` (``_bytes`` for 8-bit codes): route ``r`` against activation row ``r // x_div`` of ``rows``
     (fp16 / bf16), optionally with a nested residual ``(res_codes, res_scales, res_table)``.
     Returns None when the library says these shapes are not for the tensor-core kernels."""
     routes, in_dim = int(rhs.numel()), int(rows.shape[1])
@@ -78,7 +78,7 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
     args = _lib.GroupedProjectionArgs(
         x=_lib.ptr(rows), x_dtype=_lib.dtype_tag(rows.dtype), routes=routes, rhs=_lib.ptr(rhs), codes=_lib.ptr(codes), scales=_lib.ptr(scales),
         scales_dtype=_lib.dtype_tag(scales.dtype), slots=slots, out_dim=out_dim, in_dim=in_dim, groups=groups, codebook=_lib.ptr(table),
-        codebook_all_odd=int(code_bits == 16 and _table_all_odd(table)), code_bits=code_bits, out=_lib.ptr(out), out_dtype=_lib.dtype_tag(out_dtype),
+        codebook_all_odd=int(code_bits == 16 and _table_all_odd(table)), out=_lib.ptr(out), out_dtype=_lib.dtype_tag(out_dtype),
         workspace=_lib.ptr(ws), workspace_bytes=int(ws.numel()), x_div=int(x_div))
     keep = [rows, rhs]
     if residual is not None:
@@ -89,7 +89,7 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
         args.res_rows, args.res_groups, args.hot_of_slot = int(res_codes.shape[0]), int(res_scales.shape[2]), _lib.ptr(hot_of_slot)
         keep += [res_codes, res_scales, res_table, hot_of_slot]
     with torch.cuda.device(device):
-        status = lib.keepvq_grouped_projection(args, ctypes.c_void_p(stream))
+        status = (lib.keepvq_grouped_projection_bytes if code_bits == 8 else lib.keepvq_grouped_projection)(args, ctypes.c_void_p(stream))
     del keep
     if status == _UNSUPPORTED:
         return None

@@ -51,6 +51,27 @@ def test_struct_sizes_match_the_compiler():
         assert ctypes.sizeof(structs[name]) == int(size), name
 
 
+def test_padding_of_the_grouped_arguments_means_nothing():
+    """A C caller that fills in the fields and leaves the struct's padding as it finds it is served like
+    one that clears it.  (Calls that the library refuses for a misaligned row, before any CUDA call.)"""
+    from keep_b200 import _lib
+
+    lib, args = _lib.load(), _lib.GroupedProjectionArgs
+    pointers = "x rhs codes scales codebook out workspace res_codes res_scales res_table hot_of_slot".split()
+    numbers = "x_dtype routes scales_dtype slots out_dim in_dim groups codebook_all_odd out_dtype workspace_bytes x_div res_rows res_groups".split()
+    for filler in (0x00, 0x08, 0xFF):
+        a = args.from_buffer(bytearray([filler]) * ctypes.sizeof(args))
+        for name in pointers + numbers:  # the fields of this version of the header
+            setattr(a, name, None if name in pointers else 0)
+        for name in ("x", "rhs", "codes", "scales", "codebook", "out", "workspace"):
+            setattr(a, name, 256)
+        a.x = 264  # fp16 rows that start between two 16-byte boundaries
+        a.x_dtype = a.scales_dtype = a.out_dtype = _lib.dtype_tag(__import__("torch").float16)
+        a.routes = a.slots = a.out_dim = a.groups = a.codebook_all_odd = a.x_div = 1
+        a.in_dim, a.workspace_bytes = 256, 1 << 20
+        assert lib.keepvq_grouped_projection(a, None) == -4, filler  # KEEPVQ_ERR_ALIGN
+
+
 def test_operators_refuse_cpu_tensors():
     import pytest
     import torch
