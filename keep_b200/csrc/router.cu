@@ -176,15 +176,18 @@ __global__ void __launch_bounds__(RM_THREADS) router_logits_mma_kernel(keepvq_ro
       }
 }
 
-// 16 to 255 bf16 tokens against a bf16 router: the same 64 x 64 tile and the same arithmetic, with the
+// bf16 tokens against a bf16 router, from 24 tokens on and up to 255 tokens or 256 tiles: the same 64 x 64 tile and the same arithmetic, with the
 // hidden dimension split over a cluster of eight blocks so that a call of 64 tokens is 48 blocks
 // instead of 6.  Each block sums its eighth of K as above; the eight partial tiles meet through
 // distributed shared memory, every block adding up eight rows of the tile over the ranks in rank
 // order, so a logit is a fixed sequence of additions whatever the batch around it.
 constexpr int RC_SPLIT = 8;
-// Up to here (tiles of 64 tokens x 64 experts) a tile's serial walk over the whole hidden dimension is
-// what a call waits for: 1000 tokens x 384 experts (96 tiles) 28 against 57 us, 1021 x 192 (48 tiles,
-// 5120 wide) 20 against 70 us; with 384 tiles (4096 tokens) the GPU is full without the split: 91 against 84 us.
+// From RT_MIN_TOKENS tokens on the other kernel is the tiled one. Up to here (tiles of 64 tokens x 64
+// experts) that kernel's serial walk over the whole hidden dimension is what a call waits for: 1000 tokens
+// x 384 experts (96 tiles) 28 against 57 us, 1021 x 192 (48 tiles, 5120 wide) 20 against 70 us; with 384
+// tiles (4096 tokens) the GPU is full without the split: 91 against 84 us. With fewer tokens the other
+// kernel is the one of the fp32 pipes, which is slower at any number of tiles (200 tokens, 4096 wide:
+// 4160 experts 84 against 487 us, 16384 experts 258 against 1722 us).
 constexpr int64_t RC_MAX_TILES = 256;
 constexpr int RC_MIN_TOKENS = 24;  // below this the K-split kernel of the fp32 pipes is as fast, and shares its launch with the quantisation of the rows
 
@@ -524,7 +527,7 @@ extern "C" int keepvq_router_logits(const keepvq_router_logits_args* args, void*
   if (!aligned_to(a.x, 16) || !aligned_to(a.router_w, 16)) return KEEPVQ_ERR_ALIGN;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int64_t logit_tiles = (a.pool + RM_TILE - 1) / RM_TILE * ((a.tokens + RM_TILE - 1) / RM_TILE);
-  if (a.tokens >= RC_MIN_TOKENS && logit_tiles <= RC_MAX_TILES && a.x_dtype == KEEPVQ_BF16 && a.router_dtype == KEEPVQ_BF16 && a.hidden % (RC_SPLIT * RM_K) == 0) {
+  if (a.tokens >= RC_MIN_TOKENS && (a.tokens < RT_MIN_TOKENS || logit_tiles <= RC_MAX_TILES) && a.x_dtype == KEEPVQ_BF16 && a.router_dtype == KEEPVQ_BF16 && a.hidden % (RC_SPLIT * RM_K) == 0) {
     // the tensor-core tile with the hidden dimension split over a cluster of eight blocks
     dim3 grid(RC_SPLIT, static_cast<unsigned>((a.pool + RM_TILE - 1) / RM_TILE), static_cast<unsigned>((a.tokens + RM_TILE - 1) / RM_TILE));
     if (grid.y > 65535 || grid.z > 65535) return KEEPVQ_ERR_CAPACITY;

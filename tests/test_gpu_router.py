@@ -68,6 +68,20 @@ def test_served_demand_and_admission_match_the_oracle_exactly(cuda, tokens, pool
     assert all(resident[list(s)].all() for s in as_sets(got.served_expert.cpu()))
 
 
+@pytest.mark.parametrize("pool,tokens,fewer", [(4160, 200, 100), (8256, 65, 64)])
+def test_a_wide_pool_does_not_change_the_kernel_of_a_few_dozen_tokens(cuda, pool, tokens, fewer):
+    """24 to 255 bf16 tokens take the cluster kernel at any pool size, so a logit has the same bits
+    whatever the batch around it, also where the call has more than 256 tiles of 64 x 64."""
+    from keep_b200 import router
+
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    w = torch.randn((pool, 1024), generator=gen, device=cuda).mul_(0.02).to(torch.bfloat16)
+    x = torch.randn((tokens, 1024), generator=gen, device=cuda).to(torch.bfloat16)
+    got = router.router_logits(x, w)
+    np.testing.assert_allclose(got.cpu().numpy(), (x.double() @ w.double().t()).cpu().numpy(), rtol=0, atol=1e-5)
+    assert torch.equal(got[:fewer], router.router_logits(x[:fewer], w))
+
+
 def test_nothing_masked_means_served_equals_demand(cuda):
     from keep_b200 import router
 
