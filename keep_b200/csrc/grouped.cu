@@ -13,9 +13,21 @@
 
 namespace keepvq {
 
-// 8-bit codes: below this the general kernel, which needs no grouping and no quantised rows in front of
-// it, is as fast (2048 x 4096, 384 experts, whole calls: 82 against 42 us at 24 routes, 397 against 99 at 144).
-constexpr int64_t BYTE_CODES_MIN_ROUTES = 12;
+// 8-bit codes: whether the grouped kernel is faster than the general one, which needs no grouping, no
+// quantised rows and no 64 KB of tables in front of it, but reads an expert's codes once per four routes
+// and a code tile with one output row a thread.  Device time with cold codes, general / grouped us, over
+// matrices of 2^15 to 2^24 weights, 1 to 384 experts, 12 to 768 routes:
+//   12 routes    25 / 32 at 1024 x 2048, 47 / 30 at 2048 x 4096 (384 experts)
+//   24 routes    16 / 22 at 256 x 512, 27 / 26 at 512 x 1024, 37 / 32 at 1024 x 2048 (64 experts)
+//   48 routes    16 / 20 at 128 x 256, 23 / 22 at 256 x 512 (64 experts)
+//   96 routes    23 / 22 at 128 x 256 (384 experts), and 274 / 73 at 2048 x 4096
+// With three routes an expert some expert has more than four, and the general kernel passes over its
+// codes again: 39 / 20 for 12 routes of one 128 x 256 expert, 31 / 22 for 24 routes of eight 256 x 512.
+static bool byte_codes_pay(int64_t routes, int64_t slots, int64_t weights) {
+  if (routes < 12) return false;
+  if (routes >= 96 || routes >= 3 * slots) return true;
+  return weights >= (routes >= 48 ? int64_t{1} << 17 : routes >= 24 ? int64_t{1} << 19 : int64_t{1} << 22);
+}
 
 struct GroupedScratch {
   int64_t xq, xscale, xsums, gcount, gslot, gstart, gsize, groutes, status, total;
@@ -62,7 +74,7 @@ static int grouped_projection(const keepvq_grouped_projection_args* args, bool b
   if (!a.x || !a.rhs || !a.codes || !a.scales || !a.codebook || !a.out || !a.workspace) return KEEPVQ_ERR_NULL;
   if (a.x_dtype == KEEPVQ_F32) return KEEPVQ_ERR_UNSUPPORTED;  // these kernels keep 16 bits of a row: not what an fp32 caller asked for
   if ((!byte_codes && !a.codebook_all_odd) || !fast::shapes_supported(a.out_dim, a.in_dim, a.groups)) return KEEPVQ_ERR_UNSUPPORTED;
-  if (byte_codes && (a.res_codes || a.routes < BYTE_CODES_MIN_ROUTES || !fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups) || !aligned_to(a.codes, 16) ||
+  if (byte_codes && (a.res_codes || !byte_codes_pay(a.routes, a.slots, a.out_dim * a.in_dim) || !fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups) || !aligned_to(a.codes, 16) ||
                      a.routes > (1 << 20) || a.slots > 16384))
     return KEEPVQ_ERR_UNSUPPORTED;  // (the general kernel takes them)
   const int32_t x_div = a.x_div > 0 ? a.x_div : 1;

@@ -211,6 +211,27 @@ def test_8bit_codes_on_the_tcgen05_kernel(cuda, dtype, routes, experts, out, inp
     assert bool((with_dead[1] == 0).all()) and torch.equal(with_dead[2:], direct[2:])
 
 
+@pytest.mark.parametrize("routes,experts,out,inp,grouped", [
+    (11, 1, 2048, 2048, False), (12, 64, 1024, 2048, False), (12, 64, 2048, 2048, True), (12, 4, 128, 256, True), (24, 9, 256, 512, False), (24, 8, 256, 512, True),
+    (24, 64, 512, 1024, True), (47, 64, 256, 512, False), (48, 64, 256, 512, True), (95, 64, 128, 256, False), (96, 64, 128, 256, True),
+])
+def test_8bit_codes_take_the_kernel_that_is_faster_for_their_size(cuda, routes, experts, out, inp, grouped):
+    """Both sides of every line of the rule for 8-bit codes, and the same outputs from the operator on either."""
+    from keep_b200 import kernels, prefill, vq, vq_switch
+
+    gen = torch.Generator(device=cuda).manual_seed(29)
+    codes = torch.randint(0, 256, (experts, out, inp // 8), generator=gen, device=cuda, dtype=torch.uint8)
+    scales = torch.full((experts, out, 1), 0.02, dtype=torch.float16, device=cuda)
+    x = torch.randn((routes, inp), generator=gen, device=cuda).to(torch.bfloat16)
+    rhs = torch.randint(0, experts, (routes, 1), generator=gen, device=cuda).to(torch.int32)
+    table = vq.table_on(cuda, "e8_1bit")
+    assert (prefill.tensor_core_projection(x, codes, scales, table, rhs.reshape(-1), code_bits=8) is not None) == grouped
+    got = vq_switch.gather_vqmm(x, codes, scales, table, rhs, input_dims=inp, output_dims=out, group_size=inp, code_bits=8)
+    want = kernels.routed_matvec(x, codes, scales, table, rhs.reshape(-1), code_bits=8)
+    atol = 2.0 ** -11 * float(want.float().abs().max())  # the fixed-point step of a row against its largest output
+    np.testing.assert_allclose(f32(got).reshape(routes, out), f32(want), rtol=2.0 ** -8, atol=atol)
+
+
 @pytest.mark.parametrize("bits,inp,word,code", [
     (8, 8192, 0x00000000, 0), (8, 8704, 0x00000000, 0), (8, 66560, 0x00000000, 0),  # every weight -4
     (16, 8192, 0x11111111, 0), (16, 10240, 0x11111111, 0),  # an all-odd table: every weight -3.25
