@@ -438,6 +438,9 @@ int keepvq_grouped_projection(const keepvq_grouped_projection_args* args, void* 
  * keepvq_routed_matvec takes them.  (An entry point of its own: keepvq_grouped_projection_args stays
  * as callers of this ABI version lay it out.) */
 int keepvq_grouped_projection_bytes(const keepvq_grouped_projection_args* args, void* stream);
+/* 1 when keepvq_grouped_projection_bytes takes calls of these sizes, else 0: for callers that would
+ * rather not prepare one to be refused. */
+int keepvq_grouped_projection_bytes_served(int64_t routes, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups);
 
 /* ------------------------------------------------------------------------------------------
  * Expert parallelism: packing routes for the dispatch all-to-all and summing them after the

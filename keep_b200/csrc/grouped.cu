@@ -29,6 +29,11 @@ static bool byte_codes_pay(int64_t routes, int64_t slots, int64_t weights) {
   return weights >= (routes >= 48 ? int64_t{1} << 17 : routes >= 24 ? int64_t{1} << 19 : int64_t{1} << 22);
 }
 
+// ... and whether its limits hold the sizes.
+static bool byte_codes_served(int64_t routes, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups) {
+  return routes <= (1 << 20) && slots <= 16384 && fast::prefill_supported(slots, out_dim, in_dim, groups) && byte_codes_pay(routes, slots, out_dim * in_dim);
+}
+
 struct GroupedScratch {
   int64_t xq, xscale, xsums, gcount, gslot, gstart, gsize, groutes, status, total;
 };
@@ -58,6 +63,10 @@ extern "C" int64_t keepvq_grouped_projection_workspace_bytes(int64_t routes, int
   return keepvq::plan_grouped(routes, in_dim).total;
 }
 
+extern "C" int keepvq_grouped_projection_bytes_served(int64_t routes, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups) {
+  return routes > 0 && slots > 0 && out_dim > 0 && in_dim > 0 && groups > 0 && keepvq::byte_codes_served(routes, slots, out_dim, in_dim, groups) ? 1 : 0;
+}
+
 extern "C" int64_t keepvq_grouped_projection_status_offset(int64_t routes, int64_t in_dim) {
   if (routes < 0 || in_dim <= 0 || in_dim % 8) return KEEPVQ_ERR_SHAPE;
   return keepvq::plan_grouped(routes, in_dim).status;
@@ -74,9 +83,7 @@ static int grouped_projection(const keepvq_grouped_projection_args* args, bool b
   if (!a.x || !a.rhs || !a.codes || !a.scales || !a.codebook || !a.out || !a.workspace) return KEEPVQ_ERR_NULL;
   if (a.x_dtype == KEEPVQ_F32) return KEEPVQ_ERR_UNSUPPORTED;  // these kernels keep 16 bits of a row: not what an fp32 caller asked for
   if ((!byte_codes && !a.codebook_all_odd) || !fast::shapes_supported(a.out_dim, a.in_dim, a.groups)) return KEEPVQ_ERR_UNSUPPORTED;
-  if (byte_codes && (a.res_codes || !byte_codes_pay(a.routes, a.slots, a.out_dim * a.in_dim) || !fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups) || !aligned_to(a.codes, 16) ||
-                     a.routes > (1 << 20) || a.slots > 16384))
-    return KEEPVQ_ERR_UNSUPPORTED;  // (the general kernel takes them)
+  if (byte_codes && (a.res_codes || !aligned_to(a.codes, 16) || !byte_codes_served(a.routes, a.slots, a.out_dim, a.in_dim, a.groups))) return KEEPVQ_ERR_UNSUPPORTED;  // (the general kernel takes them)
   const int32_t x_div = a.x_div > 0 ? a.x_div : 1;
   if (a.routes % x_div) return KEEPVQ_ERR_SHAPE;
   const int64_t x_rows = a.routes / x_div;

@@ -53,6 +53,12 @@ def _scratch_bytes(routes: int, in_dim: int) -> int:
     return nbytes
 
 
+@lru_cache(maxsize=256)
+def byte_codes_served(routes: int, slots: int, out_dim: int, in_dim: int, groups: int) -> bool:
+    """Whether 8-bit calls of these sizes go to the grouped kernel (the rule and its figures: csrc/grouped.cu)."""
+    return bool(_lib.load().keepvq_grouped_projection_bytes_served(routes, slots, out_dim, in_dim, groups))
+
+
 def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, code_bits: int = 16, residual=None, hot_of_slot=None):
     """``keepvq_grouped_projection`` (``_bytes`` for 8-bit codes): route ``r`` against activation row ``r // x_div`` of ``rows``
     (fp16 / bf16), optionally with a nested residual ``(res_codes, res_scales, res_table)``.
@@ -63,6 +69,8 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
         return None
     if int(rows.shape[0]) * x_div != routes:
         return None
+    if code_bits == 8 and not byte_codes_served(routes, slots, out_dim, in_dim, groups):
+        return None  # (asked first: a call prepared to be refused cost 20 us)
     lib = _lib.load()
     device = rows.device
     stream = torch.cuda.current_stream(device).cuda_stream

@@ -23,6 +23,7 @@ import torch
 
 from . import _lib
 from .kernels import _activations, _index_tensor, qmv_output_dtype, routed_matvec
+from .prefill import byte_codes_served, grouped_matmul_sorted, tensor_core_projection
 from .vq import CODEWORD_DIM, _codebook_tensor, as_device, decode_weight_matrix
 
 __all__ = [
@@ -213,8 +214,6 @@ def gather_vqmm_sorted_routes(x, codes, scales, codebook, sorted_rhs, sorted_lhs
     if implementation == "reference":
         rows = x_t if skip_gather else x_t[lhs.long()]
         return _dense_routes(rows, codes_t, scales_t, table, rhs, code_bits).to(qmv_output_dtype(x_t.dtype))
-    from .prefill import grouped_matmul_sorted
-
     return grouped_matmul_sorted(x_t, codes_t.contiguous(), scales_t.contiguous(), table, rhs,
                                  None if skip_gather else lhs, code_bits=code_bits, tile_descriptors=tile_descriptors)
 
@@ -276,13 +275,12 @@ def gather_vqmm(x, codes, scales, codebook, rhs_indices, *, lhs_indices=None, in
             _check_range(flat_lhs, int(x_t.shape[0]), "lhs_indices")
         return _dense_routes(x_t[rows], codes_t, scales_t, table, flat_rhs, code_bits).reshape(output_shape)
 
-    if flat_lhs is None and x_t.dtype in (torch.float16, torch.bfloat16) and scales_t.dtype in (torch.float32, torch.float16, torch.bfloat16):
+    if flat_lhs is None and x_t.dtype in (torch.float16, torch.bfloat16) and scales_t.dtype in (torch.float32, torch.float16, torch.bfloat16) and (
+            code_bits == 16 or byte_codes_served(routes, codes_t.shape[0], output_dims, input_dims, input_dims // group_size)):
         # token layout with 16-bit rows: the int8 tensor-core kernels, which group the routes by
         # expert on the device, in whatever order they come, and read each touched expert's codes
         # once: sorting them here first, gathering a row per route and scattering the outputs back
         # cost 200 of the 445 us of a 1024-token call
-        from .prefill import tensor_core_projection
-
         out = tensor_core_projection(x_t, codes_t.contiguous(), scales_t.contiguous(), table, flat_rhs, x_div=x_div, code_bits=code_bits)
         if out is not None:
             return out.reshape(output_shape)

@@ -1,4 +1,4 @@
-"""Scratch of the operators' grouped kernels: every call has its own (host logic, no GPU)."""
+"""Host side of the operators' grouped kernels: scratch, remembered facts, refusals (no GPU)."""
 
 import contextlib
 import ctypes
@@ -47,3 +47,19 @@ def test_the_answer_about_a_table_survives_an_eviction(monkeypatch):
     monkeypatch.setattr(prefill, "_all_odd", Forgetful())
     assert prefill._table_all_odd(torch.full((256,), 0x11111111, dtype=torch.int32)) is True
     assert prefill._table_all_odd(torch.full((256,), 0x11111112, dtype=torch.int32)) is False
+
+
+def test_a_call_that_the_library_will_refuse_prepares_nothing(monkeypatch):
+    """8-bit calls of few routes belong to the general kernel: neither scratch nor outputs are
+    allocated, nor the library called, to find that out."""
+    from keep_b200 import prefill
+
+    rows, codes = torch.zeros((6, 256), dtype=torch.bfloat16), torch.zeros((64, 32, 32), dtype=torch.uint8)
+    scales, table, rhs = torch.ones((64, 32, 1), dtype=torch.float16), torch.zeros(256, dtype=torch.int32), torch.zeros(6, dtype=torch.int32)
+
+    def prepared(*args, **kwargs):
+        raise AssertionError("prepared a call")
+
+    monkeypatch.setattr(torch.cuda, "current_stream", prepared)
+    monkeypatch.setattr(torch, "empty", prepared)
+    assert prefill.tensor_core_projection(rows, codes, scales, table, rhs, code_bits=8) is None
