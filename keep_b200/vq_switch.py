@@ -57,6 +57,10 @@ def _record(**fields) -> None:
         records.append(fields)
 
 
+def _projection_role(input_dims: int, output_dims: int) -> str:
+    return "down" if output_dims >= input_dims else "gate_up"
+
+
 def _validate_switch_metadata(x, codes, scales, codebook, indices, *, input_dims, output_dims, group_size, code_bits):
     """Same checks, same order, same messages as ``vq_switch.py:491-544``."""
     if code_bits not in (8, 16):
@@ -207,7 +211,7 @@ def gather_vqmm_sorted_routes(x, codes, scales, codebook, sorted_rhs, sorted_lhs
         _check_range(lhs, int(x_t.shape[0]), "sorted_lhs")
         if routes > 1 and bool((rhs[1:] < rhs[:-1]).any()):
             raise ValueError("sorted_rhs must be sorted nondecreasing by expert id")
-    role = ("down" if output_dims >= input_dims else "gate_up") if projection == "auto" else projection
+    role = _projection_role(input_dims, output_dims) if projection == "auto" else projection
     skip_gather = role == "down" and x_pre_sorted and int(x_t.shape[0]) == routes
     _record(token_rows=int(x_t.shape[0]), route_count=routes, input_dims=input_dims, output_dims=output_dims,
             code_bits=code_bits, strategy="sorted_tiled", implementation=implementation, projection=role)
@@ -226,7 +230,10 @@ def gather_vqmm(x, codes, scales, codebook, rhs_indices, *, lhs_indices=None, in
 
     ``route_strategy="auto"``: expert-sorted grouped kernel when ``sorted_indices`` or at least
     128 routes, otherwise the direct few-row kernel.  ``"per_route_decoded"`` names a Metal
-    variant of the direct kernel and is served by the same CUDA kernel as ``"direct"``.
+    variant of the direct kernel and is served by the same CUDA kernel as ``"direct"``.  Without
+    ``lhs_indices``, 16-bit rows against 16-bit codes (and against 8-bit codes where the calls are
+    large enough) run on the kernels that group the routes by expert on the device, whatever the
+    strategy: it then only names the dispatch in the trace, and the outputs are the same.
     """
     if route_strategy not in _ROUTE_STRATEGIES:
         raise ValueError("route_strategy must be 'auto', 'direct', 'sorted_tiled', or 'per_route_decoded'")
@@ -283,6 +290,9 @@ def gather_vqmm(x, codes, scales, codebook, rhs_indices, *, lhs_indices=None, in
         # cost 200 of the 445 us of a 1024-token call
         out = tensor_core_projection(x_t, codes_t.contiguous(), scales_t.contiguous(), table, flat_rhs, x_div=x_div, code_bits=code_bits)
         if out is not None:
+            if strategy == "sorted_tiled":  # the grouping is the kernels' own; the expert-grouped dispatch leaves its record all the same
+                _record(token_rows=int(x_t.shape[0]), route_count=routes, input_dims=input_dims, output_dims=output_dims, code_bits=code_bits,
+                        strategy="sorted_tiled", implementation=implementation, projection=_projection_role(input_dims, output_dims))
             return out.reshape(output_shape)
 
     if strategy == "direct":

@@ -278,6 +278,25 @@ def test_calls_on_two_streams_do_not_share_scratch(cuda):
         assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i])
 
 
+@pytest.mark.parametrize("bits", [8, 16])
+@pytest.mark.parametrize("out,inp,role", [(512, 256, "down"), (256, 512, "gate_up")])
+def test_the_trace_of_a_sorted_call_names_its_projection(cuda, bits, out, inp, role):
+    """From 128 routes on (or when asked for) a call leaves the operator's record and the expert-grouped
+    dispatch's, which names the projection; a direct call leaves one."""
+    from keep_b200 import vq_switch
+
+    codes = torch.zeros((4, out, inp // 8), dtype=torch.uint8 if bits == 8 else torch.uint16, device=cuda)
+    scales = torch.ones((4, out, 1), dtype=torch.float16, device=cuda)
+    named = dict(input_dims=inp, output_dims=out, group_size=inp, code_bits=bits)
+    for tokens, strategy, records in ((64, "auto", 2), (10, "auto", 1), (10, "sorted_tiled", 2), (64, "direct", 1)):
+        x, rhs = torch.ones((tokens, inp), dtype=torch.bfloat16, device=cuda), torch.zeros((tokens, 2), dtype=torch.int32, device=cuda)
+        with vq_switch.trace_gather_vqmm_calls() as trace:
+            vq_switch.gather_vqmm(x, codes, scales, None, rhs, route_strategy=strategy, **named)
+        first = dict(token_rows=tokens, route_count=2 * tokens, input_dims=inp, output_dims=out, code_bits=bits, implementation="cuda",
+                     strategy="sorted_tiled" if records == 2 else "direct")
+        assert trace == [first, dict(first, projection=role)][:records]
+
+
 def _calls_of_one_shape(cuda, count):
     """``count`` argument lists of one shape (100 tokens of top-2 over 8 experts) with inputs of their own, and their results."""
     from keep_b200 import vq, vq_switch
