@@ -203,16 +203,25 @@ class RoutedMoELayer:
                 and ok(self.hidden, int(self.w1.res_scales.shape[2])) and ok(self.inter, int(self.w2.res_scales.shape[2]))
         return "tensor" if self.codebook_all_odd and fits else "general"
 
+    def _on_tcgen05(self, routes: int) -> bool:
+        """Whether a call of ``routes`` routes runs the tcgen05 kernels (``prefill_pays`` and
+        ``prefill_supported`` of csrc/moe_fast.cuh and csrc/prefill_umma.cu)."""
+        shapes = ((self.inter, self.hidden, int(self.w1.scales.shape[2])), (self.hidden, self.inter, int(self.w2.scales.shape[2])))
+        several = any(groups > 1 for _, _, groups in shapes)
+        fits = all(self.slots * out < 2 ** 31 - 512 and (groups == 1 or (groups <= 32 and inp // groups <= 4096)) for out, inp, groups in shapes)
+        return not self.res_rows and fits and routes >= 1024 and routes >= (8 if several else 5) * self.slots
+
     def launches_per_call(self, tokens: int, dtype: torch.dtype = torch.bfloat16) -> int:
         """Kernel launches one ``decode`` call of ``tokens`` rows enqueues.  On the tensor-core
         kernels: logits, top-k, route grouping, quantise x, gate/up, quantise h, down, combine,
-        of which two share a launch: up to 23 fp16 / bf16 tokens the logits and the quantisation
-        of x, beyond that (up to 4096 routes) the quantisation of x and the route grouping."""
-        if self.kernel_path != "tensor":
+        of which two share a launch on the decode kernels: up to 23 tokens the logits and the
+        quantisation of x, beyond that (up to 4096 routes) the quantisation of x and the route
+        grouping.  The tcgen05 kernels' rows are quantised in grouped order, behind the grouping."""
+        if self.kernel_path != "tensor" or dtype not in (torch.float16, torch.bfloat16):
             return 7
-        front = tokens <= 23 and dtype in (torch.float16, torch.bfloat16)
-        paired = tokens * self.top_k <= 4096 and self.slots * 12 <= 40 * 1024
-        return 7 if front or paired else 8
+        routes = tokens * self.top_k
+        front, paired = tokens <= 23, routes <= 4096 and self.slots * 12 <= 40 * 1024
+        return 7 if (front or paired) and not self._on_tcgen05(routes) else 8
 
     def decode_without_scratch(self, x: torch.Tensor, out: torch.Tensor, routing: Routing) -> tuple[torch.Tensor, Routing]:
         """The same layer through ``keepvq_moe_decode_layer_static``: the caller supplies the

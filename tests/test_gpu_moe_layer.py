@@ -327,6 +327,25 @@ def test_the_time_a_kernel_waits_for_its_predecessor_is_not_its_own(cuda):
     assert ms >= 4 * 2, ms
 
 
+@pytest.mark.parametrize("experts,groups,tokens,dtype", [
+    (20, (None, None), 4, torch.bfloat16), (20, (None, None), 40, torch.float16), (20, (None, None), 256, torch.bfloat16), (300, (None, None), 300, torch.bfloat16),
+    (20, (256, None), 256, torch.bfloat16), (140, (256, 256), 256, torch.bfloat16), (20, (None, None), 40, torch.float32), (900, (None, None), 1030, torch.bfloat16),
+])
+def test_launches_per_call_counts_what_a_call_enqueues(cuda, experts, groups, tokens, dtype):
+    from torch.profiler import ProfilerActivity, profile
+
+    cfg = synthetic.layer(seed=61, experts=experts, hidden=512, inter=256, group_hidden=groups[0], group_inter=groups[1])
+    layer = build_layer(cuda, cfg, top_k=4)
+    x = synthetic.tokens(62, tokens, 512).to(cuda).to(dtype)
+    layer.decode(x)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as trace:
+        layer.decode(x)
+        torch.cuda.synchronize()
+    kernels = [e.name for e in trace.events() if "keepvq" in e.name]
+    assert len(kernels) == layer.launches_per_call(tokens, dtype), kernels
+
+
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 256, 128), (7, 512, 256), (300, 512, 256)])
 def test_shared_expert_joins_the_routed_sum_before_the_one_rounding(cuda, tokens, hidden, inter):
     """``decode(x, shared=s)``: out = bf16(sum over the picks of the routes' bf16 outputs, in pick
