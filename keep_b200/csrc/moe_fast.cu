@@ -358,7 +358,7 @@ int quantize_rows_and_group(const void* x, int32_t x_dtype, int64_t rows, int64_
 
 // ------------------------------------------------------------------------------------------
 // Route grouping: routes that are served from the same slot share the code stream.  One block;
-// counting sort by slot, then each slot's routes are cut into groups of at most 8.
+// counting sort by slot, then each slot's routes are cut into groups of at most max_group.
 // ------------------------------------------------------------------------------------------
 constexpr int GR_THREADS = 1024;
 
@@ -408,15 +408,7 @@ static int few_items(const FastProjectionArgs& p) {
   return split_fits ? 1 : sweep_fits ? 2 : 0;
 }
 
-#ifdef KEEPVQ_DIAG
-static int g_force_cols = 0;
-extern "C" void keepvq_diag_set_group_cols(int cols) { g_force_cols = cols; }
-#endif
-
 int decode_group_routes(int64_t live, int64_t slots, int64_t widest_in_dim) {
-#ifdef KEEPVQ_DIAG
-  if (g_force_cols) return g_force_cols;
-#endif
   if (live < SMALL_CALL_ROUTES) return PAIRED_GROUP_ROUTES;  // the sweep kernel (the split slab kernel with a residual tier)
   if (widest_in_dim > slab_max_in_dim(MAX_GROUP_ROUTES)) return PAIRED_GROUP_ROUTES;
   return live <= 2 * slots ? PAIRED_GROUP_ROUTES : MAX_GROUP_ROUTES;

@@ -380,15 +380,8 @@ static int launch_sweep(const FastProjectionArgs& p, cudaStream_t s) {
   return launch_sweep_kernel<1, DEPTH, true>(p, s);
 }
 
-#ifdef KEEPVQ_DIAG
-static int g_sweep_variant = 0;  // measurement build only: 0 = code ring of 2 stages, 1 = of 3
-extern "C" void keepvq_diag_set_sweep(int variant) { g_sweep_variant = variant; }
-int sweep_gate_up(const FastProjectionArgs& p, cudaStream_t s) { return g_sweep_variant ? launch_sweep<2, 3>(p, s) : launch_sweep<2, 2>(p, s); }
-int sweep_down(const FastProjectionArgs& p, cudaStream_t s) { return g_sweep_variant ? launch_sweep<1, 3>(p, s) : launch_sweep<1, 2>(p, s); }
-#else
 int sweep_gate_up(const FastProjectionArgs& p, cudaStream_t s) { return launch_sweep<2, 2>(p, s); }
 int sweep_down(const FastProjectionArgs& p, cudaStream_t s) { return launch_sweep<1, 2>(p, s); }
-#endif
 
 }  // namespace fast
 }  // namespace keepvq
