@@ -6,8 +6,9 @@ Stands in for the reference's sorted-route kernels: ``gather_vqmm_tiled_down`` /
 
 16-bit E8P codes with fp16 / bf16 activations whose shapes fit go to ``keepvq_grouped_projection``
 (int8 tensor cores: the tcgen05 kernel from 5 routes per expert on, 8 where a row has several scale
-groups, the mma.sync ones below), and so do 8-bit codes from a dozen routes on (tcgen05); everything
-else (fp32 activations, odd shapes, custom 16-bit tables with even nibbles) to the general routed kernel.
+groups, the mma.sync ones below); 8-bit codes go to ``keepvq_grouped_projection_bytes`` (tcgen05) where
+``byte_codes_served`` says so; everything else (fp32 activations, odd shapes, custom 16-bit tables with
+even nibbles) to the general routed kernel.
 """
 
 from __future__ import annotations

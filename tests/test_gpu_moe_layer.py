@@ -216,7 +216,7 @@ def test_scale_groups_and_short_groups_on_the_tcgen05_kernels(cuda, tokens, expe
     check_layer(cfg, x, out, routing, top_k=top_k)
 
 
-def test_many_routes_spread_over_many_experts_stay_on_the_decode_kernels(cuda):
+def test_nineteen_routes_per_expert_take_the_48_route_items(cuda):
     """1200 routes over 64 experts, 19 per expert on average: the tcgen05 kernels' 48-route items.
     (The mma.sync kernels with several 8-route groups per expert: the next test.)"""
     cfg = synthetic.layer(seed=43, experts=64, hidden=512, inter=256)
