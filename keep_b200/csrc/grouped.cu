@@ -115,7 +115,10 @@ static int grouped_projection(const keepvq_grouped_projection_args* args, bool b
   if (!many && fast::group_with_quantize_supported(a.routes, a.slots)) {  // one launch for both
     if ((rc = fast::quantize_rows_and_group(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, false, s, nullptr, 1, a.slots, a.rhs, a.routes, group_cols, groups, wait_status, dead))) return rc;
   } else {
-    if ((rc = fast::group_routes(a.rhs, a.routes, a.slots, group_cols, groups, wait_status, s))) return rc;
+    // The projection kernel reads its codebook before it waits for its predecessors.  8-bit calls take any
+    // table, one that a kernel has just written too: their first launch is an ordinary one, and what it
+    // waited for is in place for all that follow.  (A 16-bit table has been read back by its caller.)
+    if ((rc = fast::group_routes(a.rhs, a.routes, a.slots, group_cols, groups, wait_status, s, !byte_codes))) return rc;
     if (many) rc = fast::quantize_rows_sorted(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, groups.position, x_div, s, dead);
     else rc = fast::quantize_rows_and_group(a.x, a.x_dtype, x_rows, a.in_dim, a.groups, xq, false, s, nullptr, 1, a.slots, nullptr, 0, 0, {}, nullptr, dead);
     if (rc) return rc;

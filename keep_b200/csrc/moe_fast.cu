@@ -369,14 +369,14 @@ __global__ void __launch_bounds__(GR_THREADS) group_routes_kernel(const uint32_t
   group_routes_block<GR_THREADS>(served_slot, routes, slots, max_group, out, clear, group_scratch);
 }
 
-int group_routes(const uint32_t* served_slot, int64_t routes, int64_t slots, int max_group, const RouteGroups& out, int32_t* clear, cudaStream_t s) {
+int group_routes(const uint32_t* served_slot, int64_t routes, int64_t slots, int max_group, const RouteGroups& out, int32_t* clear, cudaStream_t s, bool early) {
   if (routes > (1 << 20) || slots > 16384) return KEEPVQ_ERR_CAPACITY;
   const size_t smem = static_cast<size_t>(slots) * 3 * sizeof(int32_t);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(group_routes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return note_cuda_error(e);
   }
-  cudaError_t err = launch_after(routes <= 4 * EARLY_LAUNCH_MAX_BLOCKS, group_routes_kernel, 1, GR_THREADS, smem, s, served_slot, static_cast<int>(routes), static_cast<int>(slots), max_group, out, clear);
+  cudaError_t err = launch_after(early && routes <= 4 * EARLY_LAUNCH_MAX_BLOCKS, group_routes_kernel, 1, GR_THREADS, smem, s, served_slot, static_cast<int>(routes), static_cast<int>(slots), max_group, out, clear);
   if (err != cudaSuccess) return note_cuda_error(err);
   return KEEPVQ_OK;
 }

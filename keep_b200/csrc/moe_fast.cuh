@@ -274,7 +274,8 @@ bool group_with_quantize_supported(int64_t routes, int64_t slots);
 int quantize_rows_and_group(const void* x, int32_t x_dtype, int64_t rows, int64_t in_dim, int64_t groups, const QuantRows& out, bool planes, cudaStream_t s,
                             const uint32_t* live_slot, int32_t per_row, int64_t slots,
                             const uint32_t* served_slot, int64_t routes, int max_group, const RouteGroups& route_groups, int32_t* clear, const DeadRows& dead = {});
-int group_routes(const uint32_t* served_slot, int64_t routes, int64_t slots, int max_group, const RouteGroups& out, int32_t* clear, cudaStream_t s);
+// early = false: an ordinary launch, behind everything the stream's kernels before it wrote.
+int group_routes(const uint32_t* served_slot, int64_t routes, int64_t slots, int max_group, const RouteGroups& out, int32_t* clear, cudaStream_t s, bool early = true);
 // Routes per group for a decode call: four while experts rarely get more (the kernels then run one
 // MMA per step for both byte planes), eight beyond.  `live` = routes expected to carry a slot.
 int decode_group_routes(int64_t live, int64_t slots, int64_t widest_in_dim);

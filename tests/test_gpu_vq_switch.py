@@ -255,6 +255,27 @@ def test_wide_rows_keep_their_integer_sums(cuda, bits, inp, word, code):
     np.testing.assert_allclose(f32(got), want, rtol=2.0 ** -8)  # exact sums, one rounding to bf16
 
 
+def test_a_codebook_written_just_before_the_call(cuda):
+    """A table that a kernel on the stream changes in place between calls: each call decodes the words it finds."""
+    from keep_b200 import kernels, vq_switch
+
+    gen = torch.Generator(device=cuda).manual_seed(29)
+    codes = torch.randint(0, 256, (4, 256, 64), generator=gen, device=cuda, dtype=torch.uint8)
+    scales = torch.full((4, 256, 1), 0.02, dtype=torch.float16, device=cuda)
+    x = torch.randn((64, 512), generator=gen, device=cuda).to(torch.bfloat16)
+    rhs = torch.randint(0, 4, (64, 2), generator=gen, device=cuda, dtype=torch.int32)
+    tables = torch.randint(-2 ** 31, 2 ** 31 - 1, (8, 256), generator=gen, device=cuda, dtype=torch.int32)
+    want = [kernels.routed_matvec(x, codes, scales, t, rhs.reshape(-1), x_div=2, code_bits=8).reshape(64, 2, 256) for t in tables]
+    table = torch.empty(256, dtype=torch.int32, device=cuda)
+    torch.cuda.synchronize()
+    got = []
+    for t in tables.repeat(8, 1):
+        torch.add(t, 0, out=table)  # a kernel, not a copy
+        got.append(vq_switch.gather_vqmm(x, codes, scales, table, rhs, input_dims=512, output_dims=256, group_size=512, code_bits=8))
+    for i, y in enumerate(got):
+        assert ((y.float() - want[i % 8].float()).norm() / want[i % 8].float().norm()).item() < 4e-3  # two roundings to bf16
+
+
 def test_calls_on_two_streams_do_not_share_scratch(cuda):
     """The same shapes on two streams that may overlap, 8-bit and 16-bit codes: each call's own result."""
     from keep_b200 import vq, vq_switch
