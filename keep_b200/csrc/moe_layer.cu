@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const T* __restrict__ down
     float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     // Six at a time: their slots, then their rows, are all in flight together, and are added in pick
     // order.  (Pick by pick, a slot and then its row, a call of one token waited for twelve reads in turn.)
-    constexpr int AT_ONCE = 6;
+    constexpr int AT_ONCE = 6;  // measured with six picks; eight go as six and two, not timed apart
     constexpr int WORDS = 8 * sizeof(T) / 16;
     for (int j0 = 0; j0 < top_k; j0 += AT_ONCE) {
       bool live[AT_ONCE];
