@@ -102,6 +102,16 @@ static int grouped_projection(const keepvq_grouped_projection_args* args, bool b
   fast::RouteGroups groups = {reinterpret_cast<int32_t*>(ws + sc.gcount), reinterpret_cast<int32_t*>(ws + sc.gslot),
                               reinterpret_cast<int32_t*>(ws + sc.gstart), reinterpret_cast<int32_t*>(ws + sc.gsize),
                               reinterpret_cast<int32_t*>(ws + sc.groutes)};
+  if (!byte_codes && !residual && a.routes < fast::SMALL_CALL_ROUTES && fast::few_tokens_fits(a.routes, 1, a.slots, a.out_dim, a.in_dim, a.groups)) {
+    fast::FewTokensArgs f = {};  // few routes: one launch that quantises and groups for itself
+    f.parts = fast::FT_DOWN;
+    f.routes = static_cast<int32_t>(a.routes); f.tokens = static_cast<int32_t>(x_rows); f.top_k = x_div;
+    f.scales_dtype = a.scales_dtype; f.slots = a.slots; f.codebook = a.codebook; f.slot = a.rhs;
+    f.phase[1] = {{a.codes, nullptr}, {a.scales, nullptr}, a.x, a.out, static_cast<int32_t>(a.out_dim), static_cast<int32_t>(a.in_dim), static_cast<int32_t>(a.groups), x_div, a.out_dtype};
+    f.dead_out = a.out; f.dead_row_bytes = a.out_dim * dtype_size(a.out_dtype);
+    f.status = reinterpret_cast<int32_t*>(ws + sc.status);
+    return fast::few_tokens(f, a.x_dtype, nullptr, s);
+  }
   const bool many = byte_codes || (!residual && fast::prefill_pays(a.routes, a.slots, a.groups > 1) && fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups));
   // (the sums region has room for a scale group per codeword; these kernels' rows have at most one
   // per 256 inputs, and their sums per 256 inputs go behind those)

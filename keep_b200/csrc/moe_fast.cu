@@ -107,52 +107,22 @@ __device__ __forceinline__ void quantize_row(const XT* __restrict__ xr, int64_t 
     team_sync();  // everyone has read warp_max
     top_bits = team_max(__float_as_uint(amax));
   }
-  const float m = __uint_as_float(top_bits);
-  float s = 1.0f;
-  if (m > 0.0f && isfinite(m)) {
-    // |x| / s < 2^15 with s a power of two: the exponent of m, less 14
-    s = top_bits >= (16u << 23) ? __uint_as_float((top_bits & 0x7F800000u) - (14u << 23)) : ldexpf(1.0f, ilogbf(m) - 14);
-    if (m / s > 32639.0f) s *= 2.0f;  // 127 * 256 + 127: the largest value two signed bytes hold
-  }
-  const float inv = 1.0f / s;  // exact: a power of two
+  float inv;
+  const float s = quant_scale(top_bits, inv);
   const bool plain = !odd && isfinite(inv);
 
   auto convert = [&](const float (&v)[8], int c) {
-    uint32_t t[8];  // the low 16 bits: x' in two's complement
-    int total = 0;
-    if (plain) {    // |x / s| <= 32639: 2^23 + 2^22 added to it rounds it to nearest even, as a conversion would
-#pragma unroll
-      for (int d = 0; d < 8; ++d) {
-        t[d] = __float_as_uint(fmaf(v[d], inv, 12582912.0f));
-        total += static_cast<int>(t[d]);
-      }
-      total -= static_cast<int>(8u * 0x4B400000u);
-    } else {
-#pragma unroll
-      for (int d = 0; d < 8; ++d) {
-        const int q = max(-32639, min(32639, __float2int_rn(v[d] * inv)));
-        t[d] = static_cast<uint32_t>(q);
-        total += q;
-      }
-    }
-    const int chunk_total = __reduce_add_sync(0xFFFFFFFFu, total);
+    const QuantWords w = quantize8(v, inv, plain);
+    const int chunk_total = __reduce_add_sync(0xFFFFFFFFu, w.total);
     if (lane == 0) sm[c >> 5] = chunk_total;
-    // x' = 256 * hi + lo with both bytes signed: lo is the low byte, hi the second byte of x' + 128.
-    // byte j of word 0 pairs with table nibble 3-j = dim 6-2j; of word 1 with nibble 7-j = dim 7-2j
-    const uint32_t lo0 = __byte_perm(__byte_perm(t[6], t[4], 0x0040), __byte_perm(t[2], t[0], 0x0040), 0x5410);
-    const uint32_t lo1 = __byte_perm(__byte_perm(t[7], t[5], 0x0040), __byte_perm(t[3], t[1], 0x0040), 0x5410);
-#pragma unroll
-    for (int d = 0; d < 8; ++d) t[d] += 128u;
-    const uint32_t hi0 = __byte_perm(__byte_perm(t[6], t[4], 0x0051), __byte_perm(t[2], t[0], 0x0051), 0x5410);
-    const uint32_t hi1 = __byte_perm(__byte_perm(t[7], t[5], 0x0051), __byte_perm(t[3], t[1], 0x0051), 0x5410);
     for (int j = 0; j < targets; ++j) {
       const int64_t row = target(j);
       if (row < 0) continue;
       if (planes) {  // high bytes of every row first, then the low bytes: what the tcgen05 B tiles copy from
-        reinterpret_cast<uint2*>(out.q)[row * cw + c] = make_uint2(hi0, hi1);
-        reinterpret_cast<uint2*>(out.q + (rows + 1) * cw * 8)[row * cw + c] = make_uint2(lo0, lo1);
+        reinterpret_cast<uint2*>(out.q)[row * cw + c] = make_uint2(w.hi0, w.hi1);
+        reinterpret_cast<uint2*>(out.q + (rows + 1) * cw * 8)[row * cw + c] = make_uint2(w.lo0, w.lo1);
       } else {
-        reinterpret_cast<uint4*>(out.q)[row * cw + c] = make_uint4(hi0, hi1, lo0, lo1);
+        reinterpret_cast<uint4*>(out.q)[row * cw + c] = make_uint4(w.hi0, w.hi1, w.lo0, w.lo1);
       }
     }
   };

@@ -85,6 +85,16 @@ __device__ __forceinline__ void decode_codeword_nibble(uint32_t word, uint32_t a
   asm("lop3.b32 %0, %1, %2, 0xF0F0F0F0, 0x28;" : "=r"(top) : "r"(e), "r"(m));
   hi = top >> 4;
 }
+// The same without the shift: `odd` are the odd dims' bytes times 16, for kernels that give the odd dims
+// MMAs and accumulators of their own (whose sums are then 16 times too large, exactly).
+template <bool ODD>
+__device__ __forceinline__ void decode_codeword_halves(uint32_t word, uint32_t abs_lane, uint32_t sign_lane, uint32_t& even, uint32_t& odd) {
+  uint32_t e, m;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(e) : "r"(__byte_perm(word, abs_lane, ODD ? 0x7634 : 0x7614)));
+  asm("ld.shared.u32 %0, [%1];" : "=r"(m) : "r"(__byte_perm(word, sign_lane, ODD ? 0x7624 : 0x7604)));
+  asm("lop3.b32 %0, %1, %2, 0x0F0F0F0F, 0x28;" : "=r"(even) : "r"(e), "r"(m));
+  asm("lop3.b32 %0, %1, %2, 0xF0F0F0F0, 0x28;" : "=r"(odd) : "r"(e), "r"(m));
+}
 __device__ __forceinline__ uint32_t pack_nibbles(uint2 v) { return (v.x & 0x0F0F0F0Fu) | ((v.y & 0x0F0F0F0Fu) << 4); }
 // All `threads` threads of the CTA (whole warps) fill the 64 KB region at `region` (shared address on
 // a 64 KB boundary): a thread works out one entry (one load of the codebook, all in flight together),
@@ -125,6 +135,64 @@ __device__ __forceinline__ void decode_byte_code(uint32_t word, int byte, uint32
   lo = e & 0x0F0F0F0Fu;
   hi = (e >> 4) & 0x0F0F0F0Fu;
 }
+// ------------------------------------------------------------------------------------------
+// Activations -> 16-bit fixed point: the scale of a row from its largest magnitude (the bits of a
+// float; not finite: 1), and eight values as the bytes of a codeword's operand words.
+// ------------------------------------------------------------------------------------------
+// Returns the scale, a power of two; `inv` = 1 / scale, exact (infinite for rows of the smallest subnormals).
+static __device__ __noinline__ float quant_scale_small(uint32_t top_bits) {  // rows of zeros, of very small values, or without a finite maximum
+  const float m = __uint_as_float(top_bits);
+  float s = 1.0f;
+  if (m > 0.0f && isfinite(m)) {
+    s = ldexpf(1.0f, ilogbf(m) - 14);
+    if (m / s > 32639.0f) s *= 2.0f;
+  }
+  return s;
+}
+__device__ __forceinline__ float quant_scale(uint32_t top_bits, float& inv) {
+  if (top_bits >= (16u << 23) && top_bits < 0x7F800000u) {
+    // |x| / s < 2^15 with s a power of two: the exponent of the maximum, less 14
+    uint32_t bits = (top_bits & 0x7F800000u) - (14u << 23);
+    if (__uint_as_float(top_bits) * __uint_as_float((254u << 23) - bits) > 32639.0f) bits += 1u << 23;  // 127 * 256 + 127: the largest value two signed bytes hold
+    inv = __uint_as_float((254u << 23) - bits);
+    return __uint_as_float(bits);
+  }
+  const float s = quant_scale_small(top_bits);
+  inv = 1.0f / s;
+  return s;
+}
+struct QuantWords { uint32_t hi0, hi1, lo0, lo1; int total; };
+// `inv` = 1 / scale, exact.  plain: the values are finite and |v * inv| <= 32639.
+__device__ __forceinline__ QuantWords quantize8(const float (&v)[8], float inv, bool plain) {
+  QuantWords w;
+  uint32_t t[8];  // the low 16 bits: x' in two's complement
+  w.total = 0;
+  if (plain) {    // 2^23 + 2^22 added to v * inv rounds it to nearest even, as a conversion would
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+      t[d] = __float_as_uint(fmaf(v[d], inv, 12582912.0f));
+      w.total += static_cast<int>(t[d]);
+    }
+    w.total -= static_cast<int>(8u * 0x4B400000u);
+  } else {
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+      const int q = max(-32639, min(32639, __float2int_rn(v[d] * inv)));
+      t[d] = static_cast<uint32_t>(q);
+      w.total += q;
+    }
+  }
+  // x' = 256 * hi + lo with both bytes signed: lo is the low byte, hi the second byte of x' + 128.
+  // byte j of word 0 pairs with table nibble 3-j = dim 6-2j; of word 1 with nibble 7-j = dim 7-2j
+  w.lo0 = __byte_perm(__byte_perm(t[6], t[4], 0x0040), __byte_perm(t[2], t[0], 0x0040), 0x5410);
+  w.lo1 = __byte_perm(__byte_perm(t[7], t[5], 0x0040), __byte_perm(t[3], t[1], 0x0040), 0x5410);
+#pragma unroll
+  for (int d = 0; d < 8; ++d) t[d] += 128u;
+  w.hi0 = __byte_perm(__byte_perm(t[6], t[4], 0x0051), __byte_perm(t[2], t[0], 0x0051), 0x5410);
+  w.hi1 = __byte_perm(__byte_perm(t[7], t[5], 0x0051), __byte_perm(t[3], t[1], 0x0051), 0x5410);
+  return w;
+}
+
 // Quantised activation rows: the B operand of the projections.
 struct QuantRows {
   uint8_t* q;       // [rows + 1, in_dim/8, 16] (last row all zero): per codeword 4 words: hi(dims 6,4,2,0) hi(7,5,3,1) lo(...) lo(...)
@@ -297,6 +365,48 @@ int slab_split_down(const FastProjectionArgs& args, cudaStream_t s);
 bool sweep_supported(int64_t in_dim);
 int sweep_gate_up(const FastProjectionArgs& args, cudaStream_t s);
 int sweep_down(const FastProjectionArgs& args, cudaStream_t s);
+
+// The few-token kernel (few_tokens.cu): a whole layer call, or part of one, in one launch, for calls of
+// few routes; also a single routed projection (FT_DOWN alone).
+constexpr int FT_MAX_ROUTES = 144;  // at most one per CTA
+constexpr int FT_MAX_TOKENS = 23;   // from 24 tokens on the logits have a faster kernel of their own (router.cu)
+constexpr int FT_MAX_CTAS = 160;
+enum : uint32_t { FT_ROUTER = 1, FT_GATE_UP = 2, FT_DOWN = 4, FT_COMBINE = 8 };
+struct FewTokensPhase {
+  const uint16_t* codes[2];   // gate and up, or the one matrix and null
+  const void* scales[2];
+  const void* x;              // activation rows; route r reads row r / x_div
+  void* out;                  // [routes, out_dim]
+  int32_t out_dim, in_dim, groups, x_div, out_dtype;
+  int32_t n_chunks, chunks_per_group, units_per_group;  // the rest is filled in by the launch
+  uint64_t by_chunks, by_group_chunks, by_units;        // their divisors for ft_div
+};
+struct FewTokensArgs {
+  uint32_t parts;             // FT_ROUTER only with FT_GATE_UP; FT_COMBINE only with FT_GATE_UP and FT_DOWN
+  int32_t routes, tokens, top_k, scales_dtype;
+  int64_t slots;
+  const uint32_t* codebook;
+  FewTokensPhase phase[2];    // gate/up, down
+  keepvq_router_logits_args logits;  // FT_ROUTER
+  keepvq_routed_topk_args topk;
+  const uint32_t* slot;       // without FT_ROUTER: the routes' slots and gate weights (weight may be null: 1)
+  const float* weight;
+  float swiglu_limit;
+  void* out;                  // FT_COMBINE: the pick sums, in the activation dtype, plus `shared` (may be null)
+  const float* shared;
+  void* dead_out;             // rows of routes without a slot are zeroed here (may be null)
+  int64_t dead_row_bytes;
+  int32_t* status;            // cleared; 1: a wait of the grid ran out, 2: unexpected shared window
+  uint64_t* barrier_words;    // filled in by the launch
+  uint32_t* counters;
+  uint64_t token, by_grid;
+  uint32_t act_bytes;
+  int32_t group_shift;
+};
+bool few_tokens_fits(int64_t routes, int64_t tokens, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups);
+bool few_tokens_router_fits(const keepvq_router_logits_args& logits, const keepvq_routed_topk_args& topk);
+int64_t few_tokens_sync_bytes(int64_t tokens, int64_t out_dim);  // scratch of a call with gate/up and down, any contents
+int few_tokens(const FewTokensArgs& a, int32_t x_dtype, void* sync, cudaStream_t s);
 
 // tcgen05 kernels for many routes per expert (prefill_umma.cu).  `status` is a device word that
 // a CTA sets to 1 if one of its bounded waits expires.

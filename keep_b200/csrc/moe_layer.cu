@@ -227,28 +227,55 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
   // slots would only put a dependent load in front of every row
   const uint32_t* padded = live < routes ? a.served_slot : nullptr;
 
+  // few routes: whatever part of the layer the call asks for as one launch of the few-token kernel
+  const bool few = tensor_path && !residual && !prefill && routes < fast::SMALL_CALL_ROUTES && fast::few_tokens_fits(routes, a.tokens, a.slots, a.inter, a.hidden, a.w1.groups) &&
+                   fast::few_tokens_fits(routes, a.tokens, a.slots, a.hidden, a.inter, a.w2.groups) && a.inter % 16 == 0 && a.hidden % 32 == 0 && aligned_to(a.x, 16) && aligned_to(a.w1.codes, 16) && aligned_to(a.w3.codes, 16) && aligned_to(a.w2.codes, 16) &&
+                   fast::few_tokens_sync_bytes(a.tokens, a.hidden) <= sc.h - sc.gate;
+  bool router_fused = false;
+  fast::FewTokensArgs few_args = {};
+
   if (stages & KEEPVQ_STAGE_ROUTER) {
     keepvq_router_logits_args rl = {};
     rl.x = a.x; rl.x_dtype = a.x_dtype; rl.router_w = a.router_w; rl.router_dtype = a.router_dtype;
     rl.tokens = a.tokens; rl.pool = a.pool; rl.hidden = a.hidden; rl.gate_temp = a.gate_temp;
     rl.logits = reinterpret_cast<float*>(ws + sc.logits);
-    // few tokens: the logits and the quantised token rows of the projections in one launch
-    const bool front = (stages & KEEPVQ_STAGE_PREPARE) && tensor_path && !prefill && valid_dtype(a.router_dtype) && a.router_w && a.gate_temp > 0.0f &&
-                       aligned_to(a.x, 16) && aligned_to(a.router_w, 16) && fast::logits_and_quantize_supported(rl, a.w1.groups);
-    if (front) {
-      if ((rc = fast::logits_and_quantize(rl, a.w1.groups, xq, s))) return rc;
-      x_quantized = true;
-    } else if ((rc = keepvq_router_logits(&rl, stream))) return rc;
     keepvq_routed_topk_args tk = {};
     tk.logits = rl.logits; tk.tokens = a.tokens; tk.pool = a.pool; tk.top_k = a.top_k; tk.score_func = a.score_func;
     tk.norm_topk_prob = a.norm_topk_prob; tk.route_scale = a.route_scale; tk.tau = a.tau;
     tk.served_bias = a.served_bias; tk.pool_bias = a.pool_bias; tk.slot_of = a.slot_of;
     tk.served_expert = a.served_expert; tk.served_slot = a.served_slot; tk.served_weight = a.served_weight;
     tk.want = a.want; tk.want_score = a.want_score; tk.admit = a.admit;
-    if ((rc = keepvq_routed_topk(&tk, stream))) return rc;
+    router_fused = few && (stages & KEEPVQ_STAGE_GATE_UP) && fast::few_tokens_router_fits(rl, tk);
+    if (router_fused) {
+      few_args.logits = rl;
+      few_args.topk = tk;
+    } else {
+      // few tokens: the logits and the quantised token rows of the projections in one launch
+      const bool front = (stages & KEEPVQ_STAGE_PREPARE) && tensor_path && !prefill && !few && valid_dtype(a.router_dtype) && a.router_w && a.gate_temp > 0.0f &&
+                         aligned_to(a.x, 16) && aligned_to(a.router_w, 16) && fast::logits_and_quantize_supported(rl, a.w1.groups);
+      if (front) {
+        if ((rc = fast::logits_and_quantize(rl, a.w1.groups, xq, s))) return rc;
+        x_quantized = true;
+      } else if ((rc = keepvq_router_logits(&rl, stream))) return rc;
+      if ((rc = keepvq_routed_topk(&tk, stream))) return rc;
+    }
   }
 
-  if (tensor_path) {
+  if (few) {
+    const bool gate_up = stages & KEEPVQ_STAGE_GATE_UP, down = stages & KEEPVQ_STAGE_DOWN;
+    if (gate_up || down) {
+      const bool combine = gate_up && down && (stages & KEEPVQ_STAGE_COMBINE);
+      few_args.parts = (router_fused ? fast::FT_ROUTER : 0u) | (gate_up ? fast::FT_GATE_UP : 0u) | (down ? fast::FT_DOWN : 0u) | (combine ? fast::FT_COMBINE : 0u);
+      few_args.routes = static_cast<int32_t>(routes); few_args.tokens = static_cast<int32_t>(a.tokens); few_args.top_k = a.top_k;
+      few_args.scales_dtype = a.scales_dtype; few_args.slots = a.slots; few_args.codebook = a.codebook;
+      few_args.phase[0] = {{a.w1.codes, a.w3.codes}, {a.w1.scales, a.w3.scales}, a.x, ws + sc.h, static_cast<int32_t>(a.inter), static_cast<int32_t>(a.hidden), static_cast<int32_t>(a.w1.groups), a.top_k, a.x_dtype};
+      few_args.phase[1] = {{a.w2.codes, nullptr}, {a.w2.scales, nullptr}, ws + sc.h, ws + sc.down, static_cast<int32_t>(a.hidden), static_cast<int32_t>(a.inter), static_cast<int32_t>(a.w2.groups), 1, a.x_dtype};
+      few_args.slot = a.served_slot; few_args.weight = a.served_weight; few_args.swiglu_limit = a.swiglu_limit;
+      few_args.out = a.out; few_args.shared = a.shared; few_args.status = reinterpret_cast<int32_t*>(ws + sc.status);
+      if ((rc = fast::few_tokens(few_args, a.x_dtype, ws + sc.gate, s))) return rc;  // (only the general kernel uses the gate and up rows)
+      if (combine) return KEEPVQ_OK;
+    }
+  } else if (tensor_path) {
     fast::RouteGroups groups = {reinterpret_cast<int32_t*>(ws + sc.gcount), reinterpret_cast<int32_t*>(ws + sc.gslot),
                                 reinterpret_cast<int32_t*>(ws + sc.gstart), reinterpret_cast<int32_t*>(ws + sc.gsize),
                                 reinterpret_cast<int32_t*>(ws + sc.groutes)};

@@ -43,8 +43,7 @@
 // mbarrier full/empty pairs carry every dependency.  Every wait is bounded by a deadline on the
 // global timer: on expiry the CTA raises a flag in `status`, stops issuing work, waits (bounded)
 // for the MMAs and the copies in flight, frees its tensor memory and returns.
-#include <cuda.h>  // CUtensorMap (types only: the one driver entry point is looked up through the runtime)
-
+#include "async_copy.cuh"
 #include "moe_fast.cuh"
 
 namespace keepvq {
@@ -109,31 +108,10 @@ struct PrefillPlan {
   }
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ uint64_t global_timer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-// One lane of a converged warp.
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t chosen;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
-  return chosen;
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // One arrival for the warp, predicated instead of a branch.
 __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar, int lane) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
-}
-__device__ __forceinline__ bool mbar_complete(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  return done != 0;
 }
 // Wait of a whole warp, bounded by time.  Returns false (in every lane) when the deadline passes (the
 // caller's CTA then gives up: the flag is raised for every role) or when another warp of the CTA
@@ -209,20 +187,10 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&v)[4]) {
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr) : "memory");
 }
 
-// One TMA box of the tensor map -> shared memory; completion is counted on `bar` in bytes.
-// x (bytes along K) is a multiple of 64 or 128 here and y a row index: both inside the rules for x.
-__device__ __forceinline__ void tma_box_2d(uint32_t dst, const CUtensorMap* map, int32_t x, int32_t y, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-               ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
-}
 __device__ __forceinline__ void tma_box_3d(uint32_t dst, const CUtensorMap* map, int32_t x, int32_t y, int32_t z, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
 // Place in a ring of STAGES stages: every role walks its rings on its own, an index and a phase bit.
 template <uint32_t STAGES>
 struct RingPlace {

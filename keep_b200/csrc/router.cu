@@ -21,7 +21,7 @@
 #include <math.h>
 
 #include "common.cuh"
-#include "router_logits.cuh"
+#include "router_topk.cuh"
 
 namespace keepvq {
 
@@ -306,15 +306,8 @@ __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 constexpr int TK_WARPS = 4;
 constexpr int TK_MAX_K = 16;
 
-// Floats as unsigned keys of the same order (-inf lowest of the real values); 0 is below all of them.
-__device__ __forceinline__ uint32_t ordered_key(float v) {
-  const uint32_t u = __float_as_uint(v);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-// One warp per token with the pool in registers (NPL experts per lane, expert e = lane + 32 i).
-// A pick is a register scan, one warp max and one warp min (redux.sync); no shared memory and no
-// loads inside the selection loops.  Same arithmetic and the same results as routed_topk_kernel.
+// One warp per token with the pool in registers (NPL experts per lane).  Same arithmetic and the
+// same results as routed_topk_kernel.
 template <int NPL>
 __global__ void __launch_bounds__(TK_WARPS * 32) routed_topk_reg_kernel(keepvq_routed_topk_args a) {
   grid_launch_dependents();
@@ -322,96 +315,24 @@ __global__ void __launch_bounds__(TK_WARPS * 32) routed_topk_reg_kernel(keepvq_r
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t t = static_cast<int64_t>(blockIdx.x) * TK_WARPS + warp;
   if (t >= a.tokens) return;
-  const int P = static_cast<int>(a.pool), K = a.top_k;
-  const float* lg = a.logits + t * P;
   float sc[NPL];
-#pragma unroll
-  for (int i = 0; i < NPL; ++i) { const int e = lane + 32 * i; sc[i] = e < P ? lg[e] : -INFINITY; }
-
-  // ---- score function --------------------------------------------------------------------
-  if (a.score_func == KEEPVQ_SCORE_SOFTMAX) {
-    float m = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) m = fmaxf(m, sc[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-    float s = 0.0f;
-#pragma unroll
-    for (int i = 0; i < NPL; ++i)
-      if (lane + 32 * i < P) { sc[i] = expf(sc[i] - m); s += sc[i]; }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) sc[i] = sc[i] / s;
-  } else if (a.score_func == KEEPVQ_SCORE_SIGMOID) {
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) sc[i] = 1.0f / (1.0f + expf(-sc[i]));
-  } else {
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) { const float v = sc[i]; sc[i] = sqrtf(v > 20.0f ? v : log1pf(expf(v))); }
-  }
+  topk_scores<NPL>(a, t, lane, sc);
   if (a.scores) {
 #pragma unroll
     for (int i = 0; i < NPL; ++i)
-      if (lane + 32 * i < P) a.scores[t * P + lane + 32 * i] = sc[i];
+      if (lane + 32 * i < a.pool) a.scores[t * a.pool + lane + 32 * i] = sc[i];
   }
-
-  // ---- two selections over the same scores -------------------------------------------------
   for (int pass = 0; pass < 2; ++pass) {
-    const float* bias = pass == 0 ? a.served_bias : a.pool_bias;
-    uint32_t key[NPL];
+    uint32_t key[NPL], slot, my_key;
+    int id[NPL], my_e;
+    float weight;
 #pragma unroll
     for (int i = 0; i < NPL; ++i) {
-      const int e = lane + 32 * i;
-      key[i] = e < P ? max(ordered_key(sc[i] + (bias ? bias[e] : 0.0f)), 1u) : 0u;
+      id[i] = lane + 32 * i;
+      key[i] = id[i] < a.pool ? topk_key(pass == 0 ? a.served_bias : a.pool_bias, id[i], sc[i]) : 0u;
     }
-    int my_e = 0;       // lane j keeps pick j
-    float my_raw = 0.0f;
-    for (int j = 0; j < K; ++j) {
-      uint32_t bu = 0u, bi = 0xFFFFFFFFu;
-#pragma unroll
-      for (int i = 0; i < NPL; ++i)
-        if (key[i] > bu) { bu = key[i]; bi = lane + 32 * i; }
-      const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, bu);
-      const uint32_t win = __reduce_min_sync(0xFFFFFFFFu, bu == top ? bi : 0xFFFFFFFFu);  // ties: the lowest expert id
-      float raw = 0.0f;
-#pragma unroll
-      for (int i = 0; i < NPL; ++i)
-        if (static_cast<uint32_t>(lane + 32 * i) == win) { raw = sc[i]; key[i] = 0u; }
-      raw = __shfl_sync(0xFFFFFFFFu, raw, win & 31u);
-      if (lane == j) { my_e = static_cast<int>(win); my_raw = raw; }
-    }
-    float raw = 0.0f;
-    bool live = false;
-    if (lane < K) {
-      raw = my_raw;
-      live = pass == 1 || !a.served_bias || a.served_bias[my_e] > ABSENT_BIAS;
-      if (!live) raw = 0.0f;  // a masked pick carries no weight (local_eval.py:87)
-    }
-    float sum = raw;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    if (lane < K) {
-      const int e = my_e;
-      const int64_t o = t * K + lane;
-      if (pass == 0) {
-        float w = raw;
-        if (a.norm_topk_prob && K > 1) w = w / (sum + 1e-20f);
-        w *= a.route_scale;
-        a.served_weight[o] = w;
-        a.served_expert[o] = live ? static_cast<uint32_t>(e) : KEEPVQ_NO_RESIDUAL;
-        a.served_slot[o] = live ? (a.slot_of ? a.slot_of[e] : static_cast<uint32_t>(e)) : KEEPVQ_NO_RESIDUAL;
-      } else {
-        a.want[o] = static_cast<uint32_t>(e);
-        a.want_score[o] = raw;
-        if (a.admit) {
-          // the policy's own normalisation: always over the k demanded scores (omlx_routed.py:186)
-          const float g = raw / (sum + 1e-20f) * a.route_scale;
-          const bool absent = a.served_bias && a.served_bias[e] <= ABSENT_BIAS;
-          a.admit[o] = (absent && g >= a.tau) ? e : -1;
-        }
-      }
-    }
+    topk_select<NPL>(key, id, a.top_k, lane, my_key, my_e);
+    topk_finish(a, t, lane, pass, my_e, topk_raw_from_registers<NPL>(sc, my_e, lane, a.top_k), true, slot, weight);
   }
 }
 

@@ -1,0 +1,147 @@
+"""The few-token kernel (csrc/few_tokens.cu): a layer call of few routes as one launch.
+
+Against the CPU oracle at the sizes where its shares of the work change shape: one to seven tokens (one,
+two and four routes to a group, rows staged by token and by group, deep and shallow code rings),
+fewer chunks than warps, scale groups that close inside a warp's run, a second group that begins in
+a block's run.  Bound of the outputs: the layer's own (three roundings to the activation dtype)."""
+
+import numpy as np
+import pytest
+import torch
+
+import synthetic
+from oracle import e8
+from test_gpu_moe_layer import build_layer, check_layer
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens,experts,top_k,hidden,inter,group_hidden,group_inter,score", [
+    (1, 20, 2, 256, 256, None, None, "softmax"),      # one chunk of inputs a row: fewer chunks than warps
+    (2, 384, 6, 512, 256, None, 256, "sigmoid"),      # the largest pool the kernel's own router takes
+    (4, 6, 5, 768, 512, 256, 256, "softmax"),         # several groups of four on one expert
+    (7, 33, 6, 4096, 512, None, None, "softmax"),     # a scale group of sixteen chunks; 42 routes
+    (3, 12, 6, 5120, 768, 512, 256, "sqrtsoftplus"),  # the widest rows, scale groups of two chunks and of one
+    (8, 12, 5, 2560, 256, None, None, "softmax"),     # eight tokens staged by token, two rounds of picks
+    (9, 12, 5, 512, 2304, 256, 768, "softmax"),       # rows staged by group
+    (23, 40, 2, 512, 256, None, None, "softmax"),     # the most tokens; six rounds of picks
+    (2, 400, 3, 512, 256, None, None, "softmax"),     # a pool whose router runs in front
+])
+def test_layer_calls_of_few_routes(cuda, tokens, experts, top_k, hidden, inter, group_hidden, group_inter, score):
+    cfg = synthetic.layer(seed=71, experts=experts, hidden=hidden, inter=inter, group_hidden=group_hidden, group_inter=group_inter)
+    x = synthetic.tokens(72 + tokens, tokens, hidden)
+    layer = build_layer(cuda, cfg, top_k=top_k, score_func=score)
+    assert layer.launches_per_call(tokens) == (1 if experts <= 384 else 3)
+    layer.decode(x.to(cuda))
+    for buf in layer._buffers.values():
+        buf["workspace"].fill_(0x7F)  # whatever the scratch holds, the barrier words of an earlier call among it
+    out, routing = layer.decode(x.to(cuda))
+    assert not layer.wait_expired(tokens, x.dtype)
+    check_layer(cfg, x, out, routing, top_k=top_k, score_func=score)
+
+
+def test_stage_by_stage_and_replayed_from_a_graph(cuda):
+    """The parts of a call one after the other, and a captured call replayed (which finds its own
+    barrier words in the scratch), give what the whole call gives, to the bit."""
+    from keep_b200 import _lib
+
+    cfg = synthetic.layer(seed=73, experts=16, hidden=1024, inter=512, group_hidden=256, group_inter=256)
+    layer = build_layer(cuda, cfg, top_k=5)
+    xs = [synthetic.tokens(74 + i, 5, 1024).to(cuda) for i in range(3)]
+    want = [layer.decode(x)[0].clone() for x in xs]
+    for x, w in zip(xs, want):
+        for stage in (_lib.STAGE_ROUTER, _lib.STAGE_PREPARE, _lib.STAGE_GATE_UP, _lib.STAGE_DOWN, _lib.STAGE_COMBINE):
+            got, _ = layer.decode(x, stages=stage, state=1)
+        assert torch.equal(got, w)
+    x = xs[0].clone()
+    layer.decode(x, state=2)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got, _ = layer.decode(x, state=2)
+    for i in (1, 2, 0, 1):
+        x.copy_(xs[i])
+        graph.replay()
+        assert torch.equal(got, want[i])
+
+
+def test_calls_on_two_streams_at_once(cuda):
+    cfg = synthetic.layer(seed=75, experts=16, hidden=1024, inter=512)
+    layer = build_layer(cuda, cfg, top_k=4)
+    xs = [synthetic.tokens(76 + i, 4, 1024).to(cuda) for i in range(2)]
+    want = [layer.decode(x)[0].clone() for x in xs]
+    for i, x in enumerate(xs):
+        layer.decode(x, state=1 + i)
+    streams = [torch.cuda.Stream(cuda) for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        outs = []
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                outs.append(layer.decode(xs[i], state=1 + i)[0])
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, w) for o, w in zip(outs, want))
+
+
+def test_two_experts_of_one_slot_and_a_token_without_any(cuda):
+    """`slot_of` may name a slot twice (a token then has it twice), and every pick of a token may be absent."""
+    from oracle import router as oracle_router
+
+    pool, hidden, inter, k = 6, 512, 256, 2
+    cfg = synthetic.layer(seed=77, experts=pool, hidden=hidden, inter=inter)
+    x = synthetic.tokens(78, 1, hidden)
+    slot_of = np.array([0, 0, 1, 1, 2, 2], dtype=np.uint32)
+    slot_cfg = dict(cfg)
+    for n in ("w1", "w3", "w2"):
+        slot_cfg[n] = (cfg[n][0][:3], cfg[n][1][:3])
+    bias = np.array([0, 0, -1e30, -1e30, -1e30, -1e30], dtype=np.float32)
+    layer = build_layer(cuda, slot_cfg, top_k=k, served_bias=bias, slot_of=slot_of)
+    out, routing = layer.decode(x.to(cuda))
+    assert sorted(routing.served_slot.cpu().view(-1).tolist()) == [0, 0]
+    check_layer(slot_cfg, x, out, routing, top_k=k, served_bias=bias, slot_of=slot_of)
+    nothing = build_layer(cuda, slot_cfg, top_k=k, served_bias=np.full(pool, oracle_router.OFF, dtype=np.float32), slot_of=slot_of)
+    shared = torch.arange(hidden, dtype=torch.float32, device=cuda)[None]
+    out, _ = nothing.decode(x.to(cuda), shared=shared)
+    assert torch.equal(out, shared.to(out.dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("routes,out_dim,in_dim,group", [(1, 72, 256, 256), (5, 40, 1024, 256), (47, 8, 512, 512), (11, 2304, 5120, 512), (4, 1, 256, 256)])
+def test_single_projections_with_ragged_rows(cuda, dtype, routes, out_dim, in_dim, group):
+    """One routed product, output rows that are no multiple of a unit's, against decoded weights in fp64;
+    dead routes give zeros.  Bound: the 16-bit steps of the activations (2^-15 of a row's largest
+    magnitude each, so at most that times the sum of the weights' magnitudes) and the output's rounding."""
+    from keep_b200 import prefill, vq
+
+    rng = np.random.default_rng(79)
+    experts = 9
+    codes = torch.from_numpy(rng.integers(0, 65536, (experts, out_dim, in_dim // 8)).astype(np.uint16)).to(cuda)
+    scales = torch.from_numpy((0.02 * (0.5 + rng.random((experts, out_dim, in_dim // group)))).astype(np.float16)).to(cuda)
+    x = torch.from_numpy(rng.standard_normal((routes, in_dim)).astype(np.float32)).to(cuda).to(dtype)
+    rhs = torch.from_numpy(rng.integers(0, experts, routes).astype(np.int32)).to(cuda)
+    rhs[routes // 2] = -1 if routes > 1 else int(rhs[0])
+    y = prefill.tensor_core_projection(x, codes, scales, vq.table_on(cuda, "e8p"), rhs)
+    w = vq.decode_weight_matrix(codes, scales, code_bits=16).double()[rhs.long().clamp(min=0)]
+    want = torch.einsum("rk,rnk->rn", x.double(), w) * (rhs >= 0).double()[:, None]
+    bound = 2.0 ** -15 * x.double().abs().amax(1, keepdim=True) * w.abs().sum(2) + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * want.abs() + 1e-7
+    assert ((y.double() - want).abs() <= bound).all()
+    assert not y[rhs < 0].any()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+def test_rows_that_are_not_finite_touch_no_other(cuda, bad):
+    """A row with a NaN or an infinity beside ordinary ones: theirs do not change, and it goes through
+    the same steps as in calls of many routes (the slab kernels): equal outputs."""
+    from keep_b200 import prefill, vq
+
+    rng = np.random.default_rng(80)
+    codes = torch.from_numpy(rng.integers(0, 65536, (4, 64, 64)).astype(np.uint16)).to(cuda)
+    scales = torch.full((4, 64, 1), 0.02, dtype=torch.float16, device=cuda)
+    x = torch.randn((60, 512), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(cuda)
+    x[2, 100] = bad
+    rhs = (torch.arange(60, device=cuda) % 4).to(torch.int32)
+    table = vq.table_on(cuda, "e8p")
+    many = prefill.tensor_core_projection(x, codes, scales, table, rhs)
+    few = prefill.tensor_core_projection(x[:8].contiguous(), codes, scales, table, rhs[:8].contiguous())
+    gap = e8.relative_gap(few.float().cpu().numpy(), many[:8].float().cpu().numpy())
+    assert gap <= 2 ** -8  # fp32 sums in another order, one rounding to bf16
+    assert torch.isfinite(few).all()
