@@ -6,7 +6,9 @@ There is no CPU or eager fallback.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import struct
 import threading
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_int64, c_void_p
 from pathlib import Path
@@ -217,6 +219,35 @@ def dtype_tag(dtype: torch.dtype) -> int:
         return _DTYPE_TAG[dtype]
     except KeyError:
         raise ValueError(f"unsupported floating dtype {dtype}") from None
+
+
+_FORMAT = {c_void_p: "P", c_int32: "i", c_int64: "q", c_float: "f"}
+
+
+def packer(cls):
+    """A function from the values of all of ``cls``'s fields, in order (a nested struct's in its place;
+    pointers as integers, 0 for null), to an instance: a third of the time of keyword arguments, which
+    set their fields one by one."""
+    def fields(c):
+        return "".join(_FORMAT[kind] if kind in _FORMAT else fields(kind) for _, kind in c._fields_)
+
+    layout = struct.Struct("@" + fields(cls) + "0P")  # native alignment, and the struct's own at its end
+    assert layout.size == ctypes.sizeof(cls), cls
+    pack, make = layout.pack, cls.from_buffer_copy
+    return lambda *values: make(pack(*values))
+
+
+pack_layer_args = packer(MoELayerArgs)
+pack_grouped_args = packer(GroupedProjectionArgs)
+pack_matvec_args = packer(MatvecArgs)
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device(device)``, for nothing where that is the current one."""
+    if device.type == "cuda" and device.index == torch.cuda.current_device():
+        return _SAME_DEVICE
+    return torch.cuda.device(device)
 
 
 def ptr(t: torch.Tensor | None) -> c_void_p:

@@ -75,26 +75,17 @@ def routed_matvec(x, codes, scales, codebook, rhs, *, lhs=None, x_div=1, code_bi
     routes = int(rhs.numel())
     out_dtype = qmv_output_dtype(x.dtype) if out_dtype is None else out_dtype
     out = torch.empty((routes, out_dim), dtype=out_dtype, device=device)
-    args = _lib.MatvecArgs(
-        x=_lib.ptr(x), x_dtype=_lib.dtype_tag(x.dtype), x_rows=int(x.shape[0]),
-        codes=_lib.ptr(codes), code_bits=code_bits,
-        scales=_lib.ptr(scales), scales_dtype=_lib.dtype_tag(scales.dtype),
-        experts=experts, out_dim=out_dim, in_dim=cw * 8, groups=groups,
-        codebook=_lib.ptr(codebook), codebook_layout=layout,
-        rhs=_lib.ptr(rhs), lhs=_lib.ptr(lhs), x_div=int(x_div), routes=routes,
-        out=_lib.ptr(out), out_dtype=_lib.dtype_tag(out_dtype),
-    )
-    keep = [x, codes, scales, codebook, rhs, lhs]
+    res = (0, 0, 0, 0, 0, 0, 0)
     if residual is not None:
         res_codes, res_scales, res_table = residual
-        args.res_codes, args.res_scales = _lib.ptr(res_codes), _lib.ptr(res_scales)
-        args.res_scales_dtype = _lib.dtype_tag(res_scales.dtype)
-        args.res_rows, args.res_groups = int(res_codes.shape[0]), int(res_scales.shape[2])
-        args.res_table, args.hot_of_slot = _lib.ptr(res_table), _lib.ptr(hot_of_slot)
-        keep += [res_codes, res_scales, res_table, hot_of_slot]
-    with torch.cuda.device(device):
+        res = (res_codes.data_ptr(), res_scales.data_ptr(), _lib.dtype_tag(res_scales.dtype), res_codes.shape[0], res_scales.shape[2],
+               res_table.data_ptr(), hot_of_slot.data_ptr())
+    args = _lib.pack_matvec_args(
+        x.data_ptr(), _lib.dtype_tag(x.dtype), x.shape[0], codes.data_ptr(), code_bits, scales.data_ptr(), _lib.dtype_tag(scales.dtype),
+        experts, out_dim, cw * 8, groups, codebook.data_ptr(), layout, rhs.data_ptr(), 0 if lhs is None else lhs.data_ptr(), int(x_div), routes,
+        *res, out.data_ptr(), _lib.dtype_tag(out_dtype))
+    with _lib.on_device(device):
         _lib.check(_lib.load().keepvq_routed_matvec(args, _lib.stream_handle(device)), "keepvq_routed_matvec")
-    del keep
     return out
 
 
@@ -131,16 +122,37 @@ def _dense_reference(x2d, codes, scales, codebook, code_bits):
     return x2d.to(torch.float32) @ weights.T
 
 
-def _one_matrix(rows, codes, scales, table, rhs, code_bits):
+_zero_routes: dict = {}  # (device, stream) -> int32 zeros, read only: the expert of every route of a single matrix
+_ZEROS = 64
+
+
+def _routes_to_one(count: int, device: torch.device, stream: int) -> torch.Tensor:
+    """At least ``count`` int32 zeros (the launch that clears them was a tenth of a small call).  Kept per
+    stream, where every reader is behind the clearing, and for a few streams; a captured call's are
+    cleared in its graph and stay the graph's."""
+    if count > _ZEROS or torch.cuda.is_current_stream_capturing():
+        return torch.zeros(count, dtype=torch.int32, device=device)
+    key = (device, stream)
+    zeros = _zero_routes.get(key)
+    if zeros is None:
+        zeros = torch.zeros(_ZEROS, dtype=torch.int32, device=device)
+        if len(_zero_routes) < 16:
+            _zero_routes[key] = zeros
+    return zeros
+
+
+def _one_matrix(rows, codes, scales, table, code_bits, out_shape):
     """Every row of ``rows`` against the one matrix ``codes``: the int8 tensor-core kernels for
     16-bit codes with fp16 / bf16 rows when the shapes fit them, else the general kernel."""
-    out = None
-    if code_bits == 16 and rows.dtype in (torch.float16, torch.bfloat16):
-        from .prefill import tensor_core_projection
+    out, routes, (out_dim, cw) = None, rows.numel() // max(rows.shape[-1], 1), codes.shape
+    stream = torch.cuda.current_stream(rows.device).cuda_stream
+    rhs, scales = _routes_to_one(routes, rows.device, stream), scales.contiguous()
+    if code_bits == 16 and rows.dtype in (torch.float16, torch.bfloat16) and scales.dtype in _lib._DTYPE_TAG:
+        from .prefill import project
 
-        out = tensor_core_projection(rows, codes[None], scales.contiguous()[None], table, rhs)
+        out = project(rows, routes, cw * 8, codes, 1, out_dim, scales, scales.shape[1], table, rhs, out_shape, stream=stream)
     if out is None:
-        out = routed_matvec(rows, codes[None], scales.contiguous()[None], table, rhs, x_div=1, code_bits=code_bits)
+        out = routed_matvec(rows.reshape(routes, cw * 8), codes[None], scales[None], table, rhs[:routes], x_div=1, code_bits=code_bits).reshape(out_shape)
     return out
 
 
@@ -166,8 +178,7 @@ def vq_qmv(x, codes, scales, codebook=None, *, in_dim: int, out_dim: int, group_
     table = _codebook_tensor(codebook, code_bits, device)
     if implementation == "reference":
         return _dense_reference(x_t[None], codes_t, scales_t, table, code_bits)[0]
-    rhs = torch.zeros(1, dtype=torch.int32, device=device)
-    return _one_matrix(x_t[None], codes_t, scales_t, table, rhs, code_bits)[0]
+    return _one_matrix(x_t, codes_t, scales_t, table, code_bits, (out_dim,))
 
 
 def vq_qmm(x, codes, scales, codebook=None, *, in_dim: int, out_dim: int, group_size: int = 512, code_bits: int = 8,
@@ -189,8 +200,7 @@ def vq_qmm(x, codes, scales, codebook=None, *, in_dim: int, out_dim: int, group_
     table = _codebook_tensor(codebook, code_bits, device)
     if implementation == "reference":
         return _dense_reference(x_t, codes_t, scales_t, table, code_bits)
-    rhs = torch.zeros(int(x_t.shape[0]), dtype=torch.int32, device=device)
-    return _one_matrix(x_t, codes_t, scales_t, table, rhs, code_bits)
+    return _one_matrix(x_t, codes_t, scales_t, table, code_bits, (x_t.shape[0], out_dim))
 
 
 # --- few-token kernels -------------------------------------------------------------------------

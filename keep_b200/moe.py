@@ -24,6 +24,10 @@ from .router import Routing
 from .vq import as_device, table_on
 
 
+def _address(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
 @dataclass
 class Projection:
     """Codes ``[slots, out, in/8]`` uint16 and scales ``[slots, out, groups]`` of one projection,
@@ -34,11 +38,12 @@ class Projection:
     res_codes: torch.Tensor | None = None
     res_scales: torch.Tensor | None = None
 
-    def struct(self) -> _lib.ExpertWeights:
-        return _lib.ExpertWeights(
-            codes=_lib.ptr(self.codes), scales=_lib.ptr(self.scales), groups=int(self.scales.shape[2]),
-            res_codes=_lib.ptr(self.res_codes), res_scales=_lib.ptr(self.res_scales),
-            res_groups=int(self.res_scales.shape[2]) if self.res_scales is not None else 0)
+    def values(self) -> tuple:
+        """The fields of ``_lib.ExpertWeights``."""
+        if self.res_codes is None and self.res_scales is None:
+            return self.codes.data_ptr(), self.scales.data_ptr(), self.scales.shape[2], 0, 0, 0
+        return (self.codes.data_ptr(), self.scales.data_ptr(), self.scales.shape[2], _address(self.res_codes), _address(self.res_scales),
+                self.res_scales.shape[2] if self.res_scales is not None else 0)
 
 
 class SharedExpert:
@@ -144,21 +149,18 @@ class RoutedMoELayer:
         return self._buffers[key]
 
     def _layer_args(self, x, out, r: Routing, *, workspace, nbytes, expected_routes: int = 0, shared=None) -> _lib.MoELayerArgs:
-        """The argument struct of a layer call over the caller's tensors."""
-        return _lib.MoELayerArgs(
-            x=_lib.ptr(x), x_dtype=_lib.dtype_tag(x.dtype), tokens=int(x.shape[0]), hidden=self.hidden, inter=self.inter,
-            router_w=_lib.ptr(self.router_w), router_dtype=_lib.dtype_tag(self.router_w.dtype), pool=self.pool,
-            top_k=self.top_k, score_func=_lib.SCORE_FUNCS[self.score_func], norm_topk_prob=int(self.norm_topk_prob),
-            gate_temp=self.gate_temp, route_scale=self.route_scale, tau=self.tau,
-            served_bias=_lib.ptr(self.served_bias), pool_bias=_lib.ptr(self.pool_bias), slot_of=_lib.ptr(self.slot_of),
-            slots=self.slots, w1=self.w1.struct(), w3=self.w3.struct(), w2=self.w2.struct(),
-            scales_dtype=_lib.dtype_tag(self.w1.scales.dtype), codebook=_lib.ptr(self.codebook), res_rows=self.res_rows,
-            res_table=_lib.ptr(self.res_table), hot_of_slot=_lib.ptr(self.hot_of_slot), swiglu_limit=self.swiglu_limit,
-            codebook_all_odd=int(self.codebook_all_odd),
-            out=_lib.ptr(out), served_expert=_lib.ptr(r.served_expert), served_slot=_lib.ptr(r.served_slot),
-            served_weight=_lib.ptr(r.served_weight), want=_lib.ptr(r.want), want_score=_lib.ptr(r.want_score),
-            admit=_lib.ptr(r.admit), workspace=_lib.ptr(workspace), workspace_bytes=nbytes, expected_routes=int(expected_routes),
-            shared=_lib.ptr(shared))
+        """The argument struct of a layer call over the caller's tensors, its fields in order."""
+        return _lib.pack_layer_args(
+            x.data_ptr(), _lib.dtype_tag(x.dtype), x.shape[0], self.hidden, self.inter,
+            self.router_w.data_ptr(), _lib.dtype_tag(self.router_w.dtype), self.pool, self.top_k,
+            _lib.SCORE_FUNCS[self.score_func], int(self.norm_topk_prob), self.gate_temp, self.route_scale, self.tau,
+            _address(self.served_bias), _address(self.pool_bias), _address(self.slot_of),
+            self.slots, *self.w1.values(), *self.w3.values(), *self.w2.values(),
+            _lib.dtype_tag(self.w1.scales.dtype), self.codebook.data_ptr(), self.res_rows, _address(self.res_table),
+            _address(self.hot_of_slot), self.swiglu_limit, int(self.codebook_all_odd),
+            out.data_ptr(), r.served_expert.data_ptr(), r.served_slot.data_ptr(), r.served_weight.data_ptr(),
+            r.want.data_ptr(), r.want_score.data_ptr(), r.admit.data_ptr(),
+            _address(workspace), nbytes, int(expected_routes), _address(shared))
 
     def _scratch_rows(self, which: str, width: int, tokens: int, dtype: torch.dtype, state: int) -> torch.Tensor:
         buf = self._buffers_for(tokens, dtype, state)
@@ -269,10 +271,10 @@ class RoutedMoELayer:
         ``SharedExpert``'s output) is added to the routed sum before the one rounding.
         """
         _lib.require_cuda(x)
-        if x.ndim != 2 or int(x.shape[1]) != self.hidden:
+        if x.ndim != 2 or x.shape[1] != self.hidden:
             raise ValueError(f"x must be [tokens, {self.hidden}], found {tuple(x.shape)}")
         x = x.contiguous()
-        tokens = int(x.shape[0])
+        tokens = x.shape[0]
         if shared is not None:
             _lib.require_cuda(shared)
             if shared.dtype != torch.float32 or tuple(shared.shape) != (tokens, self.hidden) or not shared.is_contiguous():
@@ -281,6 +283,6 @@ class RoutedMoELayer:
         r: Routing = buf["routing"]
         target = buf["out"] if out is None else out
         args = self._layer_args(x, target, r, workspace=buf["workspace"], nbytes=buf["nbytes"], expected_routes=expected_routes, shared=shared)
-        with torch.cuda.device(self.device):
+        with _lib.on_device(self.device):
             _lib.check(_lib.load().keepvq_moe_decode_stages(args, int(stages), _lib.stream_handle(self.device)), "keepvq_moe_decode_stages")
         return target, r

@@ -20,7 +20,7 @@ from functools import lru_cache
 import torch
 
 from . import _lib
-from .kernels import qmv_output_dtype, routed_matvec
+from .kernels import routed_matvec
 
 _UNSUPPORTED = -5  # KEEPVQ_ERR_UNSUPPORTED
 _all_odd: dict = {}     # table data_ptr, device -> (the tensor, its version, every nibble odd): read back once per table, never per call
@@ -64,42 +64,45 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
     """``keepvq_grouped_projection`` (``_bytes`` for 8-bit codes): route ``r`` against activation row ``r // x_div`` of ``rows``
     (fp16 / bf16), optionally with a nested residual ``(res_codes, res_scales, res_table)``.
     Returns None when the library says these shapes are not for the tensor-core kernels."""
-    routes, in_dim = int(rhs.numel()), int(rows.shape[1])
-    slots, out_dim, groups = int(codes.shape[0]), int(codes.shape[1]), int(scales.shape[2])
-    if codes.dtype != (torch.uint8 if code_bits == 8 else torch.uint16) or in_dim % 256 or rows.dtype not in (torch.float16, torch.bfloat16):
+    routes = rhs.numel()
+    if rows.shape[0] * x_div != routes:
         return None
-    if int(rows.shape[0]) * x_div != routes:
+    slots, out_dim = codes.shape[0], codes.shape[1]
+    return project(rows, routes, rows.shape[1], codes, slots, out_dim, scales, scales.shape[2], table, rhs, (routes, out_dim),
+                   x_div=x_div, code_bits=code_bits, residual=residual, hot_of_slot=hot_of_slot)
+
+
+def project(rows, routes, in_dim, codes, slots, out_dim, scales, groups, table, rhs, out_shape, *, x_div=1, code_bits=16, residual=None, hot_of_slot=None, stream=None):
+    """The same with the sizes given beside the tensors (one matrix's codes and scales, say, without an
+    experts' dimension; ``rhs`` may hold more than ``routes``), and the shape of the answer."""
+    if codes.dtype != (torch.uint8 if code_bits == 8 else torch.uint16) or in_dim % 256 or rows.dtype not in (torch.float16, torch.bfloat16):
         return None
     if code_bits == 8 and not byte_codes_served(routes, slots, out_dim, in_dim, groups):
         return None  # (asked first: a call prepared to be refused cost 20 us)
     lib = _lib.load()
     device = rows.device
-    stream = torch.cuda.current_stream(device).cuda_stream
+    stream = torch.cuda.current_stream(device).cuda_stream if stream is None else stream
     nbytes = _scratch_bytes(routes, in_dim)
     # Scratch of this call alone, from the caching allocator: calls of other threads, of other streams
     # and of other captured graphs have their own, and a graph's stays the graph's.
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    out_dtype = qmv_output_dtype(rows.dtype)
-    out = torch.empty((routes, out_dim), dtype=out_dtype, device=device)
-    rows, rhs = rows.contiguous(), rhs.to(torch.int32).contiguous()
+    out = torch.empty(out_shape, dtype=rows.dtype, device=device)  # (16-bit rows: qmv_output_dtype is theirs)
+    rows = rows.contiguous()
+    if rhs.dtype != torch.int32 or not rhs.is_contiguous():
+        rhs = rhs.to(torch.int32).contiguous()
     if rows.data_ptr() % 16:  # a view that starts inside an allocation: the kernels read 16 bytes at a time
         rows = rows.clone()
-    args = _lib.GroupedProjectionArgs(
-        x=_lib.ptr(rows), x_dtype=_lib.dtype_tag(rows.dtype), routes=routes, rhs=_lib.ptr(rhs), codes=_lib.ptr(codes), scales=_lib.ptr(scales),
-        scales_dtype=_lib.dtype_tag(scales.dtype), slots=slots, out_dim=out_dim, in_dim=in_dim, groups=groups, codebook=_lib.ptr(table),
-        codebook_all_odd=int(code_bits == 16 and _table_all_odd(table)), out=_lib.ptr(out), out_dtype=_lib.dtype_tag(out_dtype),
-        workspace=_lib.ptr(ws), workspace_bytes=int(ws.numel()), x_div=int(x_div))
-    keep = [rows, rhs]
+    dtype, res = _lib.dtype_tag(rows.dtype), (0, 0, 0, 0, 0, 0)
     if residual is not None:
         res_codes, res_scales, res_table = residual
         if res_scales.dtype != scales.dtype:
             return None
-        args.res_codes, args.res_scales, args.res_table = _lib.ptr(res_codes), _lib.ptr(res_scales), _lib.ptr(res_table)
-        args.res_rows, args.res_groups, args.hot_of_slot = int(res_codes.shape[0]), int(res_scales.shape[2]), _lib.ptr(hot_of_slot)
-        keep += [res_codes, res_scales, res_table, hot_of_slot]
-    with torch.cuda.device(device):
+        res = (res_codes.data_ptr(), res_scales.data_ptr(), res_codes.shape[0], res_scales.shape[2], res_table.data_ptr(), hot_of_slot.data_ptr())
+    args = _lib.pack_grouped_args(
+        rows.data_ptr(), dtype, routes, rhs.data_ptr(), codes.data_ptr(), scales.data_ptr(), _lib.dtype_tag(scales.dtype), slots, out_dim, in_dim, groups,
+        table.data_ptr(), int(code_bits == 16 and _table_all_odd(table)), out.data_ptr(), dtype, ws.data_ptr(), nbytes, int(x_div), *res)
+    with _lib.on_device(device):
         status = (lib.keepvq_grouped_projection_bytes if code_bits == 8 else lib.keepvq_grouped_projection)(args, ctypes.c_void_p(stream))
-    del keep
     if status == _UNSUPPORTED:
         return None
     _lib.check(status, "keepvq_grouped_projection")
