@@ -27,7 +27,7 @@
 //                codewords each behind private cp.async rings, took 1290 cycles per K block at 24
 //                routes an expert; this form 740: a 1024-token product 302 -> 180 us, the two
 //                projections of a 4096-token layer 1185 + 584 -> 715 + 367 us.)  The bytes go straight into TENSOR MEMORY
-//                (tcgen05.st), two or four stages deep, so the A operand never touches shared memory.
+//                (tcgen05.st), two stages of one or two K blocks deep, so the A operand never touches shared memory.
 //                An item's accumulators are drained (tcgen05.ld: same lanes; each of the four warps
 //                of a quadrant takes a quarter of the columns) behind the warp's first K block of the
 //                NEXT item, so nobody waits for the tail of the MMAs.
@@ -86,13 +86,23 @@ struct PrefillPlan {
   static_assert(N_MAX % 16 == 0, "an item's routes pad to a multiple of sixteen columns");
   static constexpr uint32_t ACC_SET_COLS = 2 * M * N_MAX;
   static constexpr uint32_t ACC_SETS = GROUPED ? 2 : 1;
-  static constexpr uint32_t A_STAGE_COLS = M * PF_A_TILE_COLS;
+  // K blocks per stage: what the MMA warp pays once per stage (its wait, its commits, the instructions
+  // around them: some 300 cycles alone, 550 to 700 beside the decode warps) is what a K block of few routes
+  // takes, so where tensor memory has room for two stages of two K blocks they go in pairs (1000-token layer:
+  // gate/up and down 534 + 297 -> 525 + 289 us; 24 tokens of 8-bit codes 91.7 -> 87.9)
+  static constexpr uint32_t STAGE_BLOCKS = GROUPED || N_MAX > 48 ? 1 : 2;
+  // The fp32 sums of the scale groups leave no registers for a K block's 32 operand columns at once: in halves, and
+  // with the deadline in shared memory, nothing spills (layer of 1021 tokens: 631 + 448 -> 617 + 427 us)
+  static constexpr bool HALVES = GROUPED;
+  static constexpr uint32_t A_BLOCK_COLS = M * PF_A_TILE_COLS;
+  static constexpr uint32_t A_STAGE_COLS = STAGE_BLOCKS * A_BLOCK_COLS;
   static constexpr uint32_t A_COL0 = ACC_SETS * ACC_SET_COLS;
-  static constexpr uint32_t A_STAGES = GROUPED || N_MAX > 48 ? 2 : 4;
+  static constexpr uint32_t A_STAGES = 2;
   static_assert(A_COL0 + A_STAGES * A_STAGE_COLS <= PF_TMEM_COLS, "tensor memory holds the accumulators and the A stages");
-  static constexpr uint32_t B_STAGE_BYTES = 2 * N_MAX * 128;  // high-byte rows of the routes, then their low-byte rows
+  static constexpr uint32_t B_BLOCK_BYTES = 2 * N_MAX * 128;  // a K block: high-byte rows of the routes, then their low-byte rows
+  static constexpr uint32_t B_STAGE_BYTES = STAGE_BLOCKS * B_BLOCK_BYTES;
   static constexpr uint32_t LOW_B_STAGES = PF_LOW_BYTES / B_STAGE_BYTES;
-  static constexpr uint32_t B_STAGES = N_MAX > 48 ? 4 : GROUPED ? 6 : 8;    // one ring of barriers for A and B: a K block's A stage is its B stage modulo A_STAGES
+  static constexpr uint32_t B_STAGES = GROUPED ? 6 : 4;    // one ring of barriers for A and B: a stage's A columns are its index modulo A_STAGES
   static_assert(B_STAGES % A_STAGES == 0, "");
   static constexpr uint32_t CODE_ROW_BYTES = 2 * PF_KBLOCK_CODES * BITS / 8;  // two K blocks of a row's codes
   static constexpr uint32_t CODE_UNIT_BYTES = PF_ROWS * CODE_ROW_BYTES;       // ... of a tile's
@@ -117,8 +127,8 @@ __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar, int lane) {
 // caller's CTA then gives up: the flag is raised for every role) or when another warp of the CTA
 // already gave up.  RELAXED is for the loaders, which run stages ahead: their polls would take issue
 // slots from the decode warps.
-template <bool RELAXED = false>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t deadline, volatile int* abort_flag) {
+template <bool RELAXED = false, class Time>
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const Time& deadline, volatile int* abort_flag) {
   for (uint32_t spin = 0;; ++spin) {
     if (__all_sync(0xFFFFFFFFu, mbar_complete(bar, parity))) return true;
     if (RELAXED) __nanosleep(160);
@@ -144,18 +154,19 @@ template <uint32_t STAGES>
 __device__ __forceinline__ void wait_codes_landed(uint32_t full_bars, uint32_t used) {
   for (uint32_t i = used > STAGES ? used - STAGES : 0; i < used; ++i) mbar_wait_grace(full_bars + 8u * (i % STAGES), (i / STAGES) & 1u);
 }
-// ... and for those of its activation loader (`used` K blocks).  A K block's barrier also counts the
-// decode warps that fill its A stage, so the arrivals they did not come to make are made for them:
-// place[w] is where decode warp w stopped, its next K block modulo 2 STAGES.  A K block whose barrier
+// ... and for those of its activation loader (`used` stages).  A stage's barrier also counts the
+// decode warps that fill its A columns (every other stage a warp's own with one K block a stage, all with
+// two), so the arrivals they did not come to make are made for them:
+// place[w] is where decode warp w stopped, its next stage modulo 2 STAGES.  A stage whose barrier
 // is not complete has not been read, so no decode warp is as far as STAGES beyond it, none STAGES behind.
-template <uint32_t STAGES>
+template <uint32_t STAGES, int STAGE_BLOCKS>
 __device__ __forceinline__ void wait_activations_landed(uint32_t full_bars, uint32_t used, const uint32_t* place, int decode_warps) {
   for (uint32_t i = used > STAGES ? used - STAGES : 0; i < used; ++i) {
     const uint32_t bar = full_bars + 8u * (i % STAGES), phase = (i / STAGES) & 1u;
     if (mbar_complete(bar, phase)) continue;
     for (int w = 0; w < decode_warps; ++w) {
-      const uint32_t ahead = (place[w] + 2 * STAGES - i % (2 * STAGES)) % (2 * STAGES);  // its next K block less this one
-      if (((static_cast<uint32_t>(w) >> 2) & 1u) == (i & 1u) && (ahead == 0 || ahead > STAGES)) mbar_arrive(bar);
+      const uint32_t ahead = (place[w] + 2 * STAGES - i % (2 * STAGES)) % (2 * STAGES);  // its next stage less this one
+      if ((STAGE_BLOCKS == 2 || ((static_cast<uint32_t>(w) >> 2) & 1u) == (i & 1u)) && (ahead == 0 || ahead > STAGES)) mbar_arrive(bar);
     }
     mbar_wait_grace(bar, phase);
   }
@@ -178,6 +189,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
                ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
                  "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]),
                  "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
+}
+// ... and 16.
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+                 "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -224,15 +241,17 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   using Plan = PrefillPlan<M, N_MAX, GROUPED, BITS>;
   constexpr int ITEM_ROWS = GLU ? PF_ROWS : PF_ROWS * M;
   constexpr int A_STAGES = Plan::A_STAGES, B_STAGES = Plan::B_STAGES, CODE_STAGES = Plan::CODE_STAGES, ACC_SETS = Plan::ACC_SETS;
+  constexpr int SB = Plan::STAGE_BLOCKS;
   constexpr int TILE_STEP = GLU ? 0 : PF_ROWS;  // rows between the A tiles of an item
   extern __shared__ __align__(16) uint8_t smem_raw[];
   grid_launch_dependents();
-  // STAGE_FULL: the decode warps' A tiles and the activations of a K block are in place; STAGE_EMPTY: its MMAs have read them
+  // STAGE_FULL: the decode warps' A tiles and the activations of a stage's K blocks are in place; STAGE_EMPTY: its MMAs have read them
   enum { STAGE_FULL = 0, STAGE_EMPTY = STAGE_FULL + B_STAGES, CODE_FULL = STAGE_EMPTY + B_STAGES, CODE_EMPTY = CODE_FULL + CODE_STAGES,
          ACC_FULL = CODE_EMPTY + CODE_STAGES, ACC_EMPTY = ACC_FULL + ACC_SETS, INFO_FULL = ACC_EMPTY + ACC_SETS, INFO_EMPTY = INFO_FULL + PF_INFO_BUFFERS, DRAINED = INFO_EMPTY + PF_INFO_BUFFERS, N_BARS = DRAINED + 1 };
   static_assert(N_BARS * 8 <= 1024, "");
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ volatile uint64_t shared_deadline;  // (in registers it and 64-bit row numbers made the scale-group form spill, 500 cycles of reloads from L2 per K block)
   __shared__ uint32_t decode_place[PF_DECODE_WARPS], codes_issued, activations_issued;  // where the roles stopped
   __shared__ int4 route_info[PF_INFO_BUFFERS][N_MAX];  // per item (three in flight): route, x scale, x sum (one scale group only), gate weight
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -249,7 +268,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   if (tid == 0) {
     abort_flag = window_ok ? 0 : 1;
     if (window_ok) {
-      for (int s = 0; s < B_STAGES; ++s) { mbar_init(bar(STAGE_FULL, s), M * 4 + 1); mbar_init(bar(STAGE_EMPTY, s), 1); }
+      for (int s = 0; s < B_STAGES; ++s) { mbar_init(bar(STAGE_FULL, s), M * 4 * SB + 1); mbar_init(bar(STAGE_EMPTY, s), 1); }
       for (int s = 0; s < CODE_STAGES; ++s) { mbar_init(bar(CODE_FULL, s), 1); mbar_init(bar(CODE_EMPTY, s), M * 8); }
       for (int s = 0; s < ACC_SETS; ++s) { mbar_init(bar(ACC_FULL, s), 1); mbar_init(bar(ACC_EMPTY, s), PF_DECODE_WARPS); }
       for (int s = 0; s < PF_INFO_BUFFERS; ++s) { mbar_init(bar(INFO_FULL, s), 1); mbar_init(bar(INFO_EMPTY, s), PF_DECODE_WARPS); }
@@ -269,14 +288,21 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
   // an allocation of all 512 columns starts at column 0 of lane 0: a constant, which keeps the MMAs' operands in uniform registers
   constexpr uint32_t tmem = 0;
   grid_wait();  // the tables come from constants; everything below reads what the kernels before this one wrote
-  const uint64_t deadline = global_timer_ns() + (wait_ns ? wait_ns : PF_DEFAULT_WAIT_NS);  // (the time spent waiting for those is not this kernel's)
+  const uint64_t own_deadline = global_timer_ns() + (wait_ns ? wait_ns : PF_DEFAULT_WAIT_NS);  // (the time spent waiting for those is not this kernel's)
+  if constexpr (GROUPED) {
+    if (tid == 0) shared_deadline = own_deadline;
+    __syncthreads();
+  }
+  const auto& deadline = [&]() -> const auto& {
+    if constexpr (GROUPED) return shared_deadline; else return own_deadline;
+  }();
 
-  const int64_t N_out = p.out_dim;
+  const int N_out = static_cast<int>(p.out_dim);  // (slots * out_dim is below 2^31, prefill_supported)
   const int k_blocks = static_cast<int>(p.in_dim / (8 * PF_KBLOCK_CODES));
   const int code_units = k_blocks / 2;  // of two K blocks each (inputs come in multiples of 256)
   const int segments = GROUPED ? static_cast<int>(p.groups) : 1;  // drains per item
   const int segment_blocks = k_blocks / segments;
-  const int row_tiles = static_cast<int>((N_out + ITEM_ROWS - 1) / ITEM_ROWS);
+  const int row_tiles = (N_out + ITEM_ROWS - 1) / ITEM_ROWS;
   const int items = static_cast<int>(warp_uniform(p.groups_of_routes.count[0])) * row_tiles;
   volatile int* aborted = &abort_flag;
   const int items_here = set_up_ok ? items : 0;
@@ -298,19 +324,20 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     const bool scales32 = p.scales_dtype == KEEPVQ_F32;
     const float limit = p.swiglu_limit > 0.0f ? p.swiglu_limit : INFINITY;
     RingPlace<CODE_STAGES> code;
-    RingPlace<B_STAGES> stage, freed;  // of this warp's K block, and of the one A_STAGES before it
-    stage.advance(parity);
-    freed.advance(parity);
-    int fresh = A_STAGES / 2;          // this warp's first K blocks find their A stages free
+    // stage of this warp's K block, and the one A_STAGES before it: every other stage of one K block, every stage of two
+    constexpr uint32_t OWN_STEP = SB == 2 ? 1 : 2;
+    RingPlace<B_STAGES> stage, freed;
+    if (SB == 1) { stage.advance(parity); freed.advance(parity); }
+    int fresh = A_STAGES / OWN_STEP;   // this warp's first K blocks find their A stages free
     RingPlace<ACC_SETS> acc;
     RingPlace<PF_INFO_BUFFERS> info;
     bool ok = true;
 
     // the segment that waits for its drain
-    bool pending = false, last_segment = false;
+    bool pending = false;
     int pending_segment = 0;
-    int n_pad = 0, quarter = 0;
-    int64_t erow = 0;
+    int quarter = 0;  // columns of the item, by four
+    int erow = 0;
     uint32_t raw_scale[M];
     float sum[GROUPED ? M : 1][GROUPED ? N_MAX / 4 : 1];
 
@@ -326,7 +353,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
 #pragma unroll
       for (int mm = 0; mm < M; ++mm)
 #pragma unroll
-        for (int piece = 0; piece < 2; ++piece) tmem_ld4(lane_tmem + acc.index * Plan::ACC_SET_COLS + mm * (2 * N_MAX) + piece * n_pad + c, v[mm][piece]);
+        for (int piece = 0; piece < 2; ++piece) tmem_ld4(lane_tmem + acc.index * Plan::ACC_SET_COLS + mm * (2 * N_MAX) + piece * (quarter * 4) + c, v[mm][piece]);
     };
     // The accumulators are free again as soon as they are in registers: a warp gives its arrival when
     // the LAST of its columns has been read, before the arithmetic and the stores of those columns.
@@ -356,7 +383,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       for (int mm = 0; mm < M; ++mm) scale[mm] = as_scale(raw_scale[mm]);
       if constexpr (GROUPED) {
 #pragma unroll
-        for (int c = 0; c < N_MAX / 4; c += 4) {
+        for (int c = 0; c < N_MAX / 4; c += 4) {  // (eight columns behind one wait have no registers: spills, 1086 -> 1160 us a layer of 1021 tokens)
           if (c >= quarter) break;
           uint32_t v[M][2][4], less[4];
           load_columns(v, c_first + c);
@@ -374,7 +401,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             }
           }
         }
-        if (last_segment) {
+        if (pending_segment == segments - 1) {
 #pragma unroll
           for (int c = 0; c < N_MAX / 4; ++c) {
             if (c < quarter) {
@@ -414,7 +441,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     };
     auto drain = [&]() {
       pending = false;
-      ok = ok && mbar_wait(bar(INFO_FULL, info.index), info.phase, deadline, aborted);
+      if (!GROUPED || pending_segment == 0) ok = ok && mbar_wait(bar(INFO_FULL, info.index), info.phase, deadline, aborted);
       ok = ok && mbar_wait(bar(ACC_FULL, acc.index), acc.phase, deadline, aborted);
       if (!ok) return;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -427,7 +454,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       else
         drain_as([](float v) { return v; }, [&](int64_t i, float v) { static_cast<float*>(p.out)[i] = v; });
       acc.advance();
-      if (last_segment) {
+      if (pending_segment == segments - 1) {
         __syncwarp();
         mbar_arrive_warp(bar(INFO_EMPTY, info.index), lane);
         info.advance();
@@ -442,7 +469,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     }
     for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
       const int gi = item / row_tiles, tile = item - gi * row_tiles;
-      const int64_t slot = p.groups_of_routes.slot[gi];
+      const int first_row = p.groups_of_routes.slot[gi] * N_out;
       const int gsize = p.groups_of_routes.size[gi];
       for (int segment = 0; segment < segments && ok; ++segment) {
         if (m < M) {
@@ -450,36 +477,60 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
             ok = mbar_wait(bar(CODE_FULL, code.index), code.phase, deadline, aborted);
             if (!ok) break;
             const uint32_t at = code.index * Plan::CODE_STAGE_BYTES;
-            uint32_t w[8], q[32];
+            uint32_t w[8];
             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(code_chunk0 + at));
-            if constexpr (BITS == 16) {
-              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(code_chunk1 + at));
+            if constexpr (BITS == 16) asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(code_chunk1 + at));
+            const uint32_t to = lane_tmem + Plan::A_COL0 + (stage.index % A_STAGES) * Plan::A_STAGE_COLS + (SB == 2 ? parity * Plan::A_BLOCK_COLS : 0u) + m * PF_A_TILE_COLS;
+            auto decode_words = [&](const uint32_t* words, uint32_t* q, int count) {  // the operand columns of `count` columns' codewords
+              if constexpr (BITS == 16) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                decode_codeword_nibble<false>(w[i], abs_lane, sign_lane, q[4 * i], q[4 * i + 1]);
-                decode_codeword_nibble<true>(w[i], abs_lane, sign_lane, q[4 * i + 2], q[4 * i + 3]);
+                for (int i = 0; i < count / 4; ++i) {
+                  decode_codeword_nibble<false>(words[i], abs_lane, sign_lane, q[4 * i], q[4 * i + 1]);
+                  decode_codeword_nibble<true>(words[i], abs_lane, sign_lane, q[4 * i + 2], q[4 * i + 3]);
+                }
+              } else {
+#pragma unroll
+                for (int i = 0; i < count / 2; ++i) decode_byte_code(words[i >> 2], i & 3, abs_lane, q[2 * i], q[2 * i + 1]);
               }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 16; ++i) decode_byte_code(w[i >> 2], i & 3, abs_lane, q[2 * i], q[2 * i + 1]);
-            }
-            __syncwarp();
-            mbar_arrive_warp(bar(CODE_EMPTY, code.index), lane);
-            code.advance();
-            if (fresh > 0) {
-              --fresh;
-            } else {
-              ok = mbar_wait(bar(STAGE_EMPTY, freed.index), freed.phase, deadline, aborted);
+            };
+            auto codes_read = [&]() {
+              __syncwarp();
+              mbar_arrive_warp(bar(CODE_EMPTY, code.index), lane);
+              code.advance();
+            };
+            if constexpr (Plan::HALVES) {
+              // mostly the stage is free already: asked for under the reads of the codes
+              const bool free = fresh > 0 || __all_sync(0xFFFFFFFFu, mbar_test(bar(STAGE_EMPTY, freed.index), freed.phase));
+              uint32_t q[16];
+              decode_words(w, q, 16);
+              codes_read();
+              if (!free) ok = mbar_wait(bar(STAGE_EMPTY, freed.index), freed.phase, deadline, aborted);
               if (!ok) break;
-              freed.advance(2);
+              if (fresh > 0) --fresh; else freed.advance(OWN_STEP);
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              tmem_st16(to, q);  // on its way to tensor memory under the decode of the other half
+              uint32_t q2[16];
+              decode_words(w + BITS / 4, q2, 16);
+              tmem_st16(to + 16, q2);
+            } else {
+              uint32_t q[32];
+              decode_words(w, q, 32);
+              codes_read();
+              if (fresh > 0) {
+                --fresh;
+              } else {
+                ok = mbar_wait(bar(STAGE_EMPTY, freed.index), freed.phase, deadline, aborted);
+                if (!ok) break;
+                freed.advance(OWN_STEP);
+              }
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              tmem_st32(to, q);
             }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tmem_st32(lane_tmem + Plan::A_COL0 + (stage.index % A_STAGES) * Plan::A_STAGE_COLS + m * PF_A_TILE_COLS, q);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             mbar_arrive_warp(bar(STAGE_FULL, stage.index), lane);
-            stage.advance(2);
+            stage.advance(OWN_STEP);
             // the previous segment's MMAs have had this K block's decode to finish under
             if (pending) {
               drain();
@@ -491,18 +542,16 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
         // this segment is the next to be drained; what its drain needs from memory is asked for now
         pending = true;
         pending_segment = segment;
-        last_segment = segment == segments - 1;
         if (segment == 0) {
-          n_pad = (gsize + 15) & ~15;
-          quarter = n_pad >> 2;
-          erow = static_cast<int64_t>(tile) * ITEM_ROWS + row;
+          quarter = ((gsize + 15) & ~15) >> 2;
+          erow = tile * ITEM_ROWS + row;
         }
 #pragma unroll
-        for (int mm = 0; mm < M; ++mm) raw_scale[mm] = load_scale((slot * N_out + min(erow + mm * TILE_STEP, N_out - 1)) * segments + segment, mm);
+        for (int mm = 0; mm < M; ++mm) raw_scale[mm] = load_scale(static_cast<int64_t>(first_row + min(erow + mm * TILE_STEP, N_out - 1)) * segments + segment, mm);
       }
     }
     if (pending && ok) drain();
-    if (lane == 0) decode_place[warp] = (freed.phase * B_STAGES + freed.index + A_STAGES - 2 * fresh) % (2 * B_STAGES);  // its next K block
+    if (lane == 0) decode_place[warp] = (freed.phase * B_STAGES + freed.index + A_STAGES - OWN_STEP * fresh) % (2 * B_STAGES);  // its next stage
   } else if (warp == PF_MMA_WARP) {
     // ================= the MMAs ================================================================
     // One loop over all K blocks of the block's items, unrolled over the stage ring: this warp's own
@@ -515,7 +564,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     RingPlace<ACC_SETS> acc;
     uint32_t phase = 0, idesc = 0, d_cols = 0;
     bool ok = true, first_round = true;
-    int item = static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x), segment = segments - 1, kb = segment_blocks - 1;
+    int item = static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x), segment = segments - 1, kb = segment_blocks - SB;
     // the next segment: its accumulators, and at the start of an item its width
     auto next_segment = [&]() {
       kb = 0;
@@ -536,19 +585,20 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     while (ok) {
 #pragma unroll
       for (uint32_t st = 0; st < B_STAGES; ++st) {
-        if (++kb == segment_blocks) ok = ok && next_segment();
+        if ((kb += SB) == segment_blocks) ok = ok && next_segment();
         ok = ok && mbar_wait(bar(STAGE_FULL, st), phase, deadline, aborted);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t accumulate = kb != 0;
-        const bool last = kb == segment_blocks - 1;
+        const bool last = kb == segment_blocks - SB;
         if (elect_one()) {
 #pragma unroll
-          for (int m = 0; m < M; ++m) {
+          for (int mj = 0; mj < M * SB; ++mj) {
+            const int m = mj % M, j = mj / M;  // tile, K block of the stage
 #pragma unroll
             for (int k = 0; k < 4; ++k)  // 32 bytes of K per instruction: 8 columns of A, 2 x 16 bytes of the B start address
-              umma_i8_ts(d_cols + m * (2 * N_MAX), Plan::A_COL0 + (st % A_STAGES) * Plan::A_STAGE_COLS + m * PF_A_TILE_COLS + 8 * k,
-                         umma_desc(Plan::b_stage(st)) + 2 * k, idesc, accumulate | static_cast<uint32_t>(k));
+              umma_i8_ts(d_cols + m * (2 * N_MAX), Plan::A_COL0 + (st % A_STAGES) * Plan::A_STAGE_COLS + j * Plan::A_BLOCK_COLS + m * PF_A_TILE_COLS + 8 * k,
+                         umma_desc(Plan::b_stage(st) + j * Plan::B_BLOCK_BYTES) + 2 * k, idesc, accumulate | static_cast<uint32_t>(j | k));
           }
           umma_commit(bar(STAGE_EMPTY, st));  // the stage may be refilled once these MMAs have read it
           if (last) umma_commit(bar(ACC_FULL, acc.index));
@@ -576,13 +626,15 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       const int gsize = warp_uniform(p.groups_of_routes.size[gi]), gstart = warp_uniform(p.groups_of_routes.start[gi]);
       const int n_pad = (gsize + 15) & ~15;
       const CUtensorMap* map = &x_maps.rows[(n_pad >> 4) - 1];
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      for (int kb = 0; kb < k_blocks; kb += SB) {
         ok = mbar_wait<true>(bar(STAGE_EMPTY, b.index), b.phase ^ 1u, deadline, aborted);
         if (!ok) break;
         if (stall != STALL_ACTIVATIONS) {
           if (elect_one()) {
-            mbar_expect_tx(bar(STAGE_FULL, b.index), static_cast<uint32_t>(2 * n_pad * 128));
-            tma_box_3d(Plan::b_stage(b.index), map, kb * 128, gstart, 0, bar(STAGE_FULL, b.index));
+            mbar_expect_tx(bar(STAGE_FULL, b.index), static_cast<uint32_t>(SB * 2 * n_pad * 128));
+#pragma unroll
+            for (int j = 0; j < SB; ++j)
+              tma_box_3d(Plan::b_stage(b.index) + j * Plan::B_BLOCK_BYTES, map, (kb + j) * 128, gstart, 0, bar(STAGE_FULL, b.index));
           }
           ++used;
         }
@@ -600,7 +652,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
     bool ok = true;
     for (int item = blockIdx.x; item < items_here && ok; item += gridDim.x) {
       const int gi = item / row_tiles, tile = item - gi * row_tiles;
-      const int row0 = warp_uniform(static_cast<uint32_t>(p.groups_of_routes.slot[gi] * N_out + static_cast<int64_t>(tile) * ITEM_ROWS));
+      const int row0 = static_cast<int>(warp_uniform(static_cast<uint32_t>(p.groups_of_routes.slot[gi] * N_out + tile * ITEM_ROWS)));
       for (int u = 0; u < code_units; ++u) {
         ok = mbar_wait<true>(bar(CODE_EMPTY, code.index), code.phase ^ 1u, deadline, aborted);
         if (!ok) break;
@@ -665,7 +717,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_projection_kernel(FastP
       mbar_wait_grace(bar(DRAINED, 0), 0u);
     }
     if (warp == PF_CODE_WARP && lane == 0) wait_codes_landed<CODE_STAGES>(bar(CODE_FULL, 0), codes_issued);
-    if (warp == PF_B_WARP && lane == 0) wait_activations_landed<B_STAGES>(bar(STAGE_FULL, 0), activations_issued, decode_place, M * 8);
+    if (warp == PF_B_WARP && lane == 0) wait_activations_landed<B_STAGES, SB>(bar(STAGE_FULL, 0), activations_issued, decode_place, M * 8);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -679,7 +731,7 @@ bool prefill_supported(int64_t slots, int64_t out_dim, int64_t in_dim, int64_t g
 }
 
 // Routes per item.  96 fill tensor memory (accumulators of two byte planes and two tiles, two A
-// stages), 48 leave room for four A stages; rows with several scale groups take the second half of
+// stages), 48 leave room for four K blocks' A tiles (two stages of two); rows with several scale groups take the second half of
 // tensor memory for a second accumulator set instead.  An expert with more routes than that is
 // decoded once per item, so 48 serve calls whose experts rarely get more: up to 32 on average
 // (of a uniform router's experts 0.3 % then exceed 48).
