@@ -90,68 +90,70 @@ __global__ void __launch_bounds__(RT_THREADS) router_logits_tiled_kernel(keepvq_
 // Many bf16 tokens against a bf16 router: the same tile on the tensor cores (mma.sync m16n8k16:
 // bf16 products are exact, sixteen of them are summed per instruction, the partial sums are added
 // in fp32 with k ascending).  64 tokens x 64 experts per block of four warps, K staged 32 at a time through a
-// three-stage cp.async ring; rows padded to 80 bytes so that every fragment load is conflict-free.
-constexpr int RM_TILE = 64, RM_K = 32, RM_LD = 40, RM_STAGES = 3, RM_THREADS = 128;
+// four-stage cp.async ring; rows padded to 80 bytes so that every fragment load is conflict-free.
+constexpr int RM_TILE = 64, RM_K = 32, RM_LD = 40, RM_STAGES = 4, RM_THREADS = 128;
+struct RouterStages { __nv_bfloat16 x[RM_STAGES][RM_TILE][RM_LD], w[RM_STAGES][RM_TILE][RM_LD]; };
 
-__global__ void __launch_bounds__(RM_THREADS) router_logits_mma_kernel(keepvq_router_logits_args a) {
-  __shared__ __align__(16) __nv_bfloat16 xs[RM_STAGES][RM_TILE][RM_LD], ws[RM_STAGES][RM_TILE][RM_LD];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;  // this warp's 32 x 32 corner of the tile
-  const int64_t t0 = static_cast<int64_t>(blockIdx.y) * RM_TILE, e0 = static_cast<int64_t>(blockIdx.x) * RM_TILE;
-  const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(a.x);
-  const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(a.router_w);
+__device__ __forceinline__ void load_matrices(uint32_t addr, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(addr) : "memory");
+}
+
+// This thread's part of a 64 x 64 tile: acc[i][j] is MMA tile (16 i, 8 j) of its warp's 32 x 32 corner (wm, wn).
+// x and w point at the first of `k_blocks` * RM_K inputs.
+// What bounds it is the rate of mma.sync and, before that, whatever else a warp does per MMA: fragments read word
+// by word were 24 shared-memory reads per eight MMAs, so matrices are read four at a time (4 reads), and both
+// halves of a K block before the first MMA.  Copies run three blocks ahead.  (Logits and top-k of 4096 tokens x 384
+// experts, 4096 wide, 93 -> 78 us, of 2000 tokens 55 -> 52, of 251 tokens 21 -> 17; 192 experts, 5120 wide, 4096
+// tokens 70 -> 65, 251 tokens 15.1 -> 15.7.)
+__device__ __forceinline__ void router_tile_mma(RouterStages& sm, const __nv_bfloat16* x, const __nv_bfloat16* w, const keepvq_router_logits_args& a, int64_t t0, int64_t e0, int k_blocks, int wm, int wn, float (&acc)[2][4][4]) {
+  const int tid = threadIdx.x, lane = tid & 31;
   // staging: 64 rows x 4 pieces of 16 bytes per operand, two pieces per thread
   const int row_a = tid >> 2, piece = tid & 3, row_b = row_a + 32;
   const __nv_bfloat16* xsrc[2] = {x + min(t0 + row_a, a.tokens - 1) * a.hidden + piece * 8, x + min(t0 + row_b, a.tokens - 1) * a.hidden + piece * 8};
   const __nv_bfloat16* wsrc[2] = {w + min(e0 + row_a, a.pool - 1) * a.hidden + piece * 8, w + min(e0 + row_b, a.pool - 1) * a.hidden + piece * 8};
+  const uint32_t x_smem = static_cast<uint32_t>(__cvta_generic_to_shared(&sm.x[0][0][0])), w_smem = static_cast<uint32_t>(__cvta_generic_to_shared(&sm.w[0][0][0]));
+  constexpr uint32_t STAGE_BYTES = RM_TILE * RM_LD * 2;
+  const uint32_t to[2] = {static_cast<uint32_t>((row_a * RM_LD + piece * 8) * 2), static_cast<uint32_t>((row_b * RM_LD + piece * 8) * 2)};
   auto stage_in = [&](int kb) {
-    const int st = kb % RM_STAGES;
-    if (kb * RM_K < a.hidden) {
+    if (kb < k_blocks) {
+      const uint32_t at = (kb % RM_STAGES) * STAGE_BYTES;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int row = h ? row_b : row_a;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(&xs[st][row][piece * 8]))), "l"(xsrc[h] + kb * RM_K) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(&ws[st][row][piece * 8]))), "l"(wsrc[h] + kb * RM_K) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(x_smem + at + to[h]), "l"(xsrc[h] + kb * RM_K) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(w_smem + at + to[h]), "l"(wsrc[h] + kb * RM_K) : "memory");
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float acc[2][4][4];
+  // lane l gives row l % 8 of matrix l / 8: for x the matrices (rows 0-7 and 8-15) x (k 0-7, then 8-15), for w (k 0-7 and 8-15) x (experts 0-7, then 8-15)
+  const uint32_t x_row = x_smem + ((wm + ((lane >> 3) & 1) * 8 + (lane & 7)) * RM_LD + (lane >> 4) * 8) * 2;
+  const uint32_t w_row = w_smem + ((wn + (lane >> 4) * 8 + (lane & 7)) * RM_LD + ((lane >> 3) & 1) * 8) * 2;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0f;
-  const int k_blocks = static_cast<int>(a.hidden / RM_K);
-  stage_in(0);
-  stage_in(1);
+  for (int kb = 0; kb < RM_STAGES - 1; ++kb) stage_in(kb);
   for (int kb = 0; kb < k_blocks; ++kb) {
-    asm volatile("cp.async.wait_group 1;" ::: "memory");  // block kb has landed
-    __syncthreads();                                          // ... for everyone, and block kb - 1 is no longer being read
-    stage_in(kb + 2);
-    const int st = kb % RM_STAGES;
+    asm volatile("cp.async.wait_group %0;" ::"n"(RM_STAGES - 2) : "memory");  // block kb has landed
+    __syncthreads();                                                           // ... for everyone, and block kb - 1 is no longer being read
+    stage_in(kb + RM_STAGES - 1);
+    const uint32_t at = (kb % RM_STAGES) * STAGE_BYTES;
+    uint32_t af[2][2][4], bf[2][4][2];
 #pragma unroll
-    for (int ks = 0; ks < RM_K; ks += 16) {
-      uint32_t af[2][4], bf[4][2];
+    for (int ks = 0; ks < 2; ++ks) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int r = wm + 16 * i + g;
-        af[i][0] = *reinterpret_cast<const uint32_t*>(&xs[st][r][ks + 2 * t]);
-        af[i][1] = *reinterpret_cast<const uint32_t*>(&xs[st][r + 8][ks + 2 * t]);
-        af[i][2] = *reinterpret_cast<const uint32_t*>(&xs[st][r][ks + 2 * t + 8]);
-        af[i][3] = *reinterpret_cast<const uint32_t*>(&xs[st][r + 8][ks + 2 * t + 8]);
-      }
+      for (int i = 0; i < 2; ++i) load_matrices(x_row + at + i * (16 * RM_LD * 2) + ks * 32, af[ks][i][0], af[ks][i][1], af[ks][i][2], af[ks][i][3]);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int n = wn + 8 * j + g;
-        bf[j][0] = *reinterpret_cast<const uint32_t*>(&ws[st][n][ks + 2 * t]);
-        bf[j][1] = *reinterpret_cast<const uint32_t*>(&ws[st][n][ks + 2 * t + 8]);
-      }
-      // Each MMA sums its sixteen exact products from zero; the running sums are kept by ordinary
-      // fp32 additions (round to nearest).  Accumulating inside the tensor core over the whole K
-      // truncates at every step and measured 4e-5 relative on softmax scores, too close to the
-      // gaps that decide a top-k cut.
+      for (int j = 0; j < 4; j += 2) load_matrices(w_row + at + j * (8 * RM_LD * 2) + ks * 32, bf[ks][j][0], bf[ks][j][1], bf[ks][j + 1][0], bf[ks][j + 1][1]);
+    }
+    // Each MMA sums its sixteen exact products from zero; the running sums are kept by ordinary
+    // fp32 additions (round to nearest).  Accumulating inside the tensor core over the whole K
+    // truncates at every step and measured 4e-5 relative on softmax scores, too close to the
+    // gaps that decide a top-k cut.
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -159,12 +161,20 @@ __global__ void __launch_bounds__(RM_THREADS) router_logits_mma_kernel(keepvq_ro
           float d0, d1, d2, d3;
           asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                        : "=f"(d0), "=f"(d1), "=f"(d2), "=f"(d3)
-                       : "r"(af[i][0]), "r"(af[i][1]), "r"(af[i][2]), "r"(af[i][3]), "r"(bf[j][0]), "r"(bf[j][1]), "f"(0.0f));
+                       : "r"(af[ks][i][0]), "r"(af[ks][i][1]), "r"(af[ks][i][2]), "r"(af[ks][i][3]), "r"(bf[ks][j][0]), "r"(bf[ks][j][1]), "f"(0.0f));
           acc[i][j][0] += d0; acc[i][j][1] += d1; acc[i][j][2] += d2; acc[i][j][3] += d3;
         }
-    }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(RM_THREADS) router_logits_mma_kernel(keepvq_router_logits_args a) {
+  __shared__ __align__(16) RouterStages stages;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;  // this warp's 32 x 32 corner of the tile
+  const int64_t t0 = static_cast<int64_t>(blockIdx.y) * RM_TILE, e0 = static_cast<int64_t>(blockIdx.x) * RM_TILE;
+  float acc[2][4][4];
+  router_tile_mma(stages, reinterpret_cast<const __nv_bfloat16*>(a.x), reinterpret_cast<const __nv_bfloat16*>(a.router_w), a, t0, e0, static_cast<int>(a.hidden / RM_K), wm, wn, acc);
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -185,7 +195,7 @@ constexpr int RC_SPLIT = 8;
 // From RT_MIN_TOKENS tokens on the other kernel is the tiled one. Up to here (tiles of 64 tokens x 64
 // experts) that kernel's serial walk over the whole hidden dimension is what a call waits for: 1000 tokens
 // x 384 experts (96 tiles) 28 against 57 us, 1021 x 192 (48 tiles, 5120 wide) 20 against 70 us; with 384
-// tiles (4096 tokens) the GPU is full without the split: 91 against 84 us. With fewer tokens the other
+// tiles (4096 tokens) the GPU is full without the split: 91 against 84 us (both before their loads were cut anew). With fewer tokens the other
 // kernel is the one of the fp32 pipes, which is slower at any number of tiles (200 tokens, 4096 wide:
 // 4160 experts 84 against 487 us, 16384 experts 258 against 1722 us).
 constexpr int64_t RC_MAX_TILES = 256;
@@ -194,75 +204,17 @@ constexpr int RC_MIN_TOKENS = 24;  // below this the K-split kernel of the fp32 
 __global__ void __cluster_dims__(RC_SPLIT, 1, 1) __launch_bounds__(RM_THREADS) router_logits_cluster_kernel(keepvq_router_logits_args a) {
   grid_launch_dependents();
   grid_wait();
-  __shared__ __align__(16) __nv_bfloat16 xs[RM_STAGES][RM_TILE][RM_LD], ws[RM_STAGES][RM_TILE][RM_LD];
-  __shared__ __align__(16) float red[RM_TILE][RM_TILE];  // this block's partial tile [token][expert]
+  __shared__ __align__(16) RouterStages stages;
+  static_assert(sizeof(RouterStages) >= RM_TILE * RM_TILE * 4, "the partial tile takes the stages' place");
+  float (*red)[RM_TILE] = reinterpret_cast<float (*)[RM_TILE]>(&stages);  // this block's partial tile [token][expert]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
   const int rank = static_cast<int>(blockIdx.x);  // the cluster spans x: the block's share of K
   const int64_t t0 = static_cast<int64_t>(blockIdx.z) * RM_TILE, e0 = static_cast<int64_t>(blockIdx.y) * RM_TILE;
   const int64_t k_share = a.hidden / RC_SPLIT, k_first = rank * k_share;
-  const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(a.x) + k_first;
-  const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(a.router_w) + k_first;
-  const int row_a = tid >> 2, piece = tid & 3, row_b = row_a + 32;
-  const __nv_bfloat16* xsrc[2] = {x + min(t0 + row_a, a.tokens - 1) * a.hidden + piece * 8, x + min(t0 + row_b, a.tokens - 1) * a.hidden + piece * 8};
-  const __nv_bfloat16* wsrc[2] = {w + min(e0 + row_a, a.pool - 1) * a.hidden + piece * 8, w + min(e0 + row_b, a.pool - 1) * a.hidden + piece * 8};
-  const int k_blocks = static_cast<int>(k_share / RM_K);
-  auto stage_in = [&](int kb) {
-    const int st = kb % RM_STAGES;
-    if (kb < k_blocks) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int row = h ? row_b : row_a;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(&xs[st][row][piece * 8]))), "l"(xsrc[h] + kb * RM_K) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(&ws[st][row][piece * 8]))), "l"(wsrc[h] + kb * RM_K) : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
   float acc[2][4][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0f;
-  stage_in(0);
-  stage_in(1);
-  for (int kb = 0; kb < k_blocks; ++kb) {
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
-    stage_in(kb + 2);
-    const int st = kb % RM_STAGES;
-#pragma unroll
-    for (int ks = 0; ks < RM_K; ks += 16) {
-      uint32_t af[2][4], bf[4][2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int r = wm + 16 * i + g;
-        af[i][0] = *reinterpret_cast<const uint32_t*>(&xs[st][r][ks + 2 * t]);
-        af[i][1] = *reinterpret_cast<const uint32_t*>(&xs[st][r + 8][ks + 2 * t]);
-        af[i][2] = *reinterpret_cast<const uint32_t*>(&xs[st][r][ks + 2 * t + 8]);
-        af[i][3] = *reinterpret_cast<const uint32_t*>(&xs[st][r + 8][ks + 2 * t + 8]);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int n = wn + 8 * j + g;
-        bf[j][0] = *reinterpret_cast<const uint32_t*>(&ws[st][n][ks + 2 * t]);
-        bf[j][1] = *reinterpret_cast<const uint32_t*>(&ws[st][n][ks + 2 * t + 8]);
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {  // sixteen exact products summed from zero per instruction; running sums in plain fp32 (see the kernel above)
-          float d0, d1, d2, d3;
-          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                       : "=f"(d0), "=f"(d1), "=f"(d2), "=f"(d3)
-                       : "r"(af[i][0]), "r"(af[i][1]), "r"(af[i][2]), "r"(af[i][3]), "r"(bf[j][0]), "r"(bf[j][1]), "f"(0.0f));
-          acc[i][j][0] += d0; acc[i][j][1] += d1; acc[i][j][2] += d2; acc[i][j][3] += d3;
-        }
-    }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  router_tile_mma(stages, reinterpret_cast<const __nv_bfloat16*>(a.x) + k_first, reinterpret_cast<const __nv_bfloat16*>(a.router_w) + k_first, a, t0, e0, static_cast<int>(k_share / RM_K), wm, wn, acc);
+  __syncthreads();  // the last block has been read
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
