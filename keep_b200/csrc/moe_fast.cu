@@ -369,7 +369,7 @@ bool shapes_supported(int64_t out_dim, int64_t in_dim, int64_t groups) {
 static bool many_items(const FastProjectionArgs& p) {
   return p.max_routes >= SMALL_CALL_ROUTES && p.in_dim <= slab_max_in_dim(p.group_cols > PAIRED_GROUP_ROUTES ? MAX_GROUP_ROUTES : PAIRED_GROUP_ROUTES);
 }
-// Few route groups of at most four routes.  Small calls run the sweep kernel (measured on a B200 at
+// Few route groups of at most four routes (of the calls that the few-token kernel does not take).  Small calls run the sweep kernel (measured on a B200 at
 // 4096 inputs: ahead of the split slab kernel up to four tokens of top-6, behind it at eight); the
 // rest, and every layer with a residual tier (the slab kernels hold the residual pass), the split
 // form of the slab kernel when the activations leave it room.  0 = neither, 1 = split slab, 2 = sweep.

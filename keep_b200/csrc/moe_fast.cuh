@@ -17,6 +17,7 @@ namespace keepvq {
 namespace fast {
 
 constexpr int MAX_GROUP_ROUTES = 8;     // routes of one expert that share an mma.sync tile (its 8 columns)
+constexpr int FEW_TOKENS_ROUTES = 84;   // most routes of a layer call in one launch (few_tokens_pay)
 constexpr int SMALL_CALL_ROUTES = 48;   // calls with fewer routes never run the plain slab kernel
 constexpr int FEW_ROUTE_GROUPS = 96;    // below this many route groups a CTA's warps share rows AND inputs (sweep kernel, split slab kernel)
 constexpr int PAIRED_GROUP_ROUTES = 4;  // ... when a route's two byte planes take a column each (one MMA per step)
@@ -403,6 +404,12 @@ struct FewTokensArgs {
   uint32_t act_bytes;
   int32_t group_shift;
 };
+// Which layer calls the few-token kernel is the faster one for (us a layer against the chain of kernels, B200): 12 and
+// 14 tokens of top-6 of 384 experts 152 and 176 against 177 and 191, 16 tokens 192 against 178; 8, 12, 14 and 16
+// tokens of 192 experts with scale groups 158, 214, 240 and 259 against 194, 240, 265 and 259.  Where experts get
+// several routes each the chain's groups of them win earlier: of 16 experts 8 tokens 67 against 77, 10 tokens 78
+// against 77, 12 tokens 84 against 77.
+inline bool few_tokens_pay(int64_t routes, int64_t slots) { return routes < SMALL_CALL_ROUTES || (routes <= FEW_TOKENS_ROUTES && routes <= slots / 2); }
 bool few_tokens_fits(int64_t routes, int64_t tokens, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups);
 bool few_tokens_router_fits(const keepvq_router_logits_args& logits, const keepvq_routed_topk_args& topk);
 int64_t few_tokens_sync_bytes(int64_t tokens, int64_t out_dim);  // scratch of a call with gate/up and down, any contents

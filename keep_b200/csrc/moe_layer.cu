@@ -228,7 +228,7 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
   const uint32_t* padded = live < routes ? a.served_slot : nullptr;
 
   // few routes: whatever part of the layer the call asks for as one launch of the few-token kernel
-  const bool few = tensor_path && !residual && !prefill && routes < fast::SMALL_CALL_ROUTES && fast::few_tokens_fits(routes, a.tokens, a.slots, a.inter, a.hidden, a.w1.groups) &&
+  const bool few = tensor_path && !residual && !prefill && fast::few_tokens_pay(routes, a.slots) && fast::few_tokens_fits(routes, a.tokens, a.slots, a.inter, a.hidden, a.w1.groups) &&
                    fast::few_tokens_fits(routes, a.tokens, a.slots, a.hidden, a.inter, a.w2.groups) && a.inter % 16 == 0 && a.hidden % 32 == 0 && aligned_to(a.x, 16) && aligned_to(a.w1.codes, 16) && aligned_to(a.w3.codes, 16) && aligned_to(a.w2.codes, 16) &&
                    fast::few_tokens_sync_bytes(a.tokens, a.hidden) <= sc.h - sc.gate;
   bool router_fused = false;

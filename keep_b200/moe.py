@@ -216,7 +216,7 @@ class RoutedMoELayer:
     def _one_launch(self, tokens: int) -> bool:
         """Whether a call of ``tokens`` rows runs the few-token kernel (``few`` in csrc/moe_layer.cu)."""
         routes, whole = tokens * self.top_k, lambda n: (n + 255) // 256 * 256
-        return not self.res_rows and 0 < routes < 48 and tokens <= 23 and self.hidden <= 5120 and self.inter <= 5120 and not self._on_tcgen05(routes) \
+        return not self.res_rows and 0 < routes and (routes < 48 or routes <= min(84, self.slots // 2)) and tokens <= 23 and self.hidden <= 5120 and self.inter <= 5120 and not self._on_tcgen05(routes) \
             and 2 * 8 * (160 + 16) + 4 + tokens * (self.hidden // 32) * 4 <= 2 * whole(routes * self.inter * 4)
 
     def launches_per_call(self, tokens: int, dtype: torch.dtype = torch.bfloat16) -> int:

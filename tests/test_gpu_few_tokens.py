@@ -40,6 +40,22 @@ def test_layer_calls_of_few_routes(cuda, tokens, experts, top_k, hidden, inter, 
     check_layer(cfg, x, out, routing, top_k=top_k, score_func=score)
 
 
+@pytest.mark.parametrize("tokens,experts,top_k,launches", [
+    (8, 96, 6, 1),    # 48 routes, half as many as slots
+    (14, 168, 6, 1),  # the most routes
+    (8, 95, 6, 7),    # one expert fewer: the chain of kernels
+    (17, 400, 5, 7),  # one route more
+])
+def test_layer_calls_of_48_routes_and_more(cuda, tokens, experts, top_k, launches):
+    cfg = synthetic.layer(seed=79, experts=experts, hidden=512, inter=256, group_hidden=256)
+    x = synthetic.tokens(80 + tokens, tokens, 512)
+    layer = build_layer(cuda, cfg, top_k=top_k)
+    assert layer.launches_per_call(tokens) == launches
+    out, routing = layer.decode(x.to(cuda))
+    assert not layer.wait_expired(tokens, x.dtype)
+    check_layer(cfg, x, out, routing, top_k=top_k)
+
+
 def test_stage_by_stage_and_replayed_from_a_graph(cuda):
     """The parts of a call one after the other, and a captured call replayed (which finds its own
     barrier words in the scratch), give what the whole call gives, to the bit."""
