@@ -3,8 +3,8 @@
 //
 // The projection kernels themselves (HBM-bound by design: every code byte is read once per group
 // of routes) live in their own files: projection_slab.cu (calls with many route groups, and their
-// split form for a residual tier with few), projection_sweep.cu (few route groups) and
-// prefill_umma.cu (many routes per expert, tcgen05).  They share:
+// split form for a residual tier with few), projection_sweep.cu (few route groups),
+// few_tokens.cu (a whole call of few routes in one launch) and prefill_umma.cu (many routes per expert, tcgen05).  They share:
 //   - a codeword becomes the A fragment of an m16n8k32 int8 MMA through two 4-byte table reads
 //     (abs byte, sign byte; 32 replicas each so lanes never share a bank) XORed and spread from
 //     nibbles to bytes: the nibble decoder of moe_fast.cuh;
