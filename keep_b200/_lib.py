@@ -234,7 +234,23 @@ def packer(cls):
     layout = struct.Struct("@" + fields(cls) + "0P")  # native alignment, and the struct's own at its end
     assert layout.size == ctypes.sizeof(cls), cls
     pack, make = layout.pack, cls.from_buffer_copy
-    return lambda *values: make(pack(*values))
+
+    def pack_args(*values):
+        try:
+            return make(pack(*values))
+        except (OverflowError, struct.error):  # a value outside its field, a limit of 1e39 meant as "none", say: as ctypes takes it
+            return _by_field(cls(), iter(values))
+
+    return pack_args
+
+
+def _by_field(args, values):
+    for name, kind in args._fields_:
+        if kind in _FORMAT:
+            setattr(args, name, next(values))
+        else:
+            _by_field(getattr(args, name), values)
+    return args
 
 
 pack_layer_args = packer(MoELayerArgs)

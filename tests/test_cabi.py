@@ -51,6 +51,35 @@ def test_struct_sizes_match_the_compiler():
         assert ctypes.sizeof(structs[name]) == int(size), name
 
 
+def test_packed_arguments_take_what_ctypes_takes():
+    """The structs packed in one step equal those set field by field, also for a float beyond fp32's range
+    (which becomes an infinity) and an integer beyond its field's."""
+    from keep_b200 import _lib
+
+    def flat(cls):
+        for name, kind in cls._fields_:
+            yield from flat(kind) if hasattr(kind, "_fields_") else [(name, kind)]
+
+    def by_field(args, values):
+        for name, kind in args._fields_:
+            if hasattr(kind, "_fields_"):
+                by_field(getattr(args, name), values)
+            else:
+                setattr(args, name, next(values))
+        return args
+
+    for cls, pack in ((_lib.MoELayerArgs, _lib.pack_layer_args), (_lib.GroupedProjectionArgs, _lib.pack_grouped_args), (_lib.MatvecArgs, _lib.pack_matvec_args)):
+        fields = list(flat(cls))
+        plain = [1.5 if kind is ctypes.c_float else 7 for _, kind in fields]
+        for i in range(-1, len(fields)):
+            values = list(plain)
+            if i >= 0:
+                values[i] = {ctypes.c_float: -1e40, ctypes.c_int32: 2 ** 32 + 3, ctypes.c_int64: 2 ** 64 + 3}.get(fields[i][1], 2 ** 63)
+            want = by_field(cls(), iter(values))
+            got = pack(*values)
+            assert bytes(got) == bytes(want), (cls, i)
+
+
 def test_padding_of_the_grouped_arguments_means_nothing():
     """A C caller that fills in the fields and leaves the struct's padding as it finds it is served like
     one that clears it.  (Calls that the library refuses for a misaligned row, before any CUDA call.)"""
