@@ -432,6 +432,10 @@ typedef struct keepvq_grouped_projection_args {
 int64_t keepvq_grouped_projection_workspace_bytes(int64_t routes, int64_t in_dim);
 int64_t keepvq_grouped_projection_status_offset(int64_t routes, int64_t in_dim);
 int keepvq_grouped_projection(const keepvq_grouped_projection_args* args, void* stream);
+/* Zeros on the current device that the library holds for as long as it is loaded: the `rhs` of up to
+ * *count routes of a single matrix, in place for every stream.  The first call with a device current may
+ * load code there and should precede a capture. */
+int keepvq_zero_routes(const uint32_t** routes, int64_t* count);
 /* The same for 8-bit codes: `codes` is the address of uint8 [slots, out_dim, in_dim/8], `codebook` the
  * table words (dim d in nibble d), codebook_all_odd is not looked at, and there is no residual.  Calls
  * that the general kernel serves as fast (few routes) and unaligned codes are KEEPVQ_ERR_UNSUPPORTED:

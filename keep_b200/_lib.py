@@ -170,6 +170,7 @@ _SIGNATURES = {
     "keepvq_grouped_projection": (c_int, [POINTER(GroupedProjectionArgs), c_void_p]),
     "keepvq_grouped_projection_bytes": (c_int, [POINTER(GroupedProjectionArgs), c_void_p]),
     "keepvq_grouped_projection_bytes_served": (c_int, [c_int64, c_int64, c_int64, c_int64, c_int64]),
+    "keepvq_zero_routes": (c_int, [POINTER(c_void_p), POINTER(c_int64)]),
     "keepvq_wait_selftest_workspace_bytes": (c_int64, []),
     "keepvq_wait_selftest": (c_int, [c_void_p, c_int64, c_int64, c_void_p]),
     "keepvq_ep_pack": (c_int, [POINTER(EpPackArgs), c_void_p]),

@@ -58,6 +58,21 @@ static GroupedScratch plan_grouped(int64_t routes, int64_t in_dim) {
 
 }  // namespace keepvq
 
+namespace keepvq {
+constexpr int64_t ZERO_ROUTES = 64;
+static __device__ uint32_t g_zero_routes[ZERO_ROUTES];  // never written
+}  // namespace keepvq
+
+extern "C" int keepvq_zero_routes(const uint32_t** routes, int64_t* count) {
+  if (!routes || !count) return KEEPVQ_ERR_NULL;
+  void* address = nullptr;
+  const cudaError_t e = cudaGetSymbolAddress(&address, keepvq::g_zero_routes);
+  if (e != cudaSuccess) return keepvq::note_cuda_error(e);
+  *routes = static_cast<const uint32_t*>(address);
+  *count = keepvq::ZERO_ROUTES;
+  return KEEPVQ_OK;
+}
+
 extern "C" int64_t keepvq_grouped_projection_workspace_bytes(int64_t routes, int64_t in_dim) {
   if (routes < 0 || in_dim <= 0 || in_dim % 8) return KEEPVQ_ERR_SHAPE;
   return keepvq::plan_grouped(routes, in_dim).total;

@@ -16,6 +16,8 @@ that fit (inputs and scale groups in multiples of 256) run on the layer's int8 t
 
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -122,37 +124,51 @@ def _dense_reference(x2d, codes, scales, codebook, code_bits):
     return x2d.to(torch.float32) @ weights.T
 
 
-_zero_routes: dict = {}  # (device, stream) -> int32 zeros, read only: the expert of every route of a single matrix
-_ZEROS = 64
+class _ToOneMatrix:
+    """The experts of a single matrix's routes: int32 zeros on the device, which the library holds (a launch
+    that clears a tensor of them was a tenth of a small call)."""
+
+    dtype, is_cuda = torch.int32, True
+
+    def __init__(self, address: int, device: torch.device, count: int):
+        self.address, self.device, self.count = address, device, count
+
+    def data_ptr(self) -> int:
+        return self.address
+
+    def numel(self) -> int:
+        return self.count
+
+    def is_contiguous(self) -> bool:
+        return True
 
 
-def _routes_to_one(count: int, device: torch.device, stream: int) -> torch.Tensor:
-    """At least ``count`` int32 zeros (the launch that clears them was a tenth of a small call).  Kept per
-    stream, where every reader is behind the clearing, and for a few streams; a captured call's are
-    cleared in its graph and stay the graph's."""
-    if count > _ZEROS or torch.cuda.is_current_stream_capturing():
-        return torch.zeros(count, dtype=torch.int32, device=device)
-    key = (device, stream)
-    zeros = _zero_routes.get(key)
-    if zeros is None:
-        zeros = torch.zeros(_ZEROS, dtype=torch.int32, device=device)
-        if len(_zero_routes) < 16:
-            _zero_routes[key] = zeros
-    return zeros
+_zero_routes: dict = {}  # device -> (address, how many): constants of the loaded library
+
+
+def _routes_to_one(count: int, device: torch.device):
+    """``count`` int32 zeros: the library's, or a tensor where it has fewer (and where its first use falls
+    into a capture, which is no place to look the address up)."""
+    if device not in _zero_routes and not torch.cuda.is_current_stream_capturing():
+        address, have = ctypes.c_void_p(), ctypes.c_int64()
+        with _lib.on_device(device):
+            _lib.check(_lib.load().keepvq_zero_routes(ctypes.byref(address), ctypes.byref(have)), "keepvq_zero_routes")
+        _zero_routes[device] = (address.value, have.value)
+    address, have = _zero_routes.get(device, (0, 0))
+    return _ToOneMatrix(address, device, count) if count <= have else torch.zeros(count, dtype=torch.int32, device=device)
 
 
 def _one_matrix(rows, codes, scales, table, code_bits, out_shape):
     """Every row of ``rows`` against the one matrix ``codes``: the int8 tensor-core kernels for
     16-bit codes with fp16 / bf16 rows when the shapes fit them, else the general kernel."""
     out, routes, (out_dim, cw) = None, rows.numel() // max(rows.shape[-1], 1), codes.shape
-    stream = torch.cuda.current_stream(rows.device).cuda_stream
-    rhs, scales = _routes_to_one(routes, rows.device, stream), scales.contiguous()
+    rhs, scales = _routes_to_one(routes, rows.device), scales.contiguous()
     if code_bits == 16 and rows.dtype in (torch.float16, torch.bfloat16) and scales.dtype in _lib._DTYPE_TAG:
         from .prefill import project
 
-        out = project(rows, routes, cw * 8, codes, 1, out_dim, scales, scales.shape[1], table, rhs, out_shape, stream=stream)
+        out = project(rows, routes, cw * 8, codes, 1, out_dim, scales, scales.shape[1], table, rhs, out_shape)
     if out is None:
-        out = routed_matvec(rows.reshape(routes, cw * 8), codes[None], scales[None], table, rhs[:routes], x_div=1, code_bits=code_bits).reshape(out_shape)
+        out = routed_matvec(rows.reshape(routes, cw * 8), codes[None], scales[None], table, rhs, x_div=1, code_bits=code_bits).reshape(out_shape)
     return out
 
 

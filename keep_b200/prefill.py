@@ -72,16 +72,16 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
                    x_div=x_div, code_bits=code_bits, residual=residual, hot_of_slot=hot_of_slot)
 
 
-def project(rows, routes, in_dim, codes, slots, out_dim, scales, groups, table, rhs, out_shape, *, x_div=1, code_bits=16, residual=None, hot_of_slot=None, stream=None):
+def project(rows, routes, in_dim, codes, slots, out_dim, scales, groups, table, rhs, out_shape, *, x_div=1, code_bits=16, residual=None, hot_of_slot=None):
     """The same with the sizes given beside the tensors (one matrix's codes and scales, say, without an
-    experts' dimension; ``rhs`` may hold more than ``routes``), and the shape of the answer."""
+    experts' dimension), and the shape of the answer."""
     if codes.dtype != (torch.uint8 if code_bits == 8 else torch.uint16) or in_dim % 256 or rows.dtype not in (torch.float16, torch.bfloat16):
         return None
     if code_bits == 8 and not byte_codes_served(routes, slots, out_dim, in_dim, groups):
         return None  # (asked first: a call prepared to be refused cost 20 us)
     lib = _lib.load()
     device = rows.device
-    stream = torch.cuda.current_stream(device).cuda_stream if stream is None else stream
+    stream = torch.cuda.current_stream(device).cuda_stream
     nbytes = _scratch_bytes(routes, in_dim)
     # Scratch of this call alone, from the caching allocator: calls of other threads, of other streams
     # and of other captured graphs have their own, and a graph's stays the graph's.

@@ -63,3 +63,41 @@ def test_a_call_that_the_library_will_refuse_prepares_nothing(monkeypatch):
     monkeypatch.setattr(torch.cuda, "current_stream", prepared)
     monkeypatch.setattr(torch, "empty", prepared)
     assert prefill.tensor_core_projection(rows, codes, scales, table, rhs, code_bits=8) is None
+
+
+def test_the_routes_of_a_single_matrix_outlive_any_caller(monkeypatch):
+    """The expert indices of a single matrix's routes belong to no caller, stream or tracer: a call made
+    under a tracing mode (or on a stream that is gone) must not leave its own behind for the next."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from keep_b200 import _lib, kernels, prefill
+
+    held, seen = (ctypes.c_uint32 * 64)(), []
+
+    def zero_routes(address, count):
+        address._obj.value, count._obj.value = ctypes.addressof(held), 64
+        return 0
+
+    def project(rows, routes, *rest, **named):
+        seen.append(rest[7])
+        return torch.empty(routes)
+
+    monkeypatch.setattr(_lib, "load", lambda: SimpleNamespace(keepvq_zero_routes=zero_routes))
+    monkeypatch.setattr(prefill, "project", project)
+    monkeypatch.setattr(kernels, "_zero_routes", {})
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: SimpleNamespace(cuda_stream=0))
+    monkeypatch.setattr(torch.cuda, "device", lambda device: contextlib.nullcontext())
+
+    def call(routes):
+        rows = torch.zeros((routes, 256), dtype=torch.bfloat16)
+        codes, scales = torch.zeros((32, 32), dtype=torch.uint16), torch.ones((32, 1), dtype=torch.float16)
+        kernels._one_matrix(rows, codes, scales, torch.zeros(256, dtype=torch.int32), 16, (routes, 32))
+        return seen[-1]
+
+    with FakeTensorMode():
+        call(3)
+    rhs = call(3)
+    assert rhs.data_ptr()
+    assert list((ctypes.c_uint32 * 3).from_address(rhs.data_ptr())) == [0, 0, 0]
+    assert call(65).numel() == 65 and not call(65).any()  # more than the library holds
