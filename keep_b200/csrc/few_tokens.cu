@@ -32,7 +32,7 @@
 // layer took 38 us, at 97 KB 34.  Hence the loops kept rolled and the calls kept calls below.
 #include <algorithm>
 #include <atomic>
-#include <random>
+#include <chrono>
 #include <type_traits>
 #include <utility>
 
@@ -818,9 +818,11 @@ bool few_tokens_router_fits(const keepvq_router_logits_args& l, const keepvq_rou
          t.score_func >= KEEPVQ_SCORE_SOFTMAX && t.score_func <= KEEPVQ_SCORE_SQRT_SOFTPLUS && aligned_to(l.x, 16) && aligned_to(l.router_w, 16);
 }
 
-// A token for the barrier words that no other launch of this or an earlier process is likely to have left behind.
-static uint64_t next_token() {
-  static std::atomic<uint64_t> next{(static_cast<uint64_t>(std::random_device{}()) << 32) | 1u};
+// A token for the barrier words that no other launch of this or an earlier process is likely to have left
+// behind: counted on from where and when the library came to be here (nothing that may throw: the callers are C).
+static uint64_t next_token() noexcept {
+  static char here;
+  static std::atomic<uint64_t> next{(static_cast<uint64_t>(std::chrono::steady_clock::now().time_since_epoch().count()) * 0xD1342543DE82EF95ull) ^ reinterpret_cast<uintptr_t>(&here)};
   uint64_t z = next.fetch_add(0x9E3779B97F4A7C15ull, std::memory_order_relaxed);
   z ^= z >> 32;
   return z | 1u;  // (zero marks a clear word)

@@ -30,6 +30,17 @@ def test_library_exports_every_declared_symbol():
     assert lib.keepvq_status_string(-2).decode() == "inconsistent sizes"
 
 
+def test_no_source_of_randomness_that_may_throw():
+    """The entry points are C: an exception that leaves one ends the process.  ``std::random_device`` throws
+    where the host has no entropy to give (no /dev/urandom in a sandbox, no descriptor left)."""
+    import subprocess
+
+    from keep_b200 import _lib
+
+    names = subprocess.run(["nm", "-D", "--undefined-only", str(_lib.LIBRARY_PATH)], capture_output=True, text=True, check=True).stdout
+    assert "random_device" not in names
+
+
 def test_struct_sizes_match_the_compiler():
     """ctypes mirrors of the argument structs have the layout gcc gives the header."""
     import subprocess
