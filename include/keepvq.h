@@ -576,6 +576,13 @@ int keepvq_moe_decode_layer_static(const keepvq_moe_layer_args* args, void* stre
  * ------------------------------------------------------------------------------------------ */
 int64_t keepvq_wait_selftest_workspace_bytes(void);
 int keepvq_wait_selftest(void* workspace, int64_t workspace_bytes, int64_t wait_ns, void* stream);
+/* Self-test of the grid barriers of the few-token layer kernel: the stages of a layer call (of few
+ * routes, else KEEPVQ_ERR_UNSUPPORTED) with `token` as the launch's, the way every replay of a captured
+ * call has the same one, and `wait_ns` as the limit of its waits.  `absent` 0: an ordinary call; 1: one
+ * thread block never comes to the barrier behind the logits; 2: nor to the one in front of the down
+ * projection, having passed the first.  The others' waits then run out, the status word becomes 1 and
+ * every block returns, with no barrier word left set.  No counterpart in the reference. */
+int keepvq_grid_wait_selftest(const keepvq_moe_layer_args* args, int32_t stages, int32_t absent, int64_t wait_ns, uint64_t token, void* stream);
 
 #ifdef __cplusplus
 }

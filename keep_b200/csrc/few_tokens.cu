@@ -58,6 +58,7 @@ constexpr int FT_SMEM_BYTES = 217 * 1024;     // dynamic; the static arrays take
 constexpr uint32_t FT_STATIC_MIN = 9 * 1024, FT_STATIC_MAX = 11 * 1024;  // where the dynamic part begins (the kernel checks what the launch makes of it)
 constexpr int FT_BARRIER_WORDS = FT_MAX_CTAS + 16;  // a word per CTA, and on a line of its own the one all wait on
 constexpr uint64_t FT_WAIT_NS = 2000000000ull;
+constexpr int FT_ABSENT_CTA = 3;  // the one that does not come in the self-test
 constexpr uint32_t FT_PREFETCH_BYTES = 96 * 1024;  // of a CTA's down codes, asked into L2 while gate/up runs
 static_assert(FT_MAX_CHUNKS <= 32, "a warp looks at all chunks of a row at once");
 
@@ -88,31 +89,41 @@ static uint64_t ft_divisor(int64_t d) { return ((uint64_t{1} << 40) + d - 1) / d
 __device__ __forceinline__ int ft_div(uint32_t n, uint64_t divisor) { return static_cast<int>((n * divisor) >> 40); }
 // All CTAs of the (cooperative) grid meet, in two halves.  Every CTA has a word of its own, which it
 // sets to the launch's token.  A word left by another launch, or never written, does not match the
-// token, so the words need no clearing before the launch; the launch clears them at its end, so that
-// its own replay from a captured graph finds none set.
+// token, so the words need no clearing before the launch.  A replay from a captured graph has the token
+// of the launch before it, so none may be left set, however a launch ends: a CTA clears its own words on
+// every way out, and the word that the others wait on is written by the first CTA alone, which clears
+// it once every other CTA has taken its word back.  Nobody writes another's word, so this holds in
+// whatever order CTAs give up.  A CTA may take its words back only when nobody still waits for them, so
+// the last barrier of a launch is one that GATHERs, which the others pass only after the first CTA has
+// seen every word (and by then everybody has passed the barrier before it, too).
+__device__ __forceinline__ void ft_set(uint64_t* word, uint64_t value) { asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(word), "l"(value) : "memory"); }
+__device__ __forceinline__ void ft_clear(uint64_t* word) { asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(word), "l"(uint64_t{0}) : "memory"); }
+__device__ __forceinline__ uint64_t ft_get(const uint64_t* word) {
+  uint64_t seen;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(word) : "memory");
+  return seen;
+}
 __device__ __forceinline__ void ft_arrive(uint64_t* words, uint64_t token) {
   __syncthreads();
-  if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(words + blockIdx.x), "l"(token) : "memory");
+  if (threadIdx.x == 0) ft_set(words + blockIdx.x, token);
 }
-__device__ __forceinline__ int ft_poll(const uint64_t* word, uint64_t token, uint64_t deadline) {
+// Until the word holds the token (or, with `gone`, no longer does).
+__device__ __forceinline__ int ft_poll(const uint64_t* word, uint64_t token, uint64_t deadline, bool gone = false) {
   for (uint32_t spin = 0;; ++spin) {
-    uint64_t seen;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(word) : "memory");
-    if (seen == token) return 1;
+    if ((ft_get(word) == token) != gone) return 1;
     if ((spin & 63u) == 63u && global_timer_ns() > deadline) return 0;
   }
 }
-// False in every thread when the deadline passes.  GATHER: the first CTA looks at all words, then sets
+// False in every thread when the deadline passes.  Gathering, the first CTA looks at all words, then sets
 // the one that the others wait on; without it every CTA looks at every word, which is sooner done
 // where the words are mostly set already, and takes 4 to 6 us where they are not.
-template <bool GATHER>
-__device__ __forceinline__ bool ft_wait(uint64_t* words, uint64_t token, uint64_t deadline) {
+__device__ __forceinline__ bool ft_wait(uint64_t* words, uint64_t token, uint64_t deadline, bool gather) {
   uint64_t* go = words + FT_MAX_CTAS;
   int ok = 1;
-  if (!GATHER || blockIdx.x == 0) {
+  if (!gather || blockIdx.x == 0) {
     for (unsigned i = threadIdx.x; i < gridDim.x && ok; i += FT_THREADS) ok = ft_poll(words + i, token, deadline);
     ok = __syncthreads_and(ok);
-    if (GATHER && threadIdx.x == 0 && ok) asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(go), "l"(token) : "memory");
+    if (gather && threadIdx.x == 0 && ok) ft_set(go, token);
     return ok != 0;
   }
   if (threadIdx.x == 0) ok = ft_poll(go, token, deadline);
@@ -252,19 +263,28 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
   const uint32_t ring = (warp < low_rings ? base + warp * RING_BYTES : high_rings + (warp - low_rings) * RING_BYTES) + lane * 16;
   const uint32_t abs_lane = a0 + lane * 4u, sign_lane = a0 + 128u + lane * 4u;
   const bool with_router = a.parts & FT_ROUTER;
-  const bool meets = with_router || ((a.parts & FT_GATE_UP) && (a.parts & FT_DOWN));
+  const bool two_phases = (a.parts & FT_GATE_UP) && (a.parts & FT_DOWN);
   uint64_t* const words_a = a.barrier_words;
   uint64_t* const words_b = a.barrier_words + FT_BARRIER_WORDS;
   auto begin = [&]() {  // behind the wait on the previous kernel
     grid_wait();
-    if (tid == 0) deadline = global_timer_ns() + FT_WAIT_NS;  // (in shared memory: a pair of registers less in the sweep; read behind the barriers' own block barrier)
+    if (tid == 0) deadline = global_timer_ns() + a.wait_ns;  // (in shared memory: a pair of registers less in the sweep; read behind the barriers' own block barrier)
     if (cta == 0) {  // ordered before their first use by the barrier in front of the down projection
       if (a.parts & FT_COMBINE)  // the pick sum's counters
 #pragma unroll 1
-        for (int i = tid; i < a.tokens * (a.phase[1].out_dim / 32); i += FT_THREADS) a.counters[1 + i] = 0;
-      if (meets && tid == 0) a.counters[0] = 0;
+        for (int i = tid; i < a.tokens * (a.phase[1].out_dim / 32); i += FT_THREADS) a.counters[i] = 0;
       if (a.status && tid == 0) *a.status = 0;
     }
+  };
+  auto take_words_back = [&]() {  // behind the last barrier, or on the way out
+    if (tid == 0) {
+      if (with_router) ft_clear(words_a + cta);
+      if (two_phases) ft_clear(words_b + cta);
+    }
+  };
+  auto give_up = [&]() {
+    take_words_back();
+    if (a.status && tid == 0) atomicExch(a.status, 1);
   };
 
   // ---- up to eight activation rows, quantised into fragment order in shared memory
@@ -400,6 +420,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
         }
         __syncthreads();
       }
+    if (a.absent == 1 && cta == FT_ABSENT_CTA) return;
     ft_arrive(words_a, a.token);
   }
   // what needs no routing, while the others arrive (or, without a router, while the previous kernel
@@ -407,10 +428,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
   build_nibble_tables(a0, a.codebook, tid, FT_THREADS);
   if (by_token) stage_rows(a.phase[0], a.tokens, lane);
   if (with_router) {
-    if (!ft_wait<false>(words_a, a.token, deadline)) {
-      if (a.status && tid == 0) atomicExch(a.status, 1);
-      return;
-    }
+    if (!ft_wait(words_a, a.token, deadline, !two_phases)) return give_up();
+    if (!two_phases) take_words_back();
     // ---- every CTA works out every token's picks (in the rings, which are still empty)
 #pragma unroll 1
     for (int t0 = 0; t0 < a.tokens; t0 += FT_PICK_TOKENS) ft_pick(a.topk, base, t0, own_token, own_scores, route_slot, route_weight);
@@ -543,10 +562,13 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"(unit_bytes) : "memory");
       }
     }
-    if (ph == 1 && (a.parts & FT_GATE_UP) && !ft_wait<true>(words_b, a.token, deadline)) {
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      if (a.status && tid == 0) atomicExch(a.status, 1);
-      return;
+    if (ph == 1 && (a.parts & FT_GATE_UP)) {
+      const bool all_here = ft_wait(words_b, a.token, deadline, true);
+      if (!all_here) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return give_up();
+      }
+      take_words_back();
     }
 
     // ---- the activation rows of this CTA's (at most two) groups
@@ -710,8 +732,10 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
       if (tl >= units_per_group) { tl -= units_per_group; ++gr; }
       finish(head, gr, tl);
     }
-    if (ph == 0 && (a.parts & FT_DOWN)) ft_arrive(words_b, a.token);  // the hidden rows are written
-    else __syncthreads();
+    if (ph == 0 && (a.parts & FT_DOWN)) {  // the hidden rows are written
+      if (a.absent == 2 && cta == FT_ABSENT_CTA) return take_words_back();
+      ft_arrive(words_b, a.token);
+    } else __syncthreads();
     // the rings and the activation rows are free again
     if (ph == 0 && own_token >= 0 && own_token < a.tokens && warp == FT_WARPS - 1) {
       // the demanded picks of a token, which nothing here waits for
@@ -760,7 +784,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
       if ((i & 3) >= grp_size[gi]) continue;
       const int tok = grp_route[gi][i & 3] / a.top_k;
       __threadfence();
-      if (atomicAdd(&a.counters[1 + tok * units_per_group + tile], 1u) + 1u == static_cast<uint32_t>(live_picks(tok))) {
+      if (atomicAdd(&a.counters[tok * units_per_group + tile], 1u) + 1u == static_cast<uint32_t>(live_picks(tok))) {
         __threadfence();
         const int at = atomicAdd(&n_due, 1);
         asm volatile("st.shared.u32 [%0], %1;" ::"r"(acts + at * 4), "r"(tok << 16 | tile) : "memory");
@@ -795,15 +819,14 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
       store_out(o, y);
     }
   }
-  // ---- the last CTA to get here clears the barrier words: everybody has passed the barriers ----------
-  if (meets) {
-    __shared__ int last_here;
-    __syncthreads();
-    if (tid == 0) last_here = atomicAdd(&a.counters[0], 1u) + 1u == static_cast<uint32_t>(grid);
-    __syncthreads();
-    if (last_here)
-#pragma unroll 1
-      for (int i = tid; i < 2 * FT_BARRIER_WORDS; i += FT_THREADS) a.barrier_words[i] = 0;
+  // ---- the others' words are back: nobody waits on the first CTA's any more ----------------------------
+  if (cta == 0 && (with_router || two_phases)) {
+    uint64_t* const words = two_phases ? words_b : words_a;
+    const uint64_t late = deadline + a.wait_ns;  // (a CTA that does not see the word gives up by its own deadline and takes its word back all the same)
+    int ok = 1;
+    for (int i = 1 + tid; i < grid && ok; i += FT_THREADS) ok = ft_poll(words + i, a.token, late, true);
+    if (!__syncthreads_and(ok) && a.status && tid == 0) atomicExch(a.status, 1);
+    if (tid == 0) ft_clear(words + FT_MAX_CTAS);
   }
 }
 
@@ -812,7 +835,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
 bool few_tokens_fits(int64_t routes, int64_t tokens, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups) {
   return routes > 0 && slots * out_dim < (int64_t{1} << 31) - 64 && routes <= FT_MAX_ROUTES && tokens <= FT_MAX_TOKENS && in_dim <= FT_MAX_IN && out_dim > 0 && out_dim < (1 << 18) && shapes_supported(out_dim, in_dim, groups);
 }
-int64_t few_tokens_sync_bytes(int64_t tokens, int64_t out_dim) { return 2 * 8 * FT_BARRIER_WORDS + 4 + tokens * (out_dim / 32) * 4; }
+int64_t few_tokens_sync_bytes(int64_t tokens, int64_t out_dim) { return 2 * 8 * FT_BARRIER_WORDS + tokens * (out_dim / 32) * 4; }
 bool few_tokens_router_fits(const keepvq_router_logits_args& l, const keepvq_routed_topk_args& t) {
   return l.router_dtype == KEEPVQ_BF16 && l.pool <= 32 * FT_TOPK_NPL && l.hidden % 8 == 0 && t.top_k <= 16 && t.top_k <= l.pool && l.gate_temp > 0.0f &&
          t.score_func >= KEEPVQ_SCORE_SOFTMAX && t.score_func <= KEEPVQ_SCORE_SQRT_SOFTPLUS && aligned_to(l.x, 16) && aligned_to(l.router_w, 16);
@@ -859,7 +882,8 @@ static int launch_few_tokens(const FewTokensArgs& args, void* sync, cudaStream_t
     p.by_group_chunks = ft_divisor(p.chunks_per_group);
   }
   a.by_grid = ft_divisor(ctas);
-  a.token = next_token();
+  if (!a.token) a.token = next_token();
+  if (!a.wait_ns) a.wait_ns = FT_WAIT_NS;
   a.barrier_words = static_cast<uint64_t*>(sync);
   a.counters = reinterpret_cast<uint32_t*>(static_cast<uint64_t*>(sync) + 2 * FT_BARRIER_WORDS);
   cudaLaunchConfig_t config = {};

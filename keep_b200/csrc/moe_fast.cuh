@@ -400,7 +400,9 @@ struct FewTokensArgs {
   int32_t* status;            // cleared; 1: a wait of the grid ran out, 2: unexpected shared window
   uint64_t* barrier_words;    // filled in by the launch
   uint32_t* counters;
-  uint64_t token, by_grid;
+  uint64_t token, wait_ns;    // filled in by the launch where they are zero
+  uint64_t by_grid;
+  int32_t absent;             // self-test: a CTA comes to neither barrier (1), or to the first only (2)
   uint32_t act_bytes;
   int32_t group_shift;
 };

@@ -185,8 +185,15 @@ extern "C" int64_t keepvq_moe_layer_route_hidden_offset(int64_t tokens, int64_t 
   return keepvq::plan_scratch(tokens, hidden, inter, pool, top_k).h;
 }
 
-extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32_t stages, void* stream) {
-  using namespace keepvq;
+namespace keepvq {
+
+// What the self-test of the grid barriers asks of the few-token kernel (zeros: an ordinary call).
+struct GridWaitTest {
+  uint64_t token, wait_ns;
+  int32_t absent;
+};
+
+static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, const GridWaitTest& test, void* stream) {
   if (!args) return KEEPVQ_ERR_NULL;
   const keepvq_moe_layer_args& a = *args;
   if (!valid_dtype(a.x_dtype) || !valid_dtype(a.router_dtype) || !valid_dtype(a.scales_dtype)) return KEEPVQ_ERR_DTYPE;
@@ -231,8 +238,10 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
   const bool few = tensor_path && !residual && !prefill && fast::few_tokens_pay(routes, a.slots) && fast::few_tokens_fits(routes, a.tokens, a.slots, a.inter, a.hidden, a.w1.groups) &&
                    fast::few_tokens_fits(routes, a.tokens, a.slots, a.hidden, a.inter, a.w2.groups) && a.inter % 16 == 0 && a.hidden % 32 == 0 && aligned_to(a.x, 16) && aligned_to(a.w1.codes, 16) && aligned_to(a.w3.codes, 16) && aligned_to(a.w2.codes, 16) &&
                    fast::few_tokens_sync_bytes(a.tokens, a.hidden) <= sc.h - sc.gate;
+  if (test.token && !few) return KEEPVQ_ERR_UNSUPPORTED;
   bool router_fused = false;
   fast::FewTokensArgs few_args = {};
+  few_args.token = test.token; few_args.wait_ns = test.wait_ns; few_args.absent = test.absent;
 
   if (stages & KEEPVQ_STAGE_ROUTER) {
     keepvq_router_logits_args rl = {};
@@ -336,6 +345,15 @@ extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32
     KEEPVQ_CHECK_LAUNCH();
   }
   return KEEPVQ_OK;
+}
+
+}  // namespace keepvq
+
+extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32_t stages, void* stream) { return keepvq::decode_stages(args, stages, {}, stream); }
+
+extern "C" int keepvq_grid_wait_selftest(const keepvq_moe_layer_args* args, int32_t stages, int32_t absent, int64_t wait_ns, uint64_t token, void* stream) {
+  if (absent < 0 || absent > 2 || wait_ns <= 0 || wait_ns > 1000000000ll || !token) return KEEPVQ_ERR_SHAPE;  // a self-test may hold the GPU for about a second at most
+  return keepvq::decode_stages(args, stages, {token, static_cast<uint64_t>(wait_ns), absent}, stream);
 }
 
 extern "C" int keepvq_moe_decode_layer(const keepvq_moe_layer_args* args, void* stream) {

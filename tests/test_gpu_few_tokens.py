@@ -80,6 +80,42 @@ def test_stage_by_stage_and_replayed_from_a_graph(cuda):
         assert torch.equal(got, want[i])
 
 
+@pytest.mark.parametrize("stages,absent", [("all", 1), ("all", 2), ("no router", 2), ("router and gate/up", 1)])
+def test_a_block_that_stays_away_from_a_grid_barrier(cuda, stages, absent):
+    """The other blocks' waits run out after 3 ms, the status says so, and nothing of the failed call is
+    left for the next: calls with the same token (what a captured call's replays have) over the same
+    scratch, on tokens of their own, pass no barrier before everybody is there."""
+    from keep_b200 import _lib
+
+    cfg = synthetic.layer(seed=83, experts=16, hidden=1024, inter=512)
+    layer = build_layer(cuda, cfg, top_k=5)
+    mask = {"all": _lib.STAGE_ALL, "no router": _lib.STAGE_ALL & ~_lib.STAGE_ROUTER, "router and gate/up": _lib.STAGE_ROUTER | _lib.STAGE_PREPARE | _lib.STAGE_GATE_UP}[stages]
+    lib, token = _lib.load(), 0x0123456789ABCDEF
+    xs = [synthetic.tokens(84 + i, 5, 1024).to(cuda) for i in range(4)]
+    want = []
+    for x in xs:
+        out, _ = layer.decode(x)
+        want.append((out.clone(), layer.route_hidden(5, x.dtype).clone()))
+    buf = layer._buffers_for(5, torch.bfloat16)
+
+    def call(i, absent):
+        if not mask & _lib.STAGE_ROUTER:
+            layer.decode(xs[i], stages=_lib.STAGE_ROUTER)
+        args = layer._layer_args(xs[i], buf["out"], buf["routing"], workspace=buf["workspace"], nbytes=buf["nbytes"])
+        _lib.check(lib.keepvq_grid_wait_selftest(args, mask, absent, 3_000_000 if absent else 1_000_000_000, token, _lib.stream_handle(cuda)), "keepvq_grid_wait_selftest")
+        torch.cuda.synchronize()
+        words = buf["workspace"][: buf["nbytes"] // 8 * 8].view(torch.int64)
+        assert not (words == token).any()
+        return layer.wait_expired(5, torch.bfloat16)
+
+    for i, away in enumerate((0, absent, absent, 0)):
+        assert call(i, away) == bool(away)
+        if not away:
+            assert torch.equal(layer.route_hidden(5, torch.bfloat16), want[i][1])
+            if mask & _lib.STAGE_COMBINE:
+                assert torch.equal(buf["out"], want[i][0])
+
+
 def test_calls_on_two_streams_at_once(cuda):
     cfg = synthetic.layer(seed=75, experts=16, hidden=1024, inter=512)
     layer = build_layer(cuda, cfg, top_k=4)
