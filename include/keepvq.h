@@ -279,11 +279,12 @@ typedef struct keepvq_moe_layer_args {
 /* Bytes of scratch keepvq_moe_decode_layer needs for these sizes (host arithmetic only). */
 int64_t keepvq_moe_layer_workspace_bytes(int64_t tokens, int64_t hidden, int64_t inter, int64_t pool, int32_t top_k);
 int keepvq_moe_decode_layer(const keepvq_moe_layer_args* args, void* stream);
-/* Byte offset, inside the scratch, of an int32 the tcgen05 kernels set to 1 when one of their
- * bounded waits expires (they then stop, free their tensor memory and return; the call's outputs
- * are invalid).  The library clears it at the start of a call that can set it and never reads it
- * back itself: a host that wants to know copies the word out after the call.  No counterpart in
- * the reference. */
+/* Byte offset, inside the scratch, of an int32 status word: 1 when a bounded wait of the tcgen05 kernels
+ * or of the few-token kernel's grid barriers expired (the blocks then stop, release what they hold and
+ * return), 2 when a kernel found its shared memory laid out differently than it was built for (it then
+ * computes nothing); either way the call's outputs are invalid.  The library clears the word in the
+ * PREPARE stage of a call that can set it and never reads it back itself: a host that wants to know
+ * copies the word out after the call.  No counterpart in the reference. */
 int64_t keepvq_moe_layer_status_offset(int64_t tokens, int64_t hidden, int64_t inter, int64_t pool, int32_t top_k);
 
 /* Byte offset, inside the scratch, of the per-route outputs [tokens * top_k, hidden] (activation
@@ -397,8 +398,8 @@ int keepvq_residency_tick(const keepvq_residency_args* args, void* stream);
  * largest magnitude, while against the output the row would give WITHOUT the outlier channel it
  * is about 0.5 % (3 %).  Everything else is exact integer arithmetic.  Rows of routes without an
  * expert are written as zeros.
- * The scratch also holds, at keepvq_grouped_projection_status_offset, the int32 the tcgen05
- * kernel sets when a bounded wait expires (see keepvq_moe_layer_status_offset).
+ * The scratch also holds, at keepvq_grouped_projection_status_offset, the int32 in which the kernels
+ * report what went wrong (see keepvq_moe_layer_status_offset).
  * ------------------------------------------------------------------------------------------ */
 typedef struct keepvq_grouped_projection_args {
   const void* x;             /* [x_rows, in_dim]; fp16 or bf16 (fp32 rows belong to keepvq_routed_matvec, which keeps 24 bits of them) */

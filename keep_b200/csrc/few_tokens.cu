@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
       if (a.parts & FT_COMBINE)  // the pick sum's counters
 #pragma unroll 1
         for (int i = tid; i < a.tokens * (a.phase[1].out_dim / 32); i += FT_THREADS) a.counters[i] = 0;
-      if (a.status && tid == 0) *a.status = 0;
+      if (a.clear_status && a.status && tid == 0) *a.status = 0;
     }
   };
   auto take_words_back = [&]() {  // behind the last barrier, or on the way out

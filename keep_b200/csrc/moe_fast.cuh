@@ -397,7 +397,8 @@ struct FewTokensArgs {
   const float* shared;
   void* dead_out;             // rows of routes without a slot are zeroed here (may be null)
   int64_t dead_row_bytes;
-  int32_t* status;            // cleared; 1: a wait of the grid ran out, 2: unexpected shared window
+  int32_t* status;            // 1: a wait of the grid ran out, 2: unexpected shared window
+  int32_t clear_status;       // ... set to 0 first
   uint64_t* barrier_words;    // filled in by the launch
   uint32_t* counters;
   uint64_t token, wait_ns;    // filled in by the launch where they are zero

@@ -272,6 +272,12 @@ static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, cons
 
   if (few) {
     const bool gate_up = stages & KEEPVQ_STAGE_GATE_UP, down = stages & KEEPVQ_STAGE_DOWN;
+    // the status is cleared where the other kernels' PREPARE stage clears it: a later stage leaves what an earlier one reported
+    few_args.clear_status = gate_up && (stages & KEEPVQ_STAGE_PREPARE);
+    if (!gate_up && (stages & KEEPVQ_STAGE_PREPARE)) {
+      const cudaError_t e = cudaMemsetAsync(ws + sc.status, 0, 4, s);
+      if (e != cudaSuccess) return note_cuda_error(e);
+    }
     if (gate_up || down) {
       const bool combine = gate_up && down && (stages & KEEPVQ_STAGE_COMBINE);
       few_args.parts = (router_fused ? fast::FT_ROUTER : 0u) | (gate_up ? fast::FT_GATE_UP : 0u) | (down ? fast::FT_DOWN : 0u) | (combine ? fast::FT_COMBINE : 0u);

@@ -182,8 +182,10 @@ class RoutedMoELayer:
         return self._scratch_rows("keepvq_moe_layer_route_hidden_offset", self.inter, tokens, dtype, state)
 
     def wait_expired(self, tokens: int, dtype: torch.dtype, state: int = 0) -> bool:
-        """True when a bounded wait of the tcgen05 kernels expired during the last call of this
-        shape (its outputs are then invalid).  Reads one word back: synchronises the stream."""
+        """True when a bounded wait (of the tcgen05 kernels, or of the few-token kernel's grid barriers)
+        expired during the last call of this shape, or a kernel found its shared memory laid out
+        otherwise than it was built for: the call's outputs are then invalid.  Reads one word back:
+        synchronises the stream."""
         buf = self._buffers_for(tokens, dtype, state)
         offset = int(_lib.load().keepvq_moe_layer_status_offset(tokens, self.hidden, self.inter, self.pool, self.top_k))
         if offset < 0:

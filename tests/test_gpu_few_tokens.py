@@ -116,6 +116,30 @@ def test_a_block_that_stays_away_from_a_grid_barrier(cuda, stages, absent):
                 assert torch.equal(buf["out"], want[i][0])
 
 
+def test_a_reported_wait_stays_reported_through_later_stages(cuda):
+    """A wait that ran out in one stage of a call is still in the status word after the stages behind it;
+    the next call's PREPARE clears it."""
+    from keep_b200 import _lib
+
+    layer = build_layer(cuda, synthetic.layer(seed=85, experts=16, hidden=512, inter=256), top_k=4)
+    x = synthetic.tokens(86, 3, 512).to(cuda)
+    layer.decode(x)
+    buf = layer._buffers_for(3, x.dtype)
+    args = layer._layer_args(x, buf["out"], buf["routing"], workspace=buf["workspace"], nbytes=buf["nbytes"])
+    front = _lib.STAGE_ROUTER | _lib.STAGE_PREPARE | _lib.STAGE_GATE_UP
+    _lib.check(_lib.load().keepvq_grid_wait_selftest(args, front, 1, 3_000_000, 77, _lib.stream_handle(cuda)), "keepvq_grid_wait_selftest")
+    assert layer.wait_expired(3, x.dtype)
+    layer.decode(x, stages=_lib.STAGE_DOWN)
+    layer.decode(x, stages=_lib.STAGE_COMBINE)
+    assert layer.wait_expired(3, x.dtype)
+    layer.decode(x, stages=_lib.STAGE_PREPARE)
+    assert not layer.wait_expired(3, x.dtype)
+    for clearing in (front, _lib.STAGE_ALL):
+        buf["workspace"].fill_(0x7F)
+        layer.decode(x, stages=clearing)
+        assert not layer.wait_expired(3, x.dtype)
+
+
 def test_calls_on_two_streams_at_once(cuda):
     cfg = synthetic.layer(seed=75, experts=16, hidden=1024, inter=512)
     layer = build_layer(cuda, cfg, top_k=4)
