@@ -582,8 +582,10 @@ int keepvq_wait_selftest(void* workspace, int64_t workspace_bytes, int64_t wait_
  * call has the same one, and `wait_ns` as the limit of its waits.  `absent` 0: an ordinary call; 1: one
  * thread block never comes to the barrier behind the logits; 2: nor to the one in front of the down
  * projection, having passed the first.  The others' waits then run out, the status word becomes 1 and
- * every block returns, with no barrier word left set.  No counterpart in the reference. */
-int keepvq_grid_wait_selftest(const keepvq_moe_layer_args* args, int32_t stages, int32_t absent, int64_t wait_ns, uint64_t token, void* stream);
+ * every block returns, with no barrier word left set.  `ctas` 0: one block per SM; else so many, at most
+ * 160: more than the device holds at once must leave the call to the other kernels, as in a context
+ * that has only part of the SMs.  No counterpart in the reference. */
+int keepvq_grid_wait_selftest(const keepvq_moe_layer_args* args, int32_t stages, int32_t absent, int32_t ctas, int64_t wait_ns, uint64_t token, void* stream);
 
 #ifdef __cplusplus
 }

@@ -173,7 +173,7 @@ _SIGNATURES = {
     "keepvq_zero_routes": (c_int, [POINTER(c_void_p), POINTER(c_int64)]),
     "keepvq_wait_selftest_workspace_bytes": (c_int64, []),
     "keepvq_wait_selftest": (c_int, [c_void_p, c_int64, c_int64, c_void_p]),
-    "keepvq_grid_wait_selftest": (c_int, [POINTER(MoELayerArgs), c_int32, c_int32, c_int64, ctypes.c_uint64, c_void_p]),
+    "keepvq_grid_wait_selftest": (c_int, [POINTER(MoELayerArgs), c_int32, c_int32, c_int32, c_int64, ctypes.c_uint64, c_void_p]),
     "keepvq_ep_pack": (c_int, [POINTER(EpPackArgs), c_void_p]),
     "keepvq_ep_combine": (c_int, [POINTER(EpCombineArgs), c_void_p]),
     "keepvq_ep_dispatch_peer": (c_int, [POINTER(EpPackArgs), POINTER(EpPeerArgs), c_void_p]),

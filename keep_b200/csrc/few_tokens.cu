@@ -832,8 +832,32 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
 
 // ---- launch -----------------------------------------------------------------------------------
 
+// CTAs of a launch on the current device, one per SM; 0 where a grid of them cannot be launched cooperatively.
+// (Of the device: a context or stream that has only part of its SMs is told so by the launch, see below.)
+static int few_tokens_grid() {
+  static std::atomic<int> known[64];  // plus one; 0: not asked yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (dev < 0 || dev >= 64) return 0;
+  int grid = known[dev].load() - 1;
+  if (grid >= 0) return grid;
+  int sms = 0, cooperative = 0, smem = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  grid = cooperative && smem >= static_cast<int>(FT_SMEM_BYTES + FT_STATIC_MAX - 1024) ? std::min(sms, FT_MAX_CTAS) : 0;  // (1 KB of that is the system's)
+  known[dev].store(grid + 1);
+  return grid;
+}
 bool few_tokens_fits(int64_t routes, int64_t tokens, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups) {
-  return routes > 0 && slots * out_dim < (int64_t{1} << 31) - 64 && routes <= FT_MAX_ROUTES && tokens <= FT_MAX_TOKENS && in_dim <= FT_MAX_IN && out_dim > 0 && out_dim < (1 << 18) && shapes_supported(out_dim, in_dim, groups);
+  // (a CTA's share of the units must not span more than two route groups: no more routes than CTAs)
+  return routes > 0 && slots * out_dim < (int64_t{1} << 31) - 64 && routes <= FT_MAX_ROUTES && tokens <= FT_MAX_TOKENS && in_dim <= FT_MAX_IN && out_dim > 0 && out_dim < (1 << 18) && shapes_supported(out_dim, in_dim, groups) &&
+         routes <= few_tokens_grid();
 }
 int64_t few_tokens_sync_bytes(int64_t tokens, int64_t out_dim) { return 2 * 8 * FT_BARRIER_WORDS + tokens * (out_dim / 32) * 4; }
 bool few_tokens_router_fits(const keepvq_router_logits_args& l, const keepvq_routed_topk_args& t) {
@@ -855,21 +879,15 @@ template <typename XT, bool RAGGED, int DEPTH>
 static int launch_few_tokens(const FewTokensArgs& args, void* sync, cudaStream_t s) {
   auto kernel = few_tokens_kernel<XT, RAGGED, DEPTH>;
   static std::atomic<uint64_t> configured{0};  // one bit per device: the shared-memory opt-in is a per-device attribute of the function
-  static std::atomic<int> sm_count[64];
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return KEEPVQ_ERR_UNSUPPORTED;
+  const int ctas = args.ctas ? args.ctas : few_tokens_grid();
+  if (args.routes > ctas || dev < 0 || dev >= 64) return KEEPVQ_ERR_UNSUPPORTED;
   if (!((configured.load() >> dev) & 1ull)) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_BYTES);
     if (e != cudaSuccess) return note_cuda_error(e);
-    int sms = 0;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return note_cuda_error(e);
-    sm_count[dev].store(sms);
     configured.fetch_or(1ull << dev);
   }
-  const int ctas = sm_count[dev].load() < FT_MAX_CTAS ? sm_count[dev].load() : FT_MAX_CTAS;
-  if (args.routes > ctas) return KEEPVQ_ERR_UNSUPPORTED;  // a CTA's share of the units must not span more than two groups
   FewTokensArgs a = args;
   for (FewTokensPhase& p : a.phase) {
     if (!p.out_dim) continue;
@@ -902,6 +920,10 @@ static int launch_few_tokens(const FewTokensArgs& args, void* sync, cudaStream_t
   config.attrs = &attribute;
   config.numAttrs = 1;
   const cudaError_t err = cudaLaunchKernelEx(&config, kernel, a);
+  if (err == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs here than the device has: nothing was launched, and the caller has kernels whose blocks do not wait for one another
+    cudaGetLastError();
+    return KEEPVQ_ERR_UNSUPPORTED;
+  }
   return err == cudaSuccess ? KEEPVQ_OK : note_cuda_error(err);
 }
 

@@ -125,7 +125,8 @@ static int grouped_projection(const keepvq_grouped_projection_args* args, bool b
     f.phase[1] = {{a.codes, nullptr}, {a.scales, nullptr}, a.x, a.out, static_cast<int32_t>(a.out_dim), static_cast<int32_t>(a.in_dim), static_cast<int32_t>(a.groups), x_div, a.out_dtype};
     f.dead_out = a.out; f.dead_row_bytes = a.out_dim * dtype_size(a.out_dtype);
     f.status = reinterpret_cast<int32_t*>(ws + sc.status); f.clear_status = 1;
-    return fast::few_tokens(f, a.x_dtype, nullptr, s);
+    const int rc = fast::few_tokens(f, a.x_dtype, nullptr, s);
+    if (rc != KEEPVQ_ERR_UNSUPPORTED) return rc;
   }
   const bool many = byte_codes || (!residual && fast::prefill_pays(a.routes, a.slots, a.groups > 1) && fast::prefill_supported(a.slots, a.out_dim, a.in_dim, a.groups));
   // (the sums region has room for a scale group per codeword; these kernels' rows have at most one

@@ -404,6 +404,7 @@ struct FewTokensArgs {
   uint64_t token, wait_ns;    // filled in by the launch where they are zero
   uint64_t by_grid;
   int32_t absent;             // self-test: a CTA comes to neither barrier (1), or to the first only (2)
+  int32_t ctas;               // self-test: so many CTAs (0: one per SM)
   uint32_t act_bytes;
   int32_t group_shift;
 };
@@ -416,7 +417,7 @@ inline bool few_tokens_pay(int64_t routes, int64_t slots) { return routes < SMAL
 bool few_tokens_fits(int64_t routes, int64_t tokens, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups);
 bool few_tokens_router_fits(const keepvq_router_logits_args& logits, const keepvq_routed_topk_args& topk);
 int64_t few_tokens_sync_bytes(int64_t tokens, int64_t out_dim);  // scratch of a call with gate/up and down, any contents
-int few_tokens(const FewTokensArgs& a, int32_t x_dtype, void* sync, cudaStream_t s);
+int few_tokens(const FewTokensArgs& a, int32_t x_dtype, void* sync, cudaStream_t s);  // KEEPVQ_ERR_UNSUPPORTED: nothing was launched, the other kernels take the call
 
 // tcgen05 kernels for many routes per expert (prefill_umma.cu).  `status` is a device word that
 // a CTA sets to 1 if one of its bounded waits expires.

@@ -190,7 +190,7 @@ namespace keepvq {
 // What the self-test of the grid barriers asks of the few-token kernel (zeros: an ordinary call).
 struct GridWaitTest {
   uint64_t token, wait_ns;
-  int32_t absent;
+  int32_t absent, ctas;
 };
 
 static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, const GridWaitTest& test, void* stream) {
@@ -235,62 +235,68 @@ static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, cons
   const uint32_t* padded = live < routes ? a.served_slot : nullptr;
 
   // few routes: whatever part of the layer the call asks for as one launch of the few-token kernel
-  const bool few = tensor_path && !residual && !prefill && fast::few_tokens_pay(routes, a.slots) && fast::few_tokens_fits(routes, a.tokens, a.slots, a.inter, a.hidden, a.w1.groups) &&
-                   fast::few_tokens_fits(routes, a.tokens, a.slots, a.hidden, a.inter, a.w2.groups) && a.inter % 16 == 0 && a.hidden % 32 == 0 && aligned_to(a.x, 16) && aligned_to(a.w1.codes, 16) && aligned_to(a.w3.codes, 16) && aligned_to(a.w2.codes, 16) &&
-                   fast::few_tokens_sync_bytes(a.tokens, a.hidden) <= sc.h - sc.gate;
+  bool few = tensor_path && !residual && !prefill && fast::few_tokens_pay(routes, a.slots) && fast::few_tokens_fits(routes, a.tokens, a.slots, a.inter, a.hidden, a.w1.groups) &&
+             fast::few_tokens_fits(routes, a.tokens, a.slots, a.hidden, a.inter, a.w2.groups) && a.inter % 16 == 0 && a.hidden % 32 == 0 && aligned_to(a.x, 16) && aligned_to(a.w1.codes, 16) && aligned_to(a.w3.codes, 16) && aligned_to(a.w2.codes, 16) &&
+             fast::few_tokens_sync_bytes(a.tokens, a.hidden) <= sc.h - sc.gate;
   if (test.token && !few) return KEEPVQ_ERR_UNSUPPORTED;
-  bool router_fused = false;
-  fast::FewTokensArgs few_args = {};
-  few_args.token = test.token; few_args.wait_ns = test.wait_ns; few_args.absent = test.absent;
 
-  if (stages & KEEPVQ_STAGE_ROUTER) {
-    keepvq_router_logits_args rl = {};
-    rl.x = a.x; rl.x_dtype = a.x_dtype; rl.router_w = a.router_w; rl.router_dtype = a.router_dtype;
-    rl.tokens = a.tokens; rl.pool = a.pool; rl.hidden = a.hidden; rl.gate_temp = a.gate_temp;
-    rl.logits = reinterpret_cast<float*>(ws + sc.logits);
-    keepvq_routed_topk_args tk = {};
-    tk.logits = rl.logits; tk.tokens = a.tokens; tk.pool = a.pool; tk.top_k = a.top_k; tk.score_func = a.score_func;
-    tk.norm_topk_prob = a.norm_topk_prob; tk.route_scale = a.route_scale; tk.tau = a.tau;
-    tk.served_bias = a.served_bias; tk.pool_bias = a.pool_bias; tk.slot_of = a.slot_of;
-    tk.served_expert = a.served_expert; tk.served_slot = a.served_slot; tk.served_weight = a.served_weight;
-    tk.want = a.want; tk.want_score = a.want_score; tk.admit = a.admit;
-    router_fused = few && (stages & KEEPVQ_STAGE_GATE_UP) && fast::few_tokens_router_fits(rl, tk);
-    if (router_fused) {
-      few_args.logits = rl;
-      few_args.topk = tk;
-    } else {
-      // few tokens: the logits and the quantised token rows of the projections in one launch
-      const bool front = (stages & KEEPVQ_STAGE_PREPARE) && tensor_path && !prefill && !few && valid_dtype(a.router_dtype) && a.router_w && a.gate_temp > 0.0f &&
-                         aligned_to(a.x, 16) && aligned_to(a.router_w, 16) && fast::logits_and_quantize_supported(rl, a.w1.groups);
-      if (front) {
-        if ((rc = fast::logits_and_quantize(rl, a.w1.groups, xq, s))) return rc;
-        x_quantized = true;
-      } else if ((rc = keepvq_router_logits(&rl, stream))) return rc;
-      if ((rc = keepvq_routed_topk(&tk, stream))) return rc;
-    }
-  }
+  keepvq_router_logits_args rl = {};
+  rl.x = a.x; rl.x_dtype = a.x_dtype; rl.router_w = a.router_w; rl.router_dtype = a.router_dtype;
+  rl.tokens = a.tokens; rl.pool = a.pool; rl.hidden = a.hidden; rl.gate_temp = a.gate_temp;
+  rl.logits = reinterpret_cast<float*>(ws + sc.logits);
+  keepvq_routed_topk_args tk = {};
+  tk.logits = rl.logits; tk.tokens = a.tokens; tk.pool = a.pool; tk.top_k = a.top_k; tk.score_func = a.score_func;
+  tk.norm_topk_prob = a.norm_topk_prob; tk.route_scale = a.route_scale; tk.tau = a.tau;
+  tk.served_bias = a.served_bias; tk.pool_bias = a.pool_bias; tk.slot_of = a.slot_of;
+  tk.served_expert = a.served_expert; tk.served_slot = a.served_slot; tk.served_weight = a.served_weight;
+  tk.want = a.want; tk.want_score = a.want_score; tk.admit = a.admit;
+  bool router_due = stages & KEEPVQ_STAGE_ROUTER;
+  auto run_router = [&]() -> int {
+    router_due = false;
+    // few tokens: the logits and the quantised token rows of the projections in one launch
+    const bool front = (stages & KEEPVQ_STAGE_PREPARE) && tensor_path && !prefill && !few && valid_dtype(a.router_dtype) && a.router_w && a.gate_temp > 0.0f &&
+                       aligned_to(a.x, 16) && aligned_to(a.router_w, 16) && fast::logits_and_quantize_supported(rl, a.w1.groups);
+    const int status = front ? fast::logits_and_quantize(rl, a.w1.groups, xq, s) : keepvq_router_logits(&rl, stream);
+    if (status) return status;
+    x_quantized = front;
+    return keepvq_routed_topk(&tk, stream);
+  };
 
   if (few) {
     const bool gate_up = stages & KEEPVQ_STAGE_GATE_UP, down = stages & KEEPVQ_STAGE_DOWN;
     // the status is cleared where the other kernels' PREPARE stage clears it: a later stage leaves what an earlier one reported
-    few_args.clear_status = gate_up && (stages & KEEPVQ_STAGE_PREPARE);
     if (!gate_up && (stages & KEEPVQ_STAGE_PREPARE)) {
       const cudaError_t e = cudaMemsetAsync(ws + sc.status, 0, 4, s);
       if (e != cudaSuccess) return note_cuda_error(e);
     }
+    const bool router_fused = router_due && gate_up && fast::few_tokens_router_fits(rl, tk);
+    if (router_due && !router_fused && (rc = run_router())) return rc;
     if (gate_up || down) {
       const bool combine = gate_up && down && (stages & KEEPVQ_STAGE_COMBINE);
-      few_args.parts = (router_fused ? fast::FT_ROUTER : 0u) | (gate_up ? fast::FT_GATE_UP : 0u) | (down ? fast::FT_DOWN : 0u) | (combine ? fast::FT_COMBINE : 0u);
-      few_args.routes = static_cast<int32_t>(routes); few_args.tokens = static_cast<int32_t>(a.tokens); few_args.top_k = a.top_k;
-      few_args.scales_dtype = a.scales_dtype; few_args.slots = a.slots; few_args.codebook = a.codebook;
-      few_args.phase[0] = {{a.w1.codes, a.w3.codes}, {a.w1.scales, a.w3.scales}, a.x, ws + sc.h, static_cast<int32_t>(a.inter), static_cast<int32_t>(a.hidden), static_cast<int32_t>(a.w1.groups), a.top_k, a.x_dtype};
-      few_args.phase[1] = {{a.w2.codes, nullptr}, {a.w2.scales, nullptr}, ws + sc.h, ws + sc.down, static_cast<int32_t>(a.hidden), static_cast<int32_t>(a.inter), static_cast<int32_t>(a.w2.groups), 1, a.x_dtype};
-      few_args.slot = a.served_slot; few_args.weight = a.served_weight; few_args.swiglu_limit = a.swiglu_limit;
-      few_args.out = a.out; few_args.shared = a.shared; few_args.status = reinterpret_cast<int32_t*>(ws + sc.status);
-      if ((rc = fast::few_tokens(few_args, a.x_dtype, ws + sc.gate, s))) return rc;  // (only the general kernel uses the gate and up rows)
-      if (combine) return KEEPVQ_OK;
+      fast::FewTokensArgs f = {};
+      f.token = test.token; f.wait_ns = test.wait_ns; f.absent = test.absent; f.ctas = test.ctas;
+      f.parts = (router_fused ? fast::FT_ROUTER : 0u) | (gate_up ? fast::FT_GATE_UP : 0u) | (down ? fast::FT_DOWN : 0u) | (combine ? fast::FT_COMBINE : 0u);
+      if (router_fused) { f.logits = rl; f.topk = tk; }
+      f.routes = static_cast<int32_t>(routes); f.tokens = static_cast<int32_t>(a.tokens); f.top_k = a.top_k;
+      f.scales_dtype = a.scales_dtype; f.slots = a.slots; f.codebook = a.codebook;
+      f.phase[0] = {{a.w1.codes, a.w3.codes}, {a.w1.scales, a.w3.scales}, a.x, ws + sc.h, static_cast<int32_t>(a.inter), static_cast<int32_t>(a.hidden), static_cast<int32_t>(a.w1.groups), a.top_k, a.x_dtype};
+      f.phase[1] = {{a.w2.codes, nullptr}, {a.w2.scales, nullptr}, ws + sc.h, ws + sc.down, static_cast<int32_t>(a.hidden), static_cast<int32_t>(a.inter), static_cast<int32_t>(a.w2.groups), 1, a.x_dtype};
+      f.slot = a.served_slot; f.weight = a.served_weight; f.swiglu_limit = a.swiglu_limit;
+      f.out = a.out; f.shared = a.shared; f.status = reinterpret_cast<int32_t*>(ws + sc.status);
+      f.clear_status = gate_up && (stages & KEEPVQ_STAGE_PREPARE);
+      rc = fast::few_tokens(f, a.x_dtype, ws + sc.gate, s);  // (only the general kernel uses the gate and up rows)
+      if (rc == KEEPVQ_OK) {
+        router_due = false;
+        if (combine) return KEEPVQ_OK;
+      } else if (rc == KEEPVQ_ERR_UNSUPPORTED) {  // its grid cannot be resident here: the chain of kernels, with the groups and rows that the few-token kernel works out for itself
+        few = false;
+        stages |= KEEPVQ_STAGE_PREPARE;
+      } else return rc;
     }
-  } else if (tensor_path) {
+  }
+  if (router_due && (rc = run_router())) return rc;
+
+  if (tensor_path && !few) {
     fast::RouteGroups groups = {reinterpret_cast<int32_t*>(ws + sc.gcount), reinterpret_cast<int32_t*>(ws + sc.gslot),
                                 reinterpret_cast<int32_t*>(ws + sc.gstart), reinterpret_cast<int32_t*>(ws + sc.gsize),
                                 reinterpret_cast<int32_t*>(ws + sc.groutes)};
@@ -330,7 +336,7 @@ static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, cons
       p.out_dim = a.hidden; p.in_dim = a.inter; p.groups = a.w2.groups; p.x = hq; p.x_zero_row = routes; p.x_div = 1; p.out = ws + sc.down;
       if ((rc = prefill ? fast::prefill_down(p, wait_status, s) : fast::down(p, s))) return rc;
     }
-  } else {
+  } else if (!tensor_path) {
     if (stages & KEEPVQ_STAGE_GATE_UP) {
       if ((rc = projection(a, a.w1, a.x, a.tokens, a.hidden, a.inter, a.top_k, ws + sc.gate, stream))) return rc;
       if ((rc = projection(a, a.w3, a.x, a.tokens, a.hidden, a.inter, a.top_k, ws + sc.up, stream))) return rc;
@@ -357,9 +363,9 @@ static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, cons
 
 extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32_t stages, void* stream) { return keepvq::decode_stages(args, stages, {}, stream); }
 
-extern "C" int keepvq_grid_wait_selftest(const keepvq_moe_layer_args* args, int32_t stages, int32_t absent, int64_t wait_ns, uint64_t token, void* stream) {
-  if (absent < 0 || absent > 2 || wait_ns <= 0 || wait_ns > 1000000000ll || !token) return KEEPVQ_ERR_SHAPE;  // a self-test may hold the GPU for about a second at most
-  return keepvq::decode_stages(args, stages, {token, static_cast<uint64_t>(wait_ns), absent}, stream);
+extern "C" int keepvq_grid_wait_selftest(const keepvq_moe_layer_args* args, int32_t stages, int32_t absent, int32_t ctas, int64_t wait_ns, uint64_t token, void* stream) {
+  if (absent < 0 || absent > 2 || ctas < 0 || ctas > keepvq::fast::FT_MAX_CTAS || wait_ns <= 0 || wait_ns > 1000000000ll || !token) return KEEPVQ_ERR_SHAPE;  // a self-test may hold the GPU for about a second at most
+  return keepvq::decode_stages(args, stages, {token, static_cast<uint64_t>(wait_ns), absent, ctas}, stream);
 }
 
 extern "C" int keepvq_moe_decode_layer(const keepvq_moe_layer_args* args, void* stream) {

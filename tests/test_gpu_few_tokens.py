@@ -102,7 +102,7 @@ def test_a_block_that_stays_away_from_a_grid_barrier(cuda, stages, absent):
         if not mask & _lib.STAGE_ROUTER:
             layer.decode(xs[i], stages=_lib.STAGE_ROUTER)
         args = layer._layer_args(xs[i], buf["out"], buf["routing"], workspace=buf["workspace"], nbytes=buf["nbytes"])
-        _lib.check(lib.keepvq_grid_wait_selftest(args, mask, absent, 3_000_000 if absent else 1_000_000_000, token, _lib.stream_handle(cuda)), "keepvq_grid_wait_selftest")
+        _lib.check(lib.keepvq_grid_wait_selftest(args, mask, absent, 0, 3_000_000 if absent else 1_000_000_000, token, _lib.stream_handle(cuda)), "keepvq_grid_wait_selftest")
         torch.cuda.synchronize()
         words = buf["workspace"][: buf["nbytes"] // 8 * 8].view(torch.int64)
         assert not (words == token).any()
@@ -127,7 +127,7 @@ def test_a_reported_wait_stays_reported_through_later_stages(cuda):
     buf = layer._buffers_for(3, x.dtype)
     args = layer._layer_args(x, buf["out"], buf["routing"], workspace=buf["workspace"], nbytes=buf["nbytes"])
     front = _lib.STAGE_ROUTER | _lib.STAGE_PREPARE | _lib.STAGE_GATE_UP
-    _lib.check(_lib.load().keepvq_grid_wait_selftest(args, front, 1, 3_000_000, 77, _lib.stream_handle(cuda)), "keepvq_grid_wait_selftest")
+    _lib.check(_lib.load().keepvq_grid_wait_selftest(args, front, 1, 0, 3_000_000, 77, _lib.stream_handle(cuda)), "keepvq_grid_wait_selftest")
     assert layer.wait_expired(3, x.dtype)
     layer.decode(x, stages=_lib.STAGE_DOWN)
     layer.decode(x, stages=_lib.STAGE_COMBINE)
@@ -138,6 +138,35 @@ def test_a_reported_wait_stays_reported_through_later_stages(cuda):
         buf["workspace"].fill_(0x7F)
         layer.decode(x, stages=clearing)
         assert not layer.wait_expired(3, x.dtype)
+
+
+@pytest.mark.parametrize("top_k,experts", [(4, 12), (3, 400)])  # with the router in the launch, and in front of it
+def test_a_grid_that_cannot_be_resident_leaves_the_call_to_the_other_kernels(cuda, top_k, experts):
+    """One block more than there are SMs is refused by the cooperative launch, as the device's own number
+    is in a context that has fewer of them.  The layer call is then served by the chain of kernels,
+    whole and in parts, and the refusal is not left behind as an error of a later call."""
+    from keep_b200 import _lib
+
+    cfg = synthetic.layer(seed=87, experts=experts, hidden=512, inter=256, group_hidden=256)
+    layer = build_layer(cuda, cfg, top_k=top_k)
+    x = synthetic.tokens(88, 6, 512).to(cuda)
+    layer.decode(x)
+    buf = layer._buffers_for(6, x.dtype)
+    args = layer._layer_args(x, buf["out"], buf["routing"], workspace=buf["workspace"], nbytes=buf["nbytes"])
+    too_many = torch.cuda.get_device_properties(cuda).multi_processor_count + 1
+
+    def call(stages):
+        _lib.check(_lib.load().keepvq_grid_wait_selftest(args, stages, 0, too_many, 1_000_000, 1, _lib.stream_handle(cuda)), "keepvq_grid_wait_selftest")
+
+    front = _lib.STAGE_ROUTER | _lib.STAGE_PREPARE
+    for steps in ((_lib.STAGE_ALL,), (front | _lib.STAGE_GATE_UP, _lib.STAGE_DOWN | _lib.STAGE_COMBINE), (front, _lib.STAGE_GATE_UP | _lib.STAGE_DOWN, _lib.STAGE_COMBINE)):
+        buf["workspace"].fill_(0x7F)
+        buf["out"].zero_()
+        for stages in steps:
+            call(stages)
+        torch.cuda.synchronize()
+        assert not layer.wait_expired(6, x.dtype)
+        check_layer(cfg, x.cpu(), buf["out"], buf["routing"], top_k=top_k)
 
 
 def test_calls_on_two_streams_at_once(cuda):
