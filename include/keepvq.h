@@ -279,6 +279,9 @@ typedef struct keepvq_moe_layer_args {
 /* Bytes of scratch keepvq_moe_decode_layer needs for these sizes (host arithmetic only). */
 int64_t keepvq_moe_layer_workspace_bytes(int64_t tokens, int64_t hidden, int64_t inter, int64_t pool, int32_t top_k);
 int keepvq_moe_decode_layer(const keepvq_moe_layer_args* args, void* stream);
+/* Kernel launches that keepvq_moe_decode_layer enqueues for these arguments on the current device, or a
+ * negative keepvq_status (nothing is launched). */
+int keepvq_moe_layer_launches(const keepvq_moe_layer_args* args);
 /* Byte offset, inside the scratch, of an int32 status word: 1 when a bounded wait of the tcgen05 kernels
  * or of the few-token kernel's grid barriers expired (the blocks then stop, release what they hold and
  * return), 2 when a kernel found its shared memory laid out differently than it was built for (it then

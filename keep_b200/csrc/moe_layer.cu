@@ -193,7 +193,7 @@ struct GridWaitTest {
   int32_t absent, ctas;
 };
 
-static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, const GridWaitTest& test, void* stream) {
+static int check_layer_args(const keepvq_moe_layer_args* args) {
   if (!args) return KEEPVQ_ERR_NULL;
   const keepvq_moe_layer_args& a = *args;
   if (!valid_dtype(a.x_dtype) || !valid_dtype(a.router_dtype) || !valid_dtype(a.scales_dtype)) return KEEPVQ_ERR_DTYPE;
@@ -204,26 +204,68 @@ static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, cons
   if (!a.w1.codes || !a.w3.codes || !a.w2.codes || !a.w1.scales || !a.w3.scales || !a.w2.scales) return KEEPVQ_ERR_NULL;
   if (!a.served_expert || !a.served_slot || !a.served_weight || !a.want || !a.want_score) return KEEPVQ_ERR_NULL;
   if (a.w1.groups <= 0 || a.w3.groups != a.w1.groups || a.w2.groups <= 0) return KEEPVQ_ERR_SHAPE;
-  const LayerScratch sc = plan_scratch(a.tokens, a.hidden, a.inter, a.pool, a.top_k);
   if (!aligned_to(a.workspace, 256) || (a.shared && !aligned_to(a.shared, 16))) return KEEPVQ_ERR_ALIGN;
-  if (a.workspace_bytes < sc.total) return KEEPVQ_ERR_CAPACITY;
-  char* ws = reinterpret_cast<char*>(a.workspace);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int64_t routes = a.tokens * a.top_k;
-  const bool residual = a.res_rows > 0 && (a.w1.res_codes || a.w3.res_codes || a.w2.res_codes);
+  if (a.workspace_bytes < plan_scratch(a.tokens, a.hidden, a.inter, a.pool, a.top_k).total) return KEEPVQ_ERR_CAPACITY;
+  return KEEPVQ_OK;
+}
+
+// Which kernels a call gets.
+struct LayerPlan {
+  LayerScratch sc;
+  int64_t routes, live;
+  bool residual, tensor_path, prefill, few;
+  bool router_fused;                   // few: the router can be part of the launch
+  bool front;                          // else: the logits and the quantised token rows can be one launch
+  keepvq_router_logits_args logits;
+  keepvq_routed_topk_args topk;
+};
+
+static LayerPlan plan_layer(const keepvq_moe_layer_args& a) {
+  LayerPlan p = {};
+  p.sc = plan_scratch(a.tokens, a.hidden, a.inter, a.pool, a.top_k);
+  p.routes = a.tokens * a.top_k;
+  p.residual = a.res_rows > 0 && (a.w1.res_codes || a.w3.res_codes || a.w2.res_codes);
   // a residual tier stays on the tensor-core kernels when all three projections carry it and the
   // call has enough routes for the kernel that holds the residual pass
-  const bool residual_fits = !residual || (a.w1.res_codes && a.w3.res_codes && a.w2.res_codes && a.res_table && a.hot_of_slot &&
-                                           a.w3.res_groups == a.w1.res_groups && fast::residual_supported(routes, a.hidden, a.w1.res_groups) &&
-                                           fast::residual_supported(routes, a.inter, a.w2.res_groups));
+  const bool residual_fits = !p.residual || (a.w1.res_codes && a.w3.res_codes && a.w2.res_codes && a.res_table && a.hot_of_slot &&
+                                             a.w3.res_groups == a.w1.res_groups && fast::residual_supported(p.routes, a.hidden, a.w1.res_groups) &&
+                                             fast::residual_supported(p.routes, a.inter, a.w2.res_groups));
   // (fp32 activations take the general kernel, which keeps 24 bits of a row instead of 16)
-  const bool tensor_path = a.x_dtype != KEEPVQ_F32 && a.codebook_all_odd && residual_fits && fast::shapes_supported(a.inter, a.hidden, a.w1.groups) &&
-                           fast::shapes_supported(a.hidden, a.inter, a.w2.groups);
-  int rc = KEEPVQ_OK;
+  p.tensor_path = a.x_dtype != KEEPVQ_F32 && a.codebook_all_odd && residual_fits && fast::shapes_supported(a.inter, a.hidden, a.w1.groups) &&
+                  fast::shapes_supported(a.hidden, a.inter, a.w2.groups);
   // many routes per expert: the tcgen05 kernels
-  const int64_t live = a.expected_routes > 0 && a.expected_routes < routes ? a.expected_routes : routes;
-  const bool prefill = tensor_path && !residual && fast::prefill_pays(live, a.slots, a.w1.groups > 1 || a.w2.groups > 1) &&
-                       fast::prefill_supported(a.slots, a.inter, a.hidden, a.w1.groups) && fast::prefill_supported(a.slots, a.hidden, a.inter, a.w2.groups);
+  p.live = a.expected_routes > 0 && a.expected_routes < p.routes ? a.expected_routes : p.routes;
+  p.prefill = p.tensor_path && !p.residual && fast::prefill_pays(p.live, a.slots, a.w1.groups > 1 || a.w2.groups > 1) &&
+              fast::prefill_supported(a.slots, a.inter, a.hidden, a.w1.groups) && fast::prefill_supported(a.slots, a.hidden, a.inter, a.w2.groups);
+  // few routes: whatever part of the layer the call asks for as one launch of the few-token kernel
+  p.few = p.tensor_path && !p.residual && !p.prefill && fast::few_tokens_pay(p.routes, a.slots) && fast::few_tokens_fits(p.routes, a.tokens, a.slots, a.inter, a.hidden, a.w1.groups) &&
+          fast::few_tokens_fits(p.routes, a.tokens, a.slots, a.hidden, a.inter, a.w2.groups) && a.inter % 16 == 0 && a.hidden % 32 == 0 && aligned_to(a.x, 16) && aligned_to(a.w1.codes, 16) && aligned_to(a.w3.codes, 16) && aligned_to(a.w2.codes, 16) &&
+          fast::few_tokens_sync_bytes(a.tokens, a.hidden) <= p.sc.h - p.sc.gate;
+  p.logits.x = a.x; p.logits.x_dtype = a.x_dtype; p.logits.router_w = a.router_w; p.logits.router_dtype = a.router_dtype;
+  p.logits.tokens = a.tokens; p.logits.pool = a.pool; p.logits.hidden = a.hidden; p.logits.gate_temp = a.gate_temp;
+  p.logits.logits = reinterpret_cast<float*>(static_cast<char*>(a.workspace) + p.sc.logits);
+  keepvq_routed_topk_args& tk = p.topk;
+  tk.logits = p.logits.logits; tk.tokens = a.tokens; tk.pool = a.pool; tk.top_k = a.top_k; tk.score_func = a.score_func;
+  tk.norm_topk_prob = a.norm_topk_prob; tk.route_scale = a.route_scale; tk.tau = a.tau;
+  tk.served_bias = a.served_bias; tk.pool_bias = a.pool_bias; tk.slot_of = a.slot_of;
+  tk.served_expert = a.served_expert; tk.served_slot = a.served_slot; tk.served_weight = a.served_weight;
+  tk.want = a.want; tk.want_score = a.want_score; tk.admit = a.admit;
+  p.router_fused = p.few && fast::few_tokens_router_fits(p.logits, p.topk);
+  p.front = p.tensor_path && !p.prefill && a.gate_temp > 0.0f && aligned_to(a.x, 16) && aligned_to(a.router_w, 16) && fast::logits_and_quantize_supported(p.logits, a.w1.groups);
+  return p;
+}
+
+static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, const GridWaitTest& test, void* stream) {
+  int rc = check_layer_args(args);
+  if (rc || args->tokens == 0) return rc;
+  const keepvq_moe_layer_args& a = *args;
+  LayerPlan plan = plan_layer(a);
+  const LayerScratch& sc = plan.sc;
+  const int64_t routes = plan.routes, live = plan.live;
+  const bool residual = plan.residual, tensor_path = plan.tensor_path, prefill = plan.prefill;
+  bool few = plan.few;
+  char* ws = reinterpret_cast<char*>(a.workspace);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
   // (the sums regions have room for a scale group per codeword; the tensor-core kernels' rows have at
   // most one per 256 inputs, and their sums per 256 inputs go behind those)
   fast::QuantRows xq = {reinterpret_cast<uint8_t*>(ws + sc.xq), reinterpret_cast<float*>(ws + sc.xscale), reinterpret_cast<int32_t*>(ws + sc.xsums),
@@ -234,32 +276,16 @@ static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, cons
   // slots would only put a dependent load in front of every row
   const uint32_t* padded = live < routes ? a.served_slot : nullptr;
 
-  // few routes: whatever part of the layer the call asks for as one launch of the few-token kernel
-  bool few = tensor_path && !residual && !prefill && fast::few_tokens_pay(routes, a.slots) && fast::few_tokens_fits(routes, a.tokens, a.slots, a.inter, a.hidden, a.w1.groups) &&
-             fast::few_tokens_fits(routes, a.tokens, a.slots, a.hidden, a.inter, a.w2.groups) && a.inter % 16 == 0 && a.hidden % 32 == 0 && aligned_to(a.x, 16) && aligned_to(a.w1.codes, 16) && aligned_to(a.w3.codes, 16) && aligned_to(a.w2.codes, 16) &&
-             fast::few_tokens_sync_bytes(a.tokens, a.hidden) <= sc.h - sc.gate;
   if (test.token && !few) return KEEPVQ_ERR_UNSUPPORTED;
-
-  keepvq_router_logits_args rl = {};
-  rl.x = a.x; rl.x_dtype = a.x_dtype; rl.router_w = a.router_w; rl.router_dtype = a.router_dtype;
-  rl.tokens = a.tokens; rl.pool = a.pool; rl.hidden = a.hidden; rl.gate_temp = a.gate_temp;
-  rl.logits = reinterpret_cast<float*>(ws + sc.logits);
-  keepvq_routed_topk_args tk = {};
-  tk.logits = rl.logits; tk.tokens = a.tokens; tk.pool = a.pool; tk.top_k = a.top_k; tk.score_func = a.score_func;
-  tk.norm_topk_prob = a.norm_topk_prob; tk.route_scale = a.route_scale; tk.tau = a.tau;
-  tk.served_bias = a.served_bias; tk.pool_bias = a.pool_bias; tk.slot_of = a.slot_of;
-  tk.served_expert = a.served_expert; tk.served_slot = a.served_slot; tk.served_weight = a.served_weight;
-  tk.want = a.want; tk.want_score = a.want_score; tk.admit = a.admit;
   bool router_due = stages & KEEPVQ_STAGE_ROUTER;
   auto run_router = [&]() -> int {
     router_due = false;
     // few tokens: the logits and the quantised token rows of the projections in one launch
-    const bool front = (stages & KEEPVQ_STAGE_PREPARE) && tensor_path && !prefill && !few && valid_dtype(a.router_dtype) && a.router_w && a.gate_temp > 0.0f &&
-                       aligned_to(a.x, 16) && aligned_to(a.router_w, 16) && fast::logits_and_quantize_supported(rl, a.w1.groups);
-    const int status = front ? fast::logits_and_quantize(rl, a.w1.groups, xq, s) : keepvq_router_logits(&rl, stream);
+    const bool front = plan.front && !few && (stages & KEEPVQ_STAGE_PREPARE);
+    const int status = front ? fast::logits_and_quantize(plan.logits, a.w1.groups, xq, s) : keepvq_router_logits(&plan.logits, stream);
     if (status) return status;
     x_quantized = front;
-    return keepvq_routed_topk(&tk, stream);
+    return keepvq_routed_topk(&plan.topk, stream);
   };
 
   if (few) {
@@ -269,14 +295,14 @@ static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, cons
       const cudaError_t e = cudaMemsetAsync(ws + sc.status, 0, 4, s);
       if (e != cudaSuccess) return note_cuda_error(e);
     }
-    const bool router_fused = router_due && gate_up && fast::few_tokens_router_fits(rl, tk);
+    const bool router_fused = plan.router_fused && router_due && gate_up;
     if (router_due && !router_fused && (rc = run_router())) return rc;
     if (gate_up || down) {
       const bool combine = gate_up && down && (stages & KEEPVQ_STAGE_COMBINE);
       fast::FewTokensArgs f = {};
       f.token = test.token; f.wait_ns = test.wait_ns; f.absent = test.absent; f.ctas = test.ctas;
       f.parts = (router_fused ? fast::FT_ROUTER : 0u) | (gate_up ? fast::FT_GATE_UP : 0u) | (down ? fast::FT_DOWN : 0u) | (combine ? fast::FT_COMBINE : 0u);
-      if (router_fused) { f.logits = rl; f.topk = tk; }
+      if (router_fused) { f.logits = plan.logits; f.topk = plan.topk; }
       f.routes = static_cast<int32_t>(routes); f.tokens = static_cast<int32_t>(a.tokens); f.top_k = a.top_k;
       f.scales_dtype = a.scales_dtype; f.slots = a.slots; f.codebook = a.codebook;
       f.phase[0] = {{a.w1.codes, a.w3.codes}, {a.w1.scales, a.w3.scales}, a.x, ws + sc.h, static_cast<int32_t>(a.inter), static_cast<int32_t>(a.hidden), static_cast<int32_t>(a.w1.groups), a.top_k, a.x_dtype};
@@ -360,6 +386,18 @@ static int decode_stages(const keepvq_moe_layer_args* args, int32_t stages, cons
 }
 
 }  // namespace keepvq
+
+extern "C" int keepvq_moe_layer_launches(const keepvq_moe_layer_args* args) {
+  using namespace keepvq;
+  const int rc = check_layer_args(args);
+  if (rc) return rc;
+  if (args->tokens == 0) return 0;
+  const LayerPlan p = plan_layer(*args);
+  if (p.few) return p.router_fused ? 1 : 3;                             // (logits, top-k,) the rest
+  if (!p.tensor_path) return 7;                                         // logits, top-k, gate, up, SwiGLU, down, pick sum
+  const bool paired = p.front || fast::group_with_quantize_supported(p.routes, args->slots);
+  return !p.prefill && paired ? 7 : 8;                                  // logits, top-k, grouping, quantised x, gate/up, quantised h, down, pick sum; two of the first four as one
+}
 
 extern "C" int keepvq_moe_decode_stages(const keepvq_moe_layer_args* args, int32_t stages, void* stream) { return keepvq::decode_stages(args, stages, {}, stream); }
 

@@ -207,34 +207,20 @@ class RoutedMoELayer:
                 and ok(self.hidden, int(self.w1.res_scales.shape[2])) and ok(self.inter, int(self.w2.res_scales.shape[2]))
         return "tensor" if self.codebook_all_odd and fits else "general"
 
-    def _on_tcgen05(self, routes: int) -> bool:
-        """Whether a call of ``routes`` routes runs the tcgen05 kernels (``prefill_pays`` and
-        ``prefill_supported`` of csrc/moe_fast.cuh and csrc/prefill_umma.cu)."""
-        shapes = ((self.inter, self.hidden, int(self.w1.scales.shape[2])), (self.hidden, self.inter, int(self.w2.scales.shape[2])))
-        several = any(groups > 1 for _, _, groups in shapes)
-        fits = all(self.slots * out < 2 ** 31 - 512 and (groups == 1 or (groups <= 32 and inp // groups <= 4096)) for out, inp, groups in shapes)
-        return not self.res_rows and fits and routes >= 1024 and routes >= (8 if several else 5) * self.slots
-
-    def _one_launch(self, tokens: int) -> bool:
-        """Whether a call of ``tokens`` rows runs the few-token kernel (``few`` in csrc/moe_layer.cu)."""
-        routes, whole = tokens * self.top_k, lambda n: (n + 255) // 256 * 256
-        return not self.res_rows and 0 < routes and (routes < 48 or routes <= min(84, self.slots // 2)) and tokens <= 23 and self.hidden <= 5120 and self.inter <= 5120 and not self._on_tcgen05(routes) \
-            and 2 * 8 * (160 + 16) + 4 + tokens * (self.hidden // 32) * 4 <= 2 * whole(routes * self.inter * 4)
-
     def launches_per_call(self, tokens: int, dtype: torch.dtype = torch.bfloat16) -> int:
         """Kernel launches one ``decode`` call of ``tokens`` rows enqueues.  A call of few routes on the
-        tensor-core kernels is one launch (three with a router that kernel does not take: logits, top-k,
+        tensor-core kernels is one launch (three where the router is not part of it: logits, top-k,
         the rest).  Else: logits, top-k, route grouping, quantise x, gate/up, quantise h, down, combine,
         of which two share a launch on the decode kernels: up to 23 tokens the logits and the
         quantisation of x, beyond that (up to 4096 routes) the quantisation of x and the route
         grouping.  The tcgen05 kernels' rows are quantised in grouped order, behind the grouping."""
-        if self.kernel_path != "tensor" or dtype not in (torch.float16, torch.bfloat16):
-            return 7
-        if self._one_launch(tokens):
-            return 1 if self.pool <= 384 and self.router_w.dtype == torch.bfloat16 else 3
-        routes = tokens * self.top_k
-        front, paired = tokens <= 23, routes <= 4096 and self.slots * 12 <= 40 * 1024
-        return 7 if (front or paired) and not self._on_tcgen05(routes) else 8
+        buf = self._buffers_for(tokens, dtype)
+        args = self._layer_args(buf["out"], buf["out"], buf["routing"], workspace=buf["workspace"], nbytes=buf["nbytes"])
+        with _lib.on_device(self.device):
+            launches = _lib.load().keepvq_moe_layer_launches(args)
+        if launches < 0:
+            _lib.check(launches, "keepvq_moe_layer_launches")
+        return launches
 
     def decode_without_scratch(self, x: torch.Tensor, out: torch.Tensor, routing: Routing) -> tuple[torch.Tensor, Routing]:
         """The same layer through ``keepvq_moe_decode_layer_static``: the caller supplies the
