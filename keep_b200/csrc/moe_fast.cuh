@@ -414,6 +414,14 @@ struct FewTokensArgs {
 // several routes each the chain's groups of them win earlier: of 16 experts 8 tokens 67 against 77, 10 tokens 78
 // against 77, 12 tokens 84 against 77.
 inline bool few_tokens_pay(int64_t routes, int64_t slots) { return routes < SMALL_CALL_ROUTES || (routes <= FEW_TOKENS_ROUTES && routes <= slots / 2); }
+// ... and which of them have the router in the same launch.  There every CTA works out every token's picks, four tokens
+// at a time, which ends the gain of two launches less: us a layer with the router in the launch / in front of it / the
+// chain of kernels (B200; the latter two never differ by more than 1 % to the chain's side):
+//   8 experts, top-2, 4096 x 2048    12 tokens 50.4 / 52.0 / 52.7, 14 tokens 55.3 / 55.4 / 57.1, 17 tokens 62.6 / 58.1 / 60.8, 23 tokens 72.7 / 64.8 / 66.7
+//   8 experts, top-2, 1024 x 512     12 tokens 27.4 / 24.5 / 28.4, 14 tokens 29.6 / 24.7 / 29.5, 23 tokens 36.3 / 25.5 / 30.1
+//   48 experts, top-2, 512 x 256     12 tokens 27.0 / 22.6 / 27.7, 14 tokens 29.0 / 22.8 / 28.2, 23 tokens 35.4 / 23.7 / 28.6
+//   8 experts, top-2, 5120 x 2304 with scale groups  14 tokens 70.9 / 72.7 / 82.6, 16 tokens 72.2 / 73.8 / 83.1, 17 tokens 79.2 / 76.5 / 87.9
+inline bool few_tokens_router_pays(int64_t tokens, int64_t hidden) { return tokens <= (hidden > 4096 ? 16 : 12); }
 bool few_tokens_fits(int64_t routes, int64_t tokens, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups);
 bool few_tokens_router_fits(const keepvq_router_logits_args& logits, const keepvq_routed_topk_args& topk);
 int64_t few_tokens_sync_bytes(int64_t tokens, int64_t out_dim);  // scratch of a call with gate/up and down, any contents

@@ -250,7 +250,7 @@ static LayerPlan plan_layer(const keepvq_moe_layer_args& a) {
   tk.served_bias = a.served_bias; tk.pool_bias = a.pool_bias; tk.slot_of = a.slot_of;
   tk.served_expert = a.served_expert; tk.served_slot = a.served_slot; tk.served_weight = a.served_weight;
   tk.want = a.want; tk.want_score = a.want_score; tk.admit = a.admit;
-  p.router_fused = p.few && fast::few_tokens_router_fits(p.logits, p.topk);
+  p.router_fused = p.few && fast::few_tokens_router_pays(a.tokens, a.hidden) && fast::few_tokens_router_fits(p.logits, p.topk);
   p.front = p.tensor_path && !p.prefill && a.gate_temp > 0.0f && aligned_to(a.x, 16) && aligned_to(a.router_w, 16) && fast::logits_and_quantize_supported(p.logits, a.w1.groups);
   return p;
 }

@@ -24,14 +24,18 @@ pytestmark = pytest.mark.gpu
     (3, 12, 6, 5120, 768, 512, 256, "sqrtsoftplus"),  # the widest rows, scale groups of two chunks and of one
     (8, 12, 5, 2560, 256, None, None, "softmax"),     # eight tokens staged by token, two rounds of picks
     (9, 12, 5, 512, 2304, 256, 768, "softmax"),       # rows staged by group
-    (23, 40, 2, 512, 256, None, None, "softmax"),     # the most tokens; six rounds of picks
+    (23, 40, 2, 512, 256, None, None, "softmax"),     # the most tokens
     (2, 400, 3, 512, 256, None, None, "softmax"),     # a pool whose router runs in front
+    (12, 40, 2, 4096, 256, None, None, "sigmoid"),    # the most tokens with the router in the launch
+    (13, 40, 2, 4096, 256, None, None, "sigmoid"),
+    (16, 20, 2, 4352, 256, None, None, "softmax"),    # ... of wider rows; four rounds of picks
+    (17, 20, 2, 4352, 256, None, None, "softmax"),
 ])
 def test_layer_calls_of_few_routes(cuda, tokens, experts, top_k, hidden, inter, group_hidden, group_inter, score):
     cfg = synthetic.layer(seed=71, experts=experts, hidden=hidden, inter=inter, group_hidden=group_hidden, group_inter=group_inter)
     x = synthetic.tokens(72 + tokens, tokens, hidden)
     layer = build_layer(cuda, cfg, top_k=top_k, score_func=score)
-    assert layer.launches_per_call(tokens) == (1 if experts <= 384 else 3)
+    assert layer.launches_per_call(tokens) == (1 if experts <= 384 and tokens <= (16 if hidden > 4096 else 12) else 3)
     layer.decode(x.to(cuda))
     for buf in layer._buffers.values():
         buf["workspace"].fill_(0x7F)  # whatever the scratch holds, the barrier words of an earlier call among it
@@ -42,7 +46,7 @@ def test_layer_calls_of_few_routes(cuda, tokens, experts, top_k, hidden, inter, 
 
 @pytest.mark.parametrize("tokens,experts,top_k,launches", [
     (8, 96, 6, 1),    # 48 routes, half as many as slots
-    (14, 168, 6, 1),  # the most routes
+    (14, 168, 6, 3),  # the most routes
     (8, 95, 6, 7),    # one expert fewer: the chain of kernels
     (17, 400, 5, 7),  # one route more
 ])
