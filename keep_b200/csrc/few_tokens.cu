@@ -144,10 +144,12 @@ __device__ __forceinline__ uint4 ft_load_row16(const void* p) {  // (not the rea
 // The served picks of up to four tokens from t0 on, by four warps a token: each scores its share of the
 // pool and picks from it, one of them picks from the shares' picks.  (A warp alone took 2650 cycles
 // for twelve scores a lane and 3200 for six picks, and all warps reading all logits of one token 3600, from twelve
-// lines of L2 that 148 CTAs want at once.)  The arithmetic and the order of additions of topk_scores.
+// lines of L2 that 148 CTAs want at once.)  The arithmetic and the order of additions of routed_topk_reg_kernel.
 // `scratch`: FT_PICK_BYTES of shared memory.  own: the token whose outputs this CTA writes and whose scores it keeps.
 constexpr int FT_PICK_PARTS = 4, FT_PICK_TOKENS = FT_WARPS / FT_PICK_PARTS;
 constexpr uint32_t FT_PICK_ROW = 32 * FT_TOPK_NPL * 4, FT_PICK_BYTES = FT_PICK_TOKENS * (2 * FT_PICK_ROW + 64 * 8);
+static __device__ __noinline__ float ft_sigmoid(float v) { return topk_sigmoid(v); }  // (calls: see the top on the size of the code)
+static __device__ __noinline__ float ft_sqrt_softplus(float v) { return topk_sqrt_softplus(v); }
 __device__ __forceinline__ void ft_pick(const keepvq_routed_topk_args& k, uint32_t scratch, int t0, int own, float* own_scores, uint32_t* route_slot, float* route_weight) {
   constexpr int NQ = FT_TOPK_NPL / FT_PICK_PARTS, PARTS = FT_PICK_PARTS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, local = warp / PARTS, part = warp % PARTS;
@@ -187,7 +189,7 @@ __device__ __forceinline__ void ft_pick(const keepvq_routed_topk_args& k, uint32
     for (int q = 0; q < NQ; ++q) sc[q] = sc[q] / s;
   } else {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) sc[q] = k.score_func == KEEPVQ_SCORE_SIGMOID ? topk_sigmoid(sc[q]) : topk_sqrt_softplus(sc[q]);
+    for (int q = 0; q < NQ; ++q) sc[q] = k.score_func == KEEPVQ_SCORE_SIGMOID ? ft_sigmoid(sc[q]) : ft_sqrt_softplus(sc[q]);
   }
   uint32_t key[NQ], my_key;
   int my_e;

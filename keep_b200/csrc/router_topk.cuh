@@ -1,5 +1,5 @@
-// Score function and top-k of one token by one warp with the pool in registers, shared by
-// keepvq_routed_topk (router.cu) and the few-token layer kernel (few_tokens.cu).
+// Pieces of the score function and top-k of one token that keepvq_routed_topk (router.cu) and the few-token
+// layer kernel (few_tokens.cu) share: the same arithmetic in the same order, so the same picks and weights.
 #pragma once
 
 #include <math.h>
@@ -14,13 +14,6 @@ __device__ __forceinline__ uint32_t ordered_key(float v) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// The logits of token t, NPL experts per lane (expert e = lane + 32 i).  (Read from L2: blocks of the same kernel may have written them.)
-template <int NPL>
-__device__ __forceinline__ void topk_logits(const keepvq_routed_topk_args& a, int64_t t, int lane, float (&lg)[NPL]) {
-  const int P = static_cast<int>(a.pool);
-#pragma unroll
-  for (int i = 0; i < NPL; ++i) { const int e = lane + 32 * i; lg[i] = e < P ? __ldcg(a.logits + t * P + e) : -INFINITY; }
-}
 // The softmax's maximum (exact in any order), and the one-value score functions.
 template <int NPL>
 __device__ __forceinline__ float topk_max(const float (&lg)[NPL]) {
@@ -42,34 +35,13 @@ __device__ __forceinline__ float topk_sum(const float (&ex)[NPL], int pool, int 
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
   return s;
 }
-static __device__ __noinline__ float topk_sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
-static __device__ __noinline__ float topk_sqrt_softplus(float v) { return sqrtf(v > 20.0f ? v : log1pf(expf(v))); }
-
-// The scores of token t by one warp.
-template <int NPL>
-__device__ __forceinline__ void topk_scores(const keepvq_routed_topk_args& a, int64_t t, int lane, float (&sc)[NPL]) {
-  const int P = static_cast<int>(a.pool);
-  topk_logits<NPL>(a, t, lane, sc);
-  if (a.score_func == KEEPVQ_SCORE_SOFTMAX) {
-    const float m = topk_max<NPL>(sc);
-#pragma unroll
-    for (int i = 0; i < NPL; ++i)
-      if (lane + 32 * i < P) sc[i] = expf(sc[i] - m);
-    const float s = topk_sum<NPL>(sc, P, lane);
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) sc[i] = sc[i] / s;
-  } else if (a.score_func == KEEPVQ_SCORE_SIGMOID) {
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) sc[i] = topk_sigmoid(sc[i]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < NPL; ++i) sc[i] = topk_sqrt_softplus(sc[i]);
-  }
-}
+__device__ __forceinline__ float topk_sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
+__device__ __forceinline__ float topk_sqrt_softplus(float v) { return sqrtf(v > 20.0f ? v : log1pf(expf(v))); }
 
 // The top_k largest of a warp's keys, NQ per lane with their expert ids, in descending order, ties to the
 // lowest id: lane j gets pick j (key 0 where there are none left).  A pick is a tree over the lane's
-// registers, one warp max and one warp min (redux.sync).
+// registers, one warp max and one warp min (redux.sync): for warps that have the SM to themselves and wait for
+// each step (routed_topk_reg_kernel scans, which is fewer instructions).
 template <int NQ>
 __device__ __forceinline__ void topk_select(uint32_t (&key)[NQ], const int (&id)[NQ], int top_k, int lane, uint32_t& my_key, int& my_e) {
   my_key = 0u;
@@ -138,21 +110,4 @@ __device__ __forceinline__ void topk_finish(const keepvq_routed_topk_args& a, in
     }
   }
 }
-// Lane j's score of its pick, from scores that are only in the warp's registers.
-template <int NPL>
-__device__ __forceinline__ float topk_raw_from_registers(const float (&sc)[NPL], int my_e, int lane, int top_k) {
-  float my_raw = 0.0f;
-#pragma unroll 1
-  for (int j = 0; j < top_k; ++j) {
-    const int win = __shfl_sync(0xFFFFFFFFu, my_e, j);
-    float raw = 0.0f;
-#pragma unroll
-    for (int i = 0; i < NPL; ++i)
-      if (lane + 32 * i == win) raw = sc[i];
-    raw = __shfl_sync(0xFFFFFFFFu, raw, win & 31);
-    if (lane == j) my_raw = raw;
-  }
-  return my_raw;
-}
-
 }  // namespace keepvq
