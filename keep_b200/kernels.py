@@ -68,13 +68,13 @@ def should_use_e8p_m1(*, code_bits: int, tokens: int, sorted_indices: bool, rout
 
 
 def routed_matvec(x, codes, scales, codebook, rhs, *, lhs=None, x_div=1, code_bits, layout=_lib.TABLE_PACKED,
-                  residual=None, hot_of_slot=None, out_dtype=None) -> torch.Tensor:
+                  residual=None, hot_of_slot=None, out_dtype=None, routes=None) -> torch.Tensor:
     """One launch of the general routed kernel.  ``x`` [rows, in]; ``codes`` [E, out, in/8];
-    ``rhs`` flat uint32/int32 [routes]; returns [routes, out]."""
+    ``rhs`` flat uint32/int32 [routes] (or more than the given ``routes``); returns [routes, out]."""
     device = _lib.require_cuda(x, codes, scales, codebook, rhs)
     experts, out_dim, cw = (int(s) for s in codes.shape)
     groups = int(scales.shape[2])
-    routes = int(rhs.numel())
+    routes = int(rhs.numel()) if routes is None else routes
     out_dtype = qmv_output_dtype(x.dtype) if out_dtype is None else out_dtype
     out = torch.empty((routes, out_dim), dtype=out_dtype, device=device)
     res = (0, 0, 0, 0, 0, 0, 0)
@@ -124,38 +124,35 @@ def _dense_reference(x2d, codes, scales, codebook, code_bits):
     return x2d.to(torch.float32) @ weights.T
 
 
-class _ToOneMatrix:
+class _ZeroRoutes:
     """The experts of a single matrix's routes: int32 zeros on the device, which the library holds (a launch
     that clears a tensor of them was a tenth of a small call)."""
 
     dtype, is_cuda = torch.int32, True
 
-    def __init__(self, address: int, device: torch.device, count: int):
-        self.address, self.device, self.count = address, device, count
+    def __init__(self, address: int, count: int, device: torch.device):
+        self.address, self.count, self.device = address, count, device
 
     def data_ptr(self) -> int:
         return self.address
-
-    def numel(self) -> int:
-        return self.count
 
     def is_contiguous(self) -> bool:
         return True
 
 
-_zero_routes: dict = {}  # device -> (address, how many): constants of the loaded library
+_zero_routes: dict = {}  # device index -> the zeros there: a constant of the loaded library
 
 
 def _routes_to_one(count: int, device: torch.device):
-    """``count`` int32 zeros: the library's, or a tensor where it has fewer (and where its first use falls
-    into a capture, which is no place to look the address up)."""
-    if device not in _zero_routes and not torch.cuda.is_current_stream_capturing():
+    """At least ``count`` int32 zeros: the library's, or a tensor where it has fewer (and where its first
+    use falls into a capture, which is no place to look the address up)."""
+    held = _zero_routes.get(device.index)
+    if held is None and not torch.cuda.is_current_stream_capturing():
         address, have = ctypes.c_void_p(), ctypes.c_int64()
         with _lib.on_device(device):
             _lib.check(_lib.load().keepvq_zero_routes(ctypes.byref(address), ctypes.byref(have)), "keepvq_zero_routes")
-        _zero_routes[device] = (address.value, have.value)
-    address, have = _zero_routes.get(device, (0, 0))
-    return _ToOneMatrix(address, device, count) if count <= have else torch.zeros(count, dtype=torch.int32, device=device)
+        held = _zero_routes[device.index] = _ZeroRoutes(address.value, have.value, device)
+    return torch.zeros(count, dtype=torch.int32, device=device) if held is None or count > held.count else held
 
 
 def _one_matrix(rows, codes, scales, table, code_bits, out_shape):
@@ -168,7 +165,7 @@ def _one_matrix(rows, codes, scales, table, code_bits, out_shape):
 
         out = project(rows, routes, cw * 8, codes, 1, out_dim, scales, scales.shape[1], table, rhs, out_shape)
     if out is None:
-        out = routed_matvec(rows.reshape(routes, cw * 8), codes[None], scales[None], table, rhs, x_div=1, code_bits=code_bits).reshape(out_shape)
+        out = routed_matvec(rows.reshape(routes, cw * 8), codes[None], scales[None], table, rhs, routes=routes, x_div=1, code_bits=code_bits).reshape(out_shape)
     return out
 
 

@@ -74,7 +74,7 @@ def tensor_core_projection(rows, codes, scales, table, rhs, *, x_div: int = 1, c
 
 def project(rows, routes, in_dim, codes, slots, out_dim, scales, groups, table, rhs, out_shape, *, x_div=1, code_bits=16, residual=None, hot_of_slot=None):
     """The same with the sizes given beside the tensors (one matrix's codes and scales, say, without an
-    experts' dimension), and the shape of the answer."""
+    experts' dimension; ``rhs`` may hold more than ``routes``), and the shape of the answer."""
     if codes.dtype != (torch.uint8 if code_bits == 8 else torch.uint16) or in_dim % 256 or rows.dtype not in (torch.float16, torch.bfloat16):
         return None
     if code_bits == 8 and not byte_codes_served(routes, slots, out_dim, in_dim, groups):
