@@ -353,7 +353,7 @@ def operator_legs(layer, device, hbm_gbs, steps=32):
     cpu_s = time.perf_counter() - begin
     out["vq_qmv_2048x4096"] = {"us_per_call": round(us, 2), "code_gbs": round(CODE_BYTES_PER_PROJECTION / (us * 1e-6) / 1e9, 1),
                                "code_frac_of_hbm": round(CODE_BYTES_PER_PROJECTION / (us * 1e-6) / 1e9 / hbm_gbs, 4),
-                               "cpu_us_per_call": round(cpu_s * 1e6, 1), "kernel": "keepvq_grouped_projection: quantize_rows_kernel (the route grouping is one of its blocks), projection_sweep_kernel (two launches per call)"}
+                               "cpu_us_per_call": round(cpu_s * 1e6, 1), "kernel": "keepvq_grouped_projection: few_tokens_kernel (one launch per call)"}
     for tokens in (1, 4, 16):
         xs, picks, uniq = [], [], []
         for j in range(8):

@@ -420,7 +420,9 @@ extern "C" int keepvq_moe_decode_layer(const keepvq_moe_layer_args* args, void* 
 // exits.  All calls on a device share it, so two calls that overlap on the GPU (different
 // streams, or a graph replay racing a direct call) corrupt each other; serialise them.  The
 // array keeps whatever the last call left there.  Nothing in it has to start at zero: every
-// region is written by an earlier stage of the same call before a later stage reads it.
+// region is written by an earlier stage of the same call before a later stage reads it, but for the
+// few-token kernel's barrier words, which are looked at as they are found and mean nothing without
+// the token of the launch.
 // ------------------------------------------------------------------------------------------
 namespace keepvq {
 

@@ -62,7 +62,7 @@ def check_rows(got, want_by_expert, rhs, which_input):
 @pytest.mark.parametrize("family", ["few", "slab8", "slab4", "tcgen05"])
 def test_single_projection_kernels_return_scale_times_weight_exactly(cuda, family):
     """The M = 1 (down-shaped) kernels through ``keepvq_grouped_projection``.  The route count and
-    the expert count pick the kernel: under 48 routes the sweep kernel ("few" below), from there the
+    the expert count pick the kernel: under 48 routes the few-token kernel ("few" below), from there the
     slab kernel with eight routes per group (many routes per expert) or four (few), and from 1024
     routes with 5 per expert the tcgen05 kernel."""
     copies = {"few": 1, "slab8": 1, "slab4": 32, "tcgen05": 1}[family]
@@ -91,17 +91,18 @@ def test_single_projection_kernels_return_scale_times_weight_exactly(cuda, famil
         check_rows(got, want, rhs, np.tile(np.arange(IN), 4))
 
 
-@pytest.mark.parametrize("family,in_dim,routes,rows", [("sweep", 2048, 6, ROWS), ("sweep", 4096, 40, ROWS), ("sweep", 2304, 7, ROWS), ("sweep", 8192, 6, ROWS),
-                                                       ("sweep", 1024, 9, 200), ("split", 2048, 60, ROWS), ("split-residual", 2048, 5, ROWS)])
+@pytest.mark.parametrize("family,in_dim,routes,rows", [("few", 2048, 6, ROWS), ("few", 4096, 40, ROWS), ("few", 2304, 7, ROWS), ("sweep", 8192, 6, ROWS),
+                                                       ("few", 1024, 9, 200), ("sweep", 5376, 9, 200), ("sweep", 5376, 40, ROWS), ("split", 2048, 60, ROWS), ("split-residual", 2048, 5, ROWS)])
 def test_few_route_kernels_over_wide_inputs_exactly(cuda, family, in_dim, routes, rows):
-    """Calls with few routes run the sweep kernel: the sixteen warps of a CTA split the input
-    dimension (evenly or not: 2304 inputs are nine chunks over eight warps), carry the partial sums
-    of several 16-row units and add them up in shared memory.  With a residual tier the split form
-    of the slab kernel does the same per item.  (The 256-input cases above give every warp the
-    whole row.)  A one-hot row at a random input picks one weight per output row, so whichever warp
-    owns that part of the row must deliver it, exactly.  200 output rows leave the last unit of an
-    expert short (its row indices are clamped); 60 routes over 32 experts are few route groups of
-    a call too large for the sweep kernel: the split slab kernel without a residual."""
+    """Calls with few routes run the few-token kernel, with rows over 5120 inputs the sweep kernel: the
+    sixteen warps of a CTA split the input dimension (evenly or not: 2304 inputs are nine chunks
+    over sixteen warps, 5376 are 21), carry the partial sums of several units of rows and add them up
+    in shared memory.  With a residual tier the split form of the slab kernel does the same per item.
+    (The 256-input cases above give every warp the whole row.)  A one-hot row at a random input picks
+    one weight per output row, so whichever warp owns that part of the row must deliver it, exactly.
+    200 output rows leave the last unit of an expert short (its row indices are clamped); 60 routes over
+    32 experts are few route groups of a call too large for these kernels: the split slab kernel without
+    a residual."""
     from keep_b200 import vq
 
     experts, cw = (32 if family == "split" else 4), in_dim // 8  # 60 routes over 32 experts: groups of four, and few of them
@@ -163,18 +164,19 @@ def test_residual_pass_returns_base_plus_residual_exactly(cuda, cols):
     check_rows(got, want, rhs, which)
 
 
-@pytest.mark.parametrize("family", ["few", "slab4", "slab8", "tcgen05"])
+@pytest.mark.parametrize("family", ["few", "sweep", "slab4", "slab8", "tcgen05"])
 def test_gate_up_kernels_decode_both_matrices_exactly(cuda, family):
     """The M = 2 kernels fuse gate, up and SwiGLU, so G and U are not visible on their own.  With
     a one-hot activation of +-2^14 and a gate weight that is positive, G is at least 41 and
     silu(G) = G exactly in fp32 (exp(-G) is below half an ulp of 1), so
     h = round(round(G) * round(U)) is a closed form of the two decodes.  One matrix holds every
     16-bit code, the other a code whose eight weights are all positive; then the roles swap, with
-    the activation's sign chosen per output so that G stays positive."""
+    the activation's sign chosen per output so that G stays positive.  Six tokens run the few-token
+    kernel, 30 tokens of one pick each the sweep kernel."""
     from keep_b200 import _lib, moe, vq
 
-    tokens = {"few": 6, "slab4": 256, "slab8": 256, "tcgen05": 1024}[family]
-    experts = {"few": 4, "slab4": 128, "slab8": 4, "tcgen05": 4}[family]
+    tokens = {"few": 6, "sweep": 30, "slab4": 256, "slab8": 256, "tcgen05": 1024}[family]
+    experts = {"few": 4, "sweep": 4, "slab4": 128, "slab8": 4, "tcgen05": 4}[family]
     every = all_codes_experts(experts // 4)
     # a codeword whose eight weights are all positive (the first one there is)
     grid = e8.decode_e8p(np.arange(1 << 16, dtype=np.uint16))
@@ -192,6 +194,7 @@ def test_gate_up_kernels_decode_both_matrices_exactly(cuda, family):
                                    moe.Projection(dev(up_codes), dev(scales)), down, top_k=1, codebook=table)
         assert layer.kernel_path == "tensor"
         xt = torch.from_numpy(x).to(cuda).to(torch.bfloat16)
+        assert (layer.launches_per_call(tokens) == 1) == (family == "few")
         r = layer._buffers_for(int(xt.shape[0]), xt.dtype)["routing"]
         r.served_slot.copy_(torch.from_numpy(slots.reshape(-1, 1)).to(cuda))
         r.served_weight.fill_(1.0)
@@ -204,8 +207,8 @@ def test_gate_up_kernels_decode_both_matrices_exactly(cuda, family):
         return (g16 * u16).to(torch.bfloat16).float().numpy()
 
     rng = np.random.default_rng(7)
-    for call in range(8 if family == "few" else 2):
-        which = rng.integers(0, IN, tokens) if family in ("few",) else np.arange(tokens) % IN
+    for call in range(8 if family in ("few", "sweep") else 2):
+        which = rng.integers(0, IN, tokens) if family in ("few", "sweep") else np.arange(tokens) % IN
         if family == "slab4":
             slots = (np.arange(tokens) % experts).astype(np.int32)
         elif family == "slab8" or family == "tcgen05":

@@ -10,8 +10,7 @@ import pytest
 import torch
 
 import synthetic
-from oracle import e8
-from test_gpu_moe_layer import build_layer, check_layer
+from test_gpu_moe_layer import TOLERANCE, build_layer, check_layer
 
 pytestmark = pytest.mark.gpu
 
@@ -238,19 +237,51 @@ def test_single_projections_with_ragged_rows(cuda, dtype, routes, out_dim, in_di
 
 @pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
 def test_rows_that_are_not_finite_touch_no_other(cuda, bad):
-    """A row with a NaN or an infinity beside ordinary ones: theirs do not change, and it goes through
-    the same steps as in calls of many routes (the slab kernels): equal outputs."""
+    """A row with a NaN or an infinity beside ordinary ones: theirs are the same bits as without it, and
+    every row goes through the same steps as in calls of many routes (the slab kernels): equal but for
+    fp32 sums in another order, which may round to the neighbouring bf16: 2^-7 of the value."""
     from keep_b200 import prefill, vq
 
     rng = np.random.default_rng(80)
     codes = torch.from_numpy(rng.integers(0, 65536, (4, 64, 64)).astype(np.uint16)).to(cuda)
     scales = torch.full((4, 64, 1), 0.02, dtype=torch.float16, device=cuda)
     x = torch.randn((60, 512), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(cuda)
-    x[2, 100] = bad
     rhs = (torch.arange(60, device=cuda) % 4).to(torch.int32)
     table = vq.table_on(cuda, "e8p")
-    many = prefill.tensor_core_projection(x, codes, scales, table, rhs)
+    before = prefill.tensor_core_projection(x[:8].contiguous(), codes, scales, table, rhs[:8].contiguous())
+    x[2, 100] = bad
+    many = prefill.tensor_core_projection(x, codes, scales, table, rhs)[:8].float()
     few = prefill.tensor_core_projection(x[:8].contiguous(), codes, scales, table, rhs[:8].contiguous())
-    gap = e8.relative_gap(few.float().cpu().numpy(), many[:8].float().cpu().numpy())
-    assert gap <= 2 ** -8  # fp32 sums in another order, one rounding to bf16
+    others = [0, 1, 3, 4, 5, 6, 7]
+    assert torch.equal(few[others], before[others]) and not torch.equal(few[2], before[2])
+    few = few.float()
     assert torch.isfinite(few).all()
+    assert ((few - many).abs() <= 2.0 ** -7 * many.abs() + 1e-6 * many.abs().amax(1, keepdim=True)).all()
+
+
+@pytest.mark.parametrize("dtype,tolerance", [(torch.bfloat16, TOLERANCE), (torch.float16, TOLERANCE / 8)])  # three roundings of 8 or of 11 bits
+def test_masked_picks_of_the_largest_pool(cuda, dtype, tolerance):
+    """384 experts of which a third is resident, the demanded picks by a bias of their own, admissions;
+    and the output written over the tokens."""
+    from oracle import router as oracle_router
+
+    pool, hidden, inter, k, tokens = 384, 512, 256, 6, 7
+    rng = np.random.default_rng(89)
+    cfg = synthetic.layer(seed=90, experts=pool, hidden=hidden, inter=inter)
+    resident = np.sort(rng.choice(pool, pool // 3, replace=False))
+    slot_of = np.full(pool, 0xFFFFFFFF, dtype=np.uint32)
+    slot_of[resident] = rng.permutation(pool // 3).astype(np.uint32)
+    served_bias = np.full(pool, oracle_router.OFF, dtype=np.float32)
+    served_bias[resident] = rng.normal(scale=1e-3, size=pool // 3)
+    pool_bias = rng.normal(scale=1e-3, size=pool).astype(np.float32)
+    expert_of_slot = np.empty(pool // 3, dtype=np.int64)
+    expert_of_slot[slot_of[resident].astype(np.int64)] = resident
+    slot_cfg = dict(cfg, **{n: (cfg[n][0][expert_of_slot], cfg[n][1][expert_of_slot]) for n in ("w1", "w3", "w2")})
+    x = synthetic.tokens(91, tokens, hidden).to(dtype)
+    layer = build_layer(cuda, slot_cfg, top_k=k, served_bias=served_bias, pool_bias=pool_bias, slot_of=slot_of, tau=0.2)
+    assert layer.launches_per_call(tokens, dtype) == 1
+    out, routing = layer.decode(x.to(cuda))
+    assert out.dtype == dtype and (routing.admit.cpu().numpy() >= 0).any()
+    check_layer(slot_cfg, x, out, routing, top_k=k, served_bias=served_bias, pool_bias=pool_bias, slot_of=slot_of, tau=0.2, dtype=dtype, tolerance=tolerance)
+    want, over = out.clone(), x.to(cuda).clone()
+    assert torch.equal(layer.decode(over, out=over)[0], want)

@@ -26,7 +26,7 @@ def build_layer(cuda, cfg, **kw):
 
 
 def check_layer(cfg, x, out, routing, *, top_k, served_bias=None, pool_bias=None, slot_of=None, res=None, hot_of_slot=None,
-                **router_kw):
+                dtype=torch.bfloat16, tolerance=TOLERANCE, **router_kw):
     want = oracle_router.routed_topk(x, cfg["router"], served_bias, pool_bias, slot_of, top_k=top_k, **router_kw)
     assert oracle_router.min_cut_gap(want["served_keys"], top_k) > 0
     np.testing.assert_array_equal(routing.served_expert.cpu().numpy(), want["served_expert"].numpy())
@@ -37,11 +37,11 @@ def check_layer(cfg, x, out, routing, *, top_k, served_bias=None, pool_bias=None
     slots = want["served_slot"].numpy()
     dense = {n: oracle_router.dense_slots(*cfg[n], slots, res=None if res is None else res[n], hot_of_slot=hot_of_slot)
              for n in ("w1", "w3", "w2")}
-    ref = oracle_router.moe_layer(x, slots, want["served_weight"].numpy(), dense["w1"], dense["w3"], dense["w2"])
+    ref = oracle_router.moe_layer(x, slots, want["served_weight"].numpy(), dense["w1"], dense["w3"], dense["w2"], dtype=dtype)
     got = out.float().cpu().numpy()
     gap, cos = e8.relative_gap(got, ref.numpy()), e8.cosine_similarity(got, ref.numpy())
     print(f"layer output: relative gap {gap:.3e}, cosine {cos:.8f}")
-    assert gap <= TOLERANCE and cos >= 0.9999
+    assert gap <= tolerance and cos >= 0.9999
     return gap, cos
 
 
@@ -138,7 +138,7 @@ def test_fewer_residents_than_top_k_leaves_dead_picks_at_zero(cuda):
     check_layer(cfg, x, out, routing, top_k=3, served_bias=served_bias, slot_of=np.arange(6))
 
 
-@pytest.mark.parametrize("tokens", [3, 30, 400])  # the sweep kernel, the slab kernel, the tcgen05 kernel
+@pytest.mark.parametrize("tokens", [3, 30, 400])  # the few-token kernel, the slab kernel, the tcgen05 kernel
 def test_dead_picks_at_tensor_core_shapes(cuda, tokens):
     """Two residents, top-3: every token has a pick without a slot, which must add nothing,
     whichever of the grouped kernels runs (they never touch the rows of such routes)."""
@@ -166,6 +166,25 @@ def test_tensor_core_path_small_shapes(cuda, tokens, experts, top_k, group):
     assert layer.kernel_path == "tensor"
     out, routing = layer.decode(x.to(cuda))
     check_layer(cfg, x, out, routing, top_k=top_k)
+
+
+@pytest.mark.parametrize("tokens,hidden,inter,group_hidden,group_inter", [
+    (3, 5376, 512, None, None),   # 21 chunks of inputs: no even share for any number of warps
+    (2, 6144, 768, 512, 256),     # scale groups of two chunks and of one
+    (5, 512, 5376, None, 768),    # the down projection's rows are the wide ones
+])
+def test_few_routes_of_wide_layers_run_the_sweep_kernel(cuda, tokens, hidden, inter, group_hidden, group_inter):
+    """Layers over 5120 wide, which the few-token kernel does not take, with picks of absent experts."""
+    cfg = synthetic.layer(seed=25, experts=8, hidden=hidden, inter=inter, group_hidden=group_hidden, group_inter=group_inter)
+    served_bias = np.array([0, oracle_router.OFF, 0, 0, oracle_router.OFF, 0, oracle_router.OFF, 0], dtype=np.float32)
+    x = synthetic.tokens(26 + tokens, tokens, hidden)
+    layer = build_layer(cuda, cfg, top_k=6, served_bias=served_bias, slot_of=np.arange(8, dtype=np.uint32))
+    assert layer.kernel_path == "tensor" and layer.launches_per_call(tokens) == 7  # not the few-token kernel's one
+    layer.decode(x.to(cuda))
+    for buf in layer._buffers.values():
+        buf["workspace"].fill_(0x7F)
+    out, routing = layer.decode(x.to(cuda))
+    check_layer(cfg, x, out, routing, top_k=6, served_bias=served_bias, slot_of=np.arange(8))
 
 
 def test_tensor_and_general_kernels_agree(cuda):
@@ -240,8 +259,8 @@ def test_under_1024_routes_the_decode_kernels_take_several_groups_per_expert(cud
 @pytest.mark.parametrize("tokens", [2, 10])
 def test_shipped_artifact_shape_with_grouped_scales(cuda, tokens):
     """The shape and scale groups of the reference's shipped artifacts: hidden 5120 in groups of
-    512, inter 2304 in groups of 256 (keep_quant.py:13-15).  Two tokens run the sweep kernel (20
-    and 9 chunks of inputs over its 16 and 8 k parts, several scale groups per row); ten tokens x
+    512, inter 2304 in groups of 256 (keep_quant.py:13-15).  Two tokens run the few-token
+    kernel (20 and 9 chunks of inputs over its 16 warps, several scale groups per row); ten tokens x
     top-6 run the split slab kernel with eight and two scale groups per row."""
     cfg = synthetic.layer(seed=31, experts=10, hidden=5120, inter=2304, group_hidden=512, group_inter=256)
     x = synthetic.tokens(32 + tokens, tokens, 5120)
