@@ -26,7 +26,7 @@
 //                and has the time of two K blocks for them.  (All 16 warps on every K block, eight
 //                codewords each behind private cp.async rings, took 1290 cycles per K block at 24
 //                routes an expert; this form 740: a 1024-token product 302 -> 180 us, the two
-//                projections of a 4096-token layer 1185 + 584 -> 715 + 367 us.)  The bytes go straight into TENSOR MEMORY
+//                projections of a 4096-token layer 1185 + 584 -> 715 + 367 us, 736 + 400 on another GPU.)  The bytes go straight into TENSOR MEMORY
 //                (tcgen05.st), two stages of one or two K blocks deep, so the A operand never touches shared memory.
 //                An item's accumulators are drained (tcgen05.ld: same lanes; each of the four warps
 //                of a quadrant takes a quarter of the columns) behind the warp's first K block of the

@@ -104,7 +104,7 @@ __device__ __forceinline__ void load_matrices(uint32_t addr, uint32_t& a, uint32
 // by word were 24 shared-memory reads per eight MMAs, so matrices are read four at a time (4 reads), and both
 // halves of a K block before the first MMA.  Copies run three blocks ahead.  (Logits and top-k of 4096 tokens x 384
 // experts, 4096 wide, 93 -> 78 us, of 2000 tokens 55 -> 52, of 251 tokens 21 -> 17; 192 experts, 5120 wide, 4096
-// tokens 70 -> 65, 251 tokens 15.1 -> 15.7.)
+// tokens 70 -> 65, 251 tokens 15.1 -> 15.1; the least gain of 192 sizes: 384 experts, 2048 wide, 251 tokens 8.9 -> 9.2 for the logits alone.)
 __device__ __forceinline__ void router_tile_mma(RouterStages& sm, const __nv_bfloat16* x, const __nv_bfloat16* w, const keepvq_router_logits_args& a, int64_t t0, int64_t e0, int k_blocks, int wm, int wn, float (&acc)[2][4][4]) {
   const int tid = threadIdx.x, lane = tid & 31;
   // staging: 64 rows x 4 pieces of 16 bytes per operand, two pieces per thread
