@@ -259,6 +259,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
   const uint32_t high_rings = a0 + FT_TABLE_BYTES;
   const uint32_t acts = high_rings + (FT_WARPS - low_rings) * RING_BYTES;
   if (acts + a.act_bytes > base + FT_SMEM_BYTES || a0 - base < FT_PICK_BYTES) {  // uniform over the grid
+    grid_wait();  // (an early launch that ended without it would let its successor overtake its predecessor)
     if (a.status && tid == 0) atomicExch(a.status, 2);
     return;
   }
