@@ -836,7 +836,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) few_tokens_kernel(const __grid_
 // ---- launch -----------------------------------------------------------------------------------
 
 // CTAs of a launch on the current device, one per SM; 0 where a grid of them cannot be launched cooperatively.
-// (Of the device: a context or stream that has only part of its SMs is told so by the launch, see below.)
+// (Of the device; a stream may have only part of its SMs, see stream_sms.)
 static int few_tokens_grid() {
   static std::atomic<int> known[64];  // plus one; 0: not asked yet
   int dev = 0;
@@ -856,6 +856,38 @@ static int few_tokens_grid() {
   grid = cooperative && smem >= static_cast<int>(FT_SMEM_BYTES + FT_STATIC_MAX - 1024) ? std::min(sms, FT_MAX_CTAS) : 0;  // (1 KB of that is the system's)
   known[dev].store(grid + 1);
   return grid;
+}
+// SMs that the stream's kernels may run on: a green context's are part of the device's.  Asked before a
+// cooperative launch, because a launch refused as too large ends a capture under way.
+static int stream_sms(cudaStream_t s, int device_sms) {
+  struct Driver {
+    CUresult(CUDAAPI* stream_green)(CUstream, CUgreenCtx*) = nullptr;
+    CUresult(CUDAAPI* green_resource)(CUgreenCtx, CUdevResource*, CUdevResourceType) = nullptr;
+    CUresult(CUDAAPI* current)(CUcontext*) = nullptr;
+    CUresult(CUDAAPI* resource)(CUcontext, CUdevResource*, CUdevResourceType) = nullptr;
+    bool known = false;
+    Driver() {
+      auto find = [](const char* name, auto& fn) {
+        void* at = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint(name, &at, cudaEnableDefault, &found) != cudaSuccess) {
+          cudaGetLastError();
+          return false;
+        }
+        fn = reinterpret_cast<std::remove_reference_t<decltype(fn)>>(at);
+        return found == cudaDriverEntryPointSuccess && at;
+      };
+      known = find("cuStreamGetGreenCtx", stream_green) && find("cuGreenCtxGetDevResource", green_resource) && find("cuCtxGetCurrent", current) && find("cuCtxGetDevResource", resource);
+    }
+  };
+  static const Driver driver;
+  if (!driver.known) return device_sms;
+  CUdevResource r = {};
+  CUgreenCtx green = nullptr;
+  CUcontext context = nullptr;
+  const bool asked = driver.stream_green(s, &green) == CUDA_SUCCESS && green ? driver.green_resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS
+                   : driver.current(&context) == CUDA_SUCCESS && context && driver.resource(context, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS;
+  return asked && r.type == CU_DEV_RESOURCE_TYPE_SM ? static_cast<int>(r.sm.smCount) : device_sms;
 }
 bool few_tokens_fits(int64_t routes, int64_t tokens, int64_t slots, int64_t out_dim, int64_t in_dim, int64_t groups) {
   // (a CTA's share of the units must not span more than two route groups: no more routes than CTAs)
@@ -914,6 +946,7 @@ static int launch_few_tokens(const FewTokensArgs& args, void* sync, cudaStream_t
   config.stream = s;
   cudaLaunchAttribute attribute = {};
   if ((a.parts & FT_ROUTER) || ((a.parts & FT_GATE_UP) && (a.parts & FT_DOWN))) {  // its CTAs wait for one another: all of them resident
+    if (stream_sms(s, ctas) < ctas) return KEEPVQ_ERR_UNSUPPORTED;
     attribute.id = cudaLaunchAttributeCooperative;
     attribute.val.cooperative = 1;
   } else {
@@ -923,7 +956,7 @@ static int launch_few_tokens(const FewTokensArgs& args, void* sync, cudaStream_t
   config.attrs = &attribute;
   config.numAttrs = 1;
   const cudaError_t err = cudaLaunchKernelEx(&config, kernel, a);
-  if (err == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs here than the device has: nothing was launched, and the caller has kernels whose blocks do not wait for one another
+  if (err == cudaErrorCooperativeLaunchTooLarge) {  // nothing was launched, and the caller has kernels whose blocks do not wait for one another
     cudaGetLastError();
     return KEEPVQ_ERR_UNSUPPORTED;
   }

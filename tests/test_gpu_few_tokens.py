@@ -172,6 +172,43 @@ def test_a_grid_that_cannot_be_resident_leaves_the_call_to_the_other_kernels(cud
         check_layer(cfg, x.cpu(), buf["out"], buf["routing"], top_k=top_k)
 
 
+def test_a_stream_with_part_of_the_SMs(cuda):
+    """A green context's stream: the grid of one block per SM of the device cannot be resident there, so
+    the call goes to the chain of kernels, captured as well as eager, before a launch is refused."""
+    drv = pytest.importorskip("cuda.bindings.driver")
+
+    def did(result):
+        assert result[0] == drv.CUresult.CUDA_SUCCESS, result[0]
+        return result[1] if len(result) == 2 else result[1:]
+
+    cfg = synthetic.layer(seed=92, experts=12, hidden=512, inter=256)
+    layer = build_layer(cuda, cfg, top_k=4)
+    x = synthetic.tokens(93, 5, 512).to(cuda)
+    layer.decode(x)
+    torch.cuda.synchronize()
+    device = did(drv.cuDeviceGet(cuda.index))
+    every = did(drv.cuDeviceGetDevResource(device, drv.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    parts = did(drv.cuDevSmResourceSplitByCount(1, every, 0, every.sm.smCount // 2))[0]
+    green = did(drv.cuGreenCtxCreate(did(drv.cuDevResourceGenerateDesc(parts, 1)), device, drv.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM.value))
+    handle = did(drv.cuGreenCtxStreamCreate(green, drv.CUstream_flags.CU_STREAM_NON_BLOCKING.value, 0))
+    stream = torch.cuda.ExternalStream(int(handle), device=cuda)
+    with torch.cuda.stream(stream):
+        out, routing = layer.decode(x)
+    stream.synchronize()
+    check_layer(cfg, x.cpu(), out, routing, top_k=4)
+    want = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        layer.decode(x)
+    out.zero_()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        graph.replay()
+    stream.synchronize()
+    assert torch.equal(out, want)
+    # (the stream and its context stay until the process ends: the allocator may know the stream)
+
+
 def test_calls_on_two_streams_at_once(cuda):
     cfg = synthetic.layer(seed=75, experts=16, hidden=1024, inter=512)
     layer = build_layer(cuda, cfg, top_k=4)
